@@ -477,21 +477,26 @@ __global__ void k_scatter_index(const uint32_t *__restrict__ bstart, const uint3
 }
 
 constexpr int RB_NT = 512;   // one thread per tile cell in the counting sort
+static_assert(REBIN_SORT_MAX % RB_NT == 0, "whole particles per thread");
 
 template <class R> constexpr size_t rb_smem_bytes()
 {
-    // per particle: id, off[3], q[3], cell, source index, cell rank, slot, sorted index
-    return (size_t)REBIN_SORT_MAX * (sizeof(int64_t) + 3 * sizeof(double) + 3 * sizeof(R) + sizeof(uint32_t) + 3 * sizeof(uint16_t));
+    // per particle: id, off[3], q[3], cell, sorted index
+    return (size_t)REBIN_SORT_MAX * (sizeof(int64_t) + 3 * sizeof(double) + 3 * sizeof(R) + sizeof(uint32_t) + sizeof(uint16_t));
 }
 
 // Step 2: one CTA per destination tile.  The tile's particles (or, for a tile
 // of more than REBIN_SORT_MAX, each of its buckets that small) are loaded once
 // from their source positions into shared memory, sorted there -- counting
-// sort by class_ord of the cell, then insertion sort by ID inside each cell --
-// and written to the sorted destination positions (coalesced writes).  A
-// bucket larger than REBIN_SORT_MAX is copied in slot order.
+// sort by class_ord of the cell, then each particle's rank by ID among its
+// cell's -- and written to the sorted destination positions (coalesced
+// writes).  The rank is one thread per particle counting the smaller IDs of
+// its cell: an insertion sort by one thread per cell takes the square of the
+// densest cell's occupation while the block waits (clustered 128^3 particles:
+// 241 us by insertion, 84 us by rank).  A bucket larger than
+// REBIN_SORT_MAX is copied in slot order.
 template <class R>
-__global__ void __launch_bounds__(RB_NT) k_rebin_tile(PView<R> src, PView<R> dst, const uint32_t *__restrict__ bstart,
+__global__ void __launch_bounds__(RB_NT, 3) k_rebin_tile(PView<R> src, PView<R> dst, const uint32_t *__restrict__ bstart,
                                                       const uint32_t *__restrict__ inv, int nt, int *err, FastDiv fN)
 {
     constexpr int M = REBIN_SORT_MAX;
@@ -500,9 +505,7 @@ __global__ void __launch_bounds__(RB_NT) k_rebin_tile(PView<R> src, PView<R> dst
     double *s_off = reinterpret_cast<double *>(s_id + M);          // 3 planes of M
     R *s_q = reinterpret_cast<R *>(s_off + 3 * M);                 // 3 planes of M
     uint32_t *s_cell = reinterpret_cast<uint32_t *>(s_q + 3 * M);
-    uint16_t *s_ord = reinterpret_cast<uint16_t *>(s_cell + M);
-    uint16_t *s_slot = s_ord + M;
-    uint16_t *s_order = s_slot + M;
+    uint16_t *s_order = reinterpret_cast<uint16_t *>(s_cell + M);
     __shared__ int s_cnt[512], s_start[512], s_wsum[RB_NT / 32];
 
     const int t = threadIdx.x, tile = blockIdx.x;
@@ -516,33 +519,37 @@ __global__ void __launch_bounds__(RB_NT) k_rebin_tile(PView<R> src, PView<R> dst
     };
 
     auto sort_range = [&](uint32_t lo, int m) {
+        constexpr int PER = M / RB_NT;   // particles per thread
+        int64_t id[PER];
+        int ord[PER], slot[PER];
         for (int c = t; c < 512; c += RB_NT) s_cnt[c] = 0;
         __syncthreads();
-        for (int j = t; j < m; j += RB_NT) {
+#pragma unroll
+        for (int k = 0; k < PER; k++) {
+            const int j = t + k * RB_NT;
+            if (j >= m) continue;
             const uint32_t s = source(lo + (uint32_t)j);
             const uint32_t cell = src.cell[s];
-            const int64_t id = src.id[s];
+            id[k] = src.id[s];
             double o[3];
             R q[3];
 #pragma unroll
-            for (int k = 0; k < 3; k++) {
-                o[k] = src.off[k * src.cap + s];
-                q[k] = src.q[k * src.cap + s];
+            for (int c = 0; c < 3; c++) {
+                o[c] = src.off[c * src.cap + s];
+                q[c] = src.q[c * src.cap + s];
             }
             int cx, cy, cz;
             decode_cell(cell, fN, cx, cy, cz);
             int lx = cx - x0, ly = cy - y0, lz = cz - z0;
             if (lx < 0 || lx > 7 || ly < 0 || ly > 7 || lz < 0 || lz > 7) { atomicOr(err, ERR_BAD_CELL); lx = ly = lz = 0; }
-            const int c = class_ord(lx, ly, lz);
+            ord[k] = class_ord(lx, ly, lz);
             s_cell[j] = cell;
-            s_id[j] = id;
 #pragma unroll
-            for (int k = 0; k < 3; k++) {
-                s_off[k * M + j] = o[k];
-                s_q[k * M + j] = q[k];
+            for (int c = 0; c < 3; c++) {
+                s_off[c * M + j] = o[c];
+                s_q[c * M + j] = q[c];
             }
-            s_ord[j] = (uint16_t)c;
-            s_slot[j] = (uint16_t)atomicAdd(&s_cnt[c], 1);
+            slot[k] = atomicAdd(&s_cnt[ord[k]], 1);
         }
         __syncthreads();
         {   // exclusive scan of the 512 cell counts, one per thread
@@ -569,20 +576,23 @@ __global__ void __launch_bounds__(RB_NT) k_rebin_tile(PView<R> src, PView<R> dst
             s_start[t] = incl - v + s_wsum[t >> 5];
         }
         __syncthreads();
-        for (int j = t; j < m; j += RB_NT) s_order[s_start[s_ord[j]] + s_slot[j]] = (uint16_t)j;
+        // IDs grouped by cell, then every particle's place among its cell's
+#pragma unroll
+        for (int k = 0; k < PER; k++) {
+            if (t + k * RB_NT >= m) continue;
+            slot[k] += s_start[ord[k]];
+            s_id[slot[k]] = id[k];
+        }
         __syncthreads();
-        {   // insertion sort by ID inside the cell (cells hold a few particles)
-            const int k0 = s_start[t], mc = s_cnt[t];
-            for (int a1 = 1; a1 < mc; a1++) {
-                const uint16_t key = s_order[k0 + a1];
-                const int64_t kid = s_id[key];
-                int b1 = a1 - 1;
-                while (b1 >= 0 && s_id[s_order[k0 + b1]] > kid) {
-                    s_order[k0 + b1 + 1] = s_order[k0 + b1];
-                    b1--;
-                }
-                s_order[k0 + b1 + 1] = key;
-            }
+#pragma unroll
+        for (int k = 0; k < PER; k++) {
+            const int j = t + k * RB_NT;
+            if (j >= m) continue;
+            const int k0 = s_start[ord[k]], k1 = k0 + s_cnt[ord[k]];
+            int pos = k0;
+            for (int i = k0; i < k1; i++) pos += (s_id[i] < id[k] || (s_id[i] == id[k] && i < slot[k])) ? 1 : 0;
+            s_order[pos] = (uint16_t)j;
+            dst.id[lo + (uint32_t)pos] = id[k];
         }
         __syncthreads();
         for (int k = t; k < m; k += RB_NT) {
@@ -594,7 +604,6 @@ __global__ void __launch_bounds__(RB_NT) k_rebin_tile(PView<R> src, PView<R> dst
                 dst.off[c * dst.cap + i] = s_off[c * M + j];
                 dst.q[c * dst.cap + i] = s_q[c * M + j];
             }
-            dst.id[i] = s_id[j];
         }
         __syncthreads();
     };

@@ -74,165 +74,223 @@ template <class T> struct PBuf {
 
 constexpr int PM_NT = 256;
 
-// cell corner and in-cell offset of an unwrapped box-unit coordinate
-__device__ __forceinline__ void pm_cell(double x, int N, int &c, double &d)
+// cell corner and in-cell offset of an unwrapped box-unit coordinate.  The
+// cell is reduced into the box in FP64 (floor of the quotient, at most one
+// off, then one correction): a 64-bit integer remainder per coordinate costs
+// more than the whole interpolation.  A non-finite coordinate gives cell 0.
+__device__ __forceinline__ void pm_cell(double x, int N, double invN, int &c, double &d)
 {
     const double p = x * (double)N;
     const double f = floor(p);
     d = p - f;
-    long long ci = (long long)f % N;
+    int ci = (int)(f - (double)N * floor(f * invN));
     if (ci < 0) ci += N;
-    c = (int)ci;
+    if (ci >= N) ci -= N;
+    c = (unsigned)ci < (unsigned)N ? ci : 0;
 }
 
 __device__ __forceinline__ int pm_wrap1(int i, int N) { return i >= N ? i - N : (i < 0 ? i + N : i); }
 
-// CIC deposit: out[comp][corner] += w * value (value = cst, or vals[3 i + comp])
-template <class R, int NC>
-__global__ void k_pm_deposit(const double *__restrict__ x, int64_t np, int N, const double *__restrict__ vals,
-                             double cst, R *out)
-{
-    const int64_t n3 = (int64_t)N * N * N;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < np; i += (int64_t)gridDim.x * blockDim.x) {
+// A particle's cell and the grid offsets (x; N y; N^2 z, all below 2^31) of
+// the four planes c - 1 .. c + 2 per axis.
+struct PmSite {
+    double d[3];
+    int x[4], y[4], z[4];
+    __device__ __forceinline__ PmSite(const double *__restrict__ pos, int N, double invN)
+    {
         int c[3];
-        double d[3];
 #pragma unroll
-        for (int k = 0; k < 3; k++) pm_cell(x[3 * i + k], N, c[k], d[k]);
-        double v[NC];
+        for (int k = 0; k < 3; k++) pm_cell(pos[k], N, invN, c[k], d[k]);
 #pragma unroll
-        for (int m = 0; m < NC; m++) v[m] = vals ? vals[3 * i + m] : cst;
-#pragma unroll
-        for (int k = 0; k < 8; k++) {
-            const int bx = (k >> 2) & 1, by = (k >> 1) & 1, bz = k & 1;
-            const double w = (bx ? d[0] : 1.0 - d[0]) * (by ? d[1] : 1.0 - d[1]) * (bz ? d[2] : 1.0 - d[2]);
-            const int64_t g = sidx(N, pm_wrap1(c[0] + bx, N), pm_wrap1(c[1] + by, N), pm_wrap1(c[2] + bz, N));
-#pragma unroll
-            for (int m = 0; m < NC; m++) atomicAdd(out + m * n3 + g, (R)(w * v[m]));
+        for (int k = 0; k < 4; k++) {
+            x[k] = pm_wrap1(c[0] + k - 1, N);
+            y[k] = pm_wrap1(c[1] + k - 1, N) * N;
+            z[k] = pm_wrap1(c[2] + k - 1, N) * N * N;
         }
     }
-}
+    __device__ __forceinline__ int at(int bx, int by, int bz) const { return x[bx + 1] + y[by + 1] + z[bz + 1]; }
+    __device__ __forceinline__ double w(int axis, int b) const { return b ? d[axis] : 1.0 - d[axis]; }
+};
 
-template <class R>
-__device__ __forceinline__ double pm_ld(const R *f, int N, int x, int y, int z)
-{
-    return (double)__ldg(f + sidx(N, pm_wrap1(x, N), pm_wrap1(y, N), pm_wrap1(z, N)));
-}
+template <class R> __device__ __forceinline__ double pm_ld(const R *__restrict__ f, int i) { return (double)__ldg(f + i); }
 
-// G[i][k] = (psi(c_k + e_i) - psi(c_k - e_i)) / 2 at the 8 corners c_k of the cell
-template <class R>
-__device__ __forceinline__ void pm_grad_corners(const R *psi, int N, const int c[3], double G[3][8])
+// CIC deposit of cst at the particle's 8 corners
+template <class R> __device__ __forceinline__ void pm_scatter(const PmSite &s, double cst, R *out)
 {
 #pragma unroll
     for (int k = 0; k < 8; k++) {
-        const int x = c[0] + ((k >> 2) & 1), y = c[1] + ((k >> 1) & 1), z = c[2] + (k & 1);
-        G[0][k] = 0.5 * (pm_ld(psi, N, x + 1, y, z) - pm_ld(psi, N, x - 1, y, z));
-        G[1][k] = 0.5 * (pm_ld(psi, N, x, y + 1, z) - pm_ld(psi, N, x, y - 1, z));
-        G[2][k] = 0.5 * (pm_ld(psi, N, x, y, z + 1) - pm_ld(psi, N, x, y, z - 1));
+        const int bx = (k >> 2) & 1, by = (k >> 1) & 1, bz = k & 1;
+        const double w = s.w(0, bx) * s.w(1, by) * s.w(2, bz);
+        atomicAdd(out + s.at(bx, by, bz), (R)(w * cst));
     }
 }
 
-// forward kick (update_q_Newton) and drift (update_pos_Newton)
-template <class R>
-__global__ void k_pm_kick_drift(double *x, double *q, int64_t np, int N, const R *__restrict__ psi, double kq, double kx)
+// one site's three values, interleaved with a pad: a corner's three additions
+// are one 16-byte vector addition in FP32
+__device__ __forceinline__ void pm_add3(float *out, double a, double b, double c)
 {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < np; i += (int64_t)gridDim.x * blockDim.x) {
-        int c[3];
-        double d[3];
+    atomicAdd(reinterpret_cast<float4 *>(out), make_float4((float)a, (float)b, (float)c, 0.0f));
+}
+__device__ __forceinline__ void pm_add3(double *out, double a, double b, double c)
+{
+    atomicAdd(out, a);
+    atomicAdd(out + 1, b);
+    atomicAdd(out + 2, c);
+}
+
+// G[i][k] = (psi(c_k + e_i) - psi(c_k - e_i)) / 2 at the 8 corners c_k of the
+// cell: 32 distinct values (the 8 corners and the 24 one step outside them)
+template <class R>
+__device__ __forceinline__ void pm_grad_corners(const R *__restrict__ psi, const PmSite &s, double G[3][8])
+{
+    double in[8];
 #pragma unroll
-        for (int k = 0; k < 3; k++) pm_cell(x[3 * i + k], N, c[k], d[k]);
-        double G[3][8];
-        pm_grad_corners(psi, N, c, G);
+    for (int k = 0; k < 8; k++) in[k] = pm_ld(psi, s.at((k >> 2) & 1, (k >> 1) & 1, k & 1));
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+        const int bx = (k >> 2) & 1, by = (k >> 1) & 1, bz = k & 1;
+        // the neighbour inside the cell is a corner, the other one lies outside
+        const double ox = pm_ld(psi, s.at(bx ? 2 : -1, by, bz)), oy = pm_ld(psi, s.at(bx, by ? 2 : -1, bz)),
+                     oz = pm_ld(psi, s.at(bx, by, bz ? 2 : -1));
+        G[0][k] = 0.5 * (bx ? ox - in[k & 3] : in[k | 4] - ox);
+        G[1][k] = 0.5 * (by ? oy - in[k & 5] : in[k | 2] - oy);
+        G[2][k] = 0.5 * (bz ? oz - in[k & 6] : in[k | 1] - oz);
+    }
+}
+
+// mass deposit alone (the start of a run or of a recomputed segment)
+template <class R>
+__global__ void k_pm_deposit(const double *__restrict__ x, int64_t np, int N, double cst, R *out)
+{
+    const double invN = 1.0 / N;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < np; i += (int64_t)gridDim.x * blockDim.x)
+        pm_scatter(PmSite(x + 3 * i, N, invN), cst, out);
+}
+
+// forward kick (update_q_Newton) and drift (update_pos_Newton) from (xi, qi)
+// to (xo, qo) (the same arrays or others), and the deposit of cst at the new
+// position that the next step (or the final density) needs: the moved
+// positions are not read back
+template <class R>
+__global__ void k_pm_kick_drift(const double *xi, const double *qi, double *xo, double *qo, int64_t np, int N,
+                                const R *__restrict__ psi, double kq, double kx, double cst, R *rho)
+{
+    const double invN = 1.0 / N;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < np; i += (int64_t)gridDim.x * blockDim.x) {
+        double x[3] = {xi[3 * i], xi[3 * i + 1], xi[3 * i + 2]};
+        double q[3] = {qi[3 * i], qi[3 * i + 1], qi[3 * i + 2]};
+        {
+            const PmSite s(x, N, invN);
+            double G[3][8];
+            pm_grad_corners(psi, s, G);
+            double g[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+                const double w = s.w(0, (k >> 2) & 1) * s.w(1, (k >> 1) & 1) * s.w(2, k & 1);
+#pragma unroll
+                for (int a = 0; a < 3; a++) g[a] += w * G[a][k];
+            }
+#pragma unroll
+            for (int a = 0; a < 3; a++) {
+                q[a] -= kq * g[a];
+                x[a] += kx * q[a];
+            }
+        }
 #pragma unroll
         for (int a = 0; a < 3; a++) {
-            double g = 0.0;
+            qo[3 * i + a] = q[a];
+            xo[3 * i + a] = x[a];
+        }
+        if (rho) pm_scatter(PmSite(x, N, invN), cst, rho);
+    }
+}
+
+// dw_k/dd_m v_k summed over the corners: gradient of the CIC interpolation
+__device__ __forceinline__ void pm_weight_grad(const PmSite &s, const double v[8], double gm[3])
+{
+    gm[0] = gm[1] = gm[2] = 0.0;
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+        const int bx = (k >> 2) & 1, by = (k >> 1) & 1, bz = k & 1;
+        const double fx = s.w(0, bx), fy = s.w(1, by), fz = s.w(2, bz);
+        gm[0] += (bx ? fy : -fy) * fz * v[k];
+        gm[1] += (by ? fx : -fx) * fz * v[k];
+        gm[2] += (bz ? fx : -fx) * fy * v[k];
+    }
+}
+
+// One reverse pass over the particles, the end of step n + 1 and the start of
+// step n together (both update the cotangents lx):
+//   1. transpose of the CIC deposit of weight mf at xb (step n + 1's mass
+//      deposit, or the final density): lx_m += mf N sum_k dw_k/dd_m f(c_k);
+//   2. when xa is given, reverse of the drift and of the kick at fixed psi at
+//      xa = x_n: lq becomes lq' (the cotangent of the kicked momentum), and
+//      lq' is deposited into lam (three interleaved components) for the field
+//      part of the step.
+// (lxi, lqi) null: the cotangents start at zero.
+template <class R>
+__global__ void k_pm_reverse(const double *__restrict__ xb, const R *__restrict__ f, double mf, const double *__restrict__ xa,
+                             const R *__restrict__ psi, double kq, double kx, const double *lxi, const double *lqi,
+                             double *lxo, double *lqo, R *lam, int64_t np, int N)
+{
+    const double invN = 1.0 / N;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < np; i += (int64_t)gridDim.x * blockDim.x) {
+        double lx[3], lq[3];
+#pragma unroll
+        for (int a = 0; a < 3; a++) {
+            lx[a] = lxi ? lxi[3 * i + a] : 0.0;
+            lq[a] = lqi ? lqi[3 * i + a] : 0.0;
+        }
+        {
+            const PmSite s(xb + 3 * i, N, invN);
+            double v[8], gm[3];
+#pragma unroll
+            for (int k = 0; k < 8; k++) v[k] = pm_ld(f, s.at((k >> 2) & 1, (k >> 1) & 1, k & 1));
+            pm_weight_grad(s, v, gm);
+#pragma unroll
+            for (int a = 0; a < 3; a++) lx[a] += mf * (double)N * gm[a];
+        }
+        if (xa) {
+            const PmSite s(xa + 3 * i, N, invN);
+#pragma unroll
+            for (int a = 0; a < 3; a++) lq[a] += kx * lx[a];
+            double G[3][8], v[8], gm[3];
+            pm_grad_corners(psi, s, G);
+            // lx_m -= kq N sum_k dw_k/dd_m (sum_a lq'_a G[a][k])
+#pragma unroll
+            for (int k = 0; k < 8; k++) v[k] = lq[0] * G[0][k] + lq[1] * G[1][k] + lq[2] * G[2][k];
+            pm_weight_grad(s, v, gm);
+#pragma unroll
+            for (int a = 0; a < 3; a++) lx[a] -= kq * (double)N * gm[a];
 #pragma unroll
             for (int k = 0; k < 8; k++) {
                 const int bx = (k >> 2) & 1, by = (k >> 1) & 1, bz = k & 1;
-                const double w = (bx ? d[0] : 1.0 - d[0]) * (by ? d[1] : 1.0 - d[1]) * (bz ? d[2] : 1.0 - d[2]);
-                g += w * G[a][k];
+                const double w = s.w(0, bx) * s.w(1, by) * s.w(2, bz);
+                pm_add3(lam + 4 * (int64_t)s.at(bx, by, bz), w * lq[0], w * lq[1], w * lq[2]);
             }
-            const double qn = q[3 * i + a] - kq * g;
-            q[3 * i + a] = qn;
-            x[3 * i + a] += kx * qn;
-        }
-    }
-}
-
-// reverse of the drift and of the kick at fixed psi; lq becomes lq' (the
-// cotangent of the kicked momentum), which the field part then deposits
-template <class R>
-__global__ void k_pm_adj_kick(const double *__restrict__ x, int64_t np, int N, const R *__restrict__ psi, double kq,
-                              double kx, double *lx, double *lq)
-{
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < np; i += (int64_t)gridDim.x * blockDim.x) {
-        int c[3];
-        double d[3];
-#pragma unroll
-        for (int k = 0; k < 3; k++) pm_cell(x[3 * i + k], N, c[k], d[k]);
-        double lqp[3];
-#pragma unroll
-        for (int a = 0; a < 3; a++) lqp[a] = lq[3 * i + a] + kx * lx[3 * i + a];
-        double G[3][8];
-        pm_grad_corners(psi, N, c, G);
-        // s_k = sum_a lq'_a G[a][k]; lx_m -= kq N sum_k dw_k/dd_m s_k
-        double gm[3] = {0.0, 0.0, 0.0};
-#pragma unroll
-        for (int k = 0; k < 8; k++) {
-            const int bx = (k >> 2) & 1, by = (k >> 1) & 1, bz = k & 1;
-            const double fx = bx ? d[0] : 1.0 - d[0], fy = by ? d[1] : 1.0 - d[1], fz = bz ? d[2] : 1.0 - d[2];
-            const double sx = bx ? 1.0 : -1.0, sy = by ? 1.0 : -1.0, sz = bz ? 1.0 : -1.0;
-            const double s = lqp[0] * G[0][k] + lqp[1] * G[1][k] + lqp[2] * G[2][k];
-            gm[0] += sx * fy * fz * s;
-            gm[1] += fx * sy * fz * s;
-            gm[2] += fx * fy * sz * s;
         }
 #pragma unroll
         for (int a = 0; a < 3; a++) {
-            lx[3 * i + a] -= kq * (double)N * gm[a];
-            lq[3 * i + a] = lqp[a];
+            lxo[3 * i + a] = lx[a];
+            lqo[3 * i + a] = lq[a];
         }
     }
 }
 
-// lpsi(v) = -kq sum_i (Lam_i(v - e_i) - Lam_i(v + e_i)) / 2
+// lpsi(v) = -kq sum_i (Lam_i(v - e_i) - Lam_i(v + e_i)) / 2; grid (N/32 or 1, N/4, N/2), block (min(N,32), 4, 2)
 template <class R>
 __global__ void k_pm_adj_div(const R *__restrict__ lam, int N, double kq, R *lpsi)
 {
-    const int64_t n3 = (int64_t)N * N * N;
-    for (int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; g < n3; g += (int64_t)gridDim.x * blockDim.x) {
-        const int x = (int)(g % N), y = (int)((g / N) % N), z = (int)(g / ((int64_t)N * N));
-        double s = 0.0;
-        s += pm_ld(lam, N, x - 1, y, z) - pm_ld(lam, N, x + 1, y, z);
-        s += pm_ld(lam + n3, N, x, y - 1, z) - pm_ld(lam + n3, N, x, y + 1, z);
-        s += pm_ld(lam + 2 * n3, N, x, y, z - 1) - pm_ld(lam + 2 * n3, N, x, y, z + 1);
-        lpsi[g] = (R)(-kq * 0.5 * s);
-    }
-}
-
-// lx_m += mf N sum_k dw_k/dd_m f(c_k): transpose of a CIC deposit of weight mf
-template <class R>
-__global__ void k_pm_adj_deposit(const double *__restrict__ x, int64_t np, int N, const R *__restrict__ f, double mf,
-                                 double *lx)
-{
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < np; i += (int64_t)gridDim.x * blockDim.x) {
-        int c[3];
-        double d[3];
-#pragma unroll
-        for (int k = 0; k < 3; k++) pm_cell(x[3 * i + k], N, c[k], d[k]);
-        double gm[3] = {0.0, 0.0, 0.0};
-#pragma unroll
-        for (int k = 0; k < 8; k++) {
-            const int bx = (k >> 2) & 1, by = (k >> 1) & 1, bz = k & 1;
-            const double fx = bx ? d[0] : 1.0 - d[0], fy = by ? d[1] : 1.0 - d[1], fz = bz ? d[2] : 1.0 - d[2];
-            const double sx = bx ? 1.0 : -1.0, sy = by ? 1.0 : -1.0, sz = bz ? 1.0 : -1.0;
-            const double v = pm_ld(f, N, c[0] + bx, c[1] + by, c[2] + bz);
-            gm[0] += sx * fy * fz * v;
-            gm[1] += fx * sy * fz * v;
-            gm[2] += fx * fy * sz * v;
-        }
-#pragma unroll
-        for (int a = 0; a < 3; a++) lx[3 * i + a] += mf * (double)N * gm[a];
-    }
+    const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y,
+              z = blockIdx.z * blockDim.z + threadIdx.z;
+    if (x >= N || y >= N || z >= N) return;
+    auto at = [&](int xx, int yy, int zz, int c) {
+        return (double)__ldg(lam + 4 * (int64_t)(pm_wrap1(xx, N) + N * (pm_wrap1(yy, N) + N * pm_wrap1(zz, N))) + c);
+    };
+    double s = at(x - 1, y, z, 0) - at(x + 1, y, z, 0);
+    s += at(x, y - 1, z, 1) - at(x, y + 1, z, 1);
+    s += at(x, y, z - 1, 2) - at(x, y, z + 1, 2);
+    lpsi[x + N * (y + N * z)] = (R)(-kq * 0.5 * s);
 }
 
 template <class R>
@@ -264,7 +322,9 @@ template <class R> struct Pm final : PmBase {
     double mass;
     int every;
     cudaStream_t st = nullptr;
-    PBuf<R> rho, lam;
+    PBuf<R> rho;    // deposited density of the step, cleared by its first Fourier pass
+    PBuf<R> fld;    // potential of a forward step; cotangent of a density (reverse)
+    PBuf<R> lam;    // deposited momentum cotangents, [N^3][4]
     PBuf<C> W, twf, twh;
     PBuf<double> k2;
     PBuf<double2> ks;
@@ -284,7 +344,8 @@ template <class R> struct Pm final : PmBase {
         n3 = (int64_t)N * N * N;
         nk = (int64_t)(N / 2 + 2) * N * N;   // Fourier rows of pitch N/2+2
         rho.alloc(n3, "fields");
-        lam.alloc(3 * n3, "fields");
+        fld.alloc(n3, "fields");
+        lam.alloc(4 * n3, "fields");
         W.alloc(nk, "spectrum");
         x.alloc(3 * np, "particles");
         q.alloc(3 * np, "particles");
@@ -341,11 +402,11 @@ template <class R> struct Pm final : PmBase {
     unsigned fgrid() const { return (unsigned)std::min<int64_t>((n3 + PM_NT - 1) / PM_NT, 148 * 16); }
     FftTables<R> tables() const { return FftTables<R>{twf.p, twh.p, k2.p, ks.p}; }
 
-    // field <- Poisson(field) with coefficient pc (modif 0): the pass sequence of gev_solve_phi
-    void poisson(R *f, double pc)
+    // out <- Poisson(in) with coefficient pc (modif 0): the pass sequence of gev_solve_phi
+    void poisson(const R *in, R *out, double pc)
     {
         const FftTables<R> tb = tables();
-        fx_forward<R>(N, FX_COPY, f, n3, 1, 0, nullptr, nullptr, 0.0, 0.0, 0.0, 0.0, W.p, nk, nullptr, tb, st);
+        fx_forward<R>(N, FX_COPY, in, n3, 1, 0, nullptr, nullptr, 0.0, 0.0, 0.0, 0.0, W.p, nk, nullptr, tb, st);
         fy_pass<R>(N, -1, W.p, nk, 1, derr.p, tb, st);
         FzParams fp{};
         fp.op = OP_POISSON;
@@ -354,22 +415,23 @@ template <class R> struct Pm final : PmBase {
         fp.err = derr.p;
         fz_pass<R>(N, fp, W.p, nk, nullptr, nullptr, nullptr, tb, st);
         fy_pass<R>(N, 1, W.p, nk, 1, derr.p, tb, st);
-        fx_inverse<R>(N, W.p, nk, f, n3, 1, tb, st);
+        fx_inverse<R>(N, W.p, nk, out, n3, 1, tb, st);
     }
 
-    // psi_n of state x into `out`
-    void potential(const double *xs, double pc, R *out)
+    void clear(R *f, int64_t n) { pck(cudaMemsetAsync(f, 0, n * sizeof(R), st), "memset"); }
+
+    // density of the state xs into rho (the start of a chain of steps)
+    void deposit(const double *xs, double cst)
     {
-        pck(cudaMemsetAsync(out, 0, n3 * sizeof(R), st), "memset");
-        k_pm_deposit<R, 1><<<pgrid(), PM_NT, 0, st>>>(xs, np, N, nullptr, mass * (double)n3, out);
-        poisson(out, pc);
+        clear(rho.p, n3);
+        k_pm_deposit<R><<<pgrid(), PM_NT, 0, st>>>(xs, np, N, cst, rho.p);
     }
 
-    void step(int n, double *xs, double *qs, R *psi_out)
+    // potential of the density in rho, which is left cleared for the next deposit
+    void potential(double pc, R *out)
     {
-        const double kq = coefs[3 * n], kx = coefs[3 * n + 1], pc = coefs[3 * n + 2];
-        potential(xs, pc, psi_out);
-        k_pm_kick_drift<R><<<pgrid(), PM_NT, 0, st>>>(xs, qs, np, N, psi_out, kq, kx);
+        poisson(rho.p, out, pc);
+        clear(rho.p, n3);
     }
 
     void forward(int ns, const double *coef, const double *x0, const double *q0, double *delta, double *xo,
@@ -382,21 +444,26 @@ template <class R> struct Pm final : PmBase {
             ckx.emplace_back(new PBuf<double>());
             ckq.emplace_back(new PBuf<double>());
         }
-        pck(cudaMemcpyAsync(x.p, x0, 3 * np * sizeof(double), cudaMemcpyDeviceToDevice, st), "copy x0");
-        pck(cudaMemcpyAsync(q.p, q0, 3 * np * sizeof(double), cudaMemcpyDeviceToDevice, st), "copy q0");
+        for (int s = 0; s < nck; s++) {
+            ckx[s]->alloc(3 * np, "checkpoint");
+            ckq[s]->alloc(3 * np, "checkpoint");
+        }
+        pck(cudaMemcpyAsync(ckx[0]->p, x0, 3 * np * sizeof(double), cudaMemcpyDeviceToDevice, st), "copy x0");
+        pck(cudaMemcpyAsync(ckq[0]->p, q0, 3 * np * sizeof(double), cudaMemcpyDeviceToDevice, st), "copy q0");
+        const double mcell = mass * (double)n3, contrast = (double)n3 / (double)np;
+        deposit(ckx[0]->p, mcell);
         for (int n = 0; n < ns; n++) {
-            if (n % every == 0) {
-                PBuf<double> &cx = *ckx[n / every], &cq = *ckq[n / every];
-                cx.alloc(3 * np, "checkpoint");
-                cq.alloc(3 * np, "checkpoint");
-                pck(cudaMemcpyAsync(cx.p, x.p, 3 * np * sizeof(double), cudaMemcpyDeviceToDevice, st), "checkpoint");
-                pck(cudaMemcpyAsync(cq.p, q.p, 3 * np * sizeof(double), cudaMemcpyDeviceToDevice, st), "checkpoint");
-            }
-            step(n, x.p, q.p, rho.p);
+            potential(coefs[3 * n + 2], fld.p);
+            // a step reads its state where the last one wrote it; the states
+            // before steps 0, every, 2 every, ... are the checkpoints
+            const bool from = n % every == 0, to = (n + 1) % every == 0 && n + 1 < ns;
+            const int cf = n / every, ct = (n + 1) / every;
+            k_pm_kick_drift<R><<<pgrid(), PM_NT, 0, st>>>(from ? ckx[cf]->p : x.p, from ? ckq[cf]->p : q.p,
+                                                          to ? ckx[ct]->p : x.p, to ? ckq[ct]->p : q.p, np, N, fld.p,
+                                                          coefs[3 * n], coefs[3 * n + 1], n + 1 < ns ? mcell : contrast,
+                                                          rho.p);
         }
         // final CIC density contrast: mass N^3/Np per particle, minus one
-        pck(cudaMemsetAsync(rho.p, 0, n3 * sizeof(R), st), "memset");
-        k_pm_deposit<R, 1><<<pgrid(), PM_NT, 0, st>>>(x.p, np, N, nullptr, (double)n3 / (double)np, rho.p);
         k_pm_contrast<R><<<fgrid(), PM_NT, 0, st>>>(rho.p, n3, delta);
         if (xo) pck(cudaMemcpyAsync(xo, x.p, 3 * np * sizeof(double), cudaMemcpyDeviceToDevice, st), "copy x");
         if (qo) pck(cudaMemcpyAsync(qo, q.p, 3 * np * sizeof(double), cudaMemcpyDeviceToDevice, st), "copy q");
@@ -409,48 +476,50 @@ template <class R> struct Pm final : PmBase {
     void adjoint(const double *ddelta, double *gx0, double *gq0) override
     {
         if (!have_forward) throw PmError(GEV_ERR_STATE, "gev_pm_adjoint needs a preceding gev_pm_forward");
-        // cotangent of the final positions: transpose of the final deposit
-        pck(cudaMemsetAsync(lx.p, 0, 3 * np * sizeof(double), st), "memset");
-        pck(cudaMemsetAsync(lq.p, 0, 3 * np * sizeof(double), st), "memset");
-        k_pm_to_field<R><<<fgrid(), PM_NT, 0, st>>>(ddelta, n3, rho.p);
-        k_pm_adj_deposit<R><<<pgrid(), PM_NT, 0, st>>>(x.p, np, N, rho.p, (double)n3 / (double)np, lx.p);
+        const double mcell = mass * (double)n3;
         const int nseg = (nsteps + every - 1) / every;
         while ((int)segx.size() < every) {
             segx.emplace_back(new PBuf<double>());
             segpsi.emplace_back(new PBuf<R>());
         }
+        const int nb = N < 32 ? N : 32;
+        const dim3 db(nb, 4, 2), dg(N / nb, N / 4, N / 2);
+        // fld: the cotangent of the density deposited at xb (the final density first)
+        k_pm_to_field<R><<<fgrid(), PM_NT, 0, st>>>(ddelta, n3, fld.p);
+        const double *xb = x.p;
+        double mb = (double)n3 / (double)np;
+        bool first = true;
         for (int s = nseg - 1; s >= 0; s--) {
             const int n0 = s * every, n1 = std::min(nsteps, n0 + every);
             // recompute x_n and psi_n of the segment from its checkpoint; q.p (the
             // forward's final momenta were already copied out) is the working q
-            pck(cudaMemcpyAsync(q.p, ckq[s]->p, 3 * np * sizeof(double), cudaMemcpyDeviceToDevice, st), "segment");
+            auto xn = [&](int n) { return n == n0 ? ckx[s]->p : segx[n - n0]->p; };
+            deposit(ckx[s]->p, mcell);
             for (int n = n0; n < n1; n++) {
-                PBuf<double> &sx = *segx[n - n0];
                 PBuf<R> &sp = *segpsi[n - n0];
-                sx.alloc(3 * np, "segment");
                 sp.alloc(n3, "segment");
-                const double *src = (n == n0) ? ckx[s]->p : segx[n - n0 - 1]->p;
-                pck(cudaMemcpyAsync(sx.p, src, 3 * np * sizeof(double), cudaMemcpyDeviceToDevice, st), "segment");
-                if (n > n0) {
-                    // x_n = x_{n-1} advanced by step n-1 (q advanced in place in wq)
-                    const double kq = coefs[3 * (n - 1)], kx = coefs[3 * (n - 1) + 1];
-                    k_pm_kick_drift<R><<<pgrid(), PM_NT, 0, st>>>(sx.p, q.p, np, N, segpsi[n - n0 - 1]->p, kq, kx);
+                potential(coefs[3 * n + 2], sp.p);
+                if (n + 1 < n1) {
+                    segx[n + 1 - n0]->alloc(3 * np, "segment");
+                    k_pm_kick_drift<R><<<pgrid(), PM_NT, 0, st>>>(xn(n), n == n0 ? ckq[s]->p : q.p, xn(n + 1), q.p, np, N,
+                                                                  sp.p, coefs[3 * n], coefs[3 * n + 1], mcell, rho.p);
                 }
-                potential(sx.p, coefs[3 * n + 2], sp.p);
             }
             for (int n = n1 - 1; n >= n0; n--) {
                 const double kq = coefs[3 * n], kx = coefs[3 * n + 1], pc = coefs[3 * n + 2];
-                const double *xn = segx[n - n0]->p;
-                k_pm_adj_kick<R><<<pgrid(), PM_NT, 0, st>>>(xn, np, N, segpsi[n - n0]->p, kq, kx, lx.p, lq.p);
-                pck(cudaMemsetAsync(lam.p, 0, 3 * n3 * sizeof(R), st), "memset");
-                k_pm_deposit<R, 3><<<pgrid(), PM_NT, 0, st>>>(xn, np, N, lq.p, 0.0, lam.p);
-                k_pm_adj_div<R><<<fgrid(), PM_NT, 0, st>>>(lam.p, N, kq, rho.p);
-                poisson(rho.p, pc);
-                k_pm_adj_deposit<R><<<pgrid(), PM_NT, 0, st>>>(xn, np, N, rho.p, mass * (double)n3, lx.p);
+                clear(lam.p, 4 * n3);
+                k_pm_reverse<R><<<pgrid(), PM_NT, 0, st>>>(xb, fld.p, mb, xn(n), segpsi[n - n0]->p, kq, kx,
+                                                           first ? nullptr : lx.p, first ? nullptr : lq.p, lx.p, lq.p,
+                                                           lam.p, np, N);
+                first = false;
+                k_pm_adj_div<R><<<dg, db, 0, st>>>(lam.p, N, kq, fld.p);
+                poisson(fld.p, fld.p, pc);
+                mb = mcell;
+                xb = xn(n);   // of the segment's first step the checkpoint, which outlives the segment
             }
         }
-        pck(cudaMemcpyAsync(gx0, lx.p, 3 * np * sizeof(double), cudaMemcpyDeviceToDevice, st), "copy gx");
-        pck(cudaMemcpyAsync(gq0, lq.p, 3 * np * sizeof(double), cudaMemcpyDeviceToDevice, st), "copy gq");
+        k_pm_reverse<R><<<pgrid(), PM_NT, 0, st>>>(xb, fld.p, mb, nullptr, nullptr, 0.0, 0.0, lx.p, lq.p, gx0, gq0, nullptr,
+                                                   np, N);
         pck(cudaGetLastError(), "adjoint launch");
         pck(cudaStreamSynchronize(st), "adjoint");
         check_device("adjoint");

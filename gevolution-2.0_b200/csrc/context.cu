@@ -214,7 +214,7 @@ template <class R> struct Ctx final : CtxBase {
     DBuf<double> partial, scal;          // scal: [0] sum, [1] phi_hom
     DBuf<unsigned long long> u64;        // [0] vmax bits, [1] lc count, [2] prelog count
     DBuf<int> derr;
-    DBuf<double> bins;
+    DBuf<double> bins, sinc;
     DBuf<unsigned long long> occ;
     DBuf<double> rho64;                  // mixed precision: FP64 density of the spectrum measurement
     DBuf<double2> tw64_full, tw64_half;  // mixed precision: FP64 twiddles of that measurement
@@ -490,19 +490,17 @@ template <class R> struct Ctx final : CtxBase {
         if (ip.noise_out) field_get(GEV_FIELD_SOURCE, ip.noise_out);
         // 2. displacement field into the B_i planes
         const FftTables<R> tb = tables();
-        fx_forward<R>(N, FX_COPY, source.p, g.n3, 1, 0, nullptr, nullptr, 0, 0, 0, 0, W.p, g.nk, nullptr, tb, st);
-        fy_pass<R>(N, -1, W.p, g.nk, 1, derr.p, tb, st);
+        launched("forward x, y passes", fxy_forward<R>(N, FX_COPY, source.p, g.n3, 1, nullptr, nullptr, 0, 0, 0, 0, W.p, g.nk, nullptr, tb, st));
         FzParams fz{};
+        fz.err = derr.p;
         fz.op = OP_ZELD;
         fz.p0 = ip.boxsize;
         fz.p1 = ip.ksphere ? 1.0 : 0.0;
         fz.tab = dtab.p;
         fz.ntab = ip.n_pk;
-        fz.err = derr.p;
         fz_pass<R>(N, fz, W.p, g.nk, nullptr, nullptr, nullptr, tb, st);
-        fy_pass<R>(N, 1, W.p, g.nk, 3, derr.p, tb, st);
-        fx_inverse<R>(N, W.p, g.nk, Bi.p, g.n3, 3, tb, st);
-        launched("ics displacement", 5);
+        launched("inverse x, y passes", fyx_inverse<R>(N, W.p, g.nk, Bi.p, g.n3, 3, tb, st));
+        launched("ics displacement");
         // 3. the displaced lattice (part_simple_info.mass = Omega_m / Np, ic_basic.hpp:2198-2201)
         np = g.n3;
         mass = ip.Omega_m / (double)g.n3;
@@ -527,18 +525,16 @@ template <class R> struct Ctx final : CtxBase {
         project(GEV_PROJ_CIC, 1.0, 1.0, 0, 0);
         gev_cosmo cm{Om, OL, Orad, fourpiG, 0.0, 0.0, 0.0, boxsize};
         const double H = hconf(a, fourpiG, cm);
-        fx_forward<R>(N, FX_COPY, source.p, g.n3, 1, 0, nullptr, nullptr, 0, 0, 0, 0, W.p, g.nk, nullptr, tb, st);
-        fy_pass<R>(N, -1, W.p, g.nk, 1, derr.p, tb, st);
+        launched("forward x, y passes", fxy_forward<R>(N, FX_COPY, source.p, g.n3, 1, nullptr, nullptr, 0, 0, 0, 0, W.p, g.nk, nullptr, tb, st));
         FzParams fp{};
+        fp.err = derr.p;
         fp.op = OP_POISSON;
         fp.p0 = (fourpiG / a) / -((double)N * (double)N * (double)N);
         fp.p1 = gr ? 3.0 * (H * H + fourpiG * Om / a) : 0.0;
         fp.p2 = 1.0;   // remove the k = 0 mode
-        fp.err = derr.p;
         fz_pass<R>(N, fp, W.p, g.nk, nullptr, nullptr, nullptr, tb, st);
-        fy_pass<R>(N, 1, W.p, g.nk, 1, derr.p, tb, st);
-        fx_inverse<R>(N, W.p, g.nk, phi.p, g.n3, 1, tb, st);
-        launched("ics phi", 5);
+        launched("inverse x, y passes", fyx_inverse<R>(N, W.p, g.nk, phi.p, g.n3, 1, tb, st));
+        launched("ics phi", 1);
         const double den = Om + OL * a * a * a + Orad / a;
         const double om_a = Om / den;
         const double orad_a = Orad / (Om * a + OL * a * a * a * a + Orad);
@@ -604,16 +600,14 @@ template <class R> struct Ctx final : CtxBase {
         launch_ics_modes(modes.p, N, ip.seed, ip.ksphere, (float)(ip.gr ? H * H : 0.0), sp, derr.p, st);
         launched("ics modes");
         // 3. kernel transform, numerator / kernel, backward transform: the displacement potential in chi
-        fx_forward<R>(N, FX_COPY, source.p, g.n3, 1, 0, nullptr, nullptr, 0, 0, 0, 0, W.p, g.nk, nullptr, tb, st);
-        fy_pass<R>(N, -1, W.p, g.nk, 1, derr.p, tb, st);
+        launched("forward x, y passes", fxy_forward<R>(N, FX_COPY, source.p, g.n3, 1, nullptr, nullptr, 0, 0, 0, 0, W.p, g.nk, nullptr, tb, st));
         FzParams fz{};
+        fz.err = derr.p;
         fz.op = OP_ICS;
         fz.modes = modes.p;
-        fz.err = derr.p;
         fz_pass<R>(N, fz, W.p, g.nk, nullptr, nullptr, nullptr, tb, st);
-        fy_pass<R>(N, 1, W.p, g.nk, 1, derr.p, tb, st);
-        fx_inverse<R>(N, W.p, g.nk, chi.p, g.n3, 1, tb, st);
-        launched("ics displacement potential", 5);
+        launched("inverse x, y passes", fyx_inverse<R>(N, W.p, g.nk, chi.p, g.n3, 1, tb, st));
+        launched("ics displacement potential");
         // 4. the tiled, displaced template
         DBuf<float> tmpl;
         tmpl.alloc(3 * ip.template_n, "particle template");
@@ -846,7 +840,7 @@ template <class R> struct Ctx final : CtxBase {
         if (which & GEV_PROJ_CIC) {
             DepOut<R> o{};
             o.p[0] = source.p;
-            deposit(DEP_T00, false, o, 1.0, mass * coeff * n3, 0.0, 0.0, accumulate, "deposit CIC");
+            deposit(DEP_CIC, false, o, 1.0, mass * coeff * n3, 0.0, 0.0, accumulate, "deposit CIC");
         }
         if (which & GEV_PROJ_T0I) {
             DepOut<R> o{};
@@ -891,15 +885,11 @@ template <class R> struct Ctx final : CtxBase {
     {
         const int N = g.N;
         const FftTables<R> tb = tables();
-        fx_forward<R>(N, prepare ? FX_PREP_T00 : FX_COPY, source.p, g.n3, 1, 0, phi.p, chi.p, bg, c, c2, c3, W.p, g.nk,
-                      partial.p, tb, st);
-        launched("fx forward (phi)");
+        launched("forward x, y passes", fxy_forward<R>(N, prepare ? FX_PREP_T00 : FX_COPY, source.p, g.n3, 1, phi.p, chi.p, bg, c, c2, c3, W.p, g.nk, partial.p, tb, st));
         if (prepare) {
-            launch_reduce_sum(partial.p, (int64_t)(N / fx_rows_per_block(N, sizeof(R) == 8)) * N, scal.p, st);
+            launch_reduce_sum(partial.p, fxy_partials(N), scal.p, st);
             launched("reduce");
         }
-        fy_pass<R>(N, -1, W.p, g.nk, 1, derr.p, tb, st);
-        launched("fy forward (phi)");
         FzParams fp{};
         fp.err = derr.p;
         fp.op = OP_POISSON;
@@ -908,10 +898,7 @@ template <class R> struct Ctx final : CtxBase {
         fp.phi_hom = scal.p + 1;
         fz_pass<R>(N, fp, W.p, g.nk, nullptr, nullptr, nullptr, tb, st);
         launched("fz Poisson");
-        fy_pass<R>(N, 1, W.p, g.nk, 1, derr.p, tb, st);
-        launched("fy inverse (phi)");
-        fx_inverse<R>(N, W.p, g.nk, phi.p, g.n3, 1, tb, st);
-        launched("fx inverse (phi)");
+        launched("inverse x, y passes", fyx_inverse<R>(N, W.p, g.nk, phi.p, g.n3, 1, tb, st));
         if (sum || phom) {
             double h[2] = {0.0, 0.0};
             ck(cudaMemcpyAsync(h, scal.p, 2 * sizeof(double), cudaMemcpyDeviceToHost, st), "D2H");
@@ -956,10 +943,7 @@ template <class R> struct Ctx final : CtxBase {
     {
         const int N = g.N;
         const FftTables<R> tb = tables();
-        fx_forward<R>(N, FX_PREP_TIJ, Sij.p, g.n3, 6, 0, phi.p, chi.p, 0, coeff, 0, 0, W.p, g.nk, nullptr, tb, st);
-        launched("fx forward (Sij)");
-        fy_pass<R>(N, -1, W.p, g.nk, 6, derr.p, tb, st);
-        launched("fy forward (Sij)");
+        launched("forward x, y passes", fxy_forward<R>(N, FX_PREP_TIJ, Sij.p, g.n3, 6, phi.p, chi.p, 0, coeff, 0, 0, W.p, g.nk, nullptr, tb, st));
         FzParams fp{};
         fp.err = derr.p;
         fp.op = OP_SCALAR;
@@ -968,14 +952,9 @@ template <class R> struct Ctx final : CtxBase {
         fp.p0 = hubble; fp.p1 = dtau; fp.p2 = dtau_old; fp.p3 = a2dtau;
         fz_pass<R>(N, fp, W.p, g.nk, hij.p, hijp.p, bstate.p, tb, st);
         launched("fz scalar projection");
-        const int nout = parab ? 4 : 1;
-        fy_pass<R>(N, 1, W.p, g.nk, nout, derr.p, tb, st);
-        launched("fy inverse (chi)");
-        fx_inverse<R>(N, W.p, g.nk, chi.p, g.n3, 1, tb, st);
-        launched("fx inverse (chi)");
+        launched("inverse x, y passes (chi)", fyx_inverse<R>(N, W.p, g.nk, chi.p, g.n3, 1, tb, st));
         if (parab) {
-            fx_inverse<R>(N, W.p + g.nk, g.nk, Bi.p, g.n3, 3, tb, st);
-            launched("fx inverse (B)");
+            launched("inverse x, y passes (B)", fyx_inverse<R>(N, W.p + g.nk, g.nk, Bi.p, g.n3, 3, tb, st));
             bi_sums = false;
         }
     }
@@ -987,12 +966,8 @@ template <class R> struct Ctx final : CtxBase {
         // T0i straight from project(T0I), or completed from project_step's sums with the current phi
         if (t0i_pending) project(GEV_PROJ_T0I, 1.0, t0i_coeff, 1, 0);
         t0i_pending = false;
-        fx_forward<R>(N, bi_sums ? FX_PREP_T0I : FX_COPY, Bi.p, g.n3, 3, 0, phi.p, nullptr, 0, 0, 0, 0, W.p, g.nk,
-                      nullptr, tb, st);
-        launched("fx forward (T0i)");
+        launched("forward x, y passes", fxy_forward<R>(N, bi_sums ? FX_PREP_T0I : FX_COPY, Bi.p, g.n3, 3, phi.p, nullptr, 0, 0, 0, 0, W.p, g.nk, nullptr, tb, st));
         bi_sums = false;
-        fy_pass<R>(N, -1, W.p, g.nk, 3, derr.p, tb, st);
-        launched("fy forward (T0i)");
         FzParams fp{};
         fp.err = derr.p;
         fp.op = OP_VECTOR;
@@ -1000,10 +975,7 @@ template <class R> struct Ctx final : CtxBase {
         fp.p1 = modif;
         fz_pass<R>(N, fp, W.p, g.nk, nullptr, nullptr, nullptr, tb, st);
         launched("fz vector projection");
-        fy_pass<R>(N, 1, W.p, g.nk, 3, derr.p, tb, st);
-        launched("fy inverse (B)");
-        fx_inverse<R>(N, W.p, g.nk, Bi.p, g.n3, 3, tb, st);
-        launched("fx inverse (B)");
+        launched("inverse x, y passes", fyx_inverse<R>(N, W.p, g.nk, Bi.p, g.n3, 3, tb, st));
     }
 
     double kick_drift(const KickDriftParams &kp) override
@@ -1040,9 +1012,19 @@ template <class R> struct Ctx final : CtxBase {
             t *= t;
             kmax = std::sqrt(3.0 * t);
         }
-        if ((int)occ.n < nb) { bins.alloc(4 * nb, "bins"); occ.alloc(nb, "bins"); }
-        ck(cudaMemsetAsync(bins.p, 0, 4 * nb * sizeof(double), st), "memset");
-        ck(cudaMemsetAsync(occ.p, 0, nb * sizeof(unsigned long long), st), "memset");
+        if ((int64_t)occ.n < (int64_t)BIN_COPIES * nb) {
+            bins.alloc((size_t)BIN_COPIES * 4 * nb, "bins");
+            occ.alloc((size_t)BIN_COPIES * nb, "bins");
+        }
+        ck(cudaMemsetAsync(bins.p, 0, (size_t)BIN_COPIES * 4 * nb * sizeof(double), st), "memset");
+        ck(cudaMemsetAsync(occ.p, 0, (size_t)BIN_COPIES * nb * sizeof(unsigned long long), st), "memset");
+        if (!sinc.p) {   // the CIC deconvolution's sinc (tools.hpp:118-127)
+            std::vector<double> h(N / 2 + 1, 1.0);
+            for (int i = 1; i <= N / 2; i++)
+                h[i] = std::sin(M_PI * (double)(float)i / (double)(float)N) * (double)(float)N / (M_PI * (double)(float)i);
+            sinc.alloc(h.size(), "sinc table");
+            ck(cudaMemcpy(sinc.p, h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice), "sinc table");
+        }
         FzParams fp{};
         fp.err = derr.p;
         fp.op = OP_BIN;
@@ -1050,22 +1032,20 @@ template <class R> struct Ctx final : CtxBase {
         fp.p1 = kmax;
         fp.bins = bins.p;
         fp.occ = occ.p;
+        fp.tab = sinc.p;
         if constexpr (sizeof(R) == 8) {
             project(GEV_PROJ_CIC, 1.0, 1.0, 0, 0);
             const FftTables<R> tb = tables();
-            fx_forward<R>(N, FX_COPY, source.p, g.n3, 1, 0, nullptr, nullptr, 0, 0, 0, 0, W.p, g.nk, nullptr, tb, st);
-            launched("fx forward (CIC)");
-            fy_pass<R>(N, -1, W.p, g.nk, 1, derr.p, tb, st);
-            launched("fy forward (CIC)");
+            launched("forward x, y passes", fxy_forward<R>(N, FX_COPY, source.p, g.n3, 1, nullptr, nullptr, 0, 0, 0, 0, W.p, g.nk, nullptr, tb, st));
             fz_pass<R>(N, fp, W.p, g.nk, nullptr, nullptr, nullptr, tb, st);
             launched("fz binning");
         } else {
             // Mixed precision measures in FP64: the density contrast of an early,
             // nearly uniform box is ~1e-2 of the density, and FP32 rounding of the
             // density itself would set the small-scale floor of the spectrum.
-            // FP64 CIC density of the FP64 positions (atomic adds), FP64
-            // transform and binning in the first two FP32 components of W; the
-            // FP32 copy of the density is left in the source field as in FP64.
+            // FP64 CIC density of the FP64 positions, FP64 transform and
+            // binning in the first two FP32 components of W; the FP32 copy of
+            // the density is left in the source field as in FP64.
             if (!rho64.p) {
                 rho64.alloc(g.n3, "FP64 density");
                 make_tables64();
@@ -1077,13 +1057,12 @@ template <class R> struct Ctx final : CtxBase {
             launched("density to FP32");
             const FftTables<double> tb{tw64_full.p, tw64_half.p, k2.p, ks.p};
             double2 *W64 = reinterpret_cast<double2 *>(W.p);   // W holds 6 FP32 components = 3 FP64 ones
-            fx_forward<double>(N, FX_COPY, rho64.p, g.n3, 1, 0, nullptr, nullptr, 0, 0, 0, 0, W64, g.nk, nullptr, tb, st);
-            launched("fx forward (CIC, FP64)");
-            fy_pass<double>(N, -1, W64, g.nk, 1, derr.p, tb, st);
-            launched("fy forward (CIC, FP64)");
+            launched("forward x, y passes", fxy_forward<double>(N, FX_COPY, rho64.p, g.n3, 1, nullptr, nullptr, 0, 0, 0, 0, W64, g.nk, nullptr, tb, st));
             fz_pass<double>(N, fp, W64, g.nk, nullptr, nullptr, nullptr, tb, st);
             launched("fz binning (FP64)");
         }
+        launch_bin_reduce(bins.p, occ.p, nb, st);
+        launched("bin sums");
         std::vector<double> acc(4 * nb);
         std::vector<unsigned long long> oc(nb);
         ck(cudaMemcpyAsync(acc.data(), bins.p, 4 * nb * sizeof(double), cudaMemcpyDeviceToHost, st), "D2H");

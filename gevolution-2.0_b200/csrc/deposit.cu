@@ -90,19 +90,20 @@ static_assert(DepCh<float>::v <= REBIN_SORT_MAX && DepCh<float, DEP_T00_TIJ_S0I>
                   DepCh<double>::v <= REBIN_SORT_MAX,
               "a single-chunk deposit must only see buckets that the re-binning keeps sorted");
 
-// record layout: [d0 d1 d2 | T00: E F G | Tij: W00 W11 W22 W01 W02 W12 | T0i: Q0 Q1 Q2 | S: P0 P1 P2]
+// record layout: [d0 d1 d2 | T00: E F G, or CIC: E | Tij: W00 W11 W22 W01 W02 W12 | T0i: Q0 Q1 Q2 | S: P0 P1 P2]
 // (S: the T0i momenta m q_i without the potential factor, DEP_T00_TIJ_S0I)
 template <int KIND> struct DepShape {
     static constexpr bool HAS00 = (KIND == DEP_T00 || KIND == DEP_T00_TIJ || KIND == DEP_T00_TIJ_S0I);
+    static constexpr bool HASM = (KIND == DEP_CIC);   // the mass alone: no momenta, no potential
     static constexpr bool HASIJ = (KIND == DEP_TIJ || KIND == DEP_T00_TIJ || KIND == DEP_T00_TIJ_S0I);
     static constexpr bool HAS0I = (KIND == DEP_T0I);
     static constexpr bool HASS = (KIND == DEP_T00_TIJ_S0I);
-    static constexpr int NC = (HAS00 ? 1 : 0) + (HASIJ ? 6 : 0) + (HAS0I ? 3 : 0) + (HASS ? 3 : 0);
+    static constexpr int NC = (HAS00 || HASM ? 1 : 0) + (HASIJ ? 6 : 0) + (HAS0I ? 3 : 0) + (HASS ? 3 : 0);
     static constexpr int F00 = 3;
     static constexpr int FIJ = 3 + (HAS00 ? 3 : 0);
     static constexpr int F0I = 3;
     static constexpr int FS = FIJ + (HASIJ ? 6 : 0);
-    static constexpr int NF = 3 + (HAS00 ? 3 : 0) + (HASIJ ? 6 : 0) + (HAS0I ? 3 : 0) + (HASS ? 3 : 0);
+    static constexpr int NF = 3 + (HAS00 ? 3 : 0) + (HASM ? 1 : 0) + (HASIJ ? 6 : 0) + (HAS0I ? 3 : 0) + (HASS ? 3 : 0);
     static constexpr int NFP = (NF + 3) & ~3;   // padded for 16-byte record loads
     static constexpr int CIJ = HAS00 ? 1 : 0;   // first Tij output component
     static constexpr int CS = CIJ + (HASIJ ? 6 : 0);   // first S output component
@@ -144,8 +145,13 @@ __device__ __forceinline__ bool make_record(const RawParticle<R> &pr, int N, con
     if (rx < -1 || rx > 7 || ry < -1 || ry > 7 || rz < -1 || rz > 7) return false;
     lc = (rx + 1) + 9 * ((ry + 1) + 9 * (rz + 1));
     const R d[3] = {(R)pr.off[0], (R)pr.off[1], (R)pr.off[2]};
-    const R q[3] = {pr.q[0], pr.q[1], pr.q[2]};
     v[0] = d[0]; v[1] = d[1]; v[2] = d[2];
+    if constexpr (S::HASM) {
+        v[S::F00] = m00;
+        bnd[0] = fabs(m00);
+        return true;
+    } else {
+    const R q[3] = {pr.q[0], pr.q[1], pr.q[2]};
     R pm = 0, pint = 0;
     if (USE_PHI) {
 #pragma unroll
@@ -203,6 +209,7 @@ __device__ __forceinline__ bool make_record(const RawParticle<R> &pr, int N, con
         }
     }
     return true;
+    }
 }
 
 // Multiply a record's value fields by the fixed-point scales of the
@@ -210,6 +217,7 @@ __device__ __forceinline__ bool make_record(const RawParticle<R> &pr, int N, con
 template <class R, int KIND> __device__ __forceinline__ void scale_record(R *r, const R *scl)
 {
     using S = DepShape<KIND>;
+    if constexpr (S::HASM) r[S::F00] *= scl[0];
     if constexpr (S::HAS00) {
 #pragma unroll
         for (int k = 0; k < 3; k++) r[S::F00 + k] *= scl[0];
@@ -239,6 +247,7 @@ __device__ __forceinline__ void gather_one(const R *r, int bx, int by, int bz, R
     const R wy = by ? r[1] : (R)1 - r[1];
     const R wz = bz ? r[2] : (R)1 - r[2];
     const R w = wx * wy * wz;
+    if constexpr (S::HASM) acc[0] += to_fixed<R>(w * r[S::F00]);
     if constexpr (S::HAS00) {
         const R val = USE_PHI ? w * (r[S::F00] + (r[S::F00 + 1] + r[S::F00 + 2] * phv) * phv) : w * r[S::F00];
         acc[0] += to_fixed<R>(val);
@@ -277,6 +286,7 @@ __device__ __forceinline__ void gather_sum(const R *r, int bx, int by, int bz, R
     const R wy = by ? r[1] : (R)1 - r[1];
     const R wz = bz ? r[2] : (R)1 - r[2];
     const R w = wx * wy * wz;
+    if constexpr (S::HASM) acc[0] += w * r[S::F00];
     if constexpr (S::HAS00) {
         acc[0] += USE_PHI ? w * (r[S::F00] + (r[S::F00 + 1] + r[S::F00 + 2] * phv) * phv) : w * r[S::F00];
     }
@@ -369,6 +379,8 @@ __host__ __device__ constexpr size_t dep_smem_bytes()
 // shared memory of two CTAs.
 template <class R, int KIND> struct DepMinBlocks { static constexpr int v = sizeof(R) == 4 ? GEV_DEP_MINB_F : 2; };
 template <> struct DepMinBlocks<float, DEP_T0I> { static constexpr int v = GEV_DEP_MINB_T0I_F; };
+// CIC records are small in either precision
+template <> struct DepMinBlocks<double, DEP_CIC> { static constexpr int v = 3; };
 template <> struct DepMinBlocks<float, DEP_T00_TIJ_S0I> { static constexpr int v = GEV_DEP_MINB_S_F; };
 
 // The dense-tile launch holds only the paths for tiles whose reach takes
@@ -388,6 +400,7 @@ __device__ __forceinline__ void deposit_tile(int tile, uint32_t *work, const PVi
 {
     using S = DepShape<KIND>;
     constexpr int NC = S::NC, NF = S::NF, NFP = S::NFP;
+    constexpr bool LOADQ = !S::HASM;
     constexpr int CH = DepCh<R, KIND, DENSE>::v;
     constexpr int NT = DENSE ? DEP_NT : dep_tile_threads<R>();   // threads
     constexpr int VPT = DEP_NT / NT;                        // vertices per thread
@@ -433,7 +446,7 @@ __device__ __forceinline__ void deposit_tile(int tile, uint32_t *work, const PVi
 #pragma unroll
     for (int u = 0; u < PP; u++) {
         const int j = t + u * NT;
-        if ((uint32_t)j < own_n) raw[u] = load_particle(p, own_lo + (uint32_t)j);
+        if ((uint32_t)j < own_n) raw[u] = load_particle<R, LOADQ>(p, own_lo + (uint32_t)j);
     }
     // the candidate ranges, formed by warp 0 in registers and stored to shared
     // memory; the barrier below publishes them together with the phi stencil
@@ -618,7 +631,7 @@ __device__ __forceinline__ void deposit_tile(int tile, uint32_t *work, const PVi
 #pragma unroll
         for (int u = 0; u < PP; u++) {
             const int j = t + u * NT;
-            if (j < n && (uint32_t)j >= own_n) raw[u] = load_particle(p, seg_find(seg_lo, seg_pre, (uint32_t)j));
+            if (j < n && (uint32_t)j >= own_n) raw[u] = load_particle<R, LOADQ>(p, seg_find(seg_lo, seg_pre, (uint32_t)j));
         }
         build_chunk(n, raw);
         if constexpr (VPT == 2) {
@@ -663,7 +676,7 @@ __device__ __forceinline__ void deposit_tile(int tile, uint32_t *work, const PVi
 #pragma unroll
             for (int u = 0; u < PP; u++) {
                 const uint32_t j = base + (uint32_t)(t + u * NT);
-                if (t + u * NT < n && (base > 0 || j >= own_n)) raw[u] = load_particle(p, seg_index(seg_lo, seg_pre, j));
+                if (t + u * NT < n && (base > 0 || j >= own_n)) raw[u] = load_particle<R, LOADQ>(p, seg_index(seg_lo, seg_pre, j));
             }
             build_chunk(n, raw);
             gather_vertex(acc);
@@ -704,7 +717,7 @@ __device__ __forceinline__ void deposit_tile(int tile, uint32_t *work, const PVi
             const uint32_t i = seg_index(seg_lo, seg_pre, j);
             R v[NF], b[NC];
             int lc;
-            if (make_record<R, KIND, USE_PHI>(load_particle(p, i), N, fN, x0, y0, z0, phis, ra, rm00, rmij, rm0i, v, lc, b)) {
+            if (make_record<R, KIND, USE_PHI>(load_particle<R, LOADQ>(p, i), N, fN, x0, y0, z0, phis, ra, rm00, rmij, rm0i, v, lc, b)) {
 #pragma unroll
                 for (int c = 0; c < NC; c++) lb[c] = fmax(lb[c], b[c]);
             }
@@ -729,7 +742,7 @@ __device__ __forceinline__ void deposit_tile(int tile, uint32_t *work, const PVi
                 const uint32_t i = seg_index(seg_lo, seg_pre, base + (uint32_t)j);
                 R v[NF], b[NC];
                 int lc;
-                if (make_record<R, KIND, USE_PHI>(load_particle(p, i), N, fN, x0, y0, z0, phis, ra, rm00, rmij, rm0i, v, lc, b)) {
+                if (make_record<R, KIND, USE_PHI>(load_particle<R, LOADQ>(p, i), N, fN, x0, y0, z0, phis, ra, rm00, rmij, rm0i, v, lc, b)) {
                     scale_record<R, KIND>(v, scl_s);   // fixed-point scales of the components (weights unscaled)
                     store_record<R, NFP>(rec, j, v);
                     rcell[j] = (uint16_t)lc;
@@ -841,17 +854,27 @@ void launch_deposit(int kind, bool use_phi, const PView<R> &p, const uint32_t *b
                     const DepOut<R> &out, double a, double m00, double mij, double m0i, int accumulate, uint32_t *work,
                     int *err, cudaStream_t st)
 {
-#define GEV_DEP(K)                                                                                                \
-    if (kind == K) {                                                                                              \
-        if (use_phi) launch_k<R, K, true>(p, bstart, N, phi, out, a, m00, mij, m0i, accumulate, work, err, st);   \
-        else launch_k<R, K, false>(p, bstart, N, phi, out, a, m00, mij, m0i, accumulate, work, err, st);          \
-        return;                                                                                                   \
+#define GEV_DEP(K, PHI) launch_k<R, K, PHI>(p, bstart, N, phi, out, a, m00, mij, m0i, accumulate, work, err, st)
+    switch (kind) {
+    case DEP_CIC: GEV_DEP(DEP_CIC, false); break;
+    case DEP_T00:   // without the potential T00 is the CIC density
+        if (use_phi) GEV_DEP(DEP_T00, true);
+        else GEV_DEP(DEP_CIC, false);
+        break;
+    case DEP_TIJ:
+        if (use_phi) GEV_DEP(DEP_TIJ, true);
+        else GEV_DEP(DEP_TIJ, false);
+        break;
+    case DEP_T00_TIJ:
+        if (use_phi) GEV_DEP(DEP_T00_TIJ, true);
+        else GEV_DEP(DEP_T00_TIJ, false);
+        break;
+    case DEP_T0I:
+        if (use_phi) GEV_DEP(DEP_T0I, true);
+        else GEV_DEP(DEP_T0I, false);
+        break;
+    case DEP_T00_TIJ_S0I: GEV_DEP(DEP_T00_TIJ_S0I, true); break;
     }
-    GEV_DEP(DEP_T00)
-    GEV_DEP(DEP_TIJ)
-    GEV_DEP(DEP_T00_TIJ)
-    GEV_DEP(DEP_T0I)
-    GEV_DEP(DEP_T00_TIJ_S0I)
 #undef GEV_DEP
 }
 

@@ -3,7 +3,7 @@
 //
 // Fourier layout: kx + PP*(ky + N*kz) for kx < P = N/2 + 1 (half spectrum
 // along x); the row pitch PP = N/2 + 2 is even so that every row starts on a
-// 16-byte boundary (tensor-memory-access copies need 16-byte-aligned strides).
+// 16-byte boundary.
 //   fx_fwd : R2C along x for T rows (y0..y0+T-1, z); fused prepareFTsource
 //   fy     : complex FFT along y for T kx-columns at one z (in place)
 //   fz     : FFT along z, pointwise Fourier-space solver, inverse FFT along z,
@@ -12,31 +12,11 @@
 #pragma once
 
 #include "common.cuh"
-#include "fft.cuh"
+#include "fftreg.cuh"
+#include "kernels.h"
 #include "tma.cuh"
 
 namespace gev {
-
-// occupancy the z pass and the six-component x pass are compiled for
-#ifndef GEV_FZ_MINB
-#define GEV_FZ_MINB 4   // resident CTAs of 256 threads per SM (FP32)
-#endif
-#ifndef GEV_FZ_MINB_D
-#define GEV_FZ_MINB_D 3   // the same for FP64
-#endif
-#ifndef GEV_TIJ6_MINB
-#define GEV_TIJ6_MINB 3
-#endif
-// resident CTAs per SM of the FP32 x passes (256 threads) and of the FP32 bulk-copy y pass (512 threads)
-#ifndef GEV_FX_MINB
-#define GEV_FX_MINB 4
-#endif
-#ifndef GEV_FXI_MINB
-#define GEV_FXI_MINB 4
-#endif
-#ifndef GEV_FY_MINB
-#define GEV_FY_MINB 2
-#endif
 
 // ---------------------------------------------------------------------------
 // fused source preparation (PHINONLINEAR): T00 in FP64, Tij in the field precision
@@ -48,16 +28,9 @@ template <class R> struct FxArgs {
     const R *phi;
     const R *chi;
     double bg, c, c2, c3; // prepareFTsource_T00 params (bgmodel, coeff, coeff2, coeff3) / Tij coeff in c
-    int comp0;            // first Tij component of the batch (gridDim.z = number of components)
     typename CT<R>::C *out;
     double *partial;      // per-block partial sums of the source (FX_PREP_T00)
 };
-
-template <class R>
-__device__ __forceinline__ double ld(const R *f, int N, int x, int y, int z)
-{
-    return (double)f[sidx(N, wrapi(x, N), wrapi(y, N), wrapi(z, N))];
-}
 
 template <class R>
 __device__ __forceinline__ R ldr(const R *f, int N, int x, int y, int z)
@@ -65,45 +38,36 @@ __device__ __forceinline__ R ldr(const R *f, int N, int x, int y, int z)
     return __ldg(f + sidx(N, wrapi(x, N), wrapi(y, N), wrapi(z, N)));
 }
 
-// Strided fill of TOT elements (element idx = threadIdx.x + k*NT): each thread
-// issues B loads before the matching B stores, so B global loads per thread are
-// in flight instead of one (the passes are bound by load latency otherwise).
-template <int TOT, int NT, int B, class V, class LOAD, class STORE>
-__device__ __forceinline__ void staged_fill(LOAD &&load, STORE &&store)
+// two adjacent values (x even: 8- or 16-byte aligned) in one load
+template <class R> __device__ __forceinline__ typename CT<R>::C ld_pair(const R *p)
 {
-    constexpr int PER = (TOT + NT - 1) / NT;
-#pragma unroll
-    for (int k0 = 0; k0 < PER; k0 += B) {
-        V v[B];
-#pragma unroll
-        for (int k = 0; k < B; k++) {
-            const int idx = threadIdx.x + (k0 + k) * NT;
-            if (k0 + k < PER && (PER * NT == TOT || idx < TOT)) v[k] = load(idx);
-        }
-#pragma unroll
-        for (int k = 0; k < B; k++) {
-            const int idx = threadIdx.x + (k0 + k) * NT;
-            if (k0 + k < PER && (PER * NT == TOT || idx < TOT)) store(idx, v[k]);
-        }
-    }
+    return __ldg(reinterpret_cast<const typename CT<R>::C *>(p));
 }
 
-// prepareFTsource_T00: gevolution.hpp:160-171
+// prepareFTsource_T00 (gevolution.hpp:160-171) at one point, in FP64: source
+// s, phi and chi there, phi at the six neighbours
+template <class R>
+__device__ __forceinline__ double t00_point(const FxArgs<R> &a, R s_, R p_, R chi, R pxm, R pxp, R pym, R pyp, R pzm, R pzp)
+{
+    const double ph = (double)p_;
+    double r = a.c2 * ((double)s_ - a.bg);
+    r *= 1.0 - 2.0 * ph * (1.0 - ph);
+    double g;
+    g = (double)pxm - (double)pxp; r += 0.125 * g * g;
+    g = (double)pym - (double)pyp; r += 0.125 * g * g;
+    g = (double)pzm - (double)pzp; r += 0.125 * g * g;
+    r += (a.c3 * (1.0 - 3.0 * ph) - a.c) * ph - a.c3 * (double)chi;
+    return r;
+}
+
 template <class R>
 __device__ __forceinline__ double prep_t00(const FxArgs<R> &a, int N, int x, int y, int z, double &src)
 {
-    int64_t i = sidx(N, x, y, z);
-    double s = (double)a.in[i];
-    double ph = (double)a.phi[i];
-    src = s;
-    double r = a.c2 * (s - a.bg);
-    r *= 1.0 - 2.0 * ph * (1.0 - ph);
-    double g;
-    g = ld(a.phi, N, x - 1, y, z) - ld(a.phi, N, x + 1, y, z); r += 0.125 * g * g;
-    g = ld(a.phi, N, x, y - 1, z) - ld(a.phi, N, x, y + 1, z); r += 0.125 * g * g;
-    g = ld(a.phi, N, x, y, z - 1) - ld(a.phi, N, x, y, z + 1); r += 0.125 * g * g;
-    r += (a.c3 * (1.0 - 3.0 * ph) - a.c) * ph - a.c3 * (double)a.chi[i];
-    return r;
+    const int64_t i = sidx(N, x, y, z);
+    src = (double)a.in[i];
+    return t00_point(a, a.in[i], a.phi[i], a.chi[i], ldr(a.phi, N, x - 1, y, z), ldr(a.phi, N, x + 1, y, z),
+                     ldr(a.phi, N, x, y - 1, z), ldr(a.phi, N, x, y + 1, z), ldr(a.phi, N, x, y, z - 1),
+                     ldr(a.phi, N, x, y, z + 1));
 }
 
 // prepareFTsource_Tij for one symmetric component c (00,01,02,11,12,22),
@@ -134,85 +98,170 @@ __device__ __forceinline__ R prep_tij(const R *T, const R *phi, R coeff, int c, 
     return (R)2 * u * v + w * (u + v + (R)0.5 * w) + coeff * t;
 }
 
-// T0i component c completed from its potential-free sum S_c at vertex x:
-// T0i_c(x) = (1 + phi(x) + phi(x + e_c)) S_c(x) -- the per-vertex factor of
-// particle_T0i_project (gevolution.hpp:2031-2201), which does not depend on
-// the particle, applied once per vertex with the current phi
-template <class R>
-__device__ __forceinline__ R prep_t0i(const R *S, const R *phi, int c, int N, int x, int y, int z)
+// ---------------------------------------------------------------------------
+// x pass, forward: real rows -> half spectrum.  grid (N/T, N, ncomp), R2 * T
+// threads.  A row of N reals is transformed as N/2 complex pairs (two-step
+// register FFT) and unfolded into kx = 0 .. N/2.
+// ---------------------------------------------------------------------------
+// the transform of `LINES` rows whose step 1 is stored: step 2 in place (R2
+// threads per line), then each warp unfolds whole rows.  With Z the transform
+// of the row's pairs, ze = (Z[k] + conj Z[M-k]) / 2 and
+// zo = (Z[k] - conj Z[M-k]) / 2i: kx = k gets ze + w zo, kx = M - k its mirror
+// conj(ze - w zo), from the same two values.  dst(l) is the output row of
+// line l.
+template <int M, int LINES, int NT, class C, class DST>
+__device__ __forceinline__ void fx_finish(C *smem, const C *__restrict__ tw_full, DST &&dst)
 {
-    const int64_t i = sidx(N, x, y, z);
-    const R f = (R)1 + __ldg(phi + i) + ldr(phi, N, x + (c == 0), y + (c == 1), z + (c == 2));
-    return f * __ldg(S + i);
+    using R = decltype(smem->x);
+    constexpr int R1 = RegPlan<M>::R1, R2 = RegPlan<M>::R2, ES = exch_size<M, 1>();
+    constexpr int GRP = NT / R2, NW = (NT + 31) / 32;
+    const int u = threadIdx.x % R2;
+#pragma unroll 1
+    for (int l = threadIdx.x / R2; l < LINES; l += GRP) {
+        C *buf = smem + l * ES;
+        for (int q = u; q < R1; q += R2) {
+            C v[R2];
+            step2_load<M, -1, 1>(v, buf, q);
+#pragma unroll
+            for (int p = 0; p < R2; p++) buf[q * (R2 + 1) + p] = v[p];
+        }
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int l = threadIdx.x / 32; l < LINES; l += NW) {
+        const C *buf = smem + l * ES;
+        C *out = dst(l);
+#pragma unroll 4
+        for (int k = threadIdx.x % 32; k <= M / 2; k += 32) {
+            const int m = k == 0 ? 0 : M - k;
+            const C zk = buf[(k % R1) * (R2 + 1) + k / R1];
+            C zm = buf[(m % R1) * (R2 + 1) + m / R1];
+            zm.y = -zm.y;
+            const C ze = cscale(cadd(zk, zm), R(0.5)), d = csub(zk, zm);
+            const C wo = cmul(__ldg(tw_full + k), mk(R(0.5) * d.y, R(-0.5) * d.x));
+            out[k] = cadd(ze, wo);
+            if (k < M / 2) out[M - k] = cconj(csub(ze, wo));
+        }
+    }
 }
 
-// ---------------------------------------------------------------------------
-// x pass, forward: real rows -> half spectrum.  grid (N/T, N, ncomp)
-// ---------------------------------------------------------------------------
-template <class R, int N, int T, int NT, int MODE>
-__global__ void __launch_bounds__(NT, sizeof(R) == 4 ? GEV_FX_MINB : 1) k_fx_fwd(FxArgs<R> a, int64_t in_stride, int64_t out_stride,
-                                               const typename CT<R>::C *__restrict__ tw_half,
-                                               const typename CT<R>::C *__restrict__ tw_full)
+// the pair of sources at x = 2n, 2n + 1 of row (y, z)
+template <class R, int N, int MODE, int COMP>
+__device__ __forceinline__ typename CT<R>::C fx_pair(const FxArgs<R> &a, const R *in, int n, int y, int z, double &lsum)
+{
+    const int x0 = 2 * n;
+    if constexpr (MODE == FX_COPY) {
+        // a caller's own array (gev_poisson_noalloc) may be aligned to single values only
+        const R *p = in + sidx(N, x0, y, z);
+        if (reinterpret_cast<uintptr_t>(in) % (2 * sizeof(R)) == 0) return ld_pair(p);
+        return mk(__ldg(p), __ldg(p + 1));
+    } else if constexpr (MODE == FX_PREP_T00) {
+        const int xm = x0 == 0 ? N - 1 : x0 - 1, x2 = x0 + 2 == N ? 0 : x0 + 2;
+        const int ym = y == 0 ? N - 1 : y - 1, yp = y == N - 1 ? 0 : y + 1;
+        const int zm = z == 0 ? N - 1 : z - 1, zp = z == N - 1 ? 0 : z + 1;
+        const auto s = ld_pair(in + sidx(N, x0, y, z)), ch = ld_pair(a.chi + sidx(N, x0, y, z));
+        const R *row = a.phi + sidx(N, 0, y, z);
+        const auto p0 = ld_pair(row + x0);
+        const R pm = __ldg(row + xm), p2 = __ldg(row + x2);
+        const auto ya = ld_pair(a.phi + sidx(N, x0, ym, z)), yb = ld_pair(a.phi + sidx(N, x0, yp, z));
+        const auto za = ld_pair(a.phi + sidx(N, x0, y, zm)), zb = ld_pair(a.phi + sidx(N, x0, y, zp));
+        lsum += (double)s.x + (double)s.y;
+        return mk((R)t00_point(a, s.x, p0.x, ch.x, pm, p0.y, ya.x, yb.x, za.x, zb.x),
+                  (R)t00_point(a, s.y, p0.y, ch.y, p0.x, p2, ya.y, yb.y, za.y, zb.y));
+    } else if constexpr (MODE == FX_PREP_TIJ) {
+        // one component of prepareFTsource_Tij (COMP in the order 00,01,02,11,12,22),
+        // the expressions of tij6_point
+        const R rc = (R)a.c;
+        const auto t = ld_pair(in + sidx(N, x0, y, z));
+        const int ym = y == 0 ? N - 1 : y - 1, yp = y == N - 1 ? 0 : y + 1;
+        const int zm = z == 0 ? N - 1 : z - 1, zp = z == N - 1 ? 0 : z + 1;
+        const int xm = x0 == 0 ? N - 1 : x0 - 1, x2 = x0 + 2 == N ? 0 : x0 + 2;
+        auto pair = [&](int yy, int zz) { return ld_pair(a.phi + sidx(N, x0, yy, zz)); };
+        auto one = [&](int x, int yy, int zz) { return __ldg(a.phi + sidx(N, x, yy, zz)); };
+        auto diag = [&](R p, R m, R tv) { const R g = p - m; return (R)0.5 * g * g + rc * tv; };
+        auto off = [&](R p0, R pi, R pj, R pij, R tv) {
+            const R u = pi - p0, v = pj - p0, w = (pij - pi) - (pj - p0);
+            return (R)2 * u * v + w * (u + v + (R)0.5 * w) + rc * tv;
+        };
+        if constexpr (COMP == 0) {
+            const auto c = pair(y, z);
+            return mk(diag(c.y, one(xm, y, z), t.x), diag(one(x2, y, z), c.x, t.y));
+        } else if constexpr (COMP == 3 || COMP == 5) {
+            const auto p = COMP == 3 ? pair(yp, z) : pair(y, zp), m = COMP == 3 ? pair(ym, z) : pair(y, zm);
+            return mk(diag(p.x, m.x, t.x), diag(p.y, m.y, t.y));
+        } else if constexpr (COMP == 4) {
+            const auto c = pair(y, z), py = pair(yp, z), pz = pair(y, zp), pyz = pair(yp, zp);
+            return mk(off(c.x, py.x, pz.x, pyz.x, t.x), off(c.y, py.y, pz.y, pyz.y, t.y));
+        } else {
+            // 01 and 02: x and the other axis
+            const auto c = pair(y, z), o = COMP == 1 ? pair(yp, z) : pair(y, zp);
+            const R c2 = one(x2, y, z), o2 = COMP == 1 ? one(x2, yp, z) : one(x2, y, zp);
+            return mk(off(c.x, c.y, o.x, o.y, t.x), off(c.y, c2, o.y, o2, t.y));
+        }
+    } else {
+        // FX_PREP_T0I: T0i component c completed from its potential-free sum S_c at
+        // vertex x: T0i_c(x) = (1 + phi(x) + phi(x + e_c)) S_c(x) -- the per-vertex
+        // factor of particle_T0i_project (gevolution.hpp:2031-2201), applied once
+        // per vertex with the current phi
+        static_assert(MODE == FX_PREP_T0I, "mode");
+        const auto s = ld_pair(in + sidx(N, x0, y, z));
+        const R *row = a.phi + sidx(N, 0, y, z);
+        const auto p0 = ld_pair(row + x0);
+        typename CT<R>::C pe;
+        if constexpr (COMP == 0) pe = mk(p0.y, __ldg(row + (x0 + 2 == N ? 0 : x0 + 2)));
+        else if constexpr (COMP == 1) pe = ld_pair(a.phi + sidx(N, x0, y == N - 1 ? 0 : y + 1, z));
+        else pe = ld_pair(a.phi + sidx(N, x0, y, z == N - 1 ? 0 : z + 1));
+        return mk(((R)1 + p0.x + pe.x) * s.x, ((R)1 + p0.y + pe.y) * s.y);
+    }
+}
+
+// sum of v over the block's NT threads (any NT), written by thread 0
+template <int NT> __device__ __forceinline__ void block_sum(double v, double *out)
+{
+    __shared__ double red[(NT + 31) / 32];
+    for (int o = 16; o > 0; o >>= 1) {
+        const double up = __shfl_down_sync(__activemask(), v, o);
+        if ((int)(threadIdx.x & 31) + o < 32 && (int)threadIdx.x + o < NT) v += up;
+    }
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double s = 0.0;
+        for (int w = 0; w < (NT + 31) / 32; w++) s += red[w];
+        *out = s;
+    }
+}
+
+template <class R, int N, int T, int MODE, int MINB>
+__global__ void __launch_bounds__(RegPlan<N / 2>::R2 *T, MINB) k_fx_fwd(FxArgs<R> a, int64_t in_stride, int64_t out_stride,
+                                                                       const typename CT<R>::C *__restrict__ tw_half,
+                                                                       const typename CT<R>::C *__restrict__ tw_full)
 {
     using C = typename CT<R>::C;
-    constexpr int M = N / 2, P = N / 2 + 1, PP = N / 2 + 2, LD = T + 1;
+    constexpr int M = N / 2, PP = N / 2 + 2, R1 = RegPlan<M>::R1, R2 = RegPlan<M>::R2, NT = R2 * T, ES = exch_size<M, 1>();
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    C *buf = reinterpret_cast<C *>(smem_raw);
-    __shared__ double red[NT / 32];
-
+    C *smem = reinterpret_cast<C *>(smem_raw);
+    const int u = threadIdx.x % R2, l = threadIdx.x / R2;
     const int y0 = blockIdx.x * T, z = blockIdx.y, comp = blockIdx.z;
     const R *in = a.in + (int64_t)comp * in_stride;
     C *out = a.out + (int64_t)comp * out_stride;
     double lsum = 0.0;
-
-    staged_fill<M * T, NT, (MODE == FX_COPY ? 8 : 4), C>(
-        [&](int idx) {
-            const int n = idx % M, t = idx / M, y = y0 + t;
-            R v0, v1;
-            if constexpr (MODE == FX_COPY) {
-                const R *row = in + sidx(N, 0, y, z);
-                v0 = __ldg(row + 2 * n);
-                v1 = __ldg(row + 2 * n + 1);
-            } else if constexpr (MODE == FX_PREP_T00) {
-                double s0, s1;
-                v0 = (R)prep_t00(a, N, 2 * n, y, z, s0);
-                v1 = (R)prep_t00(a, N, 2 * n + 1, y, z, s1);
-                lsum += s0 + s1;
-            } else if constexpr (MODE == FX_PREP_T0I) {
-                v0 = prep_t0i(in, a.phi, a.comp0 + comp, N, 2 * n, y, z);
-                v1 = prep_t0i(in, a.phi, a.comp0 + comp, N, 2 * n + 1, y, z);
-            } else {
-                v0 = prep_tij(in, a.phi, (R)a.c, a.comp0 + comp, N, 2 * n, y, z);
-                v1 = prep_tij(in, a.phi, (R)a.c, a.comp0 + comp, N, 2 * n + 1, y, z);
-            }
-            return mk(v0, v1);
-        },
-        [&](int idx, C v) { buf[(idx % M) * LD + idx / M] = v; });
+    {
+        C v[R1];
+        auto load = [&](auto cc) {
+#pragma unroll
+            for (int r = 0; r < R1; r++) v[r] = fx_pair<R, N, MODE, decltype(cc)::v>(a, in, u + R2 * r, y0 + l, z, lsum);
+        };
+        // the component is uniform over the block: branch around the loads, not between them
+        if (MODE != FX_PREP_T0I || comp == 0) load(IntC<0>{});
+        else if (comp == 1) load(IntC<1>{});
+        else load(IntC<2>{});
+        step1_store<M, -1, 1>(v, smem + l * ES, u, tw_half);
+    }
     __syncthreads();
-    fft_lines<M, -1, T, NT>(buf, LD, tw_half);
+    fx_finish<M, T, NT>(smem, tw_full, [&](int i) { return out + (int64_t)PP * (y0 + i + (int64_t)N * z); });
 
-    for (int idx = threadIdx.x; idx < P * T; idx += NT) {
-        int k = idx % P, t = idx / P, y = y0 + t;
-        C zk = buf[(k == M ? 0 : k) * LD + t];
-        C zm = buf[(k == 0 ? 0 : M - k) * LD + t];
-        zm.y = -zm.y;                                  // conj(Z[M-k])
-        C ze = cscale(cadd(zk, zm), R(0.5));
-        C d = csub(zk, zm);
-        C zo = mk(R(0.5) * d.y, R(-0.5) * d.x);        // (zk - conj(zm)) / (2i)
-        C w = __ldg(tw_full + k);
-        out[k + (int64_t)PP * (y + (int64_t)N * z)] = cadd(ze, cmul(w, zo));
-    }
-
-    if constexpr (MODE == FX_PREP_T00) {
-        for (int o = 16; o > 0; o >>= 1) lsum += __shfl_down_sync(0xffffffffu, lsum, o);
-        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = lsum;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            double s = 0.0;
-            for (int w = 0; w < NT / 32; w++) s += red[w];
-            a.partial[blockIdx.x + gridDim.x * blockIdx.y] = s;
-        }
-    }
+    if constexpr (MODE == FX_PREP_T00) block_sum<NT>(lsum, a.partial + blockIdx.x + gridDim.x * blockIdx.y);
 }
 
 // prepareFTsource_Tij for all six components at one point from the ten
@@ -236,145 +285,321 @@ __device__ __forceinline__ void tij6_point(R p0, R pxp, R pxm, R pyp, R pym, R p
     o[4] = (R)2 * u * v + w * (u + v + (R)0.5 * w) + coeff * t[4];
 }
 
-// two adjacent values (x even: 8- or 16-byte aligned) in one load
-template <class R> __device__ __forceinline__ typename CT<R>::C ld_pair(const R *p)
-{
-    return __ldg(reinterpret_cast<const typename CT<R>::C *>(p));
-}
-
 // x pass, forward, for the six Tij components at once: each potential value
-// is loaded once for all six sources.  grid (N/T, N)
-template <class R, int N, int T, int NT>
-__global__ void __launch_bounds__(NT, GEV_TIJ6_MINB) k_fx_fwd_tij6(const R *__restrict__ Tij, int64_t n3, const R *__restrict__ phi,
-                                                    double coeff, typename CT<R>::C *out, int64_t out_stride,
-                                                    const typename CT<R>::C *__restrict__ tw_half,
-                                                    const typename CT<R>::C *__restrict__ tw_full)
+// is loaded once for all six sources.  grid (N/T, N); G thread groups per
+// line: every group forms the sources of its share of the pairs, and
+// transforms its share of the components.
+template <class R, int N, int T, int G, int MINB>
+__global__ void __launch_bounds__(RegPlan<N / 2>::R2 *T *G, MINB) k_fx_fwd_tij6(const R *__restrict__ Tij, int64_t n3,
+                                                                              const R *__restrict__ phi, double coeff,
+                                                                              typename CT<R>::C *out, int64_t out_stride,
+                                                                              const typename CT<R>::C *__restrict__ tw_half,
+                                                                              const typename CT<R>::C *__restrict__ tw_full)
 {
     using C = typename CT<R>::C;
-    // the six components' rows side by side: 6T lines of one batched transform,
-    // element n of line c*T + t at buf[n*LD + c*T + t]
-    constexpr int M = N / 2, P = N / 2 + 1, PP = N / 2 + 2, T6 = 6 * T, LD = T6 + 1;
+    constexpr int M = N / 2, PP = N / 2 + 2, R1 = RegPlan<M>::R1, R2 = RegPlan<M>::R2, NT = R2 * T * G, ES = exch_size<M, 1>();
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    C *buf = reinterpret_cast<C *>(smem_raw);
+    C *smem = reinterpret_cast<C *>(smem_raw);   // line c * T + l
     const int y0 = blockIdx.x * T, z = blockIdx.y;
     const R rc = (R)coeff;
-    struct Six { C v[6]; };
-    staged_fill<M * T, NT, 2, Six>(
-        [&](int idx) {
+    {
+        const int zm = z == 0 ? N - 1 : z - 1, zp = z == N - 1 ? 0 : z + 1;
+#pragma unroll 2
+        for (int idx = threadIdx.x; idx < M * T; idx += NT) {
             // the points x0 = 2n and x0 + 1 of row (y, z): the potential rows
             // they touch are read as aligned pairs plus the four values beyond
-            const int n = idx % M, t = idx / M, y = y0 + t;
+            const int n = idx % M, l = idx / M, y = y0 + l;
             const int x0 = 2 * n, xm = x0 == 0 ? N - 1 : x0 - 1, x2 = x0 + 2 == N ? 0 : x0 + 2;
             const int ym = y == 0 ? N - 1 : y - 1, yp = y == N - 1 ? 0 : y + 1;
-            const int zm = z == 0 ? N - 1 : z - 1, zp = z == N - 1 ? 0 : z + 1;
-            const R *r00 = phi + sidx(N, 0, y, z), *rm0 = phi + sidx(N, 0, ym, z), *rp0 = phi + sidx(N, 0, yp, z);
-            const R *r0p = phi + sidx(N, 0, y, zp), *r0m = phi + sidx(N, 0, y, zm), *rpp = phi + sidx(N, 0, yp, zp);
-            const C c00 = ld_pair(r00 + x0), cm0 = ld_pair(rm0 + x0), cp0 = ld_pair(rp0 + x0);
-            const C c0p = ld_pair(r0p + x0), c0m = ld_pair(r0m + x0), cpp = ld_pair(rpp + x0);
-            const R f00m = __ldg(r00 + xm), f002 = __ldg(r00 + x2), fp02 = __ldg(rp0 + x2), f0p2 = __ldg(r0p + x2);
-            const int64_t i0 = sidx(N, x0, y, z);
+            // 32-bit offsets (N <= 768): one base register per plane
+            auto row = [&](int yy, int zz) { return ((uint32_t)zz * N + (uint32_t)yy) * N; };
+            const uint32_t r00 = row(y, z), rp0 = row(yp, z), r0p = row(y, zp);
+            const C c00 = ld_pair(phi + (r00 + x0)), cm0 = ld_pair(phi + (row(ym, z) + x0)), cp0 = ld_pair(phi + (rp0 + x0));
+            const C c0p = ld_pair(phi + (r0p + x0)), c0m = ld_pair(phi + (row(y, zm) + x0)), cpp = ld_pair(phi + (row(yp, zp) + x0));
+            const R f00m = __ldg(phi + (r00 + xm)), f002 = __ldg(phi + (r00 + x2)), fp02 = __ldg(phi + (rp0 + x2)),
+                    f0p2 = __ldg(phi + (r0p + x2));
             R t0[6], t1[6];
 #pragma unroll
             for (int c = 0; c < 6; c++) {
-                const C tv = ld_pair(Tij + c * n3 + i0);
+                const C tv = ld_pair(Tij + c * n3 + (r00 + x0));
                 t0[c] = tv.x;
                 t1[c] = tv.y;
             }
             R a0[6], a1[6];
             tij6_point(c00.x, c00.y, f00m, cp0.x, cm0.x, c0p.x, c0m.x, cp0.y, c0p.y, cpp.x, t0, rc, a0);
             tij6_point(c00.y, f002, c00.x, cp0.y, cm0.y, c0p.y, c0m.y, fp02, f0p2, cpp.y, t1, rc, a1);
-            Six s;
+            // pair n = j + R2 r waits at slot (r, j), where step 1 of thread j reads it
+            C *b = smem + l * ES + (n / R2) * (R2 + 1) + n % R2;
 #pragma unroll
-            for (int c = 0; c < 6; c++) s.v[c] = mk(a0[c], a1[c]);
-            return s;
-        },
-        [&](int idx, Six s) {
-            const int o = (idx % M) * LD + idx / M;
+            for (int c = 0; c < 6; c++) b[c * T * ES] = mk(a0[c], a1[c]);
+        }
+    }
+    __syncthreads();
+    const int u = threadIdx.x % R2;
+#pragma unroll 1
+    for (int l = threadIdx.x / R2; l < 6 * T; l += T * G) {
+        C *b = smem + l * ES;
+        C v[R1];
 #pragma unroll
-            for (int c = 0; c < 6; c++) buf[o + c * T] = s.v[c];
-        });
-    __syncthreads();
-    fft_lines<M, -1, T6, NT>(buf, LD, tw_half);
-    for (int idx = threadIdx.x; idx < 6 * P * T; idx += NT) {
-        const int k = idx % P, r = idx / P, t = r % T, c = r / T, y = y0 + t;
-        const C *b = buf + c * T;
-        C zk = b[(k == M ? 0 : k) * LD + t];
-        C zm = b[(k == 0 ? 0 : M - k) * LD + t];
-        zm.y = -zm.y;
-        C ze = cscale(cadd(zk, zm), R(0.5));
-        C d = csub(zk, zm);
-        C zo = mk(R(0.5) * d.y, R(-0.5) * d.x);
-        C w = __ldg(tw_full + k);
-        out[c * out_stride + k + (int64_t)PP * (y + (int64_t)N * z)] = cadd(ze, cmul(w, zo));
+        for (int r = 0; r < R1; r++) v[r] = b[r * (R2 + 1) + u];
+        step1_store<M, -1, 1>(v, b, u, tw_half);
     }
-}
-
-// ---------------------------------------------------------------------------
-// y pass (in place), complex.  grid (ceil(P/T), N, ncomp)
-// ---------------------------------------------------------------------------
-template <class R, int N, int T, int NT, int S>
-__global__ void __launch_bounds__(NT, 1024 / NT) k_fy(typename CT<R>::C *data, int64_t stride,
-                                           const typename CT<R>::C *__restrict__ tw)
-{
-    using C = typename CT<R>::C;
-    constexpr int P = N / 2 + 1, PP = N / 2 + 2, LD = T + 1;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    C *buf = reinterpret_cast<C *>(smem_raw);
-    const int kx0 = blockIdx.x * T, z = blockIdx.y;
-    C *d = data + (int64_t)blockIdx.z * stride;
-    staged_fill<N * T, NT, 8, C>(
-        [&](int idx) {
-            const int t = idx % T, n = idx / T, kx = kx0 + t;
-            return (kx < P) ? d[kx + (int64_t)PP * (n + (int64_t)N * z)] : mk(R(0), R(0));
-        },
-        [&](int idx, C v) { buf[(idx / T) * LD + idx % T] = v; });
     __syncthreads();
-    fft_lines<N, S, T, NT>(buf, LD, tw);
-    for (int idx = threadIdx.x; idx < N * T; idx += NT) {
-        int t = idx % T, n = idx / T, kx = kx0 + t;
-        if (kx < P) d[kx + (int64_t)PP * (n + (int64_t)N * z)] = buf[n * LD + t];
-    }
+    fx_finish<M, 6 * T, NT>(smem, tw_full, [&](int i) {
+        return out + (i / T) * out_stride + (int64_t)PP * (y0 + i % T + (int64_t)N * z);
+    });
 }
 
 // ---------------------------------------------------------------------------
 // x pass, inverse: half spectrum -> real rows (imaginary parts of the kx = 0
 // and kx = N/2 entries do not contribute).  grid (N/T, N, ncomp)
 // ---------------------------------------------------------------------------
-template <class R, int N, int T, int NT>
-__global__ void __launch_bounds__(NT, sizeof(R) == 4 ? GEV_FXI_MINB : 1) k_fx_inv(const typename CT<R>::C *in, int64_t in_stride, R *out,
-                                               int64_t out_stride,
-                                               const typename CT<R>::C *__restrict__ tw_half,
-                                               const typename CT<R>::C *__restrict__ tw_full)
+template <class R, int N, int T, int MINB>
+__global__ void __launch_bounds__(RegPlan<N / 2>::R2 *T, MINB) k_fx_inv(const typename CT<R>::C *in, int64_t in_stride, R *out,
+                                                                       int64_t out_stride,
+                                                                       const typename CT<R>::C *__restrict__ tw_half,
+                                                                       const typename CT<R>::C *__restrict__ tw_full)
 {
     using C = typename CT<R>::C;
-    constexpr int M = N / 2, PP = N / 2 + 2, LD = T + 1;
+    constexpr int M = N / 2, PP = N / 2 + 2, R1 = RegPlan<M>::R1, R2 = RegPlan<M>::R2;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    C *buf = reinterpret_cast<C *>(smem_raw);
-    const int y0 = blockIdx.x * T, z = blockIdx.y;
-    const C *src = in + (int64_t)blockIdx.z * in_stride;
-    R *dst = out + (int64_t)blockIdx.z * out_stride;
-    staged_fill<M * T, NT, 4, C>(
-        [&](int idx) {
-            const int k = idx % M, t = idx / M, y = y0 + t;
-            const C *row = src + (int64_t)PP * (y + (int64_t)N * z);
+    const int u = threadIdx.x % R2, l = threadIdx.x / R2;   // neighbouring threads share a line
+    const int y = blockIdx.x * T + l, z = blockIdx.y;
+    C *buf = reinterpret_cast<C *>(smem_raw) + l * exch_size<M, 1>();
+    const C *row = in + (int64_t)blockIdx.z * in_stride + (int64_t)PP * (y + (int64_t)N * z);
+    {
+        C v[R1];
+#pragma unroll
+        for (int r = 0; r < R1; r++) {
+            const int k = u + R2 * r;
             C A = __ldg(row + k), B = __ldg(row + M - k);
             if (k == 0) { A.y = R(0); B.y = R(0); }
             B.y = -B.y;
             C w = __ldg(tw_full + k);
             w.y = -w.y;                                // exp(+2 pi i k / N)
-            C dd = cmul(csub(A, B), w);
-            C s = cadd(A, B);
-            return mk(s.x - dd.y, s.y + dd.x);         // (A+B) + i (A-B) w
-        },
-        [&](int idx, C v) { buf[(idx % M) * LD + idx / M] = v; });
+            const C dd = cmul(csub(A, B), w), s = cadd(A, B);
+            v[r] = mk(s.x - dd.y, s.y + dd.x);         // (A+B) + i (A-B) w
+        }
+        step1_store<M, 1, 1>(v, buf, u, tw_half);
+    }
     __syncthreads();
-    fft_lines<M, 1, T, NT>(buf, LD, tw_half);
-    for (int idx = threadIdx.x; idx < M * T; idx += NT) {
-        int n = idx % M, t = idx / M, y = y0 + t;
-        C v = buf[n * LD + t];
-        R *row = dst + sidx(N, 0, y, z);
-        row[2 * n] = v.x;
-        row[2 * n + 1] = v.y;
+    R *dst = out + (int64_t)blockIdx.z * out_stride + sidx(N, 0, y, z);
+    // a caller's own array (gev_poisson_noalloc) may be aligned to single values only
+    const bool pairs = reinterpret_cast<uintptr_t>(out) % sizeof(C) == 0;
+    for (int q = u; q < R1; q += R2) {
+        C v[R2];
+        step2_load<M, 1, 1>(v, buf, q);
+#pragma unroll
+        for (int p = 0; p < R2; p++) {
+            R *d = dst + 2 * (q + R1 * p);
+            if (pairs) {
+                *reinterpret_cast<C *>(d) = v[p];
+            } else {
+                d[0] = v[p].x;
+                d[1] = v[p].y;
+            }
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Small grids (N <= 128): the x and y transforms of a whole z plane in one
+// kernel, the plane in shared memory between them.  At these sizes a pass is
+// bound by its launch and by latency, not by its traffic: two launches of a
+// solve and one pass over the spectrum go in each direction.
+// ---------------------------------------------------------------------------
+template <int N> struct PlaneShape {
+    static constexpr int M = N / 2, P = M + 1;
+    static constexpr int XU = RegPlan<M>::R2, YU = RegPlan<N>::R2;   // threads per row, per column
+    static constexpr int NT = (P * YU + 31) / 32 * 32;               // one thread per (column, u)
+    static constexpr int XES = exch_size<M, 1>(), XITEMS = N * XU, XPER = (XITEMS + NT - 1) / NT;
+    static constexpr int VALUES = exch_size<N, P>() > N * XES ? exch_size<N, P>() : N * XES;
+    // slot of (column k, y) while the columns are the lines (k fastest)
+    __device__ __forceinline__ static int ycol(int k, int y) { return ((y / YU) * (YU + 1) + y % YU) * P + k; }
+    // slot of (k, y) after the columns' transform (row y % R1 of the exchange)
+    __device__ __forceinline__ static int yrow(int k, int y)
+    {
+        constexpr int R1 = RegPlan<N>::R1;
+        return ((y % R1) * (YU + 1) + y / R1) * P + k;
+    }
+};
+
+// resident CTAs: two FP32 planes of 128^2 fit an SM if the registers do too
+template <class R, int N> constexpr int plane_minb() { return sizeof(R) == 4 && N == 128 ? 2 : 1; }
+
+// forward: rows (with their source preparation), then columns; grid (N, ncomp)
+template <class R, int N, int MODE>
+__global__ void __launch_bounds__(PlaneShape<N>::NT, plane_minb<R, N>()) k_plane_fwd(FxArgs<R> a, int64_t in_stride, int64_t out_stride,
+                                                                 const typename CT<R>::C *__restrict__ tw_half,
+                                                                 const typename CT<R>::C *__restrict__ tw_full)
+{
+    using C = typename CT<R>::C;
+    using S = PlaneShape<N>;
+    constexpr int M = S::M, P = S::P, PP = N / 2 + 2, NT = S::NT;
+    constexpr int XR1 = RegPlan<M>::R1, XR2 = RegPlan<M>::R2, YR1 = RegPlan<N>::R1, YR2 = RegPlan<N>::R2;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    C *smem = reinterpret_cast<C *>(smem_raw);
+    const int z = blockIdx.x, comp = blockIdx.y;
+    const R *in = a.in + (int64_t)comp * in_stride;
+    double lsum = 0.0;
+    auto load = [&](auto cc) {
+#pragma unroll 1
+        for (int w = threadIdx.x; w < S::XITEMS; w += NT) {
+            const int u = w % XR2, y = w / XR2;
+            C v[XR1];
+#pragma unroll
+            for (int r = 0; r < XR1; r++) v[r] = fx_pair<R, N, MODE, decltype(cc)::v>(a, in, u + XR2 * r, y, z, lsum);
+            step1_store<M, -1, 1>(v, smem + y * S::XES, u, tw_half);
+        }
+    };
+    if constexpr (MODE == FX_PREP_T0I || MODE == FX_PREP_TIJ) {
+        if (comp == 0) load(IntC<0>{});
+        else if (comp == 1) load(IntC<1>{});
+        else if (MODE == FX_PREP_T0I || comp == 2) load(IntC<2>{});
+        if constexpr (MODE == FX_PREP_TIJ) {
+            if (comp == 3) load(IntC<3>{});
+            else if (comp == 4) load(IntC<4>{});
+            else if (comp == 5) load(IntC<5>{});
+        }
+    } else {
+        load(IntC<0>{});
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int w = threadIdx.x; w < S::XITEMS; w += NT) {
+        C *buf = smem + (w / XR2) * S::XES;
+        for (int q = w % XR2; q < XR1; q += XR2) {
+            C v[XR2];
+            step2_load<M, -1, 1>(v, buf, q);
+#pragma unroll
+            for (int p = 0; p < XR2; p++) buf[q * (XR2 + 1) + p] = v[p];
+        }
+    }
+    __syncthreads();
+    // unfold the rows through registers into the columns' layout
+    constexpr int PAIRS = N * (M / 2 + 1), PPT = (PAIRS + NT - 1) / NT;
+    C lo[PPT], hi[PPT];
+#pragma unroll
+    for (int i = 0; i < PPT; i++) {
+        const int w = threadIdx.x + i * NT, k = w % (M / 2 + 1), y = w / (M / 2 + 1);
+        if (w >= PAIRS) continue;
+        const C *buf = smem + y * S::XES;
+        const int m = k == 0 ? 0 : M - k;
+        const C zk = buf[(k % XR1) * (XR2 + 1) + k / XR1];
+        C zm = buf[(m % XR1) * (XR2 + 1) + m / XR1];
+        zm.y = -zm.y;
+        const C ze = cscale(cadd(zk, zm), R(0.5)), d = csub(zk, zm);
+        const C wo = cmul(__ldg(tw_full + k), mk(R(0.5) * d.y, R(-0.5) * d.x));
+        lo[i] = cadd(ze, wo);
+        hi[i] = cconj(csub(ze, wo));
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < PPT; i++) {
+        const int w = threadIdx.x + i * NT, k = w % (M / 2 + 1), y = w / (M / 2 + 1);
+        if (w >= PAIRS) continue;
+        smem[S::ycol(k, y)] = lo[i];
+        if (k < M / 2) smem[S::ycol(M - k, y)] = hi[i];
+    }
+    __syncthreads();
+    const int k = threadIdx.x % P, u = threadIdx.x / P;
+    if (u < YR2) {
+        C *buf = smem + k;
+        C v[YR1];
+#pragma unroll
+        for (int r = 0; r < YR1; r++) v[r] = buf[(r * (YR2 + 1) + u) * P];
+        step1_store<N, -1, P>(v, buf, u, tw_full);
+    }
+    __syncthreads();
+    if (u < YR2) {
+        C *out = a.out + (int64_t)comp * out_stride + (int64_t)PP * N * z + k;
+        for (int q = u; q < YR1; q += YR2) {
+            C v[YR2];
+            step2_load<N, -1, P>(v, smem + k, q);
+#pragma unroll
+            for (int p = 0; p < YR2; p++) out[PP * (q + YR1 * p)] = v[p];
+        }
+    }
+    if constexpr (MODE == FX_PREP_T00) block_sum<NT>(lsum, a.partial + z);
+}
+
+// inverse: columns, then rows; grid (N, ncomp)
+template <class R, int N>
+__global__ void __launch_bounds__(PlaneShape<N>::NT, plane_minb<R, N>()) k_plane_inv(const typename CT<R>::C *in, int64_t in_stride, R *out,
+                                                                 int64_t out_stride,
+                                                                 const typename CT<R>::C *__restrict__ tw_half,
+                                                                 const typename CT<R>::C *__restrict__ tw_full)
+{
+    using C = typename CT<R>::C;
+    using S = PlaneShape<N>;
+    constexpr int M = S::M, P = S::P, PP = N / 2 + 2, NT = S::NT;
+    constexpr int XR1 = RegPlan<M>::R1, XR2 = RegPlan<M>::R2, YR1 = RegPlan<N>::R1, YR2 = RegPlan<N>::R2;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    C *smem = reinterpret_cast<C *>(smem_raw);
+    const int z = blockIdx.x;
+    const int k0 = threadIdx.x % P, u0 = threadIdx.x / P;
+    if (u0 < YR2) {
+        const C *col = in + (int64_t)blockIdx.y * in_stride + (int64_t)PP * N * z + k0;
+        C v[YR1];
+#pragma unroll
+        for (int r = 0; r < YR1; r++) v[r] = __ldg(col + PP * (u0 + YR2 * r));
+        step1_store<N, 1, P>(v, smem + k0, u0, tw_full);
+    }
+    __syncthreads();
+    if (u0 < YR2) {
+        for (int q = u0; q < YR1; q += YR2) {
+            C v[YR2];
+            step2_load<N, 1, P>(v, smem + k0, q);
+#pragma unroll
+            for (int p = 0; p < YR2; p++) smem[(q * (YR2 + 1) + p) * P + k0] = v[p];
+        }
+    }
+    __syncthreads();
+    // the rows' first step in registers, then into the rows' layout
+    C v[S::XPER][XR1];
+#pragma unroll
+    for (int i = 0; i < S::XPER; i++) {
+        const int w = threadIdx.x + i * NT, u = w % XR2, y = w / XR2;
+        if (w >= S::XITEMS) continue;
+#pragma unroll
+        for (int r = 0; r < XR1; r++) {
+            const int k = u + XR2 * r;
+            C A = smem[S::yrow(k, y)], B = smem[S::yrow(M - k, y)];
+            if (k == 0) { A.y = R(0); B.y = R(0); }
+            B.y = -B.y;
+            C t = __ldg(tw_full + k);
+            t.y = -t.y;                                // exp(+2 pi i k / N)
+            const C dd = cmul(csub(A, B), t), sm = cadd(A, B);
+            v[i][r] = mk(sm.x - dd.y, sm.y + dd.x);    // (A+B) + i (A-B) w
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < S::XPER; i++) {
+        const int w = threadIdx.x + i * NT;
+        if (w < S::XITEMS) step1_store<M, 1, 1>(v[i], smem + (w / XR2) * S::XES, w % XR2, tw_half);
+    }
+    __syncthreads();
+    // a caller's own array (gev_poisson_noalloc) may be aligned to single values only
+    const bool pairs = reinterpret_cast<uintptr_t>(out) % sizeof(C) == 0;
+#pragma unroll 1
+    for (int w = threadIdx.x; w < S::XITEMS; w += NT) {
+        const int y = w / XR2;
+        R *dst = out + (int64_t)blockIdx.y * out_stride + sidx(N, 0, y, z);
+        for (int q = w % XR2; q < XR1; q += XR2) {
+            C x[XR2];
+            step2_load<M, 1, 1>(x, smem + y * S::XES, q);
+#pragma unroll
+            for (int p = 0; p < XR2; p++) {
+                R *d = dst + 2 * (q + XR1 * p);
+                if (pairs) {
+                    *reinterpret_cast<C *>(d) = x[p];
+                } else {
+                    d[0] = x[p].x;
+                    d[1] = x[p].y;
+                }
+            }
+        }
     }
 }
 
@@ -397,8 +622,8 @@ template <class R> struct FzArgs {
     typename CT<R>::C *hijp;
     typename CT<R>::C *bstate;
     double *phi_hom;           // k = 0 mode after the Poisson solve
-    double *bins;              // OP_BIN: 4*numbins accumulators (k, k^2, P, P^2)
-    unsigned long long *occ;   // OP_BIN: mode counts
+    double *bins;              // OP_BIN: BIN_COPIES x 4 x numbins accumulators (k, k^2, P, P^2)
+    unsigned long long *occ;   // OP_BIN: BIN_COPIES x numbins mode counts
     int *err;                  // device error word (may be null)
     const double *tab;         // OP_ZELD: ln k [h/Mpc] (ntab values) then ln P(k) (ntab values)
     int ntab;
@@ -441,10 +666,10 @@ template <int OP, int EXTRA> struct OpShape {
     static constexpr int COUT = (OP == OP_BIN) ? 0 : ((OP == OP_POISSON || OP == OP_ICS) ? 1 : (OP == OP_SCALAR ? ((EXTRA & EXTRA_VECTOR_EVOLVE) ? 4 : 1) : 3));
     static constexpr int CMAX = CIN > COUT ? CIN : COUT;   // columns the pass holds at once
     // projectFTscalar alone needs only three kz-independent combinations of the
-    // six S_ij (see k_fz), so the z pass transforms three columns instead of six
+    // six S_ij (see k_fz): the z pass transforms three columns instead of six
     static constexpr bool CONTRACT = (OP == OP_SCALAR && EXTRA == 0);
-    static constexpr int CBUF = CONTRACT ? 3 : CMAX;
-    static constexpr int CTMA = CONTRACT ? 4 : CMAX;   // buffers of the bulk-copy z pass (k_fz_tma)
+    static constexpr int CBUF = CONTRACT ? 3 : CMAX;   // exchange buffers of k_fz
+    static constexpr int CTMA = CONTRACT ? 4 : CMAX;   // buffers of k_fz_tma
 };
 
 // Element-wise solver for one (kx, ky, kz): reads CIN values from v, writes
@@ -456,38 +681,7 @@ __device__ __forceinline__ void fz_apply(const FzArgs<R> &a, int N, int kx, int 
     const double g[3] = {__ldg(a.k2 + kx), __ldg(a.k2 + ky), __ldg(a.k2 + kz)};
     const double2 k[3] = {__ldg(a.ks + kx), __ldg(a.ks + ky), __ldg(a.ks + kz)};
     const double k2 = g[0] + g[1] + g[2];
-    if constexpr (OP == OP_BIN) {
-        // extractCrossSpectrum binning, KTYPE_LINEAR with CIC deconvolution
-        // (tools.hpp:105-215); p0 = numbins, p1 = kmax
-        if (kx == 0 && ky == 0 && kz == 0) return;
-        const int weight = (kx == 0 || (kx == N / 2 && (N % 2) == 0)) ? 1 : 2;
-        // k^2 and the bin index with separately rounded operations (no fused
-        // multiply-add), as the reference evaluates them on the host: modes on a
-        // bin edge (|n|^2 = 3 m^2 for the default kmax) land in the same bin
-        auto lin = [&](int i) {
-            const double t = __dmul_rn(2.0 * 3.14159265358979323846, (double)(i <= N / 2 ? i : N - i));
-            return __dmul_rn(t, t);
-        };
-        auto snc = [&](int i) {
-            int j = i <= N / 2 ? i : N - i;
-            if (j == 0) return 1.0;
-            return sin(3.14159265358979323846 * (double)(float)j / (double)(float)N) * (double)(float)N / (3.14159265358979323846 * (double)(float)j);
-        };
-        double kk2 = __dadd_rn(__dadd_rn(lin(kx), lin(ky)), lin(kz));
-        double s = snc(kx) * snc(ky) * snc(kz);
-        s *= s;
-        double pw = v[0].x * v[0].x + v[0].y * v[0].y;
-        double sk = sqrt(kk2);
-        int nb = (int)a.p0;
-        int bin = (int)floor(__ddiv_rn(__dmul_rn((double)nb, sk), a.p1));
-        if (bin < nb) {
-            atomicAdd(a.bins + bin, weight * sk);
-            atomicAdd(a.bins + nb + bin, weight * kk2);
-            atomicAdd(a.bins + 2 * nb + bin, weight * pw * kk2 * sk / s);
-            atomicAdd(a.bins + 3 * nb + bin, weight * pw * pw * kk2 * kk2 * kk2 / s / s);
-            atomicAdd(a.occ + bin, (unsigned long long)weight);
-        }
-    } else if constexpr (OP == OP_ZELD) {
+    if constexpr (OP == OP_ZELD) {
         // Zel'dovich displacement of a white-noise spectrum (the generator's
         // counterpart of generateDisplacementField, ic_basic.hpp:1165-1610):
         // psi_c = i 2 pi n_c / |2 pi n|^2 * sqrt(P(k) N^3 / L^3) * w / N^3 in box
@@ -623,7 +817,79 @@ __device__ __forceinline__ void fz_apply(const FzArgs<R> &a, int N, int kx, int 
     }
 }
 
-// grid (ceil(P/T), N); T kx-columns at one ky, all CIN components of the solve.
+// OP_BIN: extractCrossSpectrum's binning (tools.hpp:105-215; KTYPE_LINEAR, CIC
+// deconvolution; p0 = numbins, p1 = kmax) of the modes (kx, ky, kz) and
+// (kx, ky, N - kz), which share their |k|: one warp, lanes at consecutive kz,
+// v0 and v1 the two values (v1 ignored unless `two`).  Along the lanes the
+// bin does not decrease, so lanes of one bin are neighbours: each run of them
+// is summed by shuffles and only its first lane adds to the bins.  Five
+// global additions per mode on a few hundred addresses take 1450 us at 256^3
+// (FP64); this takes a few of them per warp, spread over BIN_COPIES copies.
+template <class R>
+__device__ __forceinline__ void bin_modes(const FzArgs<R> &a, int N, int kx, int ky, int kz, bool on, bool two,
+                                          typename CT<R>::C v0, typename CT<R>::C v1, int copy)
+{
+    const int lane = threadIdx.x & 31, nb = (int)a.p0;
+    double s4[4] = {0.0, 0.0, 0.0, 0.0};
+    unsigned int cnt = 0;
+    int bin = nb;
+    if (on && !(kx == 0 && ky == 0 && kz == 0)) {
+        // k^2 and the bin index with separately rounded operations (no fused
+        // multiply-add), as the reference evaluates them on the host: modes on a
+        // bin edge (|n|^2 = 3 m^2 for the default kmax) land in the same bin
+        auto lin = [&](int i) {
+            const double t = __dmul_rn(2.0 * 3.14159265358979323846, (double)(i <= N / 2 ? i : N - i));
+            return __dmul_rn(t, t);
+        };
+        const double kk2 = __dadd_rn(__dadd_rn(lin(kx), lin(ky)), lin(kz)), sk = sqrt(kk2);
+        const double q = floor(__ddiv_rn(__dmul_rn((double)nb, sk), a.p1));
+        if (q < (double)nb) {
+            bin = (int)q;
+            const int weight = (kx == 0 || (kx == N / 2 && (N % 2) == 0)) ? 1 : 2;
+            double s = __ldg(a.tab + kx) * __ldg(a.tab + (ky <= N / 2 ? ky : N - ky)) * __ldg(a.tab + kz);
+            s *= s;
+            const double p0 = (double)v0.x * v0.x + (double)v0.y * v0.y, p1 = two ? (double)v1.x * v1.x + (double)v1.y * v1.y : 0.0;
+            const double wt = two ? 2.0 * weight : (double)weight, f = kk2 * sk / s;
+            cnt = two ? 2 * weight : weight;
+            s4[0] = wt * sk;
+            s4[1] = wt * kk2;
+            s4[2] = weight * ((p0 + p1) * f);
+            s4[3] = weight * ((p0 * p0 + p1 * p1) * f * f);
+        }
+    }
+    const int prev = __shfl_up_sync(0xffffffffu, bin, 1);
+    for (int o = 1; o < 32; o <<= 1) {
+        const bool same = __shfl_down_sync(0xffffffffu, bin, o) == bin && lane + o < 32;
+        if (!__any_sync(0xffffffffu, same)) break;
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const double d = __shfl_down_sync(0xffffffffu, s4[i], o);
+            if (same) s4[i] += d;
+        }
+        const unsigned int d = __shfl_down_sync(0xffffffffu, cnt, o);
+        if (same) cnt += d;
+    }
+    if (bin < nb && (lane == 0 || prev != bin)) {
+        double *b = a.bins + (size_t)copy * 4 * nb + bin;
+#pragma unroll
+        for (int i = 0; i < 4; i++) atomicAdd(b + i * nb, s4[i]);
+        atomicAdd(a.occ + (size_t)copy * nb + bin, (unsigned long long)cnt);
+    }
+}
+
+// z pass: grid (ceil(P/T), N), G * R2 * T threads; T kx-columns at one ky over
+// all kz, every component of the solve: forward transform, pointwise solver,
+// inverse transform in one kernel (two-step register FFT, fftreg.cuh), G
+// thread groups sharing the components.
+//
+//   1. step 1 of every component, from global memory: one component (and the
+//      contracted scalar sources) through registers, several by asynchronous
+//      copies into the exchange buffers;
+//   2. per row q (the modes kz = q + R1 p): step 2, the solver and the
+//      inverse's step over p.  With one component the row stays in its
+//      thread's registers; several components wait in their rows, where all
+//      threads solve the modes;
+//   3. the inverse's last step, straight to global memory.
 //
 // projectFTscalar (gevolution.hpp:251-340) without tensor or vector extras:
 //   chi 2 k^4 N = S00 (g1+g2-2g0) + S11 (g0+g2-2g1) + S22 (g0+g1-2g2)
@@ -634,100 +900,179 @@ __device__ __forceinline__ void fz_apply(const FzArgs<R> &a, int N, int kx, int 
 // A, B, C have coefficients that depend on kx, ky only, so they are formed
 // (in FP64) while the pencils load and the z transform -- linear, along kz --
 // acts on three columns instead of six.
-template <class R, int N, int T, int NT, int OP, int EXTRA>
-__global__ void __launch_bounds__(NT, GEV_FZ_MINB * 256 / NT) k_fz(FzArgs<R> a, const typename CT<R>::C *__restrict__ tw)
+template <class R, int N, int T, int G, int OP, int EXTRA, int MINB>
+__global__ void __launch_bounds__(RegPlan<N>::R2 *T *G, MINB) k_fz(FzArgs<R> a, const typename CT<R>::C *__restrict__ tw)
 {
     using C = typename CT<R>::C;
     constexpr int P = N / 2 + 1, PP = N / 2 + 2;
+    constexpr int R1 = RegPlan<N>::R1, R2 = RegPlan<N>::R2;
     constexpr int CIN = OpShape<OP, EXTRA>::CIN, COUT = OpShape<OP, EXTRA>::COUT;
     constexpr bool CONTRACT = OpShape<OP, EXTRA>::CONTRACT;
-    constexpr int CBUF = OpShape<OP, EXTRA>::CBUF;
-    constexpr int LD = CBUF * T + 1;
+    constexpr int CT1 = CONTRACT ? 3 : CIN;   // columns transformed forward
+    constexpr int ES = exch_size<N, T>();
+    static_assert(CT1 > 1 || G == 1, "one component is one group's work");
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    C *buf = reinterpret_cast<C *>(smem_raw);
-    const int kx0 = blockIdx.x * T, ky = blockIdx.y;
+    C *smem = reinterpret_cast<C *>(smem_raw);
+    const int t = threadIdx.x % T, u = (threadIdx.x / T) % R2, g = threadIdx.x / (T * R2);
+    const int kx = blockIdx.x * T + t, ky = blockIdx.y;
+    const bool live = kx < P;
+    C *buf = smem + t;   // this line's exchange buffers
+    const int64_t col = (int64_t)(live ? kx : 0) + (int64_t)PP * ky;
+    constexpr int64_t PLANE = (int64_t)PP * N;
+    // slot of mode n of line t2
+    auto slot = [](int n, int t2) { return ((n % R1) * (R2 + 1) + n / R1) * T + t2; };
 
-    if constexpr (CONTRACT) {
-        struct ABC { C v[3]; };
-        staged_fill<N * T, NT, 2, ABC>(
-            [&](int idx) {
-                const int t = idx % T, n = idx / T, kx = kx0 + t;
-                ABC o;
-                if (kx >= P) {
-                    o.v[0] = o.v[1] = o.v[2] = mk(R(0), R(0));
-                    return o;
-                }
-                const int64_t k = kx + (int64_t)PP * (ky + (int64_t)N * n);
-                double2 S[6];
+    // 1. forward step 1
+    if constexpr (CT1 > 1) {
+        // row z = j + R2 r goes where step 1 of thread j reads it
+        if constexpr (CONTRACT) {
+            const double g0 = __ldg(a.k2 + (live ? kx : 0)), g1 = __ldg(a.k2 + ky);
+            const double2 k0 = __ldg(a.ks + (live ? kx : 0)), k1 = __ldg(a.ks + ky), k01 = zmul(k0, k1);
+#pragma unroll 2
+            for (int r = g; r < R1; r += G) {
+                const C *s = a.data + col + PLANE * (u + R2 * r);
+                C x[6];
 #pragma unroll
-                for (int c = 0; c < 6; c++) S[c] = z2d(a.data[c * a.stride + k]);
-                const double g0 = __ldg(a.k2 + kx), g1 = __ldg(a.k2 + ky);
-                const double2 k0 = __ldg(a.ks + kx), k1 = __ldg(a.ks + ky);
-                const double2 A = zsub(zadd(zadd(zsc(S[0], g1 - 2.0 * g0), zsc(S[3], g0 - 2.0 * g1)), zsc(S[5], g0 + g1)),
-                                       zsc(zmul(zmul(k0, k1), S[1]), 6.0));
-                const double2 B = zsub(zadd(S[0], S[3]), zsc(S[5], 2.0));
-                const double2 Cc = zadd(zmul(k0, S[2]), zmul(k1, S[4]));
-                o.v[0] = mk(R(A.x), R(A.y));
-                o.v[1] = mk(R(B.x), R(B.y));
-                o.v[2] = mk(R(Cc.x), R(Cc.y));
-                return o;
-            },
-            [&](int idx, ABC o) {
-                const int t = idx % T, n = idx / T;
-#pragma unroll
-                for (int c = 0; c < 3; c++) buf[n * LD + c * T + t] = o.v[c];
-            });
-    } else {
-        staged_fill<N * CIN * T, NT, 8, C>(
-            [&](int idx) {
-                const int t = idx % T, r = idx / T, c = r % CIN, n = r / CIN, kx = kx0 + t;
-                return (kx < P) ? a.data[c * a.stride + kx + (int64_t)PP * (ky + (int64_t)N * n)] : mk(R(0), R(0));
-            },
-            [&](int idx, C v) {
-                const int t = idx % T, r = idx / T, c = r % CIN, n = r / CIN;
-                buf[n * LD + c * T + t] = v;
-            });
-    }
-    __syncthreads();
-    // one component at a time keeps the butterfly registers per thread small
-#pragma unroll 1
-    for (int c = 0; c < (CONTRACT ? 3 : CIN); c++) fft_lines<N, -1, T, NT>(buf + c * T, LD, tw);
-
-    if constexpr (CONTRACT) {
-        for (int idx = threadIdx.x; idx < N * T; idx += NT) {
-            const int t = idx % T, n = idx / T, kx = kx0 + t;
-            if (kx >= P) continue;
-            const double g0 = __ldg(a.k2 + kx), g1 = __ldg(a.k2 + ky), g2 = __ldg(a.k2 + n);
-            const double2 k2c = __ldg(a.ks + n);
-            const double k2 = g0 + g1 + g2;
-            double2 chi = make_double2(0.0, 0.0);
-            if (k2 > 0.0) {
-                const double2 A = z2d(buf[n * LD + t]), B = z2d(buf[n * LD + T + t]), Cc = z2d(buf[n * LD + 2 * T + t]);
-                chi = zsub(zadd(A, zsc(B, g2)), zsc(zmul(k2c, Cc), 6.0));
-                chi = zsc(chi, 1.0 / (2.0 * k2 * k2 * N));
+                for (int c = 0; c < 6; c++) x[c] = live ? __ldcs(s + c * a.stride) : mk(R(0), R(0));
+                const double2 S0 = z2d(x[0]), S1 = z2d(x[1]), S2 = z2d(x[2]), S3 = z2d(x[3]), S4 = z2d(x[4]), S5 = z2d(x[5]);
+                const double2 A = zsub(zadd(zadd(zsc(S0, g1 - 2.0 * g0), zsc(S3, g0 - 2.0 * g1)), zsc(S5, g0 + g1)),
+                                       zsc(zmul(k01, S1), 6.0));
+                const double2 B = zsub(zadd(S0, S3), zsc(S5, 2.0));
+                const double2 Cc = zadd(zmul(k0, S2), zmul(k1, S4));
+                C *o = buf + (r * (R2 + 1) + u) * T;
+                o[0] = mk(R(A.x), R(A.y));
+                o[ES] = mk(R(B.x), R(B.y));
+                o[2 * ES] = mk(R(Cc.x), R(Cc.y));
             }
-            buf[n * LD + t] = mk(R(chi.x), R(chi.y));
+            if constexpr (G > 1) __syncthreads();
+        } else {
+            // every component in flight at once, no registers held
+#pragma unroll 1
+            for (int c = g; c < CIN; c += G) {
+                const C *s = a.data + c * a.stride + col;
+#pragma unroll
+                for (int r = 0; r < R1; r++) copy_async(buf + c * ES + (r * (R2 + 1) + u) * T, s + PLANE * (u + R2 * r), live);
+            }
+            copy_async_commit();
+            copy_async_wait<0>();
+        }
+#pragma unroll 1
+        for (int c = g; c < CT1; c += G) {
+            C v[R1];
+#pragma unroll
+            for (int r = 0; r < R1; r++) v[r] = buf[c * ES + (r * (R2 + 1) + u) * T];
+            step1_store<N, -1, T>(v, buf + c * ES, u, tw);
         }
     } else {
-        for (int idx = threadIdx.x; idx < N * T; idx += NT) {
-            int t = idx % T, n = idx / T, kx = kx0 + t;
-            if (kx >= P) continue;
-            double2 v[6];
+        C v[R1];
 #pragma unroll
-            for (int c = 0; c < CIN; c++) v[c] = z2d(buf[n * LD + c * T + t]);
-            int64_t kidx = kx + (int64_t)PP * (ky + (int64_t)N * n);
-            fz_apply<R, OP, EXTRA>(a, N, kx, ky, n, kidx, v);
+        for (int r = 0; r < R1; r++) v[r] = live ? __ldcs(a.data + col + PLANE * (u + R2 * r)) : mk(R(0), R(0));
+        step1_store<N, -1, T>(v, buf, u, tw);
+    }
+    __syncthreads();
+
+    // 2. step 2, solver, inverse step 2
+    if constexpr (OP == OP_BIN) {
+        for (int q = u; q < R1; q += R2) {
+            C v[R2];
+            step2_load<N, -1, T>(v, buf, q);
 #pragma unroll
-            for (int c = 0; c < COUT; c++) buf[n * LD + c * T + t] = mk(R(v[c].x), R(v[c].y));
+            for (int p = 0; p < R2; p++) buf[(q * (R2 + 1) + p) * T] = v[p];
+        }
+        __syncthreads();
+        constexpr int NW = R2 * T / 32 > 0 ? R2 * T / 32 : 1;
+        static_assert(R2 * T % 32 == 0, "whole warps bin the modes");
+        for (int l = threadIdx.x / 32; l < T; l += NW) {
+            const int kxl = blockIdx.x * T + l;
+            for (int z0 = 0; z0 <= N / 2; z0 += 32) {
+                const int z = z0 + (threadIdx.x & 31);
+                const bool on = kxl < P && z <= N / 2, two = z > 0 && z < N / 2;
+                const C v0 = on ? smem[slot(z, l)] : mk(R(0), R(0)), v1 = on && two ? smem[slot(N - z, l)] : mk(R(0), R(0));
+                bin_modes(a, N, kxl, ky, z, on, two, v0, v1, (int)((blockIdx.x + gridDim.x * blockIdx.y) % BIN_COPIES));
+            }
+        }
+    } else if constexpr (CT1 == 1) {
+        for (int q = u; q < R1; q += R2) {
+            C v[R2];
+            step2_load<N, -1, T>(v, buf, q);
+            if (live) {
+#pragma unroll
+                for (int p = 0; p < R2; p++) {
+                    double2 w[COUT > 1 ? COUT : 1];
+                    w[0] = z2d(v[p]);
+                    const int n = q + R1 * p;
+                    fz_apply<R, OP, EXTRA>(a, N, kx, ky, n, (int64_t)kx + PP * ((int64_t)ky + (int64_t)N * n), w);
+                    if constexpr (COUT > 0) v[p] = mk(R(w[0].x), R(w[0].y));
+#pragma unroll
+                    for (int c = 1; c < COUT; c++)   // OP_ZELD: one column in, three out
+                        buf[c * ES + (q * (R2 + 1) + p) * T] = mk(R(w[c].x), R(w[c].y));
+                }
+            }
+            if constexpr (COUT > 0) step2_store<N, 1, T>(v, buf, q, tw);
+#pragma unroll 1
+            for (int c = 1; c < COUT; c++) {
+#pragma unroll
+                for (int p = 0; p < R2; p++) v[p] = buf[c * ES + (q * (R2 + 1) + p) * T];
+                step2_store<N, 1, T>(v, buf + c * ES, q, tw);
+            }
+        }
+    } else {
+#pragma unroll 1
+        for (int w = u + R2 * g; w < CT1 * R1; w += R2 * G) {
+            C *row = buf + (w / R1) * ES;
+            C v[R2];
+            step2_load<N, -1, T>(v, row, w % R1);
+#pragma unroll
+            for (int p = 0; p < R2; p++) row[((w % R1) * (R2 + 1) + p) * T] = v[p];
+        }
+        __syncthreads();
+        if (live) {
+            // threads of one line keep its kx: their kx and ky tables load once
+#pragma unroll 1
+            for (int n = u + R2 * g; n < N; n += R2 * G) {
+                const int o = slot(n, 0);
+                if constexpr (CONTRACT) {
+                    const double g0 = __ldg(a.k2 + kx), g1 = __ldg(a.k2 + ky), g2 = __ldg(a.k2 + n);
+                    const double2 k2c = __ldg(a.ks + n);
+                    const double k2 = g0 + g1 + g2;
+                    double2 chi = make_double2(0.0, 0.0);
+                    if (k2 > 0.0) {
+                        const double2 A = z2d(buf[o]), B = z2d(buf[ES + o]), Cc = z2d(buf[2 * ES + o]);
+                        chi = zsub(zadd(A, zsc(B, g2)), zsc(zmul(k2c, Cc), 6.0));
+                        chi = zsc(chi, 1.0 / (2.0 * k2 * k2 * N));
+                    }
+                    buf[o] = mk(R(chi.x), R(chi.y));
+                } else {
+                    double2 v[6];
+#pragma unroll
+                    for (int c = 0; c < CIN; c++) v[c] = z2d(buf[c * ES + o]);
+                    fz_apply<R, OP, EXTRA>(a, N, kx, ky, n, (int64_t)kx + PP * ((int64_t)ky + (int64_t)N * n), v);
+#pragma unroll
+                    for (int c = 0; c < COUT; c++) buf[c * ES + o] = mk(R(v[c].x), R(v[c].y));
+                }
+            }
+        }
+        __syncthreads();
+#pragma unroll 1
+        for (int w = u + R2 * g; w < COUT * R1; w += R2 * G) {
+            C *row = buf + (w / R1) * ES;
+            C v[R2];
+#pragma unroll
+            for (int p = 0; p < R2; p++) v[p] = row[((w % R1) * (R2 + 1) + p) * T];
+            step2_store<N, 1, T>(v, row, w % R1, tw);
         }
     }
     if constexpr (COUT > 0) {
         __syncthreads();
+        // 3. the inverse's last step
 #pragma unroll 1
-        for (int c = 0; c < COUT; c++) fft_lines<N, 1, T, NT>(buf + c * T, LD, tw);
-        for (int idx = threadIdx.x; idx < N * COUT * T; idx += NT) {
-            int t = idx % T, r = idx / T, c = r % COUT, n = r / COUT, kx = kx0 + t;
-            if (kx < P) a.data[c * a.stride + kx + (int64_t)PP * (ky + (int64_t)N * n)] = buf[n * LD + c * T + t];
+        for (int c = g; c < COUT; c += G) {
+            C v[R1];
+            step1_load<N, 1, T>(v, buf + c * ES, u);
+            if (live) {
+#pragma unroll
+                for (int r = 0; r < R1; r++) a.data[c * a.stride + col + PLANE * (u + R2 * r)] = v[r];
+            }
         }
     }
 }
@@ -737,24 +1082,25 @@ __global__ void __launch_bounds__(NT, GEV_FZ_MINB * 256 / NT) k_fz(FzArgs<R> a, 
 // copies (boxes of at most 256 kz) into dense per-component shared buffers,
 // the CTA transforms, solves and inverse-transforms them, and the results
 // leave by bulk tensor stores.  Columns kx >= P of the last CTA are zero-filled
-// on load and clipped on store.  Same arithmetic as k_fz.
+// on load and clipped on store.  Same arithmetic as k_fz, with block-wide
+// Stockham passes (fft.cuh): for FP32 lines of 512 and more, whose two-step
+// transform needs 32 values per thread and leaves too few warps to hide its
+// latency (512^3: 455 / 1425 / 1196 us for the Poisson, scalar and vector
+// passes here, 556 / 2100 / 1731 us by k_fz), and for the contracted scalar
+// pass from 256 on (187 against 222 us at 256^3), whose six input components
+// the bulk copies bring without holding registers.
 template <int N> struct ZBox {
     static constexpr int ZB = N <= 256 ? N : (N % 256 == 0 ? 256 : 128);
     static constexpr int NZB = N / ZB;
 };
 
-// the tensor extras keep six components in registers through the solve:
-// compiled for one resident CTA instead of GEV_FZ_MINB
-template <class R, int OP, int EXTRA, int NT> struct FzMinBlocks {
-    static constexpr int v = (OpShape<OP, EXTRA>::CIN == 6 && !OpShape<OP, EXTRA>::CONTRACT)
-                                 ? 1
-                                 : (sizeof(R) == 4 ? GEV_FZ_MINB : GEV_FZ_MINB_D) * 256 / NT;
-};
+// resident CTAs of 256 threads the staged z pass is compiled for
+constexpr int FZ_STAGED_MINB = 4;
 
 // PAD: the transforms use padded rows (fft.cuh), each component buffer then
 // holds N + N / 8 rows of T values
 template <class R, int N, int T, int NT, int OP, int EXTRA, bool PAD>
-__global__ void __launch_bounds__(NT, (FzMinBlocks<R, OP, EXTRA, NT>::v))
+__global__ void __launch_bounds__(NT, FZ_STAGED_MINB * 256 / NT)
     k_fz_tma(FzArgs<R> a, const typename CT<R>::C *__restrict__ tw, const __grid_constant__ CUtensorMap tmap)
 {
     using C = typename CT<R>::C;
@@ -877,37 +1223,33 @@ __global__ void __launch_bounds__(NT, (FzMinBlocks<R, OP, EXTRA, NT>::v))
     }
 }
 
-// y pass with bulk-tensor-copy staging: T kx-columns over all ky at one kz,
-// in place.  grid (ceil(P/T), N, ncomp)
-template <class R, int N, int T, int NT, int S>
-__global__ void __launch_bounds__(NT, (sizeof(R) == 4 ? GEV_FY_MINB : 2) * 512 / NT) k_fy_tma(const typename CT<R>::C *__restrict__ tw,
-                                                        int *err, const __grid_constant__ CUtensorMap tmap)
+// y pass (in place): T kx-columns over all ky at one kz; grid (ceil(P/T), N, ncomp)
+template <class R, int N, int T, int S, int MINB>
+__global__ void __launch_bounds__(RegPlan<N>::R2 *T, MINB) k_fy(typename CT<R>::C *data, int64_t stride,
+                                                               const typename CT<R>::C *__restrict__ tw)
 {
     using C = typename CT<R>::C;
-    constexpr int YB = ZBox<N>::ZB, NYB = ZBox<N>::NZB;
+    constexpr int P = N / 2 + 1, PP = N / 2 + 2, R1 = RegPlan<N>::R1, R2 = RegPlan<N>::R2;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    C *buf = reinterpret_cast<C *>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~(uintptr_t)127);
-    __shared__ __align__(8) uint64_t bar;
-    const int kx0 = blockIdx.x * T, z = blockIdx.y, comp = blockIdx.z;
-    if (threadIdx.x == 0) mbar_init(&bar, 1);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        mbar_expect_tx(&bar, (uint32_t)(N * T * sizeof(C)));
-#pragma unroll 1
-        for (int yc = 0; yc < NYB; yc++) tma_load_4d(buf + yc * YB * T, &tmap, 2 * kx0, yc * YB, z, comp, &bar);
+    const int t = threadIdx.x % T, u = threadIdx.x / T;
+    const int kx = blockIdx.x * T + t;
+    const bool live = kx < P;
+    C *buf = reinterpret_cast<C *>(smem_raw) + t;
+    C *d = data + (int64_t)blockIdx.z * stride + (live ? kx : 0) + (int64_t)PP * N * blockIdx.y;
+    {
+        C v[R1];
+#pragma unroll
+        for (int r = 0; r < R1; r++) v[r] = live ? d[PP * (u + R2 * r)] : mk(R(0), R(0));
+        step1_store<N, S, T>(v, buf, u, tw);
     }
-    const bool ok = mbar_wait(&bar, 0);
-    if (__syncthreads_or(!ok)) {   // the data never arrived: leave the array untouched and say so
-        if (threadIdx.x == 0 && err) atomicOr(err, ERR_TMA_TIMEOUT);
-        return;
-    }
-    fft_lines<N, S, T, NT>(buf, T, tw);
-    fence_async_smem();
     __syncthreads();
-    if (threadIdx.x == 0) {
-#pragma unroll 1
-        for (int yc = 0; yc < NYB; yc++) tma_store_4d(&tmap, 2 * kx0, yc * YB, z, comp, buf + yc * YB * T);
-        tma_store_drain();
+    for (int q = u; q < R1; q += R2) {
+        C v[R2];
+        step2_load<N, S, T>(v, buf, q);
+        if (live) {
+#pragma unroll
+            for (int p = 0; p < R2; p++) d[PP * (q + R1 * p)] = v[p];
+        }
     }
 }
 

@@ -12,9 +12,10 @@
 
 namespace gev {
 
+// DEP_CIC: the plain CIC mass density (no momenta read; DEP_T00 without phi).
 // DEP_T00_TIJ_S0I: T00 and Tij, plus the three T0i sums without their
 // potential factor (completed by the B solve's x pass with the new phi)
-enum { DEP_T00 = 0, DEP_TIJ = 1, DEP_T00_TIJ = 2, DEP_T0I = 3, DEP_T00_TIJ_S0I = 4 };
+enum { DEP_T00 = 0, DEP_TIJ = 1, DEP_T00_TIJ = 2, DEP_T0I = 3, DEP_T00_TIJ_S0I = 4, DEP_CIC = 5 };
 
 template <class R> struct DepOut { R *p[10]; };
 
@@ -69,16 +70,24 @@ template <class R> struct FftTables {
     const double2 *ks;                  // kshift
 };
 
+// x and y transforms, forward (mode: FX_*, the source preparation fused into
+// the row loads; with FX_PREP_T00 `partial` receives fxy_partials(N) partial
+// sums of the source) and inverse (the spectrum is overwritten).  Both return
+// the number of kernels launched.
 template <class R>
-void fx_forward(int N, int mode, const R *in, int64_t in_stride, int ncomp, int comp0, const R *phi, const R *chi,
-                double bg, double c, double c2, double c3, typename CT<R>::C *out, int64_t out_stride,
-                double *partial, const FftTables<R> &tb, cudaStream_t st);
+int fxy_forward(int N, int mode, const R *in, int64_t in_stride, int ncomp, const R *phi, const R *chi, double bg, double c,
+                double c2, double c3, typename CT<R>::C *out, int64_t out_stride, double *partial, const FftTables<R> &tb,
+                cudaStream_t st);
 template <class R>
-void fy_pass(int N, int sign, typename CT<R>::C *data, int64_t stride, int ncomp, int *err, const FftTables<R> &tb,
-             cudaStream_t st);   // err: device error word for the transfer timeout (may be null)
-template <class R>
-void fx_inverse(int N, const typename CT<R>::C *in, int64_t in_stride, R *out, int64_t out_stride, int ncomp,
-                const FftTables<R> &tb, cudaStream_t st);
+int fyx_inverse(int N, typename CT<R>::C *in, int64_t in_stride, R *out, int64_t out_stride, int ncomp, const FftTables<R> &tb,
+                cudaStream_t st);
+int64_t fxy_partials(int N);
+
+// copies of the spectrum's bins that the z pass adds into (by block), against
+// contention on a bin: bins [BIN_COPIES][4][nb], occ [BIN_COPIES][nb]
+constexpr int BIN_COPIES = 16;
+// sums the copies (in a fixed order) into the first one
+void launch_bin_reduce(double *bins, unsigned long long *occ, int nb, cudaStream_t st);
 
 struct FzParams {
     int op, extra;
@@ -87,14 +96,13 @@ struct FzParams {
     double *bins;
     unsigned long long *occ;
     int *err;   // device error word for the transfer timeout (may be null)
-    const double *tab = nullptr;   // OP_ZELD: ln k then ln P(k), device
+    const double *tab = nullptr;   // OP_ZELD: ln k then ln P(k); OP_BIN: sinc(i), i <= N/2; device
     int ntab = 0;
     const double2 *modes = nullptr;   // OP_ICS: mode numerators, device (ics.cu)
 };
 template <class R>
 void fz_pass(int N, const FzParams &fp, typename CT<R>::C *data, int64_t stride, typename CT<R>::C *hij,
              typename CT<R>::C *hijp, typename CT<R>::C *bstate, const FftTables<R> &tb, cudaStream_t st);
-int fx_rows_per_block(int N, bool fp64);   // T of the x passes (partial-sum count = N*N/T)
 // prepareFTsource in place: T00 form into source (partial[N*N]: sums of the
 // source per (y, z) row), Tij form on the six Sij planes
 template <class R>

@@ -140,14 +140,15 @@ template <class R> struct RawParticle {
     R q[3];
 };
 
-template <class R> __device__ __forceinline__ RawParticle<R> load_particle(const PView<R> &p, int64_t i)
+template <class R, bool MOMENTA = true>
+__device__ __forceinline__ RawParticle<R> load_particle(const PView<R> &p, int64_t i)
 {
     RawParticle<R> r;
     r.cell = p.cell[i];
 #pragma unroll
     for (int k = 0; k < 3; k++) {
         r.off[k] = p.off[k * p.cap + i];
-        r.q[k] = p.q[k * p.cap + i];
+        if constexpr (MOMENTA) r.q[k] = p.q[k * p.cap + i];
     }
     return r;
 }

@@ -172,7 +172,7 @@ __global__ void k_pm_deposit(const double *__restrict__ x, int64_t np, int N, do
 // position that the next step (or the final density) needs: the moved
 // positions are not read back
 template <class R>
-__global__ void k_pm_kick_drift(const double *xi, const double *qi, double *xo, double *qo, int64_t np, int N,
+__global__ void __launch_bounds__(PM_NT, 4) k_pm_kick_drift(const double *xi, const double *qi, double *xo, double *qo, int64_t np, int N,
                                 const R *__restrict__ psi, double kq, double kx, double cst, R *rho)
 {
     const double invN = 1.0 / N;
@@ -229,7 +229,7 @@ __device__ __forceinline__ void pm_weight_grad(const PmSite &s, const double v[8
 //      part of the step.
 // (lxi, lqi) null: the cotangents start at zero.
 template <class R>
-__global__ void k_pm_reverse(const double *__restrict__ xb, const R *__restrict__ f, double mf, const double *__restrict__ xa,
+__global__ void __launch_bounds__(PM_NT, 3) k_pm_reverse(const double *__restrict__ xb, const R *__restrict__ f, double mf, const double *__restrict__ xa,
                              const R *__restrict__ psi, double kq, double kx, const double *lxi, const double *lqi,
                              double *lxo, double *lqo, R *lam, int64_t np, int N)
 {
@@ -386,8 +386,8 @@ template <class R> struct Pm final : PmBase {
     }
     cudaStream_t stream() override { return st; }
 
-    // after a synchronisation: a bulk tensor copy of a Fourier pass that timed
-    // out leaves its pencils untransformed and sets the error word
+    // after a synchronisation: a bulk tensor copy of a z pass that timed out
+    // leaves its pencils untransformed and sets the error word
     void check_device(const char *what)
     {
         int e = 0;
@@ -406,16 +406,14 @@ template <class R> struct Pm final : PmBase {
     void poisson(const R *in, R *out, double pc)
     {
         const FftTables<R> tb = tables();
-        fx_forward<R>(N, FX_COPY, in, n3, 1, 0, nullptr, nullptr, 0.0, 0.0, 0.0, 0.0, W.p, nk, nullptr, tb, st);
-        fy_pass<R>(N, -1, W.p, nk, 1, derr.p, tb, st);
+        fxy_forward<R>(N, FX_COPY, in, n3, 1, nullptr, nullptr, 0.0, 0.0, 0.0, 0.0, W.p, nk, nullptr, tb, st);
         FzParams fp{};
         fp.op = OP_POISSON;
+        fp.err = derr.p;
         fp.p0 = pc / -((double)N * (double)N * (double)N);
         fp.p1 = 0.0;
-        fp.err = derr.p;
         fz_pass<R>(N, fp, W.p, nk, nullptr, nullptr, nullptr, tb, st);
-        fy_pass<R>(N, 1, W.p, nk, 1, derr.p, tb, st);
-        fx_inverse<R>(N, W.p, nk, out, n3, 1, tb, st);
+        fyx_inverse<R>(N, W.p, nk, out, n3, 1, tb, st);
     }
 
     void clear(R *f, int64_t n) { pck(cudaMemsetAsync(f, 0, n * sizeof(R), st), "memset"); }

@@ -3,5 +3,5 @@
 
 namespace gev {
 GEV_SOLVE_INST(float)
-int fx_rows_per_block(int N, bool fp64) { (void)N; return fp64 ? PassCfg<double>::TX : PassCfg<float>::TX; }
+int64_t fxy_partials(int N) { return N <= 128 ? N : (int64_t)(N / PASS_TX) * N; }
 }  // namespace gev

@@ -10,54 +10,27 @@
 
 namespace gev {
 
-// Tile shapes of the pencil passes (FP32 values; FP64 uses half the columns).
-#ifndef GEV_TX_F
-#define GEV_TX_F 16
-#endif
-#ifndef GEV_TY_F
-#define GEV_TY_F 16
-#endif
-#ifndef GEV_TZ1_F
-#define GEV_TZ1_F 8
-#endif
-#ifndef GEV_TZ3_F
-#define GEV_TZ3_F 4
-#endif
-#ifndef GEV_TZ6_F
-#define GEV_TZ6_F 4
-#endif
-#ifndef GEV_NT_Y
-#define GEV_NT_Y 512
-#endif
-#ifndef GEV_NT_Z
-#define GEV_NT_Z 256
-#endif
-#ifndef GEV_FY_TMA
-#define GEV_FY_TMA 1     // y pass staged by bulk tensor copies
-#endif
-#ifndef GEV_FZ_TMA
-#define GEV_FZ_TMA 1     // z pass staged by bulk tensor copies
-#endif
-#ifndef GEV_TZC_F
-#define GEV_TZC_F 4      // columns of the contracted scalar z pass
-#endif
-#ifndef GEV_TIJ6_T_F
-#define GEV_TIJ6_T_F 4   // rows of the six-component Tij x pass
-#endif
-template <class R> struct PassCfg {
-    static constexpr int TX = sizeof(R) == 4 ? GEV_TX_F : GEV_TX_F / 2;     // rows per x-pass CTA
-    static constexpr int TY = sizeof(R) == 4 ? GEV_TY_F : GEV_TY_F / 2;     // columns per y-pass CTA
-    static constexpr int TZ1 = sizeof(R) == 4 ? GEV_TZ1_F : GEV_TZ1_F / 2;  // Poisson
-    static constexpr int TZ3 = sizeof(R) == 4 ? GEV_TZ3_F : GEV_TZ3_F / 2;  // vector
-    static constexpr int TZ6 = sizeof(R) == 4 ? GEV_TZ6_F : GEV_TZ6_F / 2;  // scalar / tensor
-    static constexpr int NTY = GEV_NT_Y;                                    // threads per y-pass CTA
-    static constexpr int NTZ = GEV_NT_Z;                                    // threads per z-pass CTA
-    static constexpr int TZC = sizeof(R) == 4 ? GEV_TZC_F : GEV_TZC_F / 2;  // contracted scalar
-    static constexpr int TIJ6 = sizeof(R) == 4 ? GEV_TIJ6_T_F : GEV_TIJ6_T_F / 2;
-};
+// Lines (x passes) or kx-columns (y, z passes) per CTA, and the registers per
+// thread (FP32; twice that in FP64) that set the resident CTAs, from sweeps at
+// 128^3 to 512^3 (FP32) and 256^3 (FP64).
+constexpr int PASS_TX = 8, PASS_TY = 16, PASS_TZ1 = 8, PASS_TZ6 = 4, PASS_TIJ = 4, PASS_TIJ_G = 4, PASS_GZ = 3;
+constexpr int REGS_X = 72, REGS_Y = 96;
+template <class R> constexpr int REGS_TIJ = sizeof(R) == 4 ? 72 : 96;
+template <class R> constexpr int REGS_Z1 = sizeof(R) == 4 ? 72 : 96;
+constexpr int REGS_Z6 = 168;   // the tensor solve holds six components in FP64
+// three components: eight columns while a thread's values leave the registers
+// for it (256^3: 180 against 191 us with four), four columns beyond
+template <int N> constexpr int PASS_TZ3 = N <= 256 ? 8 : 4;
+template <int N> constexpr int REGS_Z3 = N <= 256 ? 80 : 64;
 
-// CTAs of `bytes` dynamic shared memory that fit one SM (228 KB, 1 KB reserved per CTA)
-constexpr int smem_ctas(size_t bytes) { return (int)(233472 / (bytes + 1024)); }
+// resident CTAs of nt threads with a budget of `regs` 32-bit registers per thread
+// (FP64 values take twice the registers)
+template <class R> constexpr int resident(int nt, int regs)
+{
+    const int r = regs * (sizeof(R) == 8 ? 2 : 1), lim = r > 248 ? 248 : r;
+    const int b = 65536 / (lim * nt);
+    return b < 1 ? 1 : (b > 32 ? 32 : b);
+}
 
 template <class K> inline void set_smem(K kernel, size_t bytes)
 {
@@ -77,13 +50,16 @@ template <class K> inline void set_smem(K kernel, size_t bytes)
     default: throw std::runtime_error("unsupported grid size"); \
     }
 
+template <class R> constexpr int cols(int t) { return sizeof(R) == 8 ? t / 2 : t; }
+template <class R, int L> constexpr int regs_for(int regs) { return RegPlan<L>::R1 >= 24 ? regs + 32 : regs; }
+
 template <class R, int N, int MODE>
 void fx_fwd_n(const FxArgs<R> &a, int ncomp, int64_t in_stride, int64_t out_stride, const FftTables<R> &tb, cudaStream_t st)
 {
     using C = typename CT<R>::C;
-    constexpr int T = PassCfg<R>::TX, NT = 256;
-    size_t smem = (size_t)(N / 2) * (T + 1) * sizeof(C);
-    auto k = k_fx_fwd<R, N, T, NT, MODE>;
+    constexpr int T = PASS_TX, NT = RegPlan<N / 2>::R2 * T;
+    size_t smem = (size_t)T * exch_size<N / 2, 1>() * sizeof(C);
+    auto k = k_fx_fwd<R, N, T, MODE, resident<R>(NT, regs_for<R, N / 2>(REGS_X))>;
     set_smem(k, smem);
     k<<<dim3(N / T, N, ncomp), NT, smem, st>>>(a, in_stride, out_stride, tb.tw_half, tb.tw_full);
 }
@@ -92,54 +68,67 @@ template <class R, int N>
 void fx_tij6_n(const FxArgs<R> &a, int64_t in_stride, int64_t out_stride, const FftTables<R> &tb, cudaStream_t st)
 {
     using C = typename CT<R>::C;
-    constexpr int T = PassCfg<R>::TIJ6, NT = 256;
-    size_t smem = (size_t)(N / 2) * (6 * T + 1) * sizeof(C);
-    auto k = k_fx_fwd_tij6<R, N, T, NT>;
+    constexpr int T = cols<R>(PASS_TIJ), G = PASS_TIJ_G, NT = RegPlan<N / 2>::R2 * T * G;
+    size_t smem = (size_t)6 * T * exch_size<N / 2, 1>() * sizeof(C);
+    auto k = k_fx_fwd_tij6<R, N, T, G, resident<R>(NT, regs_for<R, N / 2>(REGS_TIJ<R>))>;
     set_smem(k, smem);
     k<<<dim3(N / T, N), NT, smem, st>>>(a.in, in_stride, a.phi, a.c, a.out, out_stride, tb.tw_half, tb.tw_full);
 }
 
+// the x and y transforms of whole planes in one kernel (fftpass.cuh)
+template <int N> constexpr bool plane_pass() { return N <= 128; }
+
+template <class R, int N, int MODE>
+void plane_fwd_n(const FxArgs<R> &a, int ncomp, int64_t in_stride, int64_t out_stride, const FftTables<R> &tb, cudaStream_t st)
+{
+    using C = typename CT<R>::C;
+    constexpr size_t smem = (size_t)PlaneShape<N>::VALUES * sizeof(C);
+    auto k = k_plane_fwd<R, N, MODE>;
+    set_smem(k, smem);
+    k<<<dim3(N, ncomp), PlaneShape<N>::NT, smem, st>>>(a, in_stride, out_stride, tb.tw_half, tb.tw_full);
+}
+
+template <class R, int N, int S>
+void fy_n(typename CT<R>::C *data, int64_t stride, int ncomp, const FftTables<R> &tb, cudaStream_t st)
+{
+    using C = typename CT<R>::C;
+    constexpr int T = cols<R>(PASS_TY), NT = RegPlan<N>::R2 * T;
+    const size_t smem = (size_t)exch_size<N, T>() * sizeof(C);
+    auto k = k_fy<R, N, T, S, resident<R>(NT, regs_for<R, N>(REGS_Y))>;
+    set_smem(k, smem);
+    k<<<dim3((N / 2 + 1 + T - 1) / T, N, ncomp), NT, smem, st>>>(data, stride, tb.tw_full);
+}
+
+template <class R, int N, int MODE>
+int fxy_fwd_n(const FxArgs<R> &a, int ncomp, int64_t in_stride, int64_t out_stride, const FftTables<R> &tb, cudaStream_t st)
+{
+    if constexpr (plane_pass<N>()) {
+        plane_fwd_n<R, N, MODE>(a, ncomp, in_stride, out_stride, tb, st);
+        return 1;
+    } else {
+        if constexpr (MODE == FX_PREP_TIJ) fx_tij6_n<R, N>(a, in_stride, out_stride, tb, st);
+        else fx_fwd_n<R, N, MODE>(a, ncomp, in_stride, out_stride, tb, st);
+        fy_n<R, N, -1>(a.out, out_stride, ncomp, tb, st);
+        return 2;
+    }
+}
+
 template <class R>
-void fx_forward(int N, int mode, const R *in, int64_t in_stride, int ncomp, int comp0, const R *phi, const R *chi,
-                double bg, double c, double c2, double c3, typename CT<R>::C *out, int64_t out_stride,
-                double *partial, const FftTables<R> &tb, cudaStream_t st)
+int fxy_forward(int N, int mode, const R *in, int64_t in_stride, int ncomp, const R *phi, const R *chi, double bg, double c,
+                double c2, double c3, typename CT<R>::C *out, int64_t out_stride, double *partial, const FftTables<R> &tb,
+                cudaStream_t st)
 {
     FxArgs<R> a;
     a.in = in; a.phi = phi; a.chi = chi;
     a.bg = bg; a.c = c; a.c2 = c2; a.c3 = c3;
-    a.comp0 = comp0; a.out = out; a.partial = partial;
-    if (mode == FX_COPY) { GEV_SWITCH_N(N, (fx_fwd_n<R, NN, FX_COPY>(a, ncomp, in_stride, out_stride, tb, st))) }
-    else if (mode == FX_PREP_T00) { GEV_SWITCH_N(N, (fx_fwd_n<R, NN, FX_PREP_T00>(a, ncomp, in_stride, out_stride, tb, st))) }
-    else if (mode == FX_PREP_T0I) { GEV_SWITCH_N(N, (fx_fwd_n<R, NN, FX_PREP_T0I>(a, ncomp, in_stride, out_stride, tb, st))) }
-    else if (ncomp == 6 && comp0 == 0) { GEV_SWITCH_N(N, (fx_tij6_n<R, NN>(a, in_stride, out_stride, tb, st))) }
-    else { GEV_SWITCH_N(N, (fx_fwd_n<R, NN, FX_PREP_TIJ>(a, ncomp, in_stride, out_stride, tb, st))) }
-}
-
-template <class R, int N, int S>
-void fy_n(typename CT<R>::C *data, int64_t stride, int ncomp, int *err, const FftTables<R> &tb, cudaStream_t st)
-{
-    using C = typename CT<R>::C;
-    constexpr int T = PassCfg<R>::TY, NT = PassCfg<R>::NTY;
-#if GEV_FY_TMA
-    const size_t smem = (size_t)N * T * sizeof(C) + 128;
-    const CUtensorMap map = fourier_tensor_map<R>(data, N, stride, ncomp, T, ZBox<N>::ZB, 1);
-    auto k = k_fy_tma<R, N, T, NT, S>;
-    set_smem(k, smem);
-    k<<<dim3((N / 2 + 1 + T - 1) / T, N, ncomp), NT, smem, st>>>(tb.tw_full, err, map);
-#else
-    size_t smem = (size_t)N * (T + 1) * sizeof(C);
-    auto k = k_fy<R, N, T, NT, S>;
-    set_smem(k, smem);
-    k<<<dim3((N / 2 + 1 + T - 1) / T, N, ncomp), NT, smem, st>>>(data, stride, tb.tw_full);
-#endif
-}
-
-template <class R>
-void fy_pass(int N, int sign, typename CT<R>::C *data, int64_t stride, int ncomp, int *err, const FftTables<R> &tb,
-             cudaStream_t st)
-{
-    if (sign < 0) { GEV_SWITCH_N(N, (fy_n<R, NN, -1>(data, stride, ncomp, err, tb, st))) }
-    else { GEV_SWITCH_N(N, (fy_n<R, NN, 1>(data, stride, ncomp, err, tb, st))) }
+    a.out = out; a.partial = partial;
+    if (mode == FX_PREP_TIJ && ncomp != 6) throw std::runtime_error("the Tij sources are prepared together");
+    int n = 0;
+    if (mode == FX_COPY) { GEV_SWITCH_N(N, (n = fxy_fwd_n<R, NN, FX_COPY>(a, ncomp, in_stride, out_stride, tb, st))) }
+    else if (mode == FX_PREP_T00) { GEV_SWITCH_N(N, (n = fxy_fwd_n<R, NN, FX_PREP_T00>(a, ncomp, in_stride, out_stride, tb, st))) }
+    else if (mode == FX_PREP_T0I) { GEV_SWITCH_N(N, (n = fxy_fwd_n<R, NN, FX_PREP_T0I>(a, ncomp, in_stride, out_stride, tb, st))) }
+    else { GEV_SWITCH_N(N, (n = fxy_fwd_n<R, NN, FX_PREP_TIJ>(a, ncomp, in_stride, out_stride, tb, st))) }
+    return n;
 }
 
 template <class R, int N>
@@ -147,50 +136,79 @@ void fxi_n(const typename CT<R>::C *in, int64_t in_stride, R *out, int64_t out_s
            cudaStream_t st)
 {
     using C = typename CT<R>::C;
-    constexpr int T = PassCfg<R>::TX, NT = 256;
-    size_t smem = (size_t)(N / 2) * (T + 1) * sizeof(C);
-    auto k = k_fx_inv<R, N, T, NT>;
+    constexpr int T = PASS_TX, NT = RegPlan<N / 2>::R2 * T;
+    size_t smem = (size_t)T * exch_size<N / 2, 1>() * sizeof(C);
+    auto k = k_fx_inv<R, N, T, resident<R>(NT, regs_for<R, N / 2>(REGS_X))>;
     set_smem(k, smem);
     k<<<dim3(N / T, N, ncomp), NT, smem, st>>>(in, in_stride, out, out_stride, tb.tw_half, tb.tw_full);
 }
 
-template <class R>
-void fx_inverse(int N, const typename CT<R>::C *in, int64_t in_stride, R *out, int64_t out_stride, int ncomp,
-                const FftTables<R> &tb, cudaStream_t st)
+template <class R, int N>
+int fyx_inv_n(typename CT<R>::C *in, int64_t in_stride, R *out, int64_t out_stride, int ncomp, const FftTables<R> &tb,
+              cudaStream_t st)
 {
-    GEV_SWITCH_N(N, (fxi_n<R, NN>(in, in_stride, out, out_stride, ncomp, tb, st)))
+    using C = typename CT<R>::C;
+    if constexpr (plane_pass<N>()) {
+        constexpr size_t smem = (size_t)PlaneShape<N>::VALUES * sizeof(C);
+        auto k = k_plane_inv<R, N>;
+        set_smem(k, smem);
+        k<<<dim3(N, ncomp), PlaneShape<N>::NT, smem, st>>>(in, in_stride, out, out_stride, tb.tw_half, tb.tw_full);
+        return 1;
+    } else {
+        fy_n<R, N, 1>(in, in_stride, ncomp, tb, st);
+        fxi_n<R, N>(in, in_stride, out, out_stride, ncomp, tb, st);
+        return 2;
+    }
+}
+
+template <class R>
+int fyx_inverse(int N, typename CT<R>::C *in, int64_t in_stride, R *out, int64_t out_stride, int ncomp, const FftTables<R> &tb,
+                cudaStream_t st)
+{
+    int n = 0;
+    GEV_SWITCH_N(N, (n = fyx_inv_n<R, NN>(in, in_stride, out, out_stride, ncomp, tb, st)))
+    return n;
+}
+
+// CTAs of `bytes` dynamic shared memory that fit one SM (228 KB, 1 KB reserved per CTA)
+constexpr int smem_ctas(size_t bytes) { return (int)(233472 / (bytes + 1024)); }
+
+// z pass staged by bulk copies (k_fz_tma) or the two-step one (k_fz); measured
+// line between them in k_fz_tma's comment
+template <class R, int N, int OP, int EXTRA> constexpr bool z_staged()
+{
+    return sizeof(R) == 4 && OP != OP_BIN && OP != OP_ZELD && !(OP == OP_SCALAR && EXTRA != 0) &&
+           (N >= 512 || (N >= 256 && OpShape<OP, EXTRA>::CONTRACT));
 }
 
 template <class R, int N, int OP, int EXTRA>
 void fz_n(const FzArgs<R> &a, const FftTables<R> &tb, cudaStream_t st)
 {
     using C = typename CT<R>::C;
-    constexpr int T = OpShape<OP, EXTRA>::CONTRACT ? PassCfg<R>::TZC
-                      : (OP == OP_POISSON || OP == OP_BIN || OP == OP_ICS) ? PassCfg<R>::TZ1
-                      : ((OP == OP_VECTOR || OP == OP_ZELD) ? PassCfg<R>::TZ3 : PassCfg<R>::TZ6);
-    constexpr int NT = PassCfg<R>::NTZ;
-#if GEV_FZ_TMA
-    static_assert(T % 2 == 0 || sizeof(R) == 8, "TMA boxes need 16-byte rows");
-    constexpr int CMAX = OpShape<OP, EXTRA>::CMAX;
-    constexpr int CTMA = OpShape<OP, EXTRA>::CTMA;
-    constexpr size_t dense = (size_t)CTMA * N * T * sizeof(C) + 128;
-    constexpr size_t padded = (size_t)CTMA * (N + N / 8) * T * sizeof(C) + 128;
-    // padded rows where they spread the banks, keep every component buffer on
-    // a 128-byte boundary, and cost no resident CTA
-    constexpr bool PAD = pad_helps<T, C>() && ((N + N / 8) * T * sizeof(C)) % 128 == 0 &&
-                         smem_ctas(padded) >= std::min(FzMinBlocks<R, OP, EXTRA, NT>::v, smem_ctas(dense));
-    const size_t smem = PAD ? padded : dense;
-    const CUtensorMap map = fourier_tensor_map<R>(a.data, N, a.stride, CMAX, T, 1, ZBox<N>::ZB);
-    auto k = k_fz_tma<R, N, T, NT, OP, EXTRA, PAD>;
-    set_smem(k, smem);
-    k<<<dim3((N / 2 + 1 + T - 1) / T, N), NT, smem, st>>>(a, tb.tw_full, map);
-#else
-    constexpr int CBUF = OpShape<OP, EXTRA>::CBUF;
-    size_t smem = (size_t)N * (CBUF * T + 1) * sizeof(C);
-    auto k = k_fz<R, N, T, NT, OP, EXTRA>;
-    set_smem(k, smem);
-    k<<<dim3((N / 2 + 1 + T - 1) / T, N), NT, smem, st>>>(a, tb.tw_full);
-#endif
+    using S = OpShape<OP, EXTRA>;
+    if constexpr (z_staged<R, N, OP, EXTRA>()) {
+        constexpr int T = S::CMAX == 1 ? 8 : 4, NT = 256;
+        constexpr size_t dense = (size_t)S::CTMA * N * T * sizeof(C) + 128;
+        constexpr size_t padded = (size_t)S::CTMA * (N + N / 8) * T * sizeof(C) + 128;
+        // padded rows where they spread the banks, keep every component buffer on
+        // a 128-byte boundary, and cost no resident CTA
+        constexpr bool PAD = pad_helps<T, C>() && ((N + N / 8) * T * sizeof(C)) % 128 == 0 &&
+                             smem_ctas(padded) >= std::min(FZ_STAGED_MINB, smem_ctas(dense));
+        const size_t smem = PAD ? padded : dense;
+        const CUtensorMap map = fourier_tensor_map<R>(a.data, N, a.stride, S::CMAX, T, 1, ZBox<N>::ZB);
+        auto k = k_fz_tma<R, N, T, NT, OP, EXTRA, PAD>;
+        set_smem(k, smem);
+        k<<<dim3((N / 2 + 1 + T - 1) / T, N), NT, smem, st>>>(a, tb.tw_full, map);
+    } else {
+        constexpr int CT1 = S::CONTRACT ? 3 : S::CIN, G = CT1 > 1 ? PASS_GZ : 1, R2 = RegPlan<N>::R2;
+        constexpr int T0 = cols<R>(CT1 == 1 ? PASS_TZ1 : (CT1 == 3 ? PASS_TZ3<N> : PASS_TZ6));
+        constexpr int T = OP == OP_BIN && R2 * T0 < 32 ? 32 / R2 : T0, NT = R2 * T * G;   // OP_BIN works in whole warps
+        const size_t smem = (size_t)S::CBUF * exch_size<N, T>() * sizeof(C);
+        constexpr int REGS = CT1 == 6 ? REGS_Z6 : (CT1 == 3 ? REGS_Z3<N> : REGS_Z1<R>);
+        auto k = k_fz<R, N, T, G, OP, EXTRA, resident<R>(NT, regs_for<R, N>(REGS))>;
+        set_smem(k, smem);
+        k<<<dim3((N / 2 + 1 + T - 1) / T, N), NT, smem, st>>>(a, tb.tw_full);
+    }
 }
 
 template <class R, int N>
@@ -225,9 +243,9 @@ void fz_pass(int N, const FzParams &fp, typename CT<R>::C *data, int64_t stride,
     a.extra = fp.extra;
     a.hij = hij; a.hijp = hijp; a.bstate = bstate;
     a.phi_hom = fp.phi_hom;
+    a.err = fp.err;
     a.bins = fp.bins;
     a.occ = fp.occ;
-    a.err = fp.err;
     a.tab = fp.tab;
     a.ntab = fp.ntab;
     a.modes = fp.modes;
@@ -290,11 +308,9 @@ void prep_tij_pass(int N, R *Sij, const R *phi, double coeff, cudaStream_t st)
 }
 
 #define GEV_SOLVE_INST(R)                                                                                            \
-    template void fx_forward<R>(int, int, const R *, int64_t, int, int, const R *, const R *, double, double, double, \
-                                double, CT<R>::C *, int64_t, double *, const FftTables<R> &, cudaStream_t);          \
-    template void fy_pass<R>(int, int, CT<R>::C *, int64_t, int, int *, const FftTables<R> &, cudaStream_t);                \
-    template void fx_inverse<R>(int, const CT<R>::C *, int64_t, R *, int64_t, int, const FftTables<R> &,             \
-                                cudaStream_t);                                                                       \
+    template int fxy_forward<R>(int, int, const R *, int64_t, int, const R *, const R *, double, double, double, double, \
+                                CT<R>::C *, int64_t, double *, const FftTables<R> &, cudaStream_t);                  \
+    template int fyx_inverse<R>(int, CT<R>::C *, int64_t, R *, int64_t, int, const FftTables<R> &, cudaStream_t);     \
     template void fz_pass<R>(int, const FzParams &, CT<R>::C *, int64_t, CT<R>::C *, CT<R>::C *, CT<R>::C *,          \
                              const FftTables<R> &, cudaStream_t);                                                    \
     template void prep_t00_pass<R>(int, R *, const R *, const R *, double, double, double, double, double *,          \

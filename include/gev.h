@@ -279,9 +279,7 @@ double gev_particle_horizon(double a, double fourpiG, const gev_cosmo *cosmo);
  *     and re-created (cudaDeviceReset), looks it up (cudaGetSymbolAddress,
  *     which may also load the library's device code); make that call before
  *     any stream capture begins.
- *   - A Fourier pass whose bulk tensor copy does not complete within its wait
- *     limit leaves phi filled with NaN: the failure shows in the output, not
- *     in the return code, which reports argument and launch errors only. */
+ *   - The return code reports argument and launch errors only. */
 int gev_poisson_noalloc(int32_t N, int32_t precision, const void *source, void *phi,
                         double poisson_coeff, double modif, void *stream);
 

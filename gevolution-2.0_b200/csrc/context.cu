@@ -187,6 +187,13 @@ struct CtxBase {
     virtual void solve_chi(double coeff, int cycle0, double hubble, double dtau, double dtau_old, double a2dtau) = 0;
     virtual void solve_B(double coeff, double modif) = 0;
     virtual double kick_drift(const KickDriftParams &kp) = 0;
+    // kick_drift and lightcone without waiting for their results; those of a
+    // whole cycle come with one synchronisation (cycle_results, then lightcone_count)
+    virtual void kick_drift_async(const KickDriftParams &kp) = 0;
+    virtual bool lightcone_async(const gev_lightcone_args &lc, double tau, double dtau, double dtau_old, double a,
+                                 double dadtau, int64_t cap) = 0;
+    virtual void cycle_results(double *sum, double *phom, double *maxvel) = 0;
+    virtual int64_t lightcone_count() = 0;
     virtual void power_spectrum(int nb, double kmax, double *kb, double *pw, double *ks, double *ps, int32_t *occ) = 0;
     virtual void lightcone(const gev_lightcone_args &lc, double tau, double dtau, double dtau_old, double a, double dadtau,
                            int64_t cap, float *pos, float *vel, int64_t *ids, int64_t *n_out) = 0;
@@ -207,13 +214,21 @@ template <class R> struct Ctx final : CtxBase {
     DBuf<C> tw_full, tw_half;
     DBuf<double> k2;
     DBuf<double2> ks;
-    DBuf<uint32_t> cellA, cellB, bucket, rank, inv, counts, bstart, bsums, depwork;
+    DBuf<uint32_t> cellA, cellB, bucket, rank, inv, bstart, bsums, depwork;
     DBuf<double> offA, offB;
     DBuf<R> qA, qB;
     DBuf<int64_t> idA, idB;
-    DBuf<double> partial, scal;          // scal: [0] sum, [1] phi_hom
-    DBuf<unsigned long long> u64;        // [0] vmax bits, [1] lc count, [2] prelog count
-    DBuf<int> derr;
+    DBuf<double> partial;
+    // The device scalars that the host reads, in one block with the bucket
+    // counts behind them (cleared together with the largest velocity): one
+    // copy brings all of a cycle's results.
+    enum { BX_SUM = 0, BX_PHIHOM = 1, BX_ERR = 2, BX_LC = 3, BX_VMAX = 4, BX_WORDS = 5, BX_COUNTS = 6 };
+    DBuf<unsigned long long> box;
+    unsigned long long *hbox = nullptr;  // pinned host copy of the block
+    double *dsum = nullptr, *dphihom = nullptr;
+    unsigned long long *dvmax = nullptr, *dlc = nullptr;
+    uint32_t *dcounts = nullptr;
+    int *derr = nullptr;
     DBuf<double> bins, sinc;
     DBuf<unsigned long long> occ;
     DBuf<double> rho64;                  // mixed precision: FP64 density of the spectrum measurement
@@ -278,16 +293,21 @@ template <class R> struct Ctx final : CtxBase {
         idA.alloc(cap, "particles"); idB.alloc(cap, "particles");
         bucket.alloc(cap, "buckets"); rank.alloc(cap, "buckets"); inv.alloc(cap, "buckets");
         const int64_t nb = g.ntiles * 8;
-        counts.alloc(nb, "bucket counts");
         bstart.alloc(nb + 1, "bucket starts");
         bsums.alloc((nb + 1023) / 1024 + 1, "scan");
-        depwork.alloc(g.ntiles + 2, "deposit work list");
+        depwork.alloc(g.ntiles + DEP_LIST, "deposit work list");
+        ck(cudaMemsetAsync(depwork.p, 0, DEP_LIST * sizeof(uint32_t), st), "memset");
         ck(cudaMemsetAsync(bstart.p, 0, (nb + 1) * sizeof(uint32_t), st), "memset");
         partial.alloc((int64_t)N * N, "partials");
-        scal.alloc(4, "scalars");
-        u64.alloc(4, "scalars");
-        derr.alloc(1, "error word");
-        ck(cudaMemsetAsync(derr.p, 0, sizeof(int), st), "memset");
+        box.alloc(BX_COUNTS + (nb + 1) / 2, "scalars and bucket counts");
+        ck(cudaMemsetAsync(box.p, 0, BX_COUNTS * sizeof(unsigned long long), st), "memset");
+        ck(cudaMallocHost((void **)&hbox, BX_WORDS * sizeof(unsigned long long)), "pinned scalars");
+        dsum = reinterpret_cast<double *>(box.p + BX_SUM);
+        dphihom = reinterpret_cast<double *>(box.p + BX_PHIHOM);
+        derr = reinterpret_cast<int *>(box.p + BX_ERR);
+        dlc = box.p + BX_LC;
+        dvmax = box.p + BX_VMAX;
+        dcounts = reinterpret_cast<uint32_t *>(box.p + BX_COUNTS);
         ck(cudaStreamSynchronize(st), "init");
     }
 
@@ -304,6 +324,7 @@ template <class R> struct Ctx final : CtxBase {
             }
         for (cudaEvent_t e : {ev_start, ev_dn[0], ev_dn[1], ev_dn_end, ev_up_end})
             if (e) cudaEventDestroy(e);
+        if (hbox) cudaFreeHost(hbox);
     }
 
     cudaStream_t stream() override { return st; }
@@ -377,20 +398,21 @@ template <class R> struct Ctx final : CtxBase {
     void deposit(int kind, bool use_phi, const DepOut<R> &o, double a, double m00, double mij, double m0i, int accumulate,
                  const char *what)
     {
-        ck(cudaMemsetAsync(depwork.p, 0, 2 * sizeof(uint32_t), st), "memset");
-        launch_deposit<R>(kind, use_phi, cur(), bstart.p, g.N, phi.p, o, a, m00, mij, m0i, accumulate, depwork.p, derr.p,
+        launch_deposit<R>(kind, use_phi, cur(), bstart.p, g.N, phi.p, o, a, m00, mij, m0i, accumulate, depwork.p, derr,
                           st);
         launched(what, 2);
     }
     int64_t kernel_launches() const override { return launch_count; }
 
-    void check_device_error()
+    // waits for the stream and brings the scalar block to hbox; a device error
+    // raised since the last look throws
+    void sync() override
     {
-        int e = 0;
-        ck(cudaMemcpyAsync(&e, derr.p, sizeof(int), cudaMemcpyDeviceToHost, st), "error word");
+        ck(cudaMemcpyAsync(hbox, box.p, BX_WORDS * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st), "scalars");
         ck(cudaStreamSynchronize(st), "synchronize");
+        const int e = (int)(hbox[BX_ERR] & 0xffffffffu);
         if (e) {
-            ck(cudaMemsetAsync(derr.p, 0, sizeof(int), st), "memset");
+            ck(cudaMemsetAsync(derr, 0, sizeof(int), st), "memset");
             char buf[224];
             snprintf(buf, sizeof buf, "device error word 0x%x (%s%s%s%s%s)", e, (e & ERR_NONFINITE) ? "non-finite particle coordinate " : "",
                      (e & ERR_LC_OVERFLOW) ? "lightcone buffer overflow " : "", (e & ERR_BAD_CELL) ? "cell index out of range " : "",
@@ -398,11 +420,11 @@ template <class R> struct Ctx final : CtxBase {
             throw DeviceError(buf);
         }
     }
-
-    void sync() override
+    double held(int word) const
     {
-        ck(cudaStreamSynchronize(st), "synchronize");
-        check_device_error();
+        double v;
+        std::memcpy(&v, hbox + word, sizeof v);
+        return v;
     }
 
     void ensure_stage(int64_t doubles, int64_t ids)
@@ -415,8 +437,8 @@ template <class R> struct Ctx final : CtxBase {
     void rebin_from_cells()
     {
         const int64_t nb = g.ntiles * 8;
-        ck(cudaMemsetAsync(counts.p, 0, nb * sizeof(uint32_t), st), "memset");
-        launch_bin_count<R>(cur(), g.N, counts.p, bucket.p, rank.p, st);
+        ck(cudaMemsetAsync(dcounts, 0, nb * sizeof(uint32_t), st), "memset");
+        launch_bin_count<R>(cur(), g.N, dcounts, bucket.p, rank.p, st);
         launched("bin_count");
         finish_rebin();
     }
@@ -424,9 +446,8 @@ template <class R> struct Ctx final : CtxBase {
     void finish_rebin()
     {
         const int64_t nb = g.ntiles * 8;
-        launch_scan(counts.p, bstart.p, nb, bsums.p, st);
-        launched("scan", 3);
-        launch_rebin<R>(cur(), view(!cur_is_A), bstart.p, bucket.p, rank.p, inv.p, g.N, derr.p, st);
+        launched("scan", launch_scan(dcounts, bstart.p, nb, bsums.p, st));
+        launch_rebin<R>(cur(), view(!cur_is_A), bstart.p, bucket.p, rank.p, inv.p, g.N, derr, st);
         launched("rebin", 2);
         cur_is_A = !cur_is_A;
     }
@@ -448,7 +469,7 @@ template <class R> struct Ctx final : CtxBase {
             if (id) ck(cudaMemcpyAsync(stage_id.p, id + o, c * sizeof(int64_t), cudaMemcpyHostToDevice, st), "H2D");
             PView<R> vo = v;
             vo.cell += o; vo.off += o; vo.q += o; vo.id += o;
-            launch_load_particles<R>(vo, stage.p, stage.p + 3 * ch, id ? stage_id.p : nullptr, c, g.N, derr.p, st);
+            launch_load_particles<R>(vo, stage.p, stage.p + 3 * ch, id ? stage_id.p : nullptr, c, g.N, derr, st);
             launched("load_particles");
             if (!id) {
                 // default IDs: the particle's index in the caller's array
@@ -492,7 +513,7 @@ template <class R> struct Ctx final : CtxBase {
         const FftTables<R> tb = tables();
         launched("forward x, y passes", fxy_forward<R>(N, FX_COPY, source.p, g.n3, 1, nullptr, nullptr, 0, 0, 0, 0, W.p, g.nk, nullptr, tb, st));
         FzParams fz{};
-        fz.err = derr.p;
+        fz.err = derr;
         fz.op = OP_ZELD;
         fz.p0 = ip.boxsize;
         fz.p1 = ip.ksphere ? 1.0 : 0.0;
@@ -527,7 +548,7 @@ template <class R> struct Ctx final : CtxBase {
         const double H = hconf(a, fourpiG, cm);
         launched("forward x, y passes", fxy_forward<R>(N, FX_COPY, source.p, g.n3, 1, nullptr, nullptr, 0, 0, 0, 0, W.p, g.nk, nullptr, tb, st));
         FzParams fp{};
-        fp.err = derr.p;
+        fp.err = derr;
         fp.op = OP_POISSON;
         fp.p0 = (fourpiG / a) / -((double)N * (double)N * (double)N);
         fp.p1 = gr ? 3.0 * (H * H + fourpiG * Om / a) : 0.0;
@@ -597,12 +618,12 @@ template <class R> struct Ctx final : CtxBase {
         DBuf<double2> modes;
         modes.alloc((int64_t)(N / 2 + 1) * N * N, "IC modes");
         const IcsSpline sp{spl.p, spl.p + nspl, spl.p + 2 * nspl, spl.p + 3 * nspl, spl.p + 4 * nspl, nspl};
-        launch_ics_modes(modes.p, N, ip.seed, ip.ksphere, (float)(ip.gr ? H * H : 0.0), sp, derr.p, st);
+        launch_ics_modes(modes.p, N, ip.seed, ip.ksphere, (float)(ip.gr ? H * H : 0.0), sp, derr, st);
         launched("ics modes");
         // 3. kernel transform, numerator / kernel, backward transform: the displacement potential in chi
         launched("forward x, y passes", fxy_forward<R>(N, FX_COPY, source.p, g.n3, 1, nullptr, nullptr, 0, 0, 0, 0, W.p, g.nk, nullptr, tb, st));
         FzParams fz{};
-        fz.err = derr.p;
+        fz.err = derr;
         fz.op = OP_ICS;
         fz.modes = modes.p;
         fz_pass<R>(N, fz, W.p, g.nk, nullptr, nullptr, nullptr, tb, st);
@@ -715,7 +736,7 @@ template <class R> struct Ctx final : CtxBase {
             ck(cudaMemcpyAsync(si, id_in + o, c * sizeof(int64_t), cudaMemcpyHostToDevice, sup), "H2D");
             PView<R> vo = dst;
             vo.cell += o; vo.off += o; vo.q += o; vo.id += o;
-            launch_load_particles<R>(vo, sp, sp + 3 * XCHUNK, si, c, g.N, derr.p, sup);
+            launch_load_particles<R>(vo, sp, sp + 3 * XCHUNK, si, c, g.N, derr, sup);
             launched("load_particles");
         };
         for (int64_t i = 0; i < std::max(ndn, nup); i++) {
@@ -886,25 +907,24 @@ template <class R> struct Ctx final : CtxBase {
         const int N = g.N;
         const FftTables<R> tb = tables();
         launched("forward x, y passes", fxy_forward<R>(N, prepare ? FX_PREP_T00 : FX_COPY, source.p, g.n3, 1, phi.p, chi.p, bg, c, c2, c3, W.p, g.nk, partial.p, tb, st));
-        if (prepare) {
-            launch_reduce_sum(partial.p, fxy_partials(N), scal.p, st);
-            launched("reduce");
-        }
         FzParams fp{};
-        fp.err = derr.p;
+        fp.err = derr;
         fp.op = OP_POISSON;
         fp.p0 = pc / -((double)N * (double)N * (double)N);
         fp.p1 = modif;
-        fp.phi_hom = scal.p + 1;
+        fp.phi_hom = dphihom;
+        if (prepare) {   // the source's sum rides along
+            fp.partial = partial.p;
+            fp.npartial = fxy_partials(N);
+            fp.sum = dsum;
+        }
         fz_pass<R>(N, fp, W.p, g.nk, nullptr, nullptr, nullptr, tb, st);
         launched("fz Poisson");
         launched("inverse x, y passes", fyx_inverse<R>(N, W.p, g.nk, phi.p, g.n3, 1, tb, st));
         if (sum || phom) {
-            double h[2] = {0.0, 0.0};
-            ck(cudaMemcpyAsync(h, scal.p, 2 * sizeof(double), cudaMemcpyDeviceToHost, st), "D2H");
             sync();
-            if (sum) *sum = prepare ? h[0] : 0.0;
-            if (phom) *phom = h[1];
+            if (sum) *sum = prepare ? held(BX_SUM) : 0.0;
+            if (phom) *phom = held(BX_PHIHOM);
         }
     }
 
@@ -915,12 +935,10 @@ template <class R> struct Ctx final : CtxBase {
         const int N = g.N;
         prep_t00_pass<R>(N, source.p, phi.p, chi.p, bg, c, c2, c3, partial.p, st);
         launched("prepare T00");
-        launch_reduce_sum(partial.p, (int64_t)N * N, scal.p, st);
+        launch_reduce_sum(partial.p, (int64_t)N * N, dsum, st);
         launched("reduce");
-        double h = 0.0;
-        ck(cudaMemcpyAsync(&h, scal.p, sizeof(double), cudaMemcpyDeviceToHost, st), "D2H");
         sync();
-        return h;
+        return held(BX_SUM);
     }
 
     void prepare_tij(double coeff) override
@@ -945,7 +963,7 @@ template <class R> struct Ctx final : CtxBase {
         const FftTables<R> tb = tables();
         launched("forward x, y passes", fxy_forward<R>(N, FX_PREP_TIJ, Sij.p, g.n3, 6, phi.p, chi.p, 0, coeff, 0, 0, W.p, g.nk, nullptr, tb, st));
         FzParams fp{};
-        fp.err = derr.p;
+        fp.err = derr;
         fp.op = OP_SCALAR;
         fp.extra = extra;
         const bool parab = (extra & EXTRA_VECTOR_EVOLVE) != 0;
@@ -969,7 +987,7 @@ template <class R> struct Ctx final : CtxBase {
         launched("forward x, y passes", fxy_forward<R>(N, bi_sums ? FX_PREP_T0I : FX_COPY, Bi.p, g.n3, 3, phi.p, nullptr, 0, 0, 0, 0, W.p, g.nk, nullptr, tb, st));
         bi_sums = false;
         FzParams fp{};
-        fp.err = derr.p;
+        fp.err = derr;
         fp.op = OP_VECTOR;
         fp.p0 = coeff;
         fp.p1 = modif;
@@ -980,23 +998,29 @@ template <class R> struct Ctx final : CtxBase {
 
     double kick_drift(const KickDriftParams &kp) override
     {
+        kick_drift_async(kp);
+        if (!kp.do_kick) return 0.0;
+        sync();
+        return std::sqrt(held(BX_VMAX));
+    }
+
+    void kick_drift_async(const KickDriftParams &kp) override
+    {
         need_particles();
-        const int64_t nb = g.ntiles * 8;
-        if (kp.do_bin) ck(cudaMemsetAsync(counts.p, 0, nb * sizeof(uint32_t), st), "memset");
-        ck(cudaMemsetAsync(u64.p, 0, sizeof(unsigned long long), st), "memset");
-        launch_kick_drift<R>(cur(), bstart.p, g.N, phi.p, chi.p, Bi.p, g.n3, kp, counts.p, bucket.p, rank.p, u64.p, derr.p, st);
+        // the largest velocity and, behind it, the bucket counts
+        const size_t words = 2 * (BX_COUNTS - BX_VMAX) + (kp.do_bin ? g.ntiles * 8 : 0);
+        ck(cudaMemsetAsync(dvmax, 0, words * sizeof(uint32_t), st), "memset");
+        launch_kick_drift<R>(cur(), bstart.p, g.N, phi.p, chi.p, Bi.p, g.n3, kp, dcounts, bucket.p, rank.p, dvmax, derr, st);
         launched("kick/drift");
         if (kp.do_bin) finish_rebin();
-        double maxvel = 0.0;
-        if (kp.do_kick) {
-            unsigned long long bits = 0;
-            ck(cudaMemcpyAsync(&bits, u64.p, sizeof(bits), cudaMemcpyDeviceToHost, st), "D2H");
-            sync();
-            double v2;
-            std::memcpy(&v2, &bits, sizeof v2);
-            maxvel = std::sqrt(v2);
-        }
-        return maxvel;
+    }
+
+    void cycle_results(double *sum, double *phom, double *maxvel) override
+    {
+        sync();
+        *sum = held(BX_SUM);
+        *phom = held(BX_PHIHOM);
+        *maxvel = std::sqrt(held(BX_VMAX));
     }
 
     void power_spectrum(int nb, double kmax, double *kb, double *pw, double *ksc, double *ps, int32_t *occo) override
@@ -1026,7 +1050,7 @@ template <class R> struct Ctx final : CtxBase {
             ck(cudaMemcpy(sinc.p, h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice), "sinc table");
         }
         FzParams fp{};
-        fp.err = derr.p;
+        fp.err = derr;
         fp.op = OP_BIN;
         fp.p0 = nb;
         fp.p1 = kmax;
@@ -1132,36 +1156,42 @@ template <class R> struct Ctx final : CtxBase {
         const int64_t lcap = std::max<int64_t>(cap, 1);
         la.capacity = lcap;
         if ((int64_t)lc_id.n < lcap) { lc_pos.alloc(3 * lcap, "lightcone"); lc_vel.alloc(3 * lcap, "lightcone"); lc_id.alloc(lcap, "lightcone"); }
-        ck(cudaMemsetAsync(u64.p + 1, 0, sizeof(unsigned long long), st), "memset");
-        lo = LcOut{lc_pos.p, lc_vel.p, lc_id.p, u64.p + 1, newer, idset_cap};
+        ck(cudaMemsetAsync(dlc, 0, sizeof(unsigned long long), st), "memset");
+        lo = LcOut{lc_pos.p, lc_vel.p, lc_id.p, dlc, newer, idset_cap};
         return true;
     }
 
-    // after the shell's kernel: the IDs logged near the inner edge become the
-    // next cycle's backlog; returns the number selected (synchronises)
-    int64_t lightcone_count(int shell)
+    // The shell's kernel; the IDs logged near the inner edge become the next
+    // cycle's backlog.  False when the shell writes nothing this cycle.  The
+    // number selected is known after the next sync (lightcone_count).
+    bool lightcone_async(const gev_lightcone_args &lc, double tau, double dtau, double dtau_old, double a, double dadtau,
+                         int64_t cap) override
     {
-        idset_cur[shell] = 1 - idset_cur[shell];
-        backlog_valid[shell] = true;
-        unsigned long long cnt = 0;
-        ck(cudaMemcpyAsync(&cnt, u64.p + 1, sizeof(unsigned long long), cudaMemcpyDeviceToHost, st), "D2H");
-        sync();
-        lc_last = (int64_t)cnt;
-        return (int64_t)cnt;
+        LcKernelArgs la;
+        LcOut lo;
+        if (!lightcone_setup(lc, tau, dtau, dtau_old, a, dadtau, cap, la, lo)) return false;
+        launch_lightcone<R>(cur(), bstart.p, g.N, phi.p, la, lo.pos, lo.vel, lo.ids, lo.count, lo.newlog,
+                            lo.newlog_cap, derr, st);
+        launched("lightcone");
+        idset_cur[lc.shell] = 1 - idset_cur[lc.shell];
+        backlog_valid[lc.shell] = true;
+        return true;
+    }
+    int64_t lightcone_count() override
+    {
+        lc_last = (int64_t)hbox[BX_LC];
+        return lc_last;
     }
 
     void lightcone(const gev_lightcone_args &lc, double tau, double dtau, double dtau_old, double a, double dadtau,
                    int64_t cap, float *pos, float *vel, int64_t *ids, int64_t *n_out) override
     {
         *n_out = 0;
-        LcKernelArgs la;
-        LcOut lo;
-        if (!lightcone_setup(lc, tau, dtau, dtau_old, a, dadtau, cap, la, lo)) return;
-        launch_lightcone<R>(cur(), bstart.p, g.N, phi.p, la, lo.pos, lo.vel, lo.ids, lo.count, lo.newlog,
-                            lo.newlog_cap, derr.p, st);
-        launched("lightcone");
-        *n_out = lightcone_count(lc.shell);
-        if (*n_out > la.capacity) throw CapacityError("lightcone output exceeds the buffer capacity (n_out holds the required size)");
+        if (!lightcone_async(lc, tau, dtau, dtau_old, a, dadtau, cap)) return;
+        sync();
+        *n_out = lightcone_count();
+        if (*n_out > std::max<int64_t>(cap, 1))
+            throw CapacityError("lightcone output exceeds the buffer capacity (n_out holds the required size)");
         if (pos || vel || ids) fetch_lightcone(cap, pos, vel, ids, n_out);
     }
 
@@ -1425,13 +1455,11 @@ int step_cycle(gev_ctx *ctx, const gev_cosmo *cosmo, gev_state *s, const gev_lig
         const bool elliptic = c.cfg.vector_method == GEV_VECTOR_ELLIPTIC;
         c.project(GEV_PROJ_T00 | GEV_PROJ_TIJ | (elliptic ? GEV_PROJ_T0I_SUMS : 0u), a, 1.0, 1, 0);
         // phi (main.cu:719-809)
-        if (s->dtau_old > 0.) {
+        const bool solved = s->dtau_old > 0.;
+        if (solved) {
             const double H = gev::hconf(a, cm.fourpiG, cm);
-            double sum = 0.0, ph = 0.0;
             c.solve_phi(1, cm.Omega_m, 3. * H * dx * dx / s->dtau_old, cm.fourpiG * dx * dx / a, 3. * H * H * dx * dx,
-                        1. / (dx * dx), 3. * H / s->dtau_old, &sum, &ph);
-            s->T00hom = sum / ((double)N * N * N);
-            s->phi_hom = ph;
+                        1. / (dx * dx), 3. * H / s->dtau_old, nullptr, nullptr);
         }
         // chi, h_ij (main.cu:820-966)
         const double H = gev::hconf(a, cm.fourpiG, cm);
@@ -1439,12 +1467,10 @@ int step_cycle(gev_ctx *ctx, const gev_cosmo *cosmo, gev_state *s, const gev_lig
         // B elliptic with the new phi (main.cu:836-955): T0i completed in solve_B's x pass
         if (elliptic) c.solve_B(cm.fourpiG * dx * dx, 0.);
         // lightcone shell with this cycle's phi (main.cu:1040-1100)
+        bool lc_written = false;
         if (lc) {
-            try {
-                c.lightcone(*lc, s->tau, s->dtau, s->dtau_old, a, a * H, lc_cap, nullptr, nullptr, nullptr, lc_n);
-            } catch (const gev::CapacityError &) {
-                lc_overflow = true;
-            }
+            *lc_n = 0;
+            lc_written = c.lightcone_async(*lc, s->tau, s->dtau, s->dtau_old, a, a * H, lc_cap);
         }
         // kick, background half step, drift, background half step (main.cu:1225-1283)
         gev::KickDriftParams kp{};
@@ -1458,8 +1484,19 @@ int step_cycle(gev_ctx *ctx, const gev_cosmo *cosmo, gev_state *s, const gev_lig
         kp.a_d = a;
         kp.b_d = a * a * N;
         kp.nfield_d = (1. / a < cm.z_relax + 1.) ? 3 : 0;
-        double mv = c.kick_drift(kp);
+        c.kick_drift_async(kp);
         gev::rk4bg(a, cm.fourpiG, cm, 0.5 * s->dtau);
+        // the cycle's one synchronisation: every stage is queued by now
+        double sum = 0.0, ph = 0.0, mv = 0.0;
+        c.cycle_results(&sum, &ph, &mv);
+        if (solved) {
+            s->T00hom = sum / ((double)N * N * N);
+            s->phi_hom = ph;
+        }
+        if (lc_written) {
+            *lc_n = c.lightcone_count();
+            lc_overflow = *lc_n > std::max<int64_t>(lc_cap, 1);
+        }
         s->maxvel = mv / std::sqrt(mv * mv + 1.0);
         // step control (main.cu:1286-1310)
         s->tau += s->dtau;

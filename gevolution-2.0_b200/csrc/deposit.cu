@@ -391,8 +391,8 @@ template <> struct DepMinBlocks<float, DEP_T00_TIJ_S0I> { static constexpr int v
 
 // One tile's deposit; outputs: component c is written to out[c] (N^3 plane
 // each).  The tile launch (DENSE = false) finishes every tile whose reach fits
-// one chunk and appends the others to the work list work[2..] (count in
-// work[0]); the dense-tile launch (DENSE = true) takes them from the list.
+// one chunk and appends the others to the work list work[DEP_LIST..] (count
+// in work[0]); the dense-tile launch (DENSE = true) takes them from the list.
 template <class R, int KIND, bool USE_PHI, bool DENSE>
 __device__ __forceinline__ void deposit_tile(int tile, uint32_t *work, const PView<R> &p, const uint32_t *__restrict__ bstart,
                                              int N, int nt, const R *__restrict__ phi, const DepOut<R> &out, double a,
@@ -483,7 +483,7 @@ __device__ __forceinline__ void deposit_tile(int tile, uint32_t *work, const PVi
     if constexpr (!DENSE) {
         if (multi) {
             // several chunks: the dense-tile launch takes this tile
-            if (t == 0) work[2 + atomicAdd(&work[0], 1u)] = (uint32_t)tile;
+            if (t == 0) work[DEP_LIST + atomicAdd(&work[0], 1u)] = (uint32_t)tile;
             return;
         }
     }
@@ -814,9 +814,14 @@ __global__ void __launch_bounds__(DEP_NT, GEV_DEP_MINB_DENSE)
         __syncthreads();
         const uint32_t i = next;
         if (i >= count) break;
-        deposit_tile<R, KIND, USE_PHI, true>((int)work[2 + i], work, p, bstart, N, nt, phi, out, a, m00, mij, m0i,
+        deposit_tile<R, KIND, USE_PHI, true>((int)work[DEP_LIST + i], work, p, bstart, N, nt, phi, out, a, m00, mij, m0i,
                                              accumulate, err, fN);
         __syncthreads();   // shared memory and `next` are reused for the next tile
+    }
+    // the last block to get here clears the list for the next deposit
+    if (threadIdx.x == 0) {
+        __threadfence();
+        if (atomicAdd(&work[2], 1u) == gridDim.x - 1) work[0] = work[1] = work[2] = 0u;
     }
 }
 

@@ -622,6 +622,9 @@ template <class R> struct FzArgs {
     typename CT<R>::C *hijp;
     typename CT<R>::C *bstate;
     double *phi_hom;           // k = 0 mode after the Poisson solve
+    const double *partial;     // OP_POISSON: partial sums (npartial of them, null: none) summed into *sum
+    int64_t npartial;
+    double *sum;
     double *bins;              // OP_BIN: BIN_COPIES x 4 x numbins accumulators (k, k^2, P, P^2)
     unsigned long long *occ;   // OP_BIN: BIN_COPIES x numbins mode counts
     int *err;                  // device error word (may be null)
@@ -814,6 +817,17 @@ __device__ __forceinline__ void fz_apply(const FzArgs<R> &a, int N, int kx, int 
             }
         }
         v[0] = chi;
+    }
+}
+
+// OP_POISSON: the forward x pass's partial sums, by one block at the end of
+// its own work
+template <class R, int NT> __device__ __forceinline__ void sum_partials(const FzArgs<R> &a)
+{
+    if (a.partial && blockIdx.x == 0 && blockIdx.y == 0) {
+        double v = 0.0;
+        for (int64_t i = threadIdx.x; i < a.npartial; i += NT) v += a.partial[i];
+        block_sum<NT>(v, a.sum);
     }
 }
 
@@ -1075,6 +1089,7 @@ __global__ void __launch_bounds__(RegPlan<N>::R2 *T *G, MINB) k_fz(FzArgs<R> a, 
             }
         }
     }
+    if constexpr (OP == OP_POISSON) sum_partials<R, R2 * T>(a);
 }
 
 // z pass with tensor-memory-access staging: one elected thread loads the
@@ -1221,6 +1236,7 @@ __global__ void __launch_bounds__(NT, FZ_STAGED_MINB * 256 / NT)
             tma_store_drain();
         }
     }
+    if constexpr (OP == OP_POISSON) sum_partials<R, NT>(a);
 }
 
 // y pass (in place): T kx-columns over all ky at one kz; grid (ceil(P/T), N, ncomp)

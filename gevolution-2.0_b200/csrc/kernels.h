@@ -20,8 +20,10 @@ enum { DEP_T00 = 0, DEP_TIJ = 1, DEP_T00_TIJ = 2, DEP_T0I = 3, DEP_T00_TIJ_S0I =
 template <class R> struct DepOut { R *p[10]; };
 
 // Two launches: every tile whose reach fits one chunk, then the denser tiles
-// from the work list `work` (ntiles + 2 words; work[0] and work[1] must be
-// zero on entry).
+// from the work list `work` (ntiles + DEP_LIST words: tiles listed, tiles
+// taken, blocks done, then the list).  The first DEP_LIST words must be zero
+// on entry; the second launch leaves them so.
+constexpr int DEP_LIST = 3;
 template <class R>
 void launch_deposit(int kind, bool use_phi, const PView<R> &p, const uint32_t *bstart, int N, const R *phi,
                     const DepOut<R> &out, double a, double m00, double mij, double m0i, int accumulate, uint32_t *work,
@@ -49,7 +51,8 @@ void launch_store_particles(const PView<R> &p, double *pos, double *q, int64_t *
                             cudaStream_t st);
 template <class R>
 void launch_bin_count(const PView<R> &p, int N, uint32_t *counts, uint32_t *bucket, uint32_t *rank, cudaStream_t st);
-void launch_scan(const uint32_t *counts, uint32_t *start, int64_t nb, uint32_t *block_sums, cudaStream_t st);
+// returns the number of kernels launched
+int launch_scan(const uint32_t *counts, uint32_t *start, int64_t nb, uint32_t *block_sums, cudaStream_t st);
 template <class R>
 void launch_rebin(const PView<R> &src, PView<R> dst, const uint32_t *bstart, const uint32_t *bucket,
                   const uint32_t *rank, uint32_t *inv, int N, int *err, cudaStream_t st);
@@ -93,6 +96,10 @@ struct FzParams {
     int op, extra;
     double p0, p1, p2, p3;
     double *phi_hom;
+    // OP_POISSON: the sum of npartial partial sums (null: none) is left in *sum
+    const double *partial = nullptr;
+    int64_t npartial = 0;
+    double *sum = nullptr;
     double *bins;
     unsigned long long *occ;
     int *err;   // device error word for the transfer timeout (may be null)

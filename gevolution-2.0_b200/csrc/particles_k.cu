@@ -457,12 +457,74 @@ __global__ void k_scan_add(uint32_t *start, int64_t nb, const uint32_t *block_su
     if (i < nb) start[i] += block_sums[blockIdx.x];
 }
 
-void launch_scan(const uint32_t *counts, uint32_t *start, int64_t nb, uint32_t *block_sums, cudaStream_t st)
+// Small grids (N <= 128): one block scans all counts -- the three launches
+// below take longer than the work (10 us; one block 4 us).  Four counts per
+// thread and round, SCAN_ROUNDS rounds scanned side by side.
+constexpr int SCAN_ROUNDS = 8;
+
+__global__ void __launch_bounds__(SCAN_NT) k_scan_one(const uint32_t *__restrict__ counts, uint32_t *start, int nb)
 {
+    __shared__ uint32_t wsum[SCAN_ROUNDS][SCAN_NT / 32];
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+    uint4 v[SCAN_ROUNDS];
+    uint32_t incl[SCAN_ROUNDS];
+#pragma unroll
+    for (int r = 0; r < SCAN_ROUNDS; r++) {
+        const int i = 4 * (t + r * SCAN_NT);   // nb is a multiple of 8
+        v[r] = i < nb ? *reinterpret_cast<const uint4 *>(counts + i) : make_uint4(0u, 0u, 0u, 0u);
+    }
+#pragma unroll
+    for (int r = 0; r < SCAN_ROUNDS; r++) {
+        incl[r] = v[r].x + v[r].y + v[r].z + v[r].w;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t u = __shfl_up_sync(0xffffffffu, incl[r], o);
+            if (lane >= o) incl[r] += u;
+        }
+        if (lane == 31) wsum[r][w] = incl[r];
+    }
+    __syncthreads();
+    if (t < 32) {
+        uint32_t carry = 0;
+#pragma unroll
+        for (int r = 0; r < SCAN_ROUNDS; r++) {
+            const uint32_t x = wsum[r][t];
+            uint32_t xi = x;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t u = __shfl_up_sync(0xffffffffu, xi, o);
+                if (t >= o) xi += u;
+            }
+            wsum[r][t] = carry + xi - x;
+            carry += __shfl_sync(0xffffffffu, xi, 31);
+        }
+        if (t == 0) start[nb] = carry;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < SCAN_ROUNDS; r++) {
+        const int i = 4 * (t + r * SCAN_NT);
+        if (i >= nb) break;
+        uint4 o;
+        o.x = wsum[r][w] + incl[r] - (v[r].x + v[r].y + v[r].z + v[r].w);
+        o.y = o.x + v[r].x;
+        o.z = o.y + v[r].y;
+        o.w = o.z + v[r].z;
+        *reinterpret_cast<uint4 *>(start + i) = o;
+    }
+}
+
+int launch_scan(const uint32_t *counts, uint32_t *start, int64_t nb, uint32_t *block_sums, cudaStream_t st)
+{
+    if (nb <= (int64_t)SCAN_NT * 4 * SCAN_ROUNDS) {
+        k_scan_one<<<1, SCAN_NT, 0, st>>>(counts, start, (int)nb);
+        return 1;
+    }
     int64_t nblk = (nb + SCAN_NT - 1) / SCAN_NT;
     k_scan_blocks<<<(unsigned)nblk, SCAN_NT, 0, st>>>(counts, start, nb, block_sums);
     k_scan_sums<<<1, SCAN_NT, 0, st>>>(block_sums, nblk, start, nb);
     k_scan_add<<<(unsigned)nblk, SCAN_NT, 0, st>>>(start, nb, block_sums);
+    return 3;
 }
 
 // ---- re-binning into bucket order, each bucket in (cell, ID) order ----

@@ -244,6 +244,9 @@ void fz_pass(int N, const FzParams &fp, typename CT<R>::C *data, int64_t stride,
     a.hij = hij; a.hijp = hijp; a.bstate = bstate;
     a.phi_hom = fp.phi_hom;
     a.err = fp.err;
+    a.partial = fp.partial;
+    a.npartial = fp.npartial;
+    a.sum = fp.sum;
     a.bins = fp.bins;
     a.occ = fp.occ;
     a.tab = fp.tab;

@@ -91,12 +91,47 @@ __device__ __forceinline__ void pm_cell(double x, int N, double invN, int &c, do
 
 __device__ __forceinline__ int pm_wrap1(int i, int N) { return i >= N ? i - N : (i < 0 ? i + N : i); }
 
+// The run's own particle arrays are three planes of np values (the caller's
+// are triples): a warp's load of one coordinate is 256 contiguous bytes where
+// triples spread it over 768, and the particle passes are bound by the L1
+// wavefronts of their loads.
+struct Vec3 {
+    double v[3];
+};
+__device__ __forceinline__ Vec3 pm_get(const double *__restrict__ p, int64_t np, int64_t i)
+{
+    return Vec3{{p[i], p[np + i], p[2 * np + i]}};
+}
+__device__ __forceinline__ void pm_put(double *p, int64_t np, int64_t i, const double (&v)[3])
+{
+    p[i] = v[0];
+    p[np + i] = v[1];
+    p[2 * np + i] = v[2];
+}
+
+// triples -> planes and back
+__global__ void k_pm_planes(const double *__restrict__ in, double *__restrict__ out, int64_t np)
+{
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < np; i += (int64_t)gridDim.x * blockDim.x) {
+        const double v[3] = {in[3 * i], in[3 * i + 1], in[3 * i + 2]};
+        pm_put(out, np, i, v);
+    }
+}
+__global__ void k_pm_triples(const double *__restrict__ in, double *__restrict__ out, int64_t np)
+{
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < np; i += (int64_t)gridDim.x * blockDim.x) {
+        const Vec3 v = pm_get(in, np, i);
+#pragma unroll
+        for (int k = 0; k < 3; k++) out[3 * i + k] = v.v[k];
+    }
+}
+
 // A particle's cell and the grid offsets (x; N y; N^2 z, all below 2^31) of
 // the four planes c - 1 .. c + 2 per axis.
 struct PmSite {
     double d[3];
     int x[4], y[4], z[4];
-    __device__ __forceinline__ PmSite(const double *__restrict__ pos, int N, double invN)
+    __device__ __forceinline__ PmSite(const double (&pos)[3], int N, double invN)
     {
         int c[3];
 #pragma unroll
@@ -164,7 +199,7 @@ __global__ void k_pm_deposit(const double *__restrict__ x, int64_t np, int N, do
 {
     const double invN = 1.0 / N;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < np; i += (int64_t)gridDim.x * blockDim.x)
-        pm_scatter(PmSite(x + 3 * i, N, invN), cst, out);
+        pm_scatter(PmSite(pm_get(x, np, i).v, N, invN), cst, out);
 }
 
 // forward kick (update_q_Newton) and drift (update_pos_Newton) from (xi, qi)
@@ -172,13 +207,17 @@ __global__ void k_pm_deposit(const double *__restrict__ x, int64_t np, int N, do
 // position that the next step (or the final density) needs: the moved
 // positions are not read back
 template <class R>
-__global__ void __launch_bounds__(PM_NT, 4) k_pm_kick_drift(const double *xi, const double *qi, double *xo, double *qo, int64_t np, int N,
+__global__ void __launch_bounds__(PM_NT, 3) k_pm_kick_drift(const double *xi, const double *qi, double *xo, double *qo, int64_t np, int N,
                                 const R *__restrict__ psi, double kq, double kx, double cst, R *rho)
 {
     const double invN = 1.0 / N;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < np; i += (int64_t)gridDim.x * blockDim.x) {
-        double x[3] = {xi[3 * i], xi[3 * i + 1], xi[3 * i + 2]};
-        double q[3] = {qi[3 * i], qi[3 * i + 1], qi[3 * i + 2]};
+        double x[3], q[3];
+#pragma unroll
+        for (int a = 0; a < 3; a++) {
+            x[a] = xi[a * np + i];
+            q[a] = qi[a * np + i];
+        }
         {
             const PmSite s(x, N, invN);
             double G[3][8];
@@ -196,11 +235,8 @@ __global__ void __launch_bounds__(PM_NT, 4) k_pm_kick_drift(const double *xi, co
                 x[a] += kx * q[a];
             }
         }
-#pragma unroll
-        for (int a = 0; a < 3; a++) {
-            qo[3 * i + a] = q[a];
-            xo[3 * i + a] = x[a];
-        }
+        pm_put(qo, np, i, q);
+        pm_put(xo, np, i, x);
         if (rho) pm_scatter(PmSite(x, N, invN), cst, rho);
     }
 }
@@ -229,7 +265,7 @@ __device__ __forceinline__ void pm_weight_grad(const PmSite &s, const double v[8
 //      part of the step.
 // (lxi, lqi) null: the cotangents start at zero.
 template <class R>
-__global__ void __launch_bounds__(PM_NT, 3) k_pm_reverse(const double *__restrict__ xb, const R *__restrict__ f, double mf, const double *__restrict__ xa,
+__global__ void __launch_bounds__(PM_NT, 2) k_pm_reverse(const double *__restrict__ xb, const R *__restrict__ f, double mf, const double *__restrict__ xa,
                              const R *__restrict__ psi, double kq, double kx, const double *lxi, const double *lqi,
                              double *lxo, double *lqo, R *lam, int64_t np, int N)
 {
@@ -238,11 +274,11 @@ __global__ void __launch_bounds__(PM_NT, 3) k_pm_reverse(const double *__restric
         double lx[3], lq[3];
 #pragma unroll
         for (int a = 0; a < 3; a++) {
-            lx[a] = lxi ? lxi[3 * i + a] : 0.0;
-            lq[a] = lqi ? lqi[3 * i + a] : 0.0;
+            lx[a] = lxi ? lxi[a * np + i] : 0.0;
+            lq[a] = lqi ? lqi[a * np + i] : 0.0;
         }
         {
-            const PmSite s(xb + 3 * i, N, invN);
+            const PmSite s(pm_get(xb, np, i).v, N, invN);
             double v[8], gm[3];
 #pragma unroll
             for (int k = 0; k < 8; k++) v[k] = pm_ld(f, s.at((k >> 2) & 1, (k >> 1) & 1, k & 1));
@@ -251,7 +287,7 @@ __global__ void __launch_bounds__(PM_NT, 3) k_pm_reverse(const double *__restric
             for (int a = 0; a < 3; a++) lx[a] += mf * (double)N * gm[a];
         }
         if (xa) {
-            const PmSite s(xa + 3 * i, N, invN);
+            const PmSite s(pm_get(xa, np, i).v, N, invN);
 #pragma unroll
             for (int a = 0; a < 3; a++) lq[a] += kx * lx[a];
             double G[3][8], v[8], gm[3];
@@ -269,11 +305,8 @@ __global__ void __launch_bounds__(PM_NT, 3) k_pm_reverse(const double *__restric
                 pm_add3(lam + 4 * (int64_t)s.at(bx, by, bz), w * lq[0], w * lq[1], w * lq[2]);
             }
         }
-#pragma unroll
-        for (int a = 0; a < 3; a++) {
-            lxo[3 * i + a] = lx[a];
-            lqo[3 * i + a] = lq[a];
-        }
+        pm_put(lxo, np, i, lx);
+        pm_put(lqo, np, i, lq);
     }
 }
 
@@ -322,13 +355,15 @@ template <class R> struct Pm final : PmBase {
     double mass;
     int every;
     cudaStream_t st = nullptr;
-    PBuf<R> rho;    // deposited density of the step, cleared by its first Fourier pass
-    PBuf<R> fld;    // potential of a forward step; cotangent of a density (reverse)
-    PBuf<R> lam;    // deposited momentum cotangents, [N^3][4]
+    PBuf<R> fields;          // one allocation for rho, fld and lam
+    R *rho = nullptr;        // deposited density of the step
+    R *fld = nullptr;        // potential of a forward step; cotangent of a density (reverse)
+    R *lam = nullptr;        // deposited momentum cotangents, [N^3][4]
     PBuf<C> W, twf, twh;
     PBuf<double> k2;
     PBuf<double2> ks;
-    PBuf<double> x, q, lx, lq;
+    PBuf<double> state;      // one allocation for the particles and their cotangents
+    double *x = nullptr, *q = nullptr, *lx = nullptr, *lq = nullptr;
     PBuf<int> derr;                                        // device error word of the Fourier passes
     std::vector<std::unique_ptr<PBuf<double>>> ckx, ckq;   // checkpoints (x, q) before steps 0, k, 2k, ...
     std::vector<std::unique_ptr<PBuf<double>>> segx;       // x_n within the segment being reversed
@@ -343,14 +378,16 @@ template <class R> struct Pm final : PmBase {
         pck(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking), "stream");
         n3 = (int64_t)N * N * N;
         nk = (int64_t)(N / 2 + 2) * N * N;   // Fourier rows of pitch N/2+2
-        rho.alloc(n3, "fields");
-        fld.alloc(n3, "fields");
-        lam.alloc(4 * n3, "fields");
+        fields.alloc(6 * n3, "fields");
+        rho = fields.p;
+        fld = rho + n3;
+        lam = fld + n3;   // 16-byte aligned: n3 is a multiple of 4096
         W.alloc(nk, "spectrum");
-        x.alloc(3 * np, "particles");
-        q.alloc(3 * np, "particles");
-        lx.alloc(3 * np, "adjoint");
-        lq.alloc(3 * np, "adjoint");
+        state.alloc(12 * np, "particles");
+        x = state.p;
+        q = x + 3 * np;
+        lx = q + 3 * np;
+        lq = lx + 3 * np;
         derr.alloc(1, "error word");
         pck(cudaMemset(derr.p, 0, sizeof(int)), "memset");
         std::vector<C> tf(N), th(N / 2);
@@ -421,15 +458,15 @@ template <class R> struct Pm final : PmBase {
     // density of the state xs into rho (the start of a chain of steps)
     void deposit(const double *xs, double cst)
     {
-        clear(rho.p, n3);
-        k_pm_deposit<R><<<pgrid(), PM_NT, 0, st>>>(xs, np, N, cst, rho.p);
+        clear(rho, n3);
+        k_pm_deposit<R><<<pgrid(), PM_NT, 0, st>>>(xs, np, N, cst, rho);
     }
 
     // potential of the density in rho, which is left cleared for the next deposit
     void potential(double pc, R *out)
     {
-        poisson(rho.p, out, pc);
-        clear(rho.p, n3);
+        poisson(rho, out, pc);
+        clear(rho, n3);
     }
 
     void forward(int ns, const double *coef, const double *x0, const double *q0, double *delta, double *xo,
@@ -446,25 +483,25 @@ template <class R> struct Pm final : PmBase {
             ckx[s]->alloc(3 * np, "checkpoint");
             ckq[s]->alloc(3 * np, "checkpoint");
         }
-        pck(cudaMemcpyAsync(ckx[0]->p, x0, 3 * np * sizeof(double), cudaMemcpyDeviceToDevice, st), "copy x0");
-        pck(cudaMemcpyAsync(ckq[0]->p, q0, 3 * np * sizeof(double), cudaMemcpyDeviceToDevice, st), "copy q0");
+        k_pm_planes<<<pgrid(), PM_NT, 0, st>>>(x0, ckx[0]->p, np);
+        k_pm_planes<<<pgrid(), PM_NT, 0, st>>>(q0, ckq[0]->p, np);
         const double mcell = mass * (double)n3, contrast = (double)n3 / (double)np;
         deposit(ckx[0]->p, mcell);
         for (int n = 0; n < ns; n++) {
-            potential(coefs[3 * n + 2], fld.p);
+            potential(coefs[3 * n + 2], fld);
             // a step reads its state where the last one wrote it; the states
             // before steps 0, every, 2 every, ... are the checkpoints
             const bool from = n % every == 0, to = (n + 1) % every == 0 && n + 1 < ns;
             const int cf = n / every, ct = (n + 1) / every;
-            k_pm_kick_drift<R><<<pgrid(), PM_NT, 0, st>>>(from ? ckx[cf]->p : x.p, from ? ckq[cf]->p : q.p,
-                                                          to ? ckx[ct]->p : x.p, to ? ckq[ct]->p : q.p, np, N, fld.p,
+            k_pm_kick_drift<R><<<pgrid(), PM_NT, 0, st>>>(from ? ckx[cf]->p : x, from ? ckq[cf]->p : q,
+                                                          to ? ckx[ct]->p : x, to ? ckq[ct]->p : q, np, N, fld,
                                                           coefs[3 * n], coefs[3 * n + 1], n + 1 < ns ? mcell : contrast,
-                                                          rho.p);
+                                                          rho);
         }
         // final CIC density contrast: mass N^3/Np per particle, minus one
-        k_pm_contrast<R><<<fgrid(), PM_NT, 0, st>>>(rho.p, n3, delta);
-        if (xo) pck(cudaMemcpyAsync(xo, x.p, 3 * np * sizeof(double), cudaMemcpyDeviceToDevice, st), "copy x");
-        if (qo) pck(cudaMemcpyAsync(qo, q.p, 3 * np * sizeof(double), cudaMemcpyDeviceToDevice, st), "copy q");
+        k_pm_contrast<R><<<fgrid(), PM_NT, 0, st>>>(rho, n3, delta);
+        if (xo) k_pm_triples<<<pgrid(), PM_NT, 0, st>>>(x, xo, np);
+        if (qo) k_pm_triples<<<pgrid(), PM_NT, 0, st>>>(q, qo, np);
         pck(cudaGetLastError(), "forward launch");
         pck(cudaStreamSynchronize(st), "forward");
         check_device("forward");
@@ -483,13 +520,13 @@ template <class R> struct Pm final : PmBase {
         const int nb = N < 32 ? N : 32;
         const dim3 db(nb, 4, 2), dg(N / nb, N / 4, N / 2);
         // fld: the cotangent of the density deposited at xb (the final density first)
-        k_pm_to_field<R><<<fgrid(), PM_NT, 0, st>>>(ddelta, n3, fld.p);
-        const double *xb = x.p;
+        k_pm_to_field<R><<<fgrid(), PM_NT, 0, st>>>(ddelta, n3, fld);
+        const double *xb = x;
         double mb = (double)n3 / (double)np;
         bool first = true;
         for (int s = nseg - 1; s >= 0; s--) {
             const int n0 = s * every, n1 = std::min(nsteps, n0 + every);
-            // recompute x_n and psi_n of the segment from its checkpoint; q.p (the
+            // recompute x_n and psi_n of the segment from its checkpoint; q (the
             // forward's final momenta were already copied out) is the working q
             auto xn = [&](int n) { return n == n0 ? ckx[s]->p : segx[n - n0]->p; };
             deposit(ckx[s]->p, mcell);
@@ -499,25 +536,27 @@ template <class R> struct Pm final : PmBase {
                 potential(coefs[3 * n + 2], sp.p);
                 if (n + 1 < n1) {
                     segx[n + 1 - n0]->alloc(3 * np, "segment");
-                    k_pm_kick_drift<R><<<pgrid(), PM_NT, 0, st>>>(xn(n), n == n0 ? ckq[s]->p : q.p, xn(n + 1), q.p, np, N,
-                                                                  sp.p, coefs[3 * n], coefs[3 * n + 1], mcell, rho.p);
+                    k_pm_kick_drift<R><<<pgrid(), PM_NT, 0, st>>>(xn(n), n == n0 ? ckq[s]->p : q, xn(n + 1), q, np, N,
+                                                                  sp.p, coefs[3 * n], coefs[3 * n + 1], mcell, rho);
                 }
             }
             for (int n = n1 - 1; n >= n0; n--) {
                 const double kq = coefs[3 * n], kx = coefs[3 * n + 1], pc = coefs[3 * n + 2];
-                clear(lam.p, 4 * n3);
-                k_pm_reverse<R><<<pgrid(), PM_NT, 0, st>>>(xb, fld.p, mb, xn(n), segpsi[n - n0]->p, kq, kx,
-                                                           first ? nullptr : lx.p, first ? nullptr : lq.p, lx.p, lq.p,
-                                                           lam.p, np, N);
+                clear(lam, 4 * n3);
+                k_pm_reverse<R><<<pgrid(), PM_NT, 0, st>>>(xb, fld, mb, xn(n), segpsi[n - n0]->p, kq, kx,
+                                                           first ? nullptr : lx, first ? nullptr : lq, lx, lq,
+                                                           lam, np, N);
                 first = false;
-                k_pm_adj_div<R><<<dg, db, 0, st>>>(lam.p, N, kq, fld.p);
-                poisson(fld.p, fld.p, pc);
+                k_pm_adj_div<R><<<dg, db, 0, st>>>(lam, N, kq, fld);
+                poisson(fld, fld, pc);
                 mb = mcell;
                 xb = xn(n);   // of the segment's first step the checkpoint, which outlives the segment
             }
         }
-        k_pm_reverse<R><<<pgrid(), PM_NT, 0, st>>>(xb, fld.p, mb, nullptr, nullptr, 0.0, 0.0, lx.p, lq.p, gx0, gq0, nullptr,
+        k_pm_reverse<R><<<pgrid(), PM_NT, 0, st>>>(xb, fld, mb, nullptr, nullptr, 0.0, 0.0, lx, lq, lx, lq, nullptr,
                                                    np, N);
+        k_pm_triples<<<pgrid(), PM_NT, 0, st>>>(lx, gx0, np);
+        k_pm_triples<<<pgrid(), PM_NT, 0, st>>>(lq, gq0, np);
         pck(cudaGetLastError(), "adjoint launch");
         pck(cudaStreamSynchronize(st), "adjoint");
         check_device("adjoint");

@@ -795,6 +795,7 @@ __global__ void __launch_bounds__(dep_tile_threads<R>(), DepMinBlocks<R, KIND>::
     k_deposit(PView<R> p, const uint32_t *__restrict__ bstart, int N, int nt, const R *__restrict__ phi, DepOut<R> out,
               double a, double m00, double mij, double m0i, int accumulate, uint32_t *work, int *err, FastDiv fN)
 {
+    pdl_entry();
     deposit_tile<R, KIND, USE_PHI, false>((int)blockIdx.x, work, p, bstart, N, nt, phi, out, a, m00, mij, m0i, accumulate,
                                           err, fN);
 }
@@ -807,6 +808,7 @@ __global__ void __launch_bounds__(DEP_NT, GEV_DEP_MINB_DENSE)
                     DepOut<R> out, double a, double m00, double mij, double m0i, int accumulate, uint32_t *work, int *err,
                     FastDiv fN)
 {
+    pdl_entry();
     __shared__ uint32_t next;
     const uint32_t count = work[0];
     for (;;) {
@@ -846,12 +848,10 @@ static void launch_k(const PView<R> &p, const uint32_t *bstart, int N, const R *
     const int nt = N / 8;
     const unsigned tiles = (unsigned)nt * nt * nt;
     const FastDiv fN((uint32_t)N);
-    k_deposit<R, KIND, USE_PHI><<<tiles, dep_tile_threads<R>(), smem, st>>>(p, bstart, N, nt, phi, out, a, m00, mij, m0i, accumulate,
-                                                               work, err, fN);
+    pdl_launch(k_deposit<R, KIND, USE_PHI>, tiles, dep_tile_threads<R>(), smem, st, p, bstart, N, nt, phi, out, a, m00, mij, m0i, accumulate, work, err, fN);
     // one wave of resident CTAs; those that find the list empty return at once
     const unsigned grid = std::min(tiles, (unsigned)(sm_count() * GEV_DEP_MINB_DENSE));
-    k_deposit_dense<R, KIND, USE_PHI><<<grid, DEP_NT, smem_dense, st>>>(p, bstart, N, nt, phi, out, a, m00, mij, m0i,
-                                                                        accumulate, work, err, fN);
+    pdl_launch(k_deposit_dense<R, KIND, USE_PHI>, grid, DEP_NT, smem_dense, st, p, bstart, N, nt, phi, out, a, m00, mij, m0i, accumulate, work, err, fN);
 }
 
 template <class R>

@@ -237,6 +237,7 @@ __global__ void __launch_bounds__(RegPlan<N / 2>::R2 *T, MINB) k_fx_fwd(FxArgs<R
                                                                        const typename CT<R>::C *__restrict__ tw_half,
                                                                        const typename CT<R>::C *__restrict__ tw_full)
 {
+    pdl_entry();
     using C = typename CT<R>::C;
     constexpr int M = N / 2, PP = N / 2 + 2, R1 = RegPlan<M>::R1, R2 = RegPlan<M>::R2, NT = R2 * T, ES = exch_size<M, 1>();
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -296,6 +297,7 @@ __global__ void __launch_bounds__(RegPlan<N / 2>::R2 *T *G, MINB) k_fx_fwd_tij6(
                                                                               const typename CT<R>::C *__restrict__ tw_half,
                                                                               const typename CT<R>::C *__restrict__ tw_full)
 {
+    pdl_entry();
     using C = typename CT<R>::C;
     constexpr int M = N / 2, PP = N / 2 + 2, R1 = RegPlan<M>::R1, R2 = RegPlan<M>::R2, NT = R2 * T * G, ES = exch_size<M, 1>();
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -360,6 +362,7 @@ __global__ void __launch_bounds__(RegPlan<N / 2>::R2 *T, MINB) k_fx_inv(const ty
                                                                        const typename CT<R>::C *__restrict__ tw_half,
                                                                        const typename CT<R>::C *__restrict__ tw_full)
 {
+    pdl_entry();
     using C = typename CT<R>::C;
     constexpr int M = N / 2, PP = N / 2 + 2, R1 = RegPlan<M>::R1, R2 = RegPlan<M>::R2;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -433,6 +436,7 @@ __global__ void __launch_bounds__(PlaneShape<N>::NT, plane_minb<R, N>()) k_plane
                                                                  const typename CT<R>::C *__restrict__ tw_half,
                                                                  const typename CT<R>::C *__restrict__ tw_full)
 {
+    pdl_entry();
     using C = typename CT<R>::C;
     using S = PlaneShape<N>;
     constexpr int M = S::M, P = S::P, PP = N / 2 + 2, NT = S::NT;
@@ -530,6 +534,7 @@ __global__ void __launch_bounds__(PlaneShape<N>::NT, plane_minb<R, N>()) k_plane
                                                                  const typename CT<R>::C *__restrict__ tw_half,
                                                                  const typename CT<R>::C *__restrict__ tw_full)
 {
+    pdl_entry();
     using C = typename CT<R>::C;
     using S = PlaneShape<N>;
     constexpr int M = S::M, P = S::P, PP = N / 2 + 2, NT = S::NT;
@@ -917,6 +922,7 @@ __device__ __forceinline__ void bin_modes(const FzArgs<R> &a, int N, int kx, int
 template <class R, int N, int T, int G, int OP, int EXTRA, int MINB>
 __global__ void __launch_bounds__(RegPlan<N>::R2 *T *G, MINB) k_fz(FzArgs<R> a, const typename CT<R>::C *__restrict__ tw)
 {
+    pdl_entry();
     using C = typename CT<R>::C;
     constexpr int P = N / 2 + 1, PP = N / 2 + 2;
     constexpr int R1 = RegPlan<N>::R1, R2 = RegPlan<N>::R2;
@@ -1118,6 +1124,7 @@ template <class R, int N, int T, int NT, int OP, int EXTRA, bool PAD>
 __global__ void __launch_bounds__(NT, FZ_STAGED_MINB * 256 / NT)
     k_fz_tma(FzArgs<R> a, const typename CT<R>::C *__restrict__ tw, const __grid_constant__ CUtensorMap tmap)
 {
+    pdl_entry();
     using C = typename CT<R>::C;
     constexpr int P = N / 2 + 1, PP = N / 2 + 2;
     constexpr int CIN = OpShape<OP, EXTRA>::CIN, COUT = OpShape<OP, EXTRA>::COUT;
@@ -1244,6 +1251,7 @@ template <class R, int N, int T, int S, int MINB>
 __global__ void __launch_bounds__(RegPlan<N>::R2 *T, MINB) k_fy(typename CT<R>::C *data, int64_t stride,
                                                                const typename CT<R>::C *__restrict__ tw)
 {
+    pdl_entry();
     using C = typename CT<R>::C;
     constexpr int P = N / 2 + 1, PP = N / 2 + 2, R1 = RegPlan<N>::R1, R2 = RegPlan<N>::R2;
     extern __shared__ __align__(16) unsigned char smem_raw[];

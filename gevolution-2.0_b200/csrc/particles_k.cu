@@ -62,6 +62,7 @@ __global__ void __launch_bounds__(KD_NT, sizeof(R) == 4 ? 4 : 2) k_kick_drift(PV
                                                       uint32_t *counts, uint32_t *bucket, uint32_t *rank,
                                                       unsigned long long *vmax_bits, int *err, FastDiv fN)
 {
+    pdl_entry();
     extern __shared__ __align__(16) unsigned char kd_smem[];
     R(*sf)[KD_W * KD_W * KD_W] = reinterpret_cast<R(*)[KD_W * KD_W * KD_W]>(kd_smem);
     __shared__ double wmax[KD_NT / 32];
@@ -327,8 +328,7 @@ void launch_kick_drift(const PView<R> &p, const uint32_t *bstart, int N, const R
     const size_t smem = 5 * KD_W * KD_W * KD_W * sizeof(R);
     static bool attr_set[SMEM_ATTR_DEVICES] = {};
     raise_smem_limit(k_kick_drift<R>, smem, attr_set);
-    k_kick_drift<R><<<(unsigned)nt * nt * nt, KD_NT, smem, st>>>(p, bstart, N, nt, phi, chi, Bi, n3, kp, counts,
-                                                                bucket, rank, vmax_bits, err, FastDiv((uint32_t)N));
+    pdl_launch(k_kick_drift<R>, (unsigned)nt * nt * nt, KD_NT, smem, st, p, bstart, N, nt, phi, chi, Bi, n3, kp, counts, bucket, rank, vmax_bits, err, FastDiv((uint32_t)N));
 }
 
 // ---- particle I/O: host layout (box-unit positions, AoS triples) <-> cell + offset ----
@@ -464,6 +464,7 @@ constexpr int SCAN_ROUNDS = 8;
 
 __global__ void __launch_bounds__(SCAN_NT) k_scan_one(const uint32_t *__restrict__ counts, uint32_t *start, int nb)
 {
+    pdl_entry();
     __shared__ uint32_t wsum[SCAN_ROUNDS][SCAN_NT / 32];
     const int t = threadIdx.x, lane = t & 31, w = t >> 5;
     uint4 v[SCAN_ROUNDS];
@@ -517,7 +518,7 @@ __global__ void __launch_bounds__(SCAN_NT) k_scan_one(const uint32_t *__restrict
 int launch_scan(const uint32_t *counts, uint32_t *start, int64_t nb, uint32_t *block_sums, cudaStream_t st)
 {
     if (nb <= (int64_t)SCAN_NT * 4 * SCAN_ROUNDS) {
-        k_scan_one<<<1, SCAN_NT, 0, st>>>(counts, start, (int)nb);
+        pdl_launch(k_scan_one, 1, SCAN_NT, 0, st, counts, start, (int)nb);
         return 1;
     }
     int64_t nblk = (nb + SCAN_NT - 1) / SCAN_NT;
@@ -532,6 +533,7 @@ int launch_scan(const uint32_t *counts, uint32_t *start, int64_t nb, uint32_t *b
 __global__ void k_scatter_index(const uint32_t *__restrict__ bstart, const uint32_t *__restrict__ bucket,
                                 const uint32_t *__restrict__ rank, int64_t n, uint32_t *inv)
 {
+    pdl_entry();
     int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
     const uint32_t j = bstart[bucket[i]] + rank[i];
@@ -561,6 +563,7 @@ template <class R>
 __global__ void __launch_bounds__(RB_NT, 3) k_rebin_tile(PView<R> src, PView<R> dst, const uint32_t *__restrict__ bstart,
                                                       const uint32_t *__restrict__ inv, int nt, int *err, FastDiv fN)
 {
+    pdl_entry();
     constexpr int M = REBIN_SORT_MAX;
     extern __shared__ __align__(16) unsigned char rb_smem[];
     int64_t *s_id = reinterpret_cast<int64_t *>(rb_smem);
@@ -699,12 +702,11 @@ void launch_rebin(const PView<R> &src, PView<R> dst, const uint32_t *bstart, con
                   const uint32_t *rank, uint32_t *inv, int N, int *err, cudaStream_t st)
 {
     if (src.n <= 0) return;
-    k_scatter_index<<<cdiv(src.n, 256), 256, 0, st>>>(bstart, bucket, rank, src.n, inv);
+    pdl_launch(k_scatter_index, cdiv(src.n, 256), 256, 0, st, bstart, bucket, rank, src.n, inv);
     static bool attr_set[SMEM_ATTR_DEVICES] = {};
     raise_smem_limit(k_rebin_tile<R>, rb_smem_bytes<R>(), attr_set);
     const int nt = N / 8;
-    k_rebin_tile<R><<<(unsigned)nt * nt * nt, RB_NT, rb_smem_bytes<R>(), st>>>(src, dst, bstart, inv, nt, err,
-                                                                    FastDiv((uint32_t)N));
+    pdl_launch(k_rebin_tile<R>, (unsigned)nt * nt * nt, RB_NT, rb_smem_bytes<R>(), st, src, dst, bstart, inv, nt, err, FastDiv((uint32_t)N));
 }
 
 // CIC mass density in FP64 (scalarProjectionCIC_project, gevolution.hpp:1902,

@@ -112,6 +112,7 @@ __device__ __forceinline__ void pm_put(double *p, int64_t np, int64_t i, const d
 // triples -> planes and back
 __global__ void k_pm_planes(const double *__restrict__ in, double *__restrict__ out, int64_t np)
 {
+    pdl_entry();
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < np; i += (int64_t)gridDim.x * blockDim.x) {
         const double v[3] = {in[3 * i], in[3 * i + 1], in[3 * i + 2]};
         pm_put(out, np, i, v);
@@ -119,6 +120,7 @@ __global__ void k_pm_planes(const double *__restrict__ in, double *__restrict__ 
 }
 __global__ void k_pm_triples(const double *__restrict__ in, double *__restrict__ out, int64_t np)
 {
+    pdl_entry();
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < np; i += (int64_t)gridDim.x * blockDim.x) {
         const Vec3 v = pm_get(in, np, i);
 #pragma unroll
@@ -197,6 +199,7 @@ __device__ __forceinline__ void pm_grad_corners(const R *__restrict__ psi, const
 template <class R>
 __global__ void k_pm_deposit(const double *__restrict__ x, int64_t np, int N, double cst, R *out)
 {
+    pdl_entry();
     const double invN = 1.0 / N;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < np; i += (int64_t)gridDim.x * blockDim.x)
         pm_scatter(PmSite(pm_get(x, np, i).v, N, invN), cst, out);
@@ -210,6 +213,7 @@ template <class R>
 __global__ void __launch_bounds__(PM_NT, 3) k_pm_kick_drift(const double *xi, const double *qi, double *xo, double *qo, int64_t np, int N,
                                 const R *__restrict__ psi, double kq, double kx, double cst, R *rho)
 {
+    pdl_entry();
     const double invN = 1.0 / N;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < np; i += (int64_t)gridDim.x * blockDim.x) {
         double x[3], q[3];
@@ -269,6 +273,7 @@ __global__ void __launch_bounds__(PM_NT, 2) k_pm_reverse(const double *__restric
                              const R *__restrict__ psi, double kq, double kx, const double *lxi, const double *lqi,
                              double *lxo, double *lqo, R *lam, int64_t np, int N)
 {
+    pdl_entry();
     const double invN = 1.0 / N;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < np; i += (int64_t)gridDim.x * blockDim.x) {
         double lx[3], lq[3];
@@ -314,6 +319,7 @@ __global__ void __launch_bounds__(PM_NT, 2) k_pm_reverse(const double *__restric
 template <class R>
 __global__ void k_pm_adj_div(const R *__restrict__ lam, int N, double kq, R *lpsi)
 {
+    pdl_entry();
     const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y,
               z = blockIdx.z * blockDim.z + threadIdx.z;
     if (x >= N || y >= N || z >= N) return;
@@ -329,6 +335,7 @@ __global__ void k_pm_adj_div(const R *__restrict__ lam, int N, double kq, R *lps
 template <class R>
 __global__ void k_pm_contrast(const R *__restrict__ rho, int64_t n3, double *out)
 {
+    pdl_entry();
     for (int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; g < n3; g += (int64_t)gridDim.x * blockDim.x)
         out[g] = (double)rho[g] - 1.0;
 }
@@ -336,6 +343,7 @@ __global__ void k_pm_contrast(const R *__restrict__ rho, int64_t n3, double *out
 template <class R>
 __global__ void k_pm_to_field(const double *__restrict__ in, int64_t n3, R *out)
 {
+    pdl_entry();
     for (int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; g < n3; g += (int64_t)gridDim.x * blockDim.x)
         out[g] = (R)in[g];
 }
@@ -459,7 +467,7 @@ template <class R> struct Pm final : PmBase {
     void deposit(const double *xs, double cst)
     {
         clear(rho, n3);
-        k_pm_deposit<R><<<pgrid(), PM_NT, 0, st>>>(xs, np, N, cst, rho);
+        pdl_launch(k_pm_deposit<R>, pgrid(), PM_NT, 0, st, xs, np, N, cst, rho);
     }
 
     // potential of the density in rho, which is left cleared for the next deposit
@@ -483,8 +491,8 @@ template <class R> struct Pm final : PmBase {
             ckx[s]->alloc(3 * np, "checkpoint");
             ckq[s]->alloc(3 * np, "checkpoint");
         }
-        k_pm_planes<<<pgrid(), PM_NT, 0, st>>>(x0, ckx[0]->p, np);
-        k_pm_planes<<<pgrid(), PM_NT, 0, st>>>(q0, ckq[0]->p, np);
+        pdl_launch(k_pm_planes, pgrid(), PM_NT, 0, st, x0, ckx[0]->p, np);
+        pdl_launch(k_pm_planes, pgrid(), PM_NT, 0, st, q0, ckq[0]->p, np);
         const double mcell = mass * (double)n3, contrast = (double)n3 / (double)np;
         deposit(ckx[0]->p, mcell);
         for (int n = 0; n < ns; n++) {
@@ -493,15 +501,12 @@ template <class R> struct Pm final : PmBase {
             // before steps 0, every, 2 every, ... are the checkpoints
             const bool from = n % every == 0, to = (n + 1) % every == 0 && n + 1 < ns;
             const int cf = n / every, ct = (n + 1) / every;
-            k_pm_kick_drift<R><<<pgrid(), PM_NT, 0, st>>>(from ? ckx[cf]->p : x, from ? ckq[cf]->p : q,
-                                                          to ? ckx[ct]->p : x, to ? ckq[ct]->p : q, np, N, fld,
-                                                          coefs[3 * n], coefs[3 * n + 1], n + 1 < ns ? mcell : contrast,
-                                                          rho);
+            pdl_launch(k_pm_kick_drift<R>, pgrid(), PM_NT, 0, st, from ? ckx[cf]->p : x, from ? ckq[cf]->p : q, to ? ckx[ct]->p : x, to ? ckq[ct]->p : q, np, N, fld, coefs[3 * n], coefs[3 * n + 1], n + 1 < ns ? mcell : contrast, rho);
         }
         // final CIC density contrast: mass N^3/Np per particle, minus one
-        k_pm_contrast<R><<<fgrid(), PM_NT, 0, st>>>(rho, n3, delta);
-        if (xo) k_pm_triples<<<pgrid(), PM_NT, 0, st>>>(x, xo, np);
-        if (qo) k_pm_triples<<<pgrid(), PM_NT, 0, st>>>(q, qo, np);
+        pdl_launch(k_pm_contrast<R>, fgrid(), PM_NT, 0, st, rho, n3, delta);
+        if (xo) pdl_launch(k_pm_triples, pgrid(), PM_NT, 0, st, x, xo, np);
+        if (qo) pdl_launch(k_pm_triples, pgrid(), PM_NT, 0, st, q, qo, np);
         pck(cudaGetLastError(), "forward launch");
         pck(cudaStreamSynchronize(st), "forward");
         check_device("forward");
@@ -520,7 +525,7 @@ template <class R> struct Pm final : PmBase {
         const int nb = N < 32 ? N : 32;
         const dim3 db(nb, 4, 2), dg(N / nb, N / 4, N / 2);
         // fld: the cotangent of the density deposited at xb (the final density first)
-        k_pm_to_field<R><<<fgrid(), PM_NT, 0, st>>>(ddelta, n3, fld);
+        pdl_launch(k_pm_to_field<R>, fgrid(), PM_NT, 0, st, ddelta, n3, fld);
         const double *xb = x;
         double mb = (double)n3 / (double)np;
         bool first = true;
@@ -536,27 +541,23 @@ template <class R> struct Pm final : PmBase {
                 potential(coefs[3 * n + 2], sp.p);
                 if (n + 1 < n1) {
                     segx[n + 1 - n0]->alloc(3 * np, "segment");
-                    k_pm_kick_drift<R><<<pgrid(), PM_NT, 0, st>>>(xn(n), n == n0 ? ckq[s]->p : q, xn(n + 1), q, np, N,
-                                                                  sp.p, coefs[3 * n], coefs[3 * n + 1], mcell, rho);
+                    pdl_launch(k_pm_kick_drift<R>, pgrid(), PM_NT, 0, st, xn(n), n == n0 ? ckq[s]->p : q, xn(n + 1), q, np, N, sp.p, coefs[3 * n], coefs[3 * n + 1], mcell, rho);
                 }
             }
             for (int n = n1 - 1; n >= n0; n--) {
                 const double kq = coefs[3 * n], kx = coefs[3 * n + 1], pc = coefs[3 * n + 2];
                 clear(lam, 4 * n3);
-                k_pm_reverse<R><<<pgrid(), PM_NT, 0, st>>>(xb, fld, mb, xn(n), segpsi[n - n0]->p, kq, kx,
-                                                           first ? nullptr : lx, first ? nullptr : lq, lx, lq,
-                                                           lam, np, N);
+                pdl_launch(k_pm_reverse<R>, pgrid(), PM_NT, 0, st, xb, fld, mb, xn(n), segpsi[n - n0]->p, kq, kx, first ? nullptr : lx, first ? nullptr : lq, lx, lq, lam, np, N);
                 first = false;
-                k_pm_adj_div<R><<<dg, db, 0, st>>>(lam, N, kq, fld);
+                pdl_launch(k_pm_adj_div<R>, dg, db, 0, st, lam, N, kq, fld);
                 poisson(fld, fld, pc);
                 mb = mcell;
                 xb = xn(n);   // of the segment's first step the checkpoint, which outlives the segment
             }
         }
-        k_pm_reverse<R><<<pgrid(), PM_NT, 0, st>>>(xb, fld, mb, nullptr, nullptr, 0.0, 0.0, lx, lq, lx, lq, nullptr,
-                                                   np, N);
-        k_pm_triples<<<pgrid(), PM_NT, 0, st>>>(lx, gx0, np);
-        k_pm_triples<<<pgrid(), PM_NT, 0, st>>>(lq, gq0, np);
+        pdl_launch(k_pm_reverse<R>, pgrid(), PM_NT, 0, st, xb, fld, mb, nullptr, nullptr, 0.0, 0.0, lx, lq, lx, lq, nullptr, np, N);
+        pdl_launch(k_pm_triples, pgrid(), PM_NT, 0, st, lx, gx0, np);
+        pdl_launch(k_pm_triples, pgrid(), PM_NT, 0, st, lq, gq0, np);
         pck(cudaGetLastError(), "adjoint launch");
         pck(cudaStreamSynchronize(st), "adjoint");
         check_device("adjoint");

@@ -61,7 +61,7 @@ void fx_fwd_n(const FxArgs<R> &a, int ncomp, int64_t in_stride, int64_t out_stri
     size_t smem = (size_t)T * exch_size<N / 2, 1>() * sizeof(C);
     auto k = k_fx_fwd<R, N, T, MODE, resident<R>(NT, regs_for<R, N / 2>(REGS_X))>;
     set_smem(k, smem);
-    k<<<dim3(N / T, N, ncomp), NT, smem, st>>>(a, in_stride, out_stride, tb.tw_half, tb.tw_full);
+    pdl_launch(k, dim3(N / T, N, ncomp), NT, smem, st, a, in_stride, out_stride, tb.tw_half, tb.tw_full);
 }
 
 template <class R, int N>
@@ -72,7 +72,7 @@ void fx_tij6_n(const FxArgs<R> &a, int64_t in_stride, int64_t out_stride, const 
     size_t smem = (size_t)6 * T * exch_size<N / 2, 1>() * sizeof(C);
     auto k = k_fx_fwd_tij6<R, N, T, G, resident<R>(NT, regs_for<R, N / 2>(REGS_TIJ<R>))>;
     set_smem(k, smem);
-    k<<<dim3(N / T, N), NT, smem, st>>>(a.in, in_stride, a.phi, a.c, a.out, out_stride, tb.tw_half, tb.tw_full);
+    pdl_launch(k, dim3(N / T, N), NT, smem, st, a.in, in_stride, a.phi, a.c, a.out, out_stride, tb.tw_half, tb.tw_full);
 }
 
 // the x and y transforms of whole planes in one kernel (fftpass.cuh)
@@ -85,7 +85,7 @@ void plane_fwd_n(const FxArgs<R> &a, int ncomp, int64_t in_stride, int64_t out_s
     constexpr size_t smem = (size_t)PlaneShape<N>::VALUES * sizeof(C);
     auto k = k_plane_fwd<R, N, MODE>;
     set_smem(k, smem);
-    k<<<dim3(N, ncomp), PlaneShape<N>::NT, smem, st>>>(a, in_stride, out_stride, tb.tw_half, tb.tw_full);
+    pdl_launch(k, dim3(N, ncomp), PlaneShape<N>::NT, smem, st, a, in_stride, out_stride, tb.tw_half, tb.tw_full);
 }
 
 template <class R, int N, int S>
@@ -96,7 +96,7 @@ void fy_n(typename CT<R>::C *data, int64_t stride, int ncomp, const FftTables<R>
     const size_t smem = (size_t)exch_size<N, T>() * sizeof(C);
     auto k = k_fy<R, N, T, S, resident<R>(NT, regs_for<R, N>(REGS_Y))>;
     set_smem(k, smem);
-    k<<<dim3((N / 2 + 1 + T - 1) / T, N, ncomp), NT, smem, st>>>(data, stride, tb.tw_full);
+    pdl_launch(k, dim3((N / 2 + 1 + T - 1) / T, N, ncomp), NT, smem, st, data, stride, tb.tw_full);
 }
 
 template <class R, int N, int MODE>
@@ -140,7 +140,7 @@ void fxi_n(const typename CT<R>::C *in, int64_t in_stride, R *out, int64_t out_s
     size_t smem = (size_t)T * exch_size<N / 2, 1>() * sizeof(C);
     auto k = k_fx_inv<R, N, T, resident<R>(NT, regs_for<R, N / 2>(REGS_X))>;
     set_smem(k, smem);
-    k<<<dim3(N / T, N, ncomp), NT, smem, st>>>(in, in_stride, out, out_stride, tb.tw_half, tb.tw_full);
+    pdl_launch(k, dim3(N / T, N, ncomp), NT, smem, st, in, in_stride, out, out_stride, tb.tw_half, tb.tw_full);
 }
 
 template <class R, int N>
@@ -152,7 +152,7 @@ int fyx_inv_n(typename CT<R>::C *in, int64_t in_stride, R *out, int64_t out_stri
         constexpr size_t smem = (size_t)PlaneShape<N>::VALUES * sizeof(C);
         auto k = k_plane_inv<R, N>;
         set_smem(k, smem);
-        k<<<dim3(N, ncomp), PlaneShape<N>::NT, smem, st>>>(in, in_stride, out, out_stride, tb.tw_half, tb.tw_full);
+        pdl_launch(k, dim3(N, ncomp), PlaneShape<N>::NT, smem, st, in, in_stride, out, out_stride, tb.tw_half, tb.tw_full);
         return 1;
     } else {
         fy_n<R, N, 1>(in, in_stride, ncomp, tb, st);
@@ -198,7 +198,7 @@ void fz_n(const FzArgs<R> &a, const FftTables<R> &tb, cudaStream_t st)
         const CUtensorMap map = fourier_tensor_map<R>(a.data, N, a.stride, S::CMAX, T, 1, ZBox<N>::ZB);
         auto k = k_fz_tma<R, N, T, NT, OP, EXTRA, PAD>;
         set_smem(k, smem);
-        k<<<dim3((N / 2 + 1 + T - 1) / T, N), NT, smem, st>>>(a, tb.tw_full, map);
+        pdl_launch(k, dim3((N / 2 + 1 + T - 1) / T, N), NT, smem, st, a, tb.tw_full, map);
     } else {
         constexpr int CT1 = S::CONTRACT ? 3 : S::CIN, G = CT1 > 1 ? PASS_GZ : 1, R2 = RegPlan<N>::R2;
         constexpr int T0 = cols<R>(CT1 == 1 ? PASS_TZ1 : (CT1 == 3 ? PASS_TZ3<N> : PASS_TZ6));
@@ -207,7 +207,7 @@ void fz_n(const FzArgs<R> &a, const FftTables<R> &tb, cudaStream_t st)
         constexpr int REGS = CT1 == 6 ? REGS_Z6 : (CT1 == 3 ? REGS_Z3<N> : REGS_Z1<R>);
         auto k = k_fz<R, N, T, G, OP, EXTRA, resident<R>(NT, regs_for<R, N>(REGS))>;
         set_smem(k, smem);
-        k<<<dim3((N / 2 + 1 + T - 1) / T, N), NT, smem, st>>>(a, tb.tw_full);
+        pdl_launch(k, dim3((N / 2 + 1 + T - 1) / T, N), NT, smem, st, a, tb.tw_full);
     }
 }
 

@@ -20,11 +20,33 @@ namespace gev {
 
 constexpr int KD_NT = 256;
 constexpr int KD_W = 11;   // staged extent per axis
+// Staged fields, by precision.  FP64: rows have a pitch of 39 values and planes
+// one of 433 (7 and 17 mod 32), so that the cells of a tile in particle order
+// -- rows of 7, planes of 49 -- follow each other in the banks and the
+// particles of a warp read different ones; three fields of 11 + 1 values share
+// a row, so the padding costs half as much again, not four times (256^3 FP64
+// kick 1056 -> 1002 us).  FP32: dense rows of 11; the same layout halves its
+// bank conflicts as well (50 to 25 million at 256^3) but not its time, which
+// instruction issue bounds (ncu: issue 70 %; 548 and 547 us).
+template <class R> struct KdLayout;
+template <> struct KdLayout<float> {
+    static constexpr int PX = KD_W, PZ = KD_W * KD_W, TOTAL = 5 * KD_W * PZ;
+    __host__ __device__ static constexpr int field(int f) { return f * KD_W * PZ; }
+};
+template <> struct KdLayout<double> {
+    static constexpr int PX = 39, PZ = 433, ARRAY = KD_W * PZ, TOTAL = 2 * ARRAY;
+    static_assert(PX % 32 == 7 && PZ % 32 == 17 && PZ >= KD_W * PX && 3 * (KD_W + 1) <= PX, "staged layout");
+    __host__ __device__ static constexpr int field(int f) { return (f / 3) * ARRAY + (f % 3) * (KD_W + 1); }
+};
+template <class R> __host__ __device__ constexpr int kd_slot(int rx, int ry, int rz)
+{
+    return (rx + 1) + KdLayout<R>::PX * (ry + 1) + KdLayout<R>::PZ * (rz + 1);
+}
 
 template <class R>
 __device__ __forceinline__ R SF(const R *s, int rx, int ry, int rz, int dx, int dy, int dz)
 {
-    return s[(rx + 1 + dx) + KD_W * ((ry + 1 + dy) + KD_W * (rz + 1 + dz))];
+    return s[kd_slot<R>(rx + dx, ry + dy, rz + dz)];
 }
 
 __device__ __forceinline__ uint32_t lanemask_lt()
@@ -64,7 +86,7 @@ __global__ void __launch_bounds__(KD_NT, sizeof(R) == 4 ? 4 : 2) k_kick_drift(PV
 {
     pdl_entry();
     extern __shared__ __align__(16) unsigned char kd_smem[];
-    R(*sf)[KD_W * KD_W * KD_W] = reinterpret_cast<R(*)[KD_W * KD_W * KD_W]>(kd_smem);
+    R *sf = reinterpret_cast<R *>(kd_smem);
     __shared__ double wmax[KD_NT / 32];
     const int tile = blockIdx.x;
     const int tx = tile % nt, ty = (tile / nt) % nt, tz = tile / (nt * nt);
@@ -79,6 +101,7 @@ __global__ void __launch_bounds__(KD_NT, sizeof(R) == 4 ? 4 : 2) k_kick_drift(PV
         constexpr int NS = KD_W * KD_W * KD_W;
         constexpr int PER = (NS + KD_NT - 1) / KD_NT;
         int64_t gi[PER];
+        int so[PER];
         R v[PER][5];
 #pragma unroll
         for (int k = 0; k < PER; k++) {
@@ -86,6 +109,7 @@ __global__ void __launch_bounds__(KD_NT, sizeof(R) == 4 ? 4 : 2) k_kick_drift(PV
             const int ii = i < NS ? i : NS - 1;
             const int vx = ii % KD_W - 1, vy = (ii / KD_W) % KD_W - 1, vz = ii / (KD_W * KD_W) - 1;
             gi[k] = sidx(N, wrapi(x0 + vx, N), wrapi(y0 + vy, N), wrapi(z0 + vz, N));
+            so[k] = kd_slot<R>(vx, vy, vz);
         }
 #pragma unroll
         for (int k = 0; k < PER; k++) {
@@ -101,14 +125,18 @@ __global__ void __launch_bounds__(KD_NT, sizeof(R) == 4 ? 4 : 2) k_kick_drift(PV
         for (int k = 0; k < PER; k++) {
             const int i = threadIdx.x + k * KD_NT;
             if (i < NS) {
-                if (need_phi) sf[0][i] = v[k][0];
-                if (need_chi) sf[1][i] = v[k][1];
-                if (need_B) { sf[2][i] = v[k][2]; sf[3][i] = v[k][3]; sf[4][i] = v[k][4]; }
+                if (need_phi) sf[KdLayout<R>::field(0) + so[k]] = v[k][0];
+                if (need_chi) sf[KdLayout<R>::field(1) + so[k]] = v[k][1];
+                if (need_B) {
+                    sf[KdLayout<R>::field(2) + so[k]] = v[k][2];
+                    sf[KdLayout<R>::field(3) + so[k]] = v[k][3];
+                    sf[KdLayout<R>::field(4) + so[k]] = v[k][4];
+                }
             }
         }
     }
     __syncthreads();
-    const R *P_ = sf[0], *X_ = sf[1], *B0 = sf[2], *B1 = sf[3], *B2 = sf[4];
+    const R *P_ = sf + KdLayout<R>::field(0), *X_ = sf + KdLayout<R>::field(1), *B0 = sf + KdLayout<R>::field(2), *B1 = sf + KdLayout<R>::field(3), *B2 = sf + KdLayout<R>::field(4);
 
     const uint32_t lo = bstart[8 * tile], hi = bstart[8 * tile + 8];
     R lmax = 0;   // max of q^2 / a^2 (converted to FP64 once, at the end)
@@ -325,7 +353,7 @@ void launch_kick_drift(const PView<R> &p, const uint32_t *bstart, int N, const R
                        unsigned long long *vmax_bits, int *err, cudaStream_t st)
 {
     int nt = N / 8;
-    const size_t smem = 5 * KD_W * KD_W * KD_W * sizeof(R);
+    const size_t smem = KdLayout<R>::TOTAL * sizeof(R);
     static bool attr_set[SMEM_ATTR_DEVICES] = {};
     raise_smem_limit(k_kick_drift<R>, smem, attr_set);
     pdl_launch(k_kick_drift<R>, (unsigned)nt * nt * nt, KD_NT, smem, st, p, bstart, N, nt, phi, chi, Bi, n3, kp, counts, bucket, rank, vmax_bits, err, FastDiv((uint32_t)N));

@@ -13,11 +13,14 @@ namespace gev {
 // Lines (x passes) or kx-columns (y, z passes) per CTA, and the registers per
 // thread (FP32; twice that in FP64) that set the resident CTAs, from sweeps at
 // 128^3 to 512^3 (FP32) and 256^3 (FP64).
-constexpr int PASS_TX = 8, PASS_TY = 16, PASS_TZ1 = 8, PASS_TZ6 = 4, PASS_TIJ = 4, PASS_TIJ_G = 4, PASS_GZ = 3;
+constexpr int PASS_TX = 8, PASS_TY = 16, PASS_TZ1 = 8, PASS_TZ6 = 8, PASS_TIJ = 4, PASS_TIJ_G = 4, PASS_GZ = 3;
 constexpr int REGS_X = 72, REGS_Y = 96;
 template <class R> constexpr int REGS_TIJ = sizeof(R) == 4 ? 72 : 96;
 template <class R> constexpr int REGS_Z1 = sizeof(R) == 4 ? 72 : 96;
-constexpr int REGS_Z6 = 168;   // the tensor solve holds six components in FP64
+// The tensor solve holds six components in FP64 and moves 24 values of tensor
+// state per mode: eight columns make its rows 64-byte segments (256^3 mixed,
+// parabolic B_i and h_ij: cycle 4075 us with four columns, 3936 with eight).
+constexpr int REGS_Z6 = 168;
 // three components: eight columns while a thread's values leave the registers
 // for it (256^3: 180 against 191 us with four), four columns beyond
 template <int N> constexpr int PASS_TZ3 = N <= 256 ? 8 : 4;

@@ -30,6 +30,7 @@ template <class R> struct FxArgs {
     double bg, c, c2, c3; // prepareFTsource_T00 params (bgmodel, coeff, coeff2, coeff3) / Tij coeff in c
     typename CT<R>::C *out;
     double *partial;      // per-block partial sums of the source (FX_PREP_T00)
+    bool clear;           // FX_COPY: leave zeros in place of the values read
 };
 
 template <class R>
@@ -153,8 +154,8 @@ __device__ __forceinline__ typename CT<R>::C fx_pair(const FxArgs<R> &a, const R
     if constexpr (MODE == FX_COPY) {
         // a caller's own array (gev_poisson_noalloc) may be aligned to single values only
         const R *p = in + sidx(N, x0, y, z);
-        if (reinterpret_cast<uintptr_t>(in) % (2 * sizeof(R)) == 0) return ld_pair(p);
-        return mk(__ldg(p), __ldg(p + 1));
+        if (reinterpret_cast<uintptr_t>(in) % (2 * sizeof(R)) == 0) return *reinterpret_cast<const typename CT<R>::C *>(p);
+        return mk(p[0], p[1]);
     } else if constexpr (MODE == FX_PREP_T00) {
         const int xm = x0 == 0 ? N - 1 : x0 - 1, x2 = x0 + 2 == N ? 0 : x0 + 2;
         const int ym = y == 0 ? N - 1 : y - 1, yp = y == N - 1 ? 0 : y + 1;
@@ -232,6 +233,20 @@ template <int NT> __device__ __forceinline__ void block_sum(double v, double *ou
     }
 }
 
+// zeros in place of the pairs that thread u of row (y, z) has read (every pair
+// has one reader), after all of its loads
+template <class R, int N>
+__device__ __forceinline__ void fx_clear(const R *in, int u, int y, int z)
+{
+    constexpr int R1 = RegPlan<N / 2>::R1, R2 = RegPlan<N / 2>::R2;
+#pragma unroll
+    for (int r = 0; r < R1; r++) {
+        R *w = const_cast<R *>(in) + sidx(N, 2 * (u + R2 * r), y, z);
+        w[0] = R(0);
+        w[1] = R(0);
+    }
+}
+
 template <class R, int N, int T, int MODE, int MINB>
 __global__ void __launch_bounds__(RegPlan<N / 2>::R2 *T, MINB) k_fx_fwd(FxArgs<R> a, int64_t in_stride, int64_t out_stride,
                                                                        const typename CT<R>::C *__restrict__ tw_half,
@@ -257,6 +272,7 @@ __global__ void __launch_bounds__(RegPlan<N / 2>::R2 *T, MINB) k_fx_fwd(FxArgs<R
         if (MODE != FX_PREP_T0I || comp == 0) load(IntC<0>{});
         else if (comp == 1) load(IntC<1>{});
         else load(IntC<2>{});
+        if (MODE == FX_COPY && a.clear) fx_clear<R, N>(in, u, y0 + l, z);
         step1_store<M, -1, 1>(v, smem + l * ES, u, tw_half);
     }
     __syncthreads();
@@ -453,6 +469,7 @@ __global__ void __launch_bounds__(PlaneShape<N>::NT, plane_minb<R, N>()) k_plane
             C v[XR1];
 #pragma unroll
             for (int r = 0; r < XR1; r++) v[r] = fx_pair<R, N, MODE, decltype(cc)::v>(a, in, u + XR2 * r, y, z, lsum);
+            if (MODE == FX_COPY && a.clear) fx_clear<R, N>(in, u, y, z);
             step1_store<M, -1, 1>(v, smem + y * S::XES, u, tw_half);
         }
     };

@@ -75,12 +75,13 @@ template <class R> struct FftTables {
 
 // x and y transforms, forward (mode: FX_*, the source preparation fused into
 // the row loads; with FX_PREP_T00 `partial` receives fxy_partials(N) partial
-// sums of the source) and inverse (the spectrum is overwritten).  Both return
+// sums of the source; with FX_COPY and `clear` the input is left zero) and
+// inverse (the spectrum is overwritten).  Both return
 // the number of kernels launched.
 template <class R>
 int fxy_forward(int N, int mode, const R *in, int64_t in_stride, int ncomp, const R *phi, const R *chi, double bg, double c,
                 double c2, double c3, typename CT<R>::C *out, int64_t out_stride, double *partial, const FftTables<R> &tb,
-                cudaStream_t st);
+                cudaStream_t st, bool clear = false);
 template <class R>
 int fyx_inverse(int N, typename CT<R>::C *in, int64_t in_stride, R *out, int64_t out_stride, int ncomp, const FftTables<R> &tb,
                 cudaStream_t st);

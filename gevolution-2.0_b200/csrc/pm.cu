@@ -448,10 +448,11 @@ template <class R> struct Pm final : PmBase {
     FftTables<R> tables() const { return FftTables<R>{twf.p, twh.p, k2.p, ks.p}; }
 
     // out <- Poisson(in) with coefficient pc (modif 0): the pass sequence of gev_solve_phi
-    void poisson(const R *in, R *out, double pc)
+    // (clear: `in`, another array, is left zero)
+    void poisson(const R *in, R *out, double pc, bool clear = false)
     {
         const FftTables<R> tb = tables();
-        fxy_forward<R>(N, FX_COPY, in, n3, 1, nullptr, nullptr, 0.0, 0.0, 0.0, 0.0, W.p, nk, nullptr, tb, st);
+        fxy_forward<R>(N, FX_COPY, in, n3, 1, nullptr, nullptr, 0.0, 0.0, 0.0, 0.0, W.p, nk, nullptr, tb, st, clear);
         FzParams fp{};
         fp.op = OP_POISSON;
         fp.err = derr.p;
@@ -473,8 +474,7 @@ template <class R> struct Pm final : PmBase {
     // potential of the density in rho, which is left cleared for the next deposit
     void potential(double pc, R *out)
     {
-        poisson(rho, out, pc);
-        clear(rho, n3);
+        poisson(rho, out, pc, true);
     }
 
     void forward(int ns, const double *coef, const double *x0, const double *q0, double *delta, double *xo,

@@ -119,12 +119,12 @@ int fxy_fwd_n(const FxArgs<R> &a, int ncomp, int64_t in_stride, int64_t out_stri
 template <class R>
 int fxy_forward(int N, int mode, const R *in, int64_t in_stride, int ncomp, const R *phi, const R *chi, double bg, double c,
                 double c2, double c3, typename CT<R>::C *out, int64_t out_stride, double *partial, const FftTables<R> &tb,
-                cudaStream_t st)
+                cudaStream_t st, bool clear)
 {
     FxArgs<R> a;
     a.in = in; a.phi = phi; a.chi = chi;
     a.bg = bg; a.c = c; a.c2 = c2; a.c3 = c3;
-    a.out = out; a.partial = partial;
+    a.out = out; a.partial = partial; a.clear = clear;
     if (mode == FX_PREP_TIJ && ncomp != 6) throw std::runtime_error("the Tij sources are prepared together");
     int n = 0;
     if (mode == FX_COPY) { GEV_SWITCH_N(N, (n = fxy_fwd_n<R, NN, FX_COPY>(a, ncomp, in_stride, out_stride, tb, st))) }
@@ -315,7 +315,7 @@ void prep_tij_pass(int N, R *Sij, const R *phi, double coeff, cudaStream_t st)
 
 #define GEV_SOLVE_INST(R)                                                                                            \
     template int fxy_forward<R>(int, int, const R *, int64_t, int, const R *, const R *, double, double, double, double, \
-                                CT<R>::C *, int64_t, double *, const FftTables<R> &, cudaStream_t);                  \
+                                CT<R>::C *, int64_t, double *, const FftTables<R> &, cudaStream_t, bool);            \
     template int fyx_inverse<R>(int, CT<R>::C *, int64_t, R *, int64_t, int, const FftTables<R> &, cudaStream_t);     \
     template void fz_pass<R>(int, const FzParams &, CT<R>::C *, int64_t, CT<R>::C *, CT<R>::C *, CT<R>::C *,          \
                              const FftTables<R> &, cudaStream_t);                                                    \

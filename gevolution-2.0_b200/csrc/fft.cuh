@@ -1,4 +1,5 @@
-// fft.cuh -- batched in-shared-memory FFTs for the pencil passes.
+// fft.cuh -- batched in-shared-memory FFTs of the staged z pass (k_fz_tma), and
+// the small in-register DFTs that the two-step transforms (fftreg.cuh) use too.
 //
 // T independent lines of length L sit in shared memory as buf[n*ld + t]
 // (n = position along the transform, t = line, ld >= T).  The transform is the
@@ -27,14 +28,8 @@ template <int L> struct Plan;
         static constexpr int ns = NS;                                                      \
         __host__ __device__ static constexpr int r(int i) { return i == 0 ? R0 : (i == 1 ? R1 : (i == 2 ? R2 : R3)); } \
     };
-GEV_PLAN(8, 1, 8, 1, 1, 1)
-GEV_PLAN(16, 2, 4, 4, 1, 1)
-GEV_PLAN(32, 2, 4, 8, 1, 1)
-GEV_PLAN(64, 2, 8, 8, 1, 1)
 // radix-8 passes first: with padded rows every pass of a dense buffer is then
 // free of bank conflicts
-GEV_PLAN(128, 3, 8, 8, 2, 1)
-GEV_PLAN(192, 3, 3, 8, 8, 1)
 GEV_PLAN(256, 3, 4, 8, 8, 1)
 GEV_PLAN(384, 4, 8, 8, 2, 3)
 GEV_PLAN(512, 3, 8, 8, 8, 1)

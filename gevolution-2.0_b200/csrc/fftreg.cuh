@@ -48,7 +48,16 @@ __host__ __device__ constexpr double root_cos(int k)   // cos(2 pi k / 96), any 
 }
 __host__ __device__ constexpr double root_sin(int k) { return root_cos(k + 72); }
 
-// a * exp(S 2 pi i K / R), R a divisor of 96
+// a * exp(S 2 pi i K / R), R a divisor of 96.
+// FP32 radices of 16 and 32 carry the rounding errors of the root's two
+// constants along, four operations more: such a radix multiplies by one root
+// per value more than the radix-8 steps of a Stockham transform, and without
+// this the FP32 transforms were the less exact ones (forward and back of white
+// noise against 64 bits, x 1e-7; Stockham / two-step / with the constants:
+// 128^3 2.49 / 2.50 / 2.36, 256^3 2.71 / 2.77 / 2.43, 384^3 3.05 / 3.13 / 2.87,
+// 512^3 2.86 / 2.96 / 2.63, 768^3 3.14 / 3.28 / 3.04).  Time: a phi solve at
+// 384^3 917 -> 926 us, none that shows at the other sizes.  With the radices of
+// 12 and 24 too it would be 933 us.
 template <int R, int K, int S, class C> __device__ __forceinline__ C mul_root(C a)
 {
     static_assert(96 % R == 0, "roots are tabulated for divisors of 96");
@@ -67,8 +76,14 @@ template <int R, int K, int S, class C> __device__ __forceinline__ C mul_root(C 
         return o;
     } else {
         constexpr F c = F(root_cos(k)), s = F(S * root_sin(k));
-        o.x = a.x * c - a.y * s;
-        o.y = a.y * c + a.x * s;
+        if constexpr (sizeof(F) == 4 && (R == 16 || R == 32)) {
+            constexpr F cl = F(root_cos(k) - (double)c), sl = F(S * root_sin(k) - (double)s);
+            o.x = fmaf(a.x, c, fmaf(-a.y, s, a.x * cl - a.y * sl));
+            o.y = fmaf(a.y, c, fmaf(a.x, s, a.y * cl + a.x * sl));
+        } else {
+            o.x = a.x * c - a.y * s;
+            o.y = a.y * c + a.x * s;
+        }
         return o;
     }
 }

@@ -154,3 +154,19 @@ def test_solve_B_sizes(N):
             c.set_field(gev.FIELD_BI, T0i)
             c.solve_B(coeff)
             assert rel_err(c.get_field(gev.FIELD_BI).ravel(), B_ref) < TOL[prec], prec
+
+
+@pytest.mark.parametrize("N,bound", [(128, 2.487e-7), (256, 2.715e-7), (384, 3.054e-7), (512, 2.860e-7), (768, 3.138e-7)])
+def test_transform_rounding_fp32(N, bound):
+    """Rounding error of the FP32 transforms alone: a screening far above every
+    k^2 makes the solve a multiplication by -1, so that forward and back of
+    white noise return its negative.  The bound is what radix-8 Stockham
+    transforms of the same lines show for these inputs (it scatters by 0.1 %
+    between seeds): the transforms must not be less exact than those."""
+    f = np.random.default_rng(140).standard_normal(N ** 3, dtype=np.float32).astype(np.float64)
+    with ctx(N, gev.MIXED) as c:
+        c.set_field(gev.FIELD_SOURCE, f)
+        c.solve_phi(False, 0.0, 0.0, 0.0, 0.0, 1e18, 1e18)
+        d = c.get_field(gev.FIELD_PHI).ravel()
+    d += f
+    assert np.linalg.norm(d) / np.linalg.norm(f) < 1.002 * bound

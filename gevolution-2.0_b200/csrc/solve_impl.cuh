@@ -4,6 +4,7 @@
 
 #include <algorithm>
 #include <stdexcept>
+#include <string>
 
 #include "fftpass.cuh"
 #include "kernels.h"
@@ -13,13 +14,17 @@ namespace gev {
 // Lines (x passes) or kx-columns (y, z passes) per CTA, and the registers per
 // thread (FP32; twice that in FP64) that set the resident CTAs, from sweeps at
 // 128^3 to 512^3 (FP32) and 256^3 (FP64).
-constexpr int PASS_TX = 8, PASS_TY = 16, PASS_TZ1 = 8, PASS_TZ6 = 8, PASS_TIJ = 4, PASS_TIJ_G = 4, PASS_GZ = 3;
+constexpr int PASS_TX = 8, PASS_TY = 16, PASS_TZ1 = 8, PASS_TIJ = 4, PASS_TIJ_G = 4, PASS_GZ = 3;
 constexpr int REGS_X = 72, REGS_Y = 96;
 template <class R> constexpr int REGS_TIJ = sizeof(R) == 4 ? 72 : 96;
 template <class R> constexpr int REGS_Z1 = sizeof(R) == 4 ? 72 : 96;
 // The tensor solve holds six components in FP64 and moves 24 values of tensor
-// state per mode: eight columns make its rows 64-byte segments (256^3 mixed,
-// parabolic B_i and h_ij: cycle 4075 us with four columns, 3936 with eight).
+// state per mode: eight columns make its rows 64-byte segments.  Chi solves
+// with parabolic B_i and h_ij, eight against four columns (FP64: four against
+// two): 256^3 1523 and 1696 us, FP64 2655 and 2780; 384^3 5.20 and 6.68 ms;
+// 512^3 12.5 and 15.7 ms.  At 768 the six lines of eight columns (307,200
+// bytes) are beyond a block's shared memory: four columns, 58.6 ms.
+template <int N> constexpr int PASS_TZ6 = N <= 512 ? 8 : 4;
 constexpr int REGS_Z6 = 168;
 // three components: eight columns while a thread's values leave the registers
 // for it (256^3: 180 against 191 us with four), four columns beyond
@@ -35,9 +40,19 @@ template <class R> constexpr int resident(int nt, int regs)
     return b < 1 ? 1 : (b > 32 ? 32 : b);
 }
 
-template <class K> inline void set_smem(K kernel, size_t bytes)
+// dynamic shared memory that every block here may ask for: the 227 KB of a
+// block less 1 KB for the kernels' static arrays
+constexpr size_t BLOCK_SMEM = 226 * 1024;
+
+template <size_t BYTES, class K> inline void set_smem(K kernel)
 {
-    if (bytes > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    static_assert(BYTES <= BLOCK_SMEM, "more shared memory than a block may have");
+    if (BYTES <= 48 * 1024) return;
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BYTES);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        throw std::runtime_error(std::string("shared memory limit: ") + cudaGetErrorString(e));
+    }
 }
 
 #define GEV_SWITCH_N(N, CALL)                          \
@@ -61,9 +76,9 @@ void fx_fwd_n(const FxArgs<R> &a, int ncomp, int64_t in_stride, int64_t out_stri
 {
     using C = typename CT<R>::C;
     constexpr int T = PASS_TX, NT = RegPlan<N / 2>::R2 * T;
-    size_t smem = (size_t)T * exch_size<N / 2, 1>() * sizeof(C);
+    constexpr size_t smem = (size_t)T * exch_size<N / 2, 1>() * sizeof(C);
     auto k = k_fx_fwd<R, N, T, MODE, resident<R>(NT, regs_for<R, N / 2>(REGS_X))>;
-    set_smem(k, smem);
+    set_smem<smem>(k);
     pdl_launch(k, dim3(N / T, N, ncomp), NT, smem, st, a, in_stride, out_stride, tb.tw_half, tb.tw_full);
 }
 
@@ -72,9 +87,9 @@ void fx_tij6_n(const FxArgs<R> &a, int64_t in_stride, int64_t out_stride, const 
 {
     using C = typename CT<R>::C;
     constexpr int T = cols<R>(PASS_TIJ), G = PASS_TIJ_G, NT = RegPlan<N / 2>::R2 * T * G;
-    size_t smem = (size_t)6 * T * exch_size<N / 2, 1>() * sizeof(C);
+    constexpr size_t smem = (size_t)6 * T * exch_size<N / 2, 1>() * sizeof(C);
     auto k = k_fx_fwd_tij6<R, N, T, G, resident<R>(NT, regs_for<R, N / 2>(REGS_TIJ<R>))>;
-    set_smem(k, smem);
+    set_smem<smem>(k);
     pdl_launch(k, dim3(N / T, N), NT, smem, st, a.in, in_stride, a.phi, a.c, a.out, out_stride, tb.tw_half, tb.tw_full);
 }
 
@@ -87,7 +102,7 @@ void plane_fwd_n(const FxArgs<R> &a, int ncomp, int64_t in_stride, int64_t out_s
     using C = typename CT<R>::C;
     constexpr size_t smem = (size_t)PlaneShape<N>::VALUES * sizeof(C);
     auto k = k_plane_fwd<R, N, MODE>;
-    set_smem(k, smem);
+    set_smem<smem>(k);
     pdl_launch(k, dim3(N, ncomp), PlaneShape<N>::NT, smem, st, a, in_stride, out_stride, tb.tw_half, tb.tw_full);
 }
 
@@ -96,9 +111,9 @@ void fy_n(typename CT<R>::C *data, int64_t stride, int ncomp, const FftTables<R>
 {
     using C = typename CT<R>::C;
     constexpr int T = cols<R>(PASS_TY), NT = RegPlan<N>::R2 * T;
-    const size_t smem = (size_t)exch_size<N, T>() * sizeof(C);
+    constexpr size_t smem = (size_t)exch_size<N, T>() * sizeof(C);
     auto k = k_fy<R, N, T, S, resident<R>(NT, regs_for<R, N>(REGS_Y))>;
-    set_smem(k, smem);
+    set_smem<smem>(k);
     pdl_launch(k, dim3((N / 2 + 1 + T - 1) / T, N, ncomp), NT, smem, st, data, stride, tb.tw_full);
 }
 
@@ -140,9 +155,9 @@ void fxi_n(const typename CT<R>::C *in, int64_t in_stride, R *out, int64_t out_s
 {
     using C = typename CT<R>::C;
     constexpr int T = PASS_TX, NT = RegPlan<N / 2>::R2 * T;
-    size_t smem = (size_t)T * exch_size<N / 2, 1>() * sizeof(C);
+    constexpr size_t smem = (size_t)T * exch_size<N / 2, 1>() * sizeof(C);
     auto k = k_fx_inv<R, N, T, resident<R>(NT, regs_for<R, N / 2>(REGS_X))>;
-    set_smem(k, smem);
+    set_smem<smem>(k);
     pdl_launch(k, dim3(N / T, N, ncomp), NT, smem, st, in, in_stride, out, out_stride, tb.tw_half, tb.tw_full);
 }
 
@@ -154,7 +169,7 @@ int fyx_inv_n(typename CT<R>::C *in, int64_t in_stride, R *out, int64_t out_stri
     if constexpr (plane_pass<N>()) {
         constexpr size_t smem = (size_t)PlaneShape<N>::VALUES * sizeof(C);
         auto k = k_plane_inv<R, N>;
-        set_smem(k, smem);
+        set_smem<smem>(k);
         pdl_launch(k, dim3(N, ncomp), PlaneShape<N>::NT, smem, st, in, in_stride, out, out_stride, tb.tw_half, tb.tw_full);
         return 1;
     } else {
@@ -197,19 +212,19 @@ void fz_n(const FzArgs<R> &a, const FftTables<R> &tb, cudaStream_t st)
         // a 128-byte boundary, and cost no resident CTA
         constexpr bool PAD = pad_helps<T, C>() && ((N + N / 8) * T * sizeof(C)) % 128 == 0 &&
                              smem_ctas(padded) >= std::min(FZ_STAGED_MINB, smem_ctas(dense));
-        const size_t smem = PAD ? padded : dense;
+        constexpr size_t smem = PAD ? padded : dense;
         const CUtensorMap map = fourier_tensor_map<R>(a.data, N, a.stride, S::CMAX, T, 1, ZBox<N>::ZB);
         auto k = k_fz_tma<R, N, T, NT, OP, EXTRA, PAD>;
-        set_smem(k, smem);
+        set_smem<smem>(k);
         pdl_launch(k, dim3((N / 2 + 1 + T - 1) / T, N), NT, smem, st, a, tb.tw_full, map);
     } else {
         constexpr int CT1 = S::CONTRACT ? 3 : S::CIN, G = CT1 > 1 ? PASS_GZ : 1, R2 = RegPlan<N>::R2;
-        constexpr int T0 = cols<R>(CT1 == 1 ? PASS_TZ1 : (CT1 == 3 ? PASS_TZ3<N> : PASS_TZ6));
+        constexpr int T0 = cols<R>(CT1 == 1 ? PASS_TZ1 : (CT1 == 3 ? PASS_TZ3<N> : PASS_TZ6<N>));
         constexpr int T = OP == OP_BIN && R2 * T0 < 32 ? 32 / R2 : T0, NT = R2 * T * G;   // OP_BIN works in whole warps
-        const size_t smem = (size_t)S::CBUF * exch_size<N, T>() * sizeof(C);
+        constexpr size_t smem = (size_t)S::CBUF * exch_size<N, T>() * sizeof(C);
         constexpr int REGS = CT1 == 6 ? REGS_Z6 : (CT1 == 3 ? REGS_Z3<N> : REGS_Z1<R>);
         auto k = k_fz<R, N, T, G, OP, EXTRA, resident<R>(NT, regs_for<R, N>(REGS))>;
-        set_smem(k, smem);
+        set_smem<smem>(k);
         pdl_launch(k, dim3((N / 2 + 1 + T - 1) / T, N), NT, smem, st, a, tb.tw_full);
     }
 }

@@ -1,9 +1,10 @@
 """GPU parity of the Fourier solves at production grid sizes.
 
-The kernels that the 512^3 cycle runs are specialised per N: the y and z
-passes load their pencils as one bulk tensor box up to N = 256 and as several
-boxes beyond (N = 384: three boxes of 128; N = 512: two of 256; N = 768: three
-of 256), and every N has its own twiddle tables and radix sequence.  These
+The kernels that the 512^3 cycle runs are specialised per N: the transforms'
+radices, rows and columns per block and twiddle tables, and the z pass, which
+in FP32 loads its pencils by bulk tensor boxes for some solves (one box up to
+N = 256; N = 384: three boxes of 128; N = 512: two of 256; N = 768: three of
+256) and through registers for the others.  These
 tests compare each solve with an independent FP64 reference at those sizes:
 pocketfft (scipy.fft, the same transform numpy uses, pinned to the oracle's
 FFT in test_oracle_pin.py) for the transforms and the oracle's C restatements
@@ -77,7 +78,7 @@ def test_solve_phi_sizes(N):
 
 
 def test_solve_phi_768_mixed():
-    """The 768^3 z and y passes (three bulk tensor boxes of 256 per pencil) in
+    """The 768^3 passes (z: three bulk tensor boxes of 256 per pencil) in
     mixed precision, without prepareFTsource: R2C, solveModifiedPoissonFT with
     a screening term, C2R."""
     N = 768
@@ -147,13 +148,65 @@ def test_solve_B_sizes(N):
         FT[k] = rfft3(T0i[k * n3:(k + 1) * n3], N)
     coeff = FOURPIG * dx * dx
     o.project_vector(N, ptr(FT), ptr(FT), coeff, 0.0)
-    B_ref = np.concatenate([irfft3(FT[k], N) for k in range(3)])
+    B_ref = np.concatenate@pytest.mark.parametrize("tensor,parabolic", [(True, False), (False, True)])irfft3(FT[k], N) for k in range(3)])
     del FT
     for prec in PRECS:
         with ctx(N, prec) as c:
             c.set_field(gev.FIELD_BI, T0i)
             c.solve_B(coeff)
             assert rel_err(c.get_field(gev.FIELD_BI).ravel(), B_ref) < TOL[prec], prec
+
+
+@pytest.mark.parametrize("tensor,parabolic", [(True, False), (False, True)])
+def test_solve_chi_extras_768_mixed(tensor, parabolic):
+    """h_ij and parabolic B_i on the largest grid.  The sources are a 256^3
+    white-noise box repeated three times along each axis: its modes are the
+    multiples of three of the 768^3 grid, where every k of the lattice is three
+    times that of the small grid.  With the time step a third, the Hubble rate
+    three times and a^2 dtau a ninth, chi, B_i and h_ij are those of the small
+    box, and h_ij vanishes at all other modes; the small box is the oracle's.
+    h_ij goes through both cycles: projectFTtensor, then evolveFTtensor."""
+    n, N = 256, 768
+    o = oracle()
+    n3 = n ** 3
+    Tij = noise(n, 150, 1e-3, 6)
+    phi = noise(n, 151, 1e-5)
+    coeff, hubble, dtau, dtau_old, a2dtau = 1e-3, 0.9, 0.01, 0.012, 0.3
+    S = np.zeros(6 * n3)
+    o.prepare_Tij(n, ptr(phi), ptr(Tij), coeff, ptr(S))
+    SFT = np.stack@pytest.mark.parametrize("tensor,parabolic", [(True, False), (False, True)])rfft3(S[k * n3:(k + 1) * n3], n) for k in range(6)])
+    G = np.zeros((n, n, n // 2 + 1), dtype=np.complex128)
+    o.project_scalar(n, ptr(SFT), ptr(G), 0)
+    chi_ref = irfft3(G, n)
+    B = np.zeros((3, n, n, n // 2 + 1), dtype=np.complex128)
+    o.evolve_vector(n, ptr(SFT), ptr(B), a2dtau)
+    B_ref = [irfft3(B[k], n) for k in range(3)]
+    h = np.zeros_like(SFT)
+    hp = np.zeros_like(SFT)
+    o.project_tensor(n, ptr(SFT), ptr(h))
+    o.evolve_tensor(n, ptr(SFT), ptr(h), ptr(hp), hubble, dtau, dtau_old)
+    tile = lambda f: np.tile(f.reshape(-1, n, n, n), (1, 3, 3, 3)).ravel()  # noqa: E731
+    kw = dict(tensor=tensor, vector_method=gev.VECTOR_PARABOLIC if parabolic else gev.VECTOR_ELLIPTIC)
+    with ctx(N, gev.MIXED, **kw) as c:
+        c.set_field(gev.FIELD_PHI, tile(phi))
+        tiled = tile(Tij)
+        for cycle0 in (True, False):
+            c.set_field(gev.FIELD_SIJ, tiled)
+            c.solve_chi(coeff, cycle0=cycle0, hubble=3 * hubble, dtau=dtau / 3, dtau_old=dtau_old / 3,
+                        a2dtau=0.0 if cycle0 else a2dtau / 9)
+        del tiled
+        assert rel_err(c.get_field(gev.FIELD_CHI), tile(chi_ref)) < TOL[gev.MIXED]
+        if parabolic:
+            got = c.get_field(gev.FIELD_BI)
+            for k in range(3):
+                assert rel_err(got[k], tile(B_ref[k])) < TOL[gev.MIXED], k
+            del got
+        if tensor:
+            got = c.get_field(gev.FIELD_HIJ_FT)
+            sub = got[:, ::3, ::3, ::3]
+            assert rel_err(sub, h) < TOL[gev.MIXED]
+            sub[...] = 0.0
+            assert max(np.abs(g).max() for g in got) < TOL[gev.MIXED] * np.abs(h).max()
 
 
 @pytest.mark.parametrize("N,bound", [(128, 2.487e-7), (256, 2.715e-7), (384, 3.054e-7), (512, 2.860e-7), (768, 3.138e-7)])

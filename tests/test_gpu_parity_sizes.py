@@ -148,7 +148,7 @@ def test_solve_B_sizes(N):
         FT[k] = rfft3(T0i[k * n3:(k + 1) * n3], N)
     coeff = FOURPIG * dx * dx
     o.project_vector(N, ptr(FT), ptr(FT), coeff, 0.0)
-    B_ref = np.concatenate@pytest.mark.parametrize("tensor,parabolic", [(True, False), (False, True)])irfft3(FT[k], N) for k in range(3)])
+    B_ref = np.concatenate([irfft3(FT[k], N) for k in range(3)])
     del FT
     for prec in PRECS:
         with ctx(N, prec) as c:
@@ -174,7 +174,7 @@ def test_solve_chi_extras_768_mixed(tensor, parabolic):
     coeff, hubble, dtau, dtau_old, a2dtau = 1e-3, 0.9, 0.01, 0.012, 0.3
     S = np.zeros(6 * n3)
     o.prepare_Tij(n, ptr(phi), ptr(Tij), coeff, ptr(S))
-    SFT = np.stack@pytest.mark.parametrize("tensor,parabolic", [(True, False), (False, True)])rfft3(S[k * n3:(k + 1) * n3], n) for k in range(6)])
+    SFT = np.stack([rfft3(S[k * n3:(k + 1) * n3], n) for k in range(6)])
     G = np.zeros((n, n, n // 2 + 1), dtype=np.complex128)
     o.project_scalar(n, ptr(SFT), ptr(G), 0)
     chi_ref = irfft3(G, n)

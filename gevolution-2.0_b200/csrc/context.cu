@@ -359,7 +359,7 @@ template <class R> struct Ctx final : CtxBase {
         ck(cudaMemcpy(ks.p, hks.data(), N * sizeof(double2), cudaMemcpyHostToDevice), "tables");
     }
 
-    FftTables<R> tables() const { return FftTables<R>{tw_full.p, tw_half.p, k2.p, ks.p}; }
+    FftTables<R> tables() const { return FftTables<R>{tw_full.p, tw_half.p, k2.p, ks.p, derr}; }
 
     void make_tables64()
     {
@@ -1079,7 +1079,7 @@ template <class R> struct Ctx final : CtxBase {
             launched("CIC density (FP64)");
             launch_f64_to_f32(rho64.p, g.n3, reinterpret_cast<float *>(source.p), st);
             launched("density to FP32");
-            const FftTables<double> tb{tw64_full.p, tw64_half.p, k2.p, ks.p};
+            const FftTables<double> tb{tw64_full.p, tw64_half.p, k2.p, ks.p, derr};
             double2 *W64 = reinterpret_cast<double2 *>(W.p);   // W holds 6 FP32 components = 3 FP64 ones
             launched("forward x, y passes", fxy_forward<double>(N, FX_COPY, rho64.p, g.n3, 1, nullptr, nullptr, 0, 0, 0, 0, W64, g.nk, nullptr, tb, st));
             fz_pass<double>(N, fp, W64, g.nk, nullptr, nullptr, nullptr, tb, st);

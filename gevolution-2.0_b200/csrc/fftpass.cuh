@@ -1121,24 +1121,36 @@ __global__ void __launch_bounds__(RegPlan<N>::R2 *T *G, MINB) k_fz(FzArgs<R> a, 
 // the CTA transforms, solves and inverse-transforms them, and the results
 // leave by bulk tensor stores.  Columns kx >= P of the last CTA are zero-filled
 // on load and clipped on store.  Same arithmetic as k_fz, with block-wide
-// Stockham passes (fft.cuh): for FP32 lines of 512 and more, whose two-step
-// transform needs 32 values per thread and leaves too few warps to hide its
-// latency (512^3: 455 / 1425 / 1196 us for the Poisson, scalar and vector
-// passes here, 556 / 2100 / 1731 us by k_fz), and for the contracted scalar
-// pass from 256 on (187 against 222 us at 256^3), whose six input components
-// the bulk copies bring without holding registers.
+// Stockham passes (fft.cuh).  Taken (z_staged) where it is the faster of the
+// two, which is where the two-step form holds too many registers for the
+// warps that would hide its latency; us here / by k_fz:
+//   FP32 contracted scalar   256: 187 / 222      512: 1425 / 2100
+//   FP32 vector              256: 202 / 180      384: 726 / 686     512: 1196 / 1731
+//   FP32 Poisson             256: 72 / 60        384: 246 / 272     512: 455 / 556
+//   FP32 displacement        128: 40 / 41        256: 239 / 336     512: 1594 / 3666
+//   FP64 contracted scalar   256: 471 / 334      384: 1941 / 1452   512: 3811 / 6495   768: 20.8 / 15.6 ms
+//   FP64 vector              384: 2329 / 1192    768: 25.1 / 13.7 ms
+//   FP64 Poisson             256: 126 / 104      384: 397 / 482     512: 801 / 1120    768: 3.0 / 5.0 ms
+//   FP64 displacement        128: 84 / 68        256: 452 / 537     384: 1747 / 3639   512: 3612 / 6962
+// The scalar solve with h_ij or parabolic B_i and the binning are k_fz's.
 template <int N> struct ZBox {
     static constexpr int ZB = N <= 256 ? N : (N % 256 == 0 ? 256 : 128);
     static constexpr int NZB = N / ZB;
 };
 
-// resident CTAs of 256 threads the staged z pass is compiled for
-constexpr int FZ_STAGED_MINB = 4;
+// resident CTAs of 256 threads the staged z pass is compiled for.  FP64: three
+// where a thread's share of the lines is larger than one butterfly (the
+// Poisson pass at 512: 801 us with three, 1664 with four, which spill), four
+// otherwise (the scalar pass at 512: 4434 us with three, 3811 with four).
+template <class R, int N, int OP, int EXTRA> constexpr int fz_staged_minb()
+{
+    return sizeof(R) == 8 && (OpShape<OP, EXTRA>::CMAX == 1 || N > 512) ? 3 : 4;
+}
 
 // PAD: the transforms use padded rows (fft.cuh), each component buffer then
 // holds N + N / 8 rows of T values
-template <class R, int N, int T, int NT, int OP, int EXTRA, bool PAD>
-__global__ void __launch_bounds__(NT, FZ_STAGED_MINB * 256 / NT)
+template <class R, int N, int T, int NT, int OP, int EXTRA, bool PAD, int MINB>
+__global__ void __launch_bounds__(NT, MINB)
     k_fz_tma(FzArgs<R> a, const typename CT<R>::C *__restrict__ tw, const __grid_constant__ CUtensorMap tmap)
 {
     pdl_entry();
@@ -1291,6 +1303,48 @@ __global__ void __launch_bounds__(RegPlan<N>::R2 *T, MINB) k_fy(typename CT<R>::
 #pragma unroll
             for (int p = 0; p < R2; p++) d[PP * (q + R1 * p)] = v[p];
         }
+    }
+}
+
+// y pass with bulk-tensor-copy staging, the same grid and Stockham passes in
+// shared memory: for the FP64 lines of 512, whose two-step form holds 32
+// values per thread and two blocks of 128 threads per SM (six components
+// forward 1517 us by k_fy, 1304 here; one back 734 and 661; with half or twice
+// the columns k_fy takes 1480 and 1662).  Elsewhere k_fy is the faster one
+// (FP64 256: 139 against 224 us, 384: 505 and 637, 768: 6.1 and 6.6 ms; FP32
+// 512: 691 and 710 us).
+constexpr int FY_STAGED_NT = 512;
+
+template <class R, int N, int T, int S>
+__global__ void __launch_bounds__(FY_STAGED_NT, 2) k_fy_tma(const typename CT<R>::C *__restrict__ tw, int *err,
+                                                            const __grid_constant__ CUtensorMap tmap)
+{
+    pdl_entry();
+    using C = typename CT<R>::C;
+    constexpr int YB = ZBox<N>::ZB, NYB = ZBox<N>::NZB;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    C *buf = reinterpret_cast<C *>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~(uintptr_t)127);
+    __shared__ __align__(8) uint64_t bar;
+    const int kx0 = blockIdx.x * T, z = blockIdx.y, comp = blockIdx.z;
+    if (threadIdx.x == 0) mbar_init(&bar, 1);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        mbar_expect_tx(&bar, (uint32_t)(N * T * sizeof(C)));
+#pragma unroll 1
+        for (int yc = 0; yc < NYB; yc++) tma_load_4d(buf + yc * YB * T, &tmap, 2 * kx0, yc * YB, z, comp, &bar);
+    }
+    const bool ok = mbar_wait(&bar, 0);
+    if (__syncthreads_or(!ok)) {   // the data never arrived: leave the array untouched and say so
+        if (threadIdx.x == 0 && err) atomicOr(err, ERR_TMA_TIMEOUT);
+        return;
+    }
+    fft_lines<N, S, T, FY_STAGED_NT>(buf, T, tw);
+    fence_async_smem();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+#pragma unroll 1
+        for (int yc = 0; yc < NYB; yc++) tma_store_4d(&tmap, 2 * kx0, yc * YB, z, comp, buf + yc * YB * T);
+        tma_store_drain();
     }
 }
 

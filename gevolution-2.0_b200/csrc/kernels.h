@@ -71,6 +71,7 @@ template <class R> struct FftTables {
     const typename CT<R>::C *tw_half;   // exp(-2 pi i k / (N/2)), k < N/2
     const double *k2;                   // gridk2
     const double2 *ks;                  // kshift
+    int *err = nullptr;                 // device error word for the transfer timeout of the y pass (may be null)
 };
 
 // x and y transforms, forward (mode: FX_*, the source preparation fused into

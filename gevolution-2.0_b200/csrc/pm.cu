@@ -431,7 +431,7 @@ template <class R> struct Pm final : PmBase {
     }
     cudaStream_t stream() override { return st; }
 
-    // after a synchronisation: a bulk tensor copy of a z pass that timed out
+    // after a synchronisation: a bulk tensor copy of a y or z pass that timed out
     // leaves its pencils untransformed and sets the error word
     void check_device(const char *what)
     {
@@ -445,7 +445,7 @@ template <class R> struct Pm final : PmBase {
 
     unsigned pgrid() const { return (unsigned)std::min<int64_t>((np + PM_NT - 1) / PM_NT, 148 * 16); }
     unsigned fgrid() const { return (unsigned)std::min<int64_t>((n3 + PM_NT - 1) / PM_NT, 148 * 16); }
-    FftTables<R> tables() const { return FftTables<R>{twf.p, twh.p, k2.p, ks.p}; }
+    FftTables<R> tables() const { return FftTables<R>{twf.p, twh.p, k2.p, ks.p, derr.p}; }
 
     // out <- Poisson(in) with coefficient pc (modif 0): the pass sequence of gev_solve_phi
     // (clear: `in`, another array, is left zero)

@@ -70,6 +70,12 @@ template <size_t BYTES, class K> inline void set_smem(K kernel)
 
 template <class R> constexpr int cols(int t) { return sizeof(R) == 8 ? t / 2 : t; }
 template <class R, int L> constexpr int regs_for(int regs) { return RegPlan<L>::R1 >= 24 ? regs + 32 : regs; }
+// forward x passes.  The T00 source in FP32 waits for its seven loads per pair
+// and wants warps more than registers (768^3: 3.58 ms with 104, 3.06 with 80)
+template <class R, int N, int MODE> constexpr int regs_fx()
+{
+    return MODE == FX_PREP_T00 && sizeof(R) == 4 && RegPlan<N / 2>::R1 >= 24 ? 80 : regs_for<R, N / 2>(REGS_X);
+}
 
 template <class R, int N, int MODE>
 void fx_fwd_n(const FxArgs<R> &a, int ncomp, int64_t in_stride, int64_t out_stride, const FftTables<R> &tb, cudaStream_t st)
@@ -77,7 +83,7 @@ void fx_fwd_n(const FxArgs<R> &a, int ncomp, int64_t in_stride, int64_t out_stri
     using C = typename CT<R>::C;
     constexpr int T = PASS_TX, NT = RegPlan<N / 2>::R2 * T;
     constexpr size_t smem = (size_t)T * exch_size<N / 2, 1>() * sizeof(C);
-    auto k = k_fx_fwd<R, N, T, MODE, resident<R>(NT, regs_for<R, N / 2>(REGS_X))>;
+    auto k = k_fx_fwd<R, N, T, MODE, resident<R>(NT, regs_fx<R, N, MODE>())>;
     set_smem<smem>(k);
     pdl_launch(k, dim3(N / T, N, ncomp), NT, smem, st, a, in_stride, out_stride, tb.tw_half, tb.tw_full);
 }
@@ -106,15 +112,28 @@ void plane_fwd_n(const FxArgs<R> &a, int ncomp, int64_t in_stride, int64_t out_s
     pdl_launch(k, dim3(N, ncomp), PlaneShape<N>::NT, smem, st, a, in_stride, out_stride, tb.tw_half, tb.tw_full);
 }
 
+// y pass staged by bulk copies (k_fy_tma) or the two-step one (k_fy)
+template <class R, int N> constexpr bool y_staged() { return sizeof(R) == 8 && N == 512; }
+
 template <class R, int N, int S>
 void fy_n(typename CT<R>::C *data, int64_t stride, int ncomp, const FftTables<R> &tb, cudaStream_t st)
 {
     using C = typename CT<R>::C;
-    constexpr int T = cols<R>(PASS_TY), NT = RegPlan<N>::R2 * T;
-    constexpr size_t smem = (size_t)exch_size<N, T>() * sizeof(C);
-    auto k = k_fy<R, N, T, S, resident<R>(NT, regs_for<R, N>(REGS_Y))>;
-    set_smem<smem>(k);
-    pdl_launch(k, dim3((N / 2 + 1 + T - 1) / T, N, ncomp), NT, smem, st, data, stride, tb.tw_full);
+    constexpr int T = cols<R>(PASS_TY);
+    const dim3 grid((N / 2 + 1 + T - 1) / T, N, ncomp);
+    if constexpr (y_staged<R, N>()) {
+        constexpr size_t smem = (size_t)N * T * sizeof(C) + 128;
+        const CUtensorMap map = fourier_tensor_map<R>(data, N, stride, ncomp, T, ZBox<N>::ZB, 1);
+        auto k = k_fy_tma<R, N, T, S>;
+        set_smem<smem>(k);
+        pdl_launch(k, grid, FY_STAGED_NT, smem, st, tb.tw_full, tb.err, map);
+    } else {
+        constexpr int NT = RegPlan<N>::R2 * T;
+        constexpr size_t smem = (size_t)exch_size<N, T>() * sizeof(C);
+        auto k = k_fy<R, N, T, S, resident<R>(NT, regs_for<R, N>(REGS_Y))>;
+        set_smem<smem>(k);
+        pdl_launch(k, grid, NT, smem, st, data, stride, tb.tw_full);
+    }
 }
 
 template <class R, int N, int MODE>
@@ -191,12 +210,16 @@ int fyx_inverse(int N, typename CT<R>::C *in, int64_t in_stride, R *out, int64_t
 // CTAs of `bytes` dynamic shared memory that fit one SM (228 KB, 1 KB reserved per CTA)
 constexpr int smem_ctas(size_t bytes) { return (int)(233472 / (bytes + 1024)); }
 
-// z pass staged by bulk copies (k_fz_tma) or the two-step one (k_fz); measured
-// line between them in k_fz_tma's comment
+// z pass staged by bulk copies (k_fz_tma) or the two-step one (k_fz); the
+// measured lines between them are in k_fz_tma's comment
 template <class R, int N, int OP, int EXTRA> constexpr bool z_staged()
 {
-    return sizeof(R) == 4 && OP != OP_BIN && OP != OP_ZELD && !(OP == OP_SCALAR && EXTRA != 0) &&
-           (N >= 512 || (N >= 256 && OpShape<OP, EXTRA>::CONTRACT));
+    using S = OpShape<OP, EXTRA>;
+    if (OP == OP_BIN || (OP == OP_SCALAR && !S::CONTRACT)) return false;
+    if (OP == OP_ZELD) return N >= 256;
+    if (S::CMAX == 1) return N >= 384;
+    if (sizeof(R) == 8) return N == 512 && S::CONTRACT;
+    return N >= 512 || (N >= 256 && S::CONTRACT);
 }
 
 template <class R, int N, int OP, int EXTRA>
@@ -205,16 +228,16 @@ void fz_n(const FzArgs<R> &a, const FftTables<R> &tb, cudaStream_t st)
     using C = typename CT<R>::C;
     using S = OpShape<OP, EXTRA>;
     if constexpr (z_staged<R, N, OP, EXTRA>()) {
-        constexpr int T = S::CMAX == 1 ? 8 : 4, NT = 256;
+        constexpr int T = S::CMAX == 1 ? cols<R>(8) : 4, NT = 256, MINB = fz_staged_minb<R, N, OP, EXTRA>();
         constexpr size_t dense = (size_t)S::CTMA * N * T * sizeof(C) + 128;
         constexpr size_t padded = (size_t)S::CTMA * (N + N / 8) * T * sizeof(C) + 128;
         // padded rows where they spread the banks, keep every component buffer on
         // a 128-byte boundary, and cost no resident CTA
         constexpr bool PAD = pad_helps<T, C>() && ((N + N / 8) * T * sizeof(C)) % 128 == 0 &&
-                             smem_ctas(padded) >= std::min(FZ_STAGED_MINB, smem_ctas(dense));
+                             smem_ctas(padded) >= std::min(MINB, smem_ctas(dense));
         constexpr size_t smem = PAD ? padded : dense;
         const CUtensorMap map = fourier_tensor_map<R>(a.data, N, a.stride, S::CMAX, T, 1, ZBox<N>::ZB);
-        auto k = k_fz_tma<R, N, T, NT, OP, EXTRA, PAD>;
+        auto k = k_fz_tma<R, N, T, NT, OP, EXTRA, PAD, MINB>;
         set_smem<smem>(k);
         pdl_launch(k, dim3((N / 2 + 1 + T - 1) / T, N), NT, smem, st, a, tb.tw_full, map);
     } else {

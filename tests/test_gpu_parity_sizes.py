@@ -223,3 +223,18 @@ def test_transform_rounding_fp32(N, bound):
         d = c.get_field(gev.FIELD_PHI).ravel()
     d += f
     assert np.linalg.norm(d) / np.linalg.norm(f) < 1.002 * bound
+
+
+@pytest.mark.parametrize("N", [256, 384, 512, 768])
+def test_transforms_fp64(N):
+    """The same round trip in FP64, on each side of the sizes from which the z
+    pass (384) and the y pass (512 only) are staged by bulk copies.  A chain of
+    60 butterfly levels rounds by about 60^(1/2) x 1.1e-16; the bound is ten
+    times that."""
+    f = np.random.default_rng(141).standard_normal(N ** 3)
+    with ctx(N, gev.FP64) as c:
+        c.set_field(gev.FIELD_SOURCE, f)
+        c.solve_phi(False, 0.0, 0.0, 0.0, 0.0, 1e22, 1e22)
+        d = c.get_field(gev.FIELD_PHI).ravel()
+    d += f
+    assert np.linalg.norm(d) / np.linalg.norm(f) < 1e-14

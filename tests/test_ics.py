@@ -130,3 +130,22 @@ def test_positions_phi_and_momenta(prec):
     q_ref = np.zeros_like(pos)
     o.initialize_q(N, len(pos), ptr(np.ascontiguousarray(pos)), ptr(q_ref), ptr(phi_ref), A / H / (1.5 * om_a))
     assert rel_err(q, q_ref) < (1e-9 if prec == gev.FP64 else 1e-4)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("prec", [gev.FP64, gev.MIXED])
+@pytest.mark.parametrize("N", [128, 256, 384])
+def test_displacements_of_larger_grids(N, prec):
+    """The displacement solve on each side of the size from which its z pass is
+    staged by bulk copies (256: one box per pencil, 384: three).  Tolerances as
+    above: the displacements are sums of the same power law."""
+    k, pk = _pk_table()
+    w = np.random.default_rng(5).standard_normal(N ** 3)
+    with gev.Context(N, precision=prec, capacity=N ** 3, boxsize=BOX) as c:
+        c.ics_zeldovich(BOX, A, _fourpiG(), OM, OL, k, pk, noise=w)
+        pos, _, ids = c.get_particles()
+    d = np.empty_like(pos)
+    d[ids] = pos
+    d -= _zeldovich_numpy(N, w, k, pk)
+    d -= np.round(d)
+    assert np.abs(d).max() < (1e-12 if prec == gev.FP64 else 2e-6), np.abs(d).max()

@@ -25,13 +25,15 @@ constexpr int KD_W = 11;   // staged extent per axis
 // -- rows of 7, planes of 49 -- follow each other in the banks and the
 // particles of a warp read different ones; three fields of 11 + 1 values share
 // a row, so the padding costs half as much again, not four times (256^3 FP64
-// kick 1056 -> 1002 us).  FP32: dense rows of 11; the same layout halves its
-// bank conflicts as well (50 to 25 million at 256^3) but not its time, which
-// instruction issue bounds (ncu: issue 70 %; 548 and 547 us).
+// kick 1056 -> 1002 us).  FP32: dense rows of 11, in which a thread's staged
+// value keeps its linear index; the same layout halves its bank conflicts as
+// well (50 to 25 million at 256^3) but not its time, which instruction issue
+// bounds (ncu: issue 70 %; 548 and 547 us), and slots of their own for the
+// staging stores cost it 2.5 % (512^3: 5560 -> 5695 us).
 template <class R> struct KdLayout;
 template <> struct KdLayout<float> {
-    static constexpr int PX = KD_W, PZ = KD_W * KD_W, TOTAL = 5 * KD_W * PZ;
-    __host__ __device__ static constexpr int field(int f) { return f * KD_W * PZ; }
+    static constexpr int FIELD = KD_W * KD_W * KD_W, TOTAL = 5 * FIELD;
+    __host__ __device__ static constexpr int field(int f) { return f * FIELD; }
 };
 template <> struct KdLayout<double> {
     static constexpr int PX = 39, PZ = 433, ARRAY = KD_W * PZ, TOTAL = 2 * ARRAY;
@@ -40,7 +42,8 @@ template <> struct KdLayout<double> {
 };
 template <class R> __host__ __device__ constexpr int kd_slot(int rx, int ry, int rz)
 {
-    return (rx + 1) + KdLayout<R>::PX * (ry + 1) + KdLayout<R>::PZ * (rz + 1);
+    if constexpr (sizeof(R) == 4) return (rx + 1) + KD_W * ((ry + 1) + KD_W * (rz + 1));
+    else return (rx + 1) + KdLayout<R>::PX * (ry + 1) + KdLayout<R>::PZ * (rz + 1);
 }
 
 template <class R>
@@ -101,7 +104,7 @@ __global__ void __launch_bounds__(KD_NT, sizeof(R) == 4 ? 4 : 2) k_kick_drift(PV
         constexpr int NS = KD_W * KD_W * KD_W;
         constexpr int PER = (NS + KD_NT - 1) / KD_NT;
         int64_t gi[PER];
-        int so[PER];
+        int so[PER];   // FP64: slot of the staged value (FP32: its linear index)
         R v[PER][5];
 #pragma unroll
         for (int k = 0; k < PER; k++) {
@@ -109,7 +112,7 @@ __global__ void __launch_bounds__(KD_NT, sizeof(R) == 4 ? 4 : 2) k_kick_drift(PV
             const int ii = i < NS ? i : NS - 1;
             const int vx = ii % KD_W - 1, vy = (ii / KD_W) % KD_W - 1, vz = ii / (KD_W * KD_W) - 1;
             gi[k] = sidx(N, wrapi(x0 + vx, N), wrapi(y0 + vy, N), wrapi(z0 + vz, N));
-            so[k] = kd_slot<R>(vx, vy, vz);
+            if constexpr (sizeof(R) == 8) so[k] = kd_slot<R>(vx, vy, vz);
         }
 #pragma unroll
         for (int k = 0; k < PER; k++) {
@@ -125,18 +128,20 @@ __global__ void __launch_bounds__(KD_NT, sizeof(R) == 4 ? 4 : 2) k_kick_drift(PV
         for (int k = 0; k < PER; k++) {
             const int i = threadIdx.x + k * KD_NT;
             if (i < NS) {
-                if (need_phi) sf[KdLayout<R>::field(0) + so[k]] = v[k][0];
-                if (need_chi) sf[KdLayout<R>::field(1) + so[k]] = v[k][1];
+                const int w = sizeof(R) == 8 ? so[k] : i;
+                if (need_phi) sf[KdLayout<R>::field(0) + w] = v[k][0];
+                if (need_chi) sf[KdLayout<R>::field(1) + w] = v[k][1];
                 if (need_B) {
-                    sf[KdLayout<R>::field(2) + so[k]] = v[k][2];
-                    sf[KdLayout<R>::field(3) + so[k]] = v[k][3];
-                    sf[KdLayout<R>::field(4) + so[k]] = v[k][4];
+                    sf[KdLayout<R>::field(2) + w] = v[k][2];
+                    sf[KdLayout<R>::field(3) + w] = v[k][3];
+                    sf[KdLayout<R>::field(4) + w] = v[k][4];
                 }
             }
         }
     }
     __syncthreads();
-    const R *P_ = sf + KdLayout<R>::field(0), *X_ = sf + KdLayout<R>::field(1), *B0 = sf + KdLayout<R>::field(2), *B1 = sf + KdLayout<R>::field(3), *B2 = sf + KdLayout<R>::field(4);
+    const R *P_ = sf + KdLayout<R>::field(0), *X_ = sf + KdLayout<R>::field(1);
+    const R *B0 = sf + KdLayout<R>::field(2), *B1 = sf + KdLayout<R>::field(3), *B2 = sf + KdLayout<R>::field(4);
 
     const uint32_t lo = bstart[8 * tile], hi = bstart[8 * tile + 8];
     R lmax = 0;   // max of q^2 / a^2 (converted to FP64 once, at the end)

@@ -147,17 +147,24 @@ constexpr int ERR_DOMAIN = 32;         // a tabulated function was evaluated out
 // and visible.  No global memory is touched before that wait, so the results
 // are those of plain stream order; what goes is the launch latency between
 // short kernels (about 1 us of 4-5 us per pass on small grids: 64^3 FP64 cycle
-// 206 -> 179 us).  Only launches of up to PDL_BLOCKS blocks, about one wave,
+// 208 -> 176 us).  Only launches of up to PDL_BLOCKS blocks, about one wave,
 // ask for it: early blocks of a large kernel take the place of the kernel
-// before it (256^3 FP64 cycle 6.10 -> 6.53 ms with every launch asking).
+// before it (256^3 FP64 cycle 6.10 -> 6.53 ms with every launch asking).  The
+// larger launches leave the two instructions out as well: in every block of
+// 512^3 they took the re-bin from 2911 to 3022 us and the index scatter from
+// 502 to 546 us.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void pdl_entry()
+constexpr uint64_t PDL_BLOCKS = 1024;
+
+__device__ __forceinline__ void pdl_wait()
 {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
-
-constexpr uint64_t PDL_BLOCKS = 1024;
+__device__ __forceinline__ void pdl_entry()
+{
+    if ((uint64_t)gridDim.x * gridDim.y * gridDim.z <= PDL_BLOCKS) pdl_wait();
+}
 
 template <class... P, class... A>
 inline void pdl_launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A &&...args)

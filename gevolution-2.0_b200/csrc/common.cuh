@@ -153,6 +153,15 @@ constexpr int ERR_DOMAIN = 32;         // a tabulated function was evaluated out
 // larger launches leave the two instructions out as well: in every block of
 // 512^3 they took the re-bin from 2911 to 3022 us and the index scatter from
 // 502 to 546 us.
+//
+// A kernel launched early is already running while the kernels before it write
+// its inputs, so these are not read-only for its lifetime and must not be read
+// through the read-only path (__ldg, or pointers declared const __restrict__):
+// the compiler may move such loads over the wait, and does (a re-bin that read
+// its bucket starts so found particles in wrong cells).  ld<EARLY> reads them
+// by plain loads where the launch can be early and by __ldg where it cannot;
+// kernels that gain nothing from the latter use plain loads throughout.
+// Tables written before any launch are read either way.
 // ---------------------------------------------------------------------------
 constexpr uint64_t PDL_BLOCKS = 1024;
 
@@ -161,9 +170,24 @@ __device__ __forceinline__ void pdl_wait()
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
-__device__ __forceinline__ void pdl_entry()
+// returns whether the launch was an early one
+__device__ __forceinline__ bool pdl_entry()
 {
-    if ((uint64_t)gridDim.x * gridDim.y * gridDim.z <= PDL_BLOCKS) pdl_wait();
+    const bool early = (uint64_t)gridDim.x * gridDim.y * gridDim.z <= PDL_BLOCKS;
+    if (early) pdl_wait();
+    return early;
+}
+// the same for kernels compiled once for each kind of launch
+template <bool EARLY> __device__ __forceinline__ void pdl_entry()
+{
+    if constexpr (EARLY) pdl_wait();
+}
+
+// a load of what an earlier kernel of the stream wrote
+template <bool EARLY = true, class T> __device__ __forceinline__ T ld(const T *p)
+{
+    if constexpr (EARLY) return *p;
+    else return __ldg(p);
 }
 
 template <class... P, class... A>
@@ -180,6 +204,12 @@ inline void pdl_launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
     cfg.attrs = at;
     cfg.numAttrs = (uint64_t)grid.x * grid.y * grid.z <= PDL_BLOCKS ? 1 : 0;
     cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+// of a kernel compiled once for each kind of launch
+template <class... P, class... A>
+inline void pdl_launch(void (*early)(P...), void (*other)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A &&...args)
+{
+    pdl_launch((uint64_t)grid.x * grid.y * grid.z <= PDL_BLOCKS ? early : other, grid, block, smem, st, static_cast<A &&>(args)...);
 }
 
 // kernel launch helper

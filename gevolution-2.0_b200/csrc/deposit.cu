@@ -393,9 +393,9 @@ template <> struct DepMinBlocks<float, DEP_T00_TIJ_S0I> { static constexpr int v
 // each).  The tile launch (DENSE = false) finishes every tile whose reach fits
 // one chunk and appends the others to the work list work[DEP_LIST..] (count
 // in work[0]); the dense-tile launch (DENSE = true) takes them from the list.
-template <class R, int KIND, bool USE_PHI, bool DENSE>
-__device__ __forceinline__ void deposit_tile(int tile, uint32_t *work, const PView<R> &p, const uint32_t *__restrict__ bstart,
-                                             int N, int nt, const R *__restrict__ phi, const DepOut<R> &out, double a,
+template <class R, int KIND, bool USE_PHI, bool DENSE, bool EARLY>
+__device__ __forceinline__ void deposit_tile(int tile, uint32_t *work, const PView<R> &p, const uint32_t *bstart,
+                                             int N, int nt, const R *phi, const DepOut<R> &out, double a,
                                              double m00, double mij, double m0i, int accumulate, int *err, FastDiv fN)
 {
     using S = DepShape<KIND>;
@@ -434,7 +434,7 @@ __device__ __forceinline__ void deposit_tile(int tile, uint32_t *work, const PVi
             int s = t + k * NT;
             if (s < 1000) {
                 int vx = s % 10 - 1, vy = (s / 10) % 10 - 1, vz = s / 100 - 1;
-                pv[k] = __ldg(phi + sidx(N, wrapi(x0 + vx, N), wrapi(y0 + vy, N), wrapi(z0 + vz, N)));
+                pv[k] = ld<EARLY>(phi + sidx(N, wrapi(x0 + vx, N), wrapi(y0 + vy, N), wrapi(z0 + vz, N)));
             }
         }
     }
@@ -442,7 +442,7 @@ __device__ __forceinline__ void deposit_tile(int tile, uint32_t *work, const PVi
     // head of the concatenation) are loaded as well, for the single-chunk path
     constexpr int PP = (CH + NT - 1) / NT;   // particles per thread (two or three)
     RawParticle<R> raw[PP];
-    const uint32_t own_lo = bstart[8 * tile], own_n = bstart[8 * tile + 8] - own_lo;
+    const uint32_t own_lo = ld<EARLY>(bstart + 8 * tile), own_n = ld<EARLY>(bstart + 8 * tile + 8) - own_lo;
 #pragma unroll
     for (int u = 0; u < PP; u++) {
         const int j = t + u * NT;
@@ -452,7 +452,7 @@ __device__ __forceinline__ void deposit_tile(int tile, uint32_t *work, const PVi
     // memory; the barrier below publishes them together with the phi stencil
     // and the per-cell run bounds (no barrier of their own)
     if (t < 32) {
-        const TileSegs ts = tile_segments_warp(bstart, nt, tx, ty, tz);
+        const TileSegs ts = tile_segments_warp<EARLY>(bstart, nt, tx, ty, tz);
         tile_segments_store(ts, seg_lo, seg_hi, seg_pre);
     }
     if (t < NC) vmax[t] = 0ull;
@@ -790,25 +790,25 @@ __device__ __forceinline__ void deposit_tile(int tile, uint32_t *work, const PVi
     }
 }
 
-template <class R, int KIND, bool USE_PHI>
+template <class R, int KIND, bool USE_PHI, bool EARLY>
 __global__ void __launch_bounds__(dep_tile_threads<R>(), DepMinBlocks<R, KIND>::v)
-    k_deposit(PView<R> p, const uint32_t *__restrict__ bstart, int N, int nt, const R *__restrict__ phi, DepOut<R> out,
+    k_deposit(PView<R> p, const uint32_t *bstart, int N, int nt, const R *phi, DepOut<R> out,
               double a, double m00, double mij, double m0i, int accumulate, uint32_t *work, int *err, FastDiv fN)
 {
-    pdl_entry();
-    deposit_tile<R, KIND, USE_PHI, false>((int)blockIdx.x, work, p, bstart, N, nt, phi, out, a, m00, mij, m0i, accumulate,
-                                          err, fN);
+    pdl_entry<EARLY>();
+    deposit_tile<R, KIND, USE_PHI, false, EARLY>((int)blockIdx.x, work, p, bstart, N, nt, phi, out, a, m00, mij, m0i, accumulate,
+                                                 err, fN);
 }
 
 // The dense tiles, one at a time per CTA, each CTA claiming the next listed
 // tile when it is done with one (their costs differ widely).
 template <class R, int KIND, bool USE_PHI>
 __global__ void __launch_bounds__(DEP_NT, GEV_DEP_MINB_DENSE)
-    k_deposit_dense(PView<R> p, const uint32_t *__restrict__ bstart, int N, int nt, const R *__restrict__ phi,
+    k_deposit_dense(PView<R> p, const uint32_t *bstart, int N, int nt, const R *phi,
                     DepOut<R> out, double a, double m00, double mij, double m0i, int accumulate, uint32_t *work, int *err,
                     FastDiv fN)
 {
-    pdl_entry();
+    pdl_entry<true>();   // one wave of blocks
     __shared__ uint32_t next;
     const uint32_t count = work[0];
     for (;;) {
@@ -816,8 +816,8 @@ __global__ void __launch_bounds__(DEP_NT, GEV_DEP_MINB_DENSE)
         __syncthreads();
         const uint32_t i = next;
         if (i >= count) break;
-        deposit_tile<R, KIND, USE_PHI, true>((int)work[DEP_LIST + i], work, p, bstart, N, nt, phi, out, a, m00, mij, m0i,
-                                             accumulate, err, fN);
+        deposit_tile<R, KIND, USE_PHI, true, true>((int)work[DEP_LIST + i], work, p, bstart, N, nt, phi, out, a, m00, mij, m0i,
+                                                   accumulate, err, fN);
         __syncthreads();   // shared memory and `next` are reused for the next tile
     }
     // the last block to get here clears the list for the next deposit
@@ -842,16 +842,19 @@ static void launch_k(const PView<R> &p, const uint32_t *bstart, int N, const R *
                      double m00, double mij, double m0i, int accumulate, uint32_t *work, int *err, cudaStream_t st)
 {
     constexpr size_t smem = dep_smem_bytes<R, KIND>(), smem_dense = dep_smem_bytes<R, KIND, true>();
-    static bool attr_set[SMEM_ATTR_DEVICES] = {}, attr_set_dense[SMEM_ATTR_DEVICES] = {};
-    raise_smem_limit(k_deposit<R, KIND, USE_PHI>, smem, attr_set);
+    static bool attr_set[2][SMEM_ATTR_DEVICES] = {}, attr_set_dense[SMEM_ATTR_DEVICES] = {};
+    raise_smem_limit(k_deposit<R, KIND, USE_PHI, true>, smem, attr_set[0]);
+    raise_smem_limit(k_deposit<R, KIND, USE_PHI, false>, smem, attr_set[1]);
     raise_smem_limit(k_deposit_dense<R, KIND, USE_PHI>, smem_dense, attr_set_dense);
     const int nt = N / 8;
     const unsigned tiles = (unsigned)nt * nt * nt;
     const FastDiv fN((uint32_t)N);
-    pdl_launch(k_deposit<R, KIND, USE_PHI>, tiles, dep_tile_threads<R>(), smem, st, p, bstart, N, nt, phi, out, a, m00, mij, m0i, accumulate, work, err, fN);
+    pdl_launch(k_deposit<R, KIND, USE_PHI, true>, k_deposit<R, KIND, USE_PHI, false>, tiles, dep_tile_threads<R>(), smem, st, p,
+               bstart, N, nt, phi, out, a, m00, mij, m0i, accumulate, work, err, fN);
     // one wave of resident CTAs; those that find the list empty return at once
     const unsigned grid = std::min(tiles, (unsigned)(sm_count() * GEV_DEP_MINB_DENSE));
-    pdl_launch(k_deposit_dense<R, KIND, USE_PHI>, grid, DEP_NT, smem_dense, st, p, bstart, N, nt, phi, out, a, m00, mij, m0i, accumulate, work, err, fN);
+    pdl_launch(k_deposit_dense<R, KIND, USE_PHI>, grid, DEP_NT, smem_dense, st, p, bstart, N, nt, phi, out, a, m00, mij, m0i,
+               accumulate, work, err, fN);
 }
 
 template <class R>

@@ -39,10 +39,14 @@ __device__ __forceinline__ R ldr(const R *f, int N, int x, int y, int z)
     return __ldg(f + sidx(N, wrapi(x, N), wrapi(y, N), wrapi(z, N)));
 }
 
+// grids whose x and y transforms run as plane kernels, launched early
+// (pdl_entry); the pass kernels of the others have more blocks than that
+template <int N> __host__ __device__ constexpr bool plane_pass() { return N <= 128; }
+
 // two adjacent values (x even: 8- or 16-byte aligned) in one load
-template <class R> __device__ __forceinline__ typename CT<R>::C ld_pair(const R *p)
+template <bool EARLY, class R> __device__ __forceinline__ typename CT<R>::C ld_pair(const R *p)
 {
-    return __ldg(reinterpret_cast<const typename CT<R>::C *>(p));
+    return ld<EARLY>(reinterpret_cast<const typename CT<R>::C *>(p));
 }
 
 // prepareFTsource_T00 (gevolution.hpp:160-171) at one point, in FP64: source
@@ -150,6 +154,7 @@ __device__ __forceinline__ void fx_finish(C *smem, const C *__restrict__ tw_full
 template <class R, int N, int MODE, int COMP>
 __device__ __forceinline__ typename CT<R>::C fx_pair(const FxArgs<R> &a, const R *in, int n, int y, int z, double &lsum)
 {
+    constexpr bool E = plane_pass<N>();
     const int x0 = 2 * n;
     if constexpr (MODE == FX_COPY) {
         // a caller's own array (gev_poisson_noalloc) may be aligned to single values only
@@ -160,12 +165,12 @@ __device__ __forceinline__ typename CT<R>::C fx_pair(const FxArgs<R> &a, const R
         const int xm = x0 == 0 ? N - 1 : x0 - 1, x2 = x0 + 2 == N ? 0 : x0 + 2;
         const int ym = y == 0 ? N - 1 : y - 1, yp = y == N - 1 ? 0 : y + 1;
         const int zm = z == 0 ? N - 1 : z - 1, zp = z == N - 1 ? 0 : z + 1;
-        const auto s = ld_pair(in + sidx(N, x0, y, z)), ch = ld_pair(a.chi + sidx(N, x0, y, z));
+        const auto s = ld_pair<E>(in + sidx(N, x0, y, z)), ch = ld_pair<E>(a.chi + sidx(N, x0, y, z));
         const R *row = a.phi + sidx(N, 0, y, z);
-        const auto p0 = ld_pair(row + x0);
-        const R pm = __ldg(row + xm), p2 = __ldg(row + x2);
-        const auto ya = ld_pair(a.phi + sidx(N, x0, ym, z)), yb = ld_pair(a.phi + sidx(N, x0, yp, z));
-        const auto za = ld_pair(a.phi + sidx(N, x0, y, zm)), zb = ld_pair(a.phi + sidx(N, x0, y, zp));
+        const auto p0 = ld_pair<E>(row + x0);
+        const R pm = ld<E>(row + xm), p2 = ld<E>(row + x2);
+        const auto ya = ld_pair<E>(a.phi + sidx(N, x0, ym, z)), yb = ld_pair<E>(a.phi + sidx(N, x0, yp, z));
+        const auto za = ld_pair<E>(a.phi + sidx(N, x0, y, zm)), zb = ld_pair<E>(a.phi + sidx(N, x0, y, zp));
         lsum += (double)s.x + (double)s.y;
         return mk((R)t00_point(a, s.x, p0.x, ch.x, pm, p0.y, ya.x, yb.x, za.x, zb.x),
                   (R)t00_point(a, s.y, p0.y, ch.y, p0.x, p2, ya.y, yb.y, za.y, zb.y));
@@ -173,12 +178,12 @@ __device__ __forceinline__ typename CT<R>::C fx_pair(const FxArgs<R> &a, const R
         // one component of prepareFTsource_Tij (COMP in the order 00,01,02,11,12,22),
         // the expressions of tij6_point
         const R rc = (R)a.c;
-        const auto t = ld_pair(in + sidx(N, x0, y, z));
+        const auto t = ld_pair<E>(in + sidx(N, x0, y, z));
         const int ym = y == 0 ? N - 1 : y - 1, yp = y == N - 1 ? 0 : y + 1;
         const int zm = z == 0 ? N - 1 : z - 1, zp = z == N - 1 ? 0 : z + 1;
         const int xm = x0 == 0 ? N - 1 : x0 - 1, x2 = x0 + 2 == N ? 0 : x0 + 2;
-        auto pair = [&](int yy, int zz) { return ld_pair(a.phi + sidx(N, x0, yy, zz)); };
-        auto one = [&](int x, int yy, int zz) { return __ldg(a.phi + sidx(N, x, yy, zz)); };
+        auto pair = [&](int yy, int zz) { return ld_pair<E>(a.phi + sidx(N, x0, yy, zz)); };
+        auto one = [&](int x, int yy, int zz) { return ld<E>(a.phi + sidx(N, x, yy, zz)); };
         auto diag = [&](R p, R m, R tv) { const R g = p - m; return (R)0.5 * g * g + rc * tv; };
         auto off = [&](R p0, R pi, R pj, R pij, R tv) {
             const R u = pi - p0, v = pj - p0, w = (pij - pi) - (pj - p0);
@@ -205,13 +210,13 @@ __device__ __forceinline__ typename CT<R>::C fx_pair(const FxArgs<R> &a, const R
         // factor of particle_T0i_project (gevolution.hpp:2031-2201), applied once
         // per vertex with the current phi
         static_assert(MODE == FX_PREP_T0I, "mode");
-        const auto s = ld_pair(in + sidx(N, x0, y, z));
+        const auto s = ld_pair<E>(in + sidx(N, x0, y, z));
         const R *row = a.phi + sidx(N, 0, y, z);
-        const auto p0 = ld_pair(row + x0);
+        const auto p0 = ld_pair<E>(row + x0);
         typename CT<R>::C pe;
-        if constexpr (COMP == 0) pe = mk(p0.y, __ldg(row + (x0 + 2 == N ? 0 : x0 + 2)));
-        else if constexpr (COMP == 1) pe = ld_pair(a.phi + sidx(N, x0, y == N - 1 ? 0 : y + 1, z));
-        else pe = ld_pair(a.phi + sidx(N, x0, y, z == N - 1 ? 0 : z + 1));
+        if constexpr (COMP == 0) pe = mk(p0.y, ld<E>(row + (x0 + 2 == N ? 0 : x0 + 2)));
+        else if constexpr (COMP == 1) pe = ld_pair<E>(a.phi + sidx(N, x0, y == N - 1 ? 0 : y + 1, z));
+        else pe = ld_pair<E>(a.phi + sidx(N, x0, y, z == N - 1 ? 0 : z + 1));
         return mk(((R)1 + p0.x + pe.x) * s.x, ((R)1 + p0.y + pe.y) * s.y);
     }
 }
@@ -252,7 +257,7 @@ __global__ void __launch_bounds__(RegPlan<N / 2>::R2 *T, MINB) k_fx_fwd(FxArgs<R
                                                                        const typename CT<R>::C *__restrict__ tw_half,
                                                                        const typename CT<R>::C *__restrict__ tw_full)
 {
-    pdl_entry();
+    pdl_entry<false>();
     using C = typename CT<R>::C;
     constexpr int M = N / 2, PP = N / 2 + 2, R1 = RegPlan<M>::R1, R2 = RegPlan<M>::R2, NT = R2 * T, ES = exch_size<M, 1>();
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -313,7 +318,7 @@ __global__ void __launch_bounds__(RegPlan<N / 2>::R2 *T *G, MINB) k_fx_fwd_tij6(
                                                                               const typename CT<R>::C *__restrict__ tw_half,
                                                                               const typename CT<R>::C *__restrict__ tw_full)
 {
-    pdl_entry();
+    pdl_entry<false>();
     using C = typename CT<R>::C;
     constexpr int M = N / 2, PP = N / 2 + 2, R1 = RegPlan<M>::R1, R2 = RegPlan<M>::R2, NT = R2 * T * G, ES = exch_size<M, 1>();
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -332,14 +337,14 @@ __global__ void __launch_bounds__(RegPlan<N / 2>::R2 *T *G, MINB) k_fx_fwd_tij6(
             // 32-bit offsets (N <= 768): one base register per plane
             auto row = [&](int yy, int zz) { return ((uint32_t)zz * N + (uint32_t)yy) * N; };
             const uint32_t r00 = row(y, z), rp0 = row(yp, z), r0p = row(y, zp);
-            const C c00 = ld_pair(phi + (r00 + x0)), cm0 = ld_pair(phi + (row(ym, z) + x0)), cp0 = ld_pair(phi + (rp0 + x0));
-            const C c0p = ld_pair(phi + (r0p + x0)), c0m = ld_pair(phi + (row(y, zm) + x0)), cpp = ld_pair(phi + (row(yp, zp) + x0));
-            const R f00m = __ldg(phi + (r00 + xm)), f002 = __ldg(phi + (r00 + x2)), fp02 = __ldg(phi + (rp0 + x2)),
-                    f0p2 = __ldg(phi + (r0p + x2));
+            const C c00 = ld_pair<false>(phi + (r00 + x0)), cm0 = ld_pair<false>(phi + (row(ym, z) + x0)), cp0 = ld_pair<false>(phi + (rp0 + x0));
+            const C c0p = ld_pair<false>(phi + (r0p + x0)), c0m = ld_pair<false>(phi + (row(y, zm) + x0)), cpp = ld_pair<false>(phi + (row(yp, zp) + x0));
+            const R f00m = ld<false>(phi + (r00 + xm)), f002 = ld<false>(phi + (r00 + x2)), fp02 = ld<false>(phi + (rp0 + x2)),
+                    f0p2 = ld<false>(phi + (r0p + x2));
             R t0[6], t1[6];
 #pragma unroll
             for (int c = 0; c < 6; c++) {
-                const C tv = ld_pair(Tij + c * n3 + (r00 + x0));
+                const C tv = ld_pair<false>(Tij + c * n3 + (r00 + x0));
                 t0[c] = tv.x;
                 t1[c] = tv.y;
             }
@@ -378,7 +383,7 @@ __global__ void __launch_bounds__(RegPlan<N / 2>::R2 *T, MINB) k_fx_inv(const ty
                                                                        const typename CT<R>::C *__restrict__ tw_half,
                                                                        const typename CT<R>::C *__restrict__ tw_full)
 {
-    pdl_entry();
+    pdl_entry<false>();
     using C = typename CT<R>::C;
     constexpr int M = N / 2, PP = N / 2 + 2, R1 = RegPlan<M>::R1, R2 = RegPlan<M>::R2;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -391,7 +396,7 @@ __global__ void __launch_bounds__(RegPlan<N / 2>::R2 *T, MINB) k_fx_inv(const ty
 #pragma unroll
         for (int r = 0; r < R1; r++) {
             const int k = u + R2 * r;
-            C A = __ldg(row + k), B = __ldg(row + M - k);
+            C A = ld<false>(row + k), B = ld<false>(row + M - k);
             if (k == 0) { A.y = R(0); B.y = R(0); }
             B.y = -B.y;
             C w = __ldg(tw_full + k);
@@ -452,7 +457,7 @@ __global__ void __launch_bounds__(PlaneShape<N>::NT, plane_minb<R, N>()) k_plane
                                                                  const typename CT<R>::C *__restrict__ tw_half,
                                                                  const typename CT<R>::C *__restrict__ tw_full)
 {
-    pdl_entry();
+    pdl_entry<true>();
     using C = typename CT<R>::C;
     using S = PlaneShape<N>;
     constexpr int M = S::M, P = S::P, PP = N / 2 + 2, NT = S::NT;
@@ -551,7 +556,7 @@ __global__ void __launch_bounds__(PlaneShape<N>::NT, plane_minb<R, N>()) k_plane
                                                                  const typename CT<R>::C *__restrict__ tw_half,
                                                                  const typename CT<R>::C *__restrict__ tw_full)
 {
-    pdl_entry();
+    pdl_entry<true>();
     using C = typename CT<R>::C;
     using S = PlaneShape<N>;
     constexpr int M = S::M, P = S::P, PP = N / 2 + 2, NT = S::NT;
@@ -564,7 +569,7 @@ __global__ void __launch_bounds__(PlaneShape<N>::NT, plane_minb<R, N>()) k_plane
         const C *col = in + (int64_t)blockIdx.y * in_stride + (int64_t)PP * N * z + k0;
         C v[YR1];
 #pragma unroll
-        for (int r = 0; r < YR1; r++) v[r] = __ldg(col + PP * (u0 + YR2 * r));
+        for (int r = 0; r < YR1; r++) v[r] = ld(col + PP * (u0 + YR2 * r));
         step1_store<N, 1, P>(v, smem + k0, u0, tw_full);
     }
     __syncthreads();
@@ -741,7 +746,7 @@ __device__ __forceinline__ void fz_apply(const FzArgs<R> &a, int N, int kx, int 
         // transform of the CIC kernel; modes the generator sets to zero stay
         // zero (their numerator is exactly zero).  Complex division as
         // (n ker*) / |ker|^2.
-        const double2 num = __ldg(a.modes + (int64_t)kx + (int64_t)(N / 2 + 1) * ((int64_t)ky + (int64_t)N * kz));
+        const double2 num = ld(a.modes + (int64_t)kx + (int64_t)(N / 2 + 1) * ((int64_t)ky + (int64_t)N * kz));
         if (num.x == 0.0 && num.y == 0.0) {
             v[0] = make_double2(0.0, 0.0);
         } else {
@@ -939,7 +944,8 @@ __device__ __forceinline__ void bin_modes(const FzArgs<R> &a, int N, int kx, int
 template <class R, int N, int T, int G, int OP, int EXTRA, int MINB>
 __global__ void __launch_bounds__(RegPlan<N>::R2 *T *G, MINB) k_fz(FzArgs<R> a, const typename CT<R>::C *__restrict__ tw)
 {
-    pdl_entry();
+    constexpr bool EARLY = (uint64_t)((N / 2 + 1 + T - 1) / T) * N <= PDL_BLOCKS;   // the launch's grid
+    pdl_entry<EARLY>();
     using C = typename CT<R>::C;
     constexpr int P = N / 2 + 1, PP = N / 2 + 2;
     constexpr int R1 = RegPlan<N>::R1, R2 = RegPlan<N>::R2;
@@ -1153,7 +1159,7 @@ template <class R, int N, int T, int NT, int OP, int EXTRA, bool PAD, int MINB>
 __global__ void __launch_bounds__(NT, MINB)
     k_fz_tma(FzArgs<R> a, const typename CT<R>::C *__restrict__ tw, const __grid_constant__ CUtensorMap tmap)
 {
-    pdl_entry();
+    pdl_entry<false>();
     using C = typename CT<R>::C;
     constexpr int P = N / 2 + 1, PP = N / 2 + 2;
     constexpr int CIN = OpShape<OP, EXTRA>::CIN, COUT = OpShape<OP, EXTRA>::COUT;
@@ -1280,7 +1286,7 @@ template <class R, int N, int T, int S, int MINB>
 __global__ void __launch_bounds__(RegPlan<N>::R2 *T, MINB) k_fy(typename CT<R>::C *data, int64_t stride,
                                                                const typename CT<R>::C *__restrict__ tw)
 {
-    pdl_entry();
+    pdl_entry<false>();
     using C = typename CT<R>::C;
     constexpr int P = N / 2 + 1, PP = N / 2 + 2, R1 = RegPlan<N>::R1, R2 = RegPlan<N>::R2;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1319,7 +1325,7 @@ template <class R, int N, int T, int S>
 __global__ void __launch_bounds__(FY_STAGED_NT, 2) k_fy_tma(const typename CT<R>::C *__restrict__ tw, int *err,
                                                             const __grid_constant__ CUtensorMap tmap)
 {
-    pdl_entry();
+    pdl_entry<false>();
     using C = typename CT<R>::C;
     constexpr int YB = ZBox<N>::ZB, NYB = ZBox<N>::NZB;
     extern __shared__ __align__(16) unsigned char smem_raw[];

@@ -61,6 +61,7 @@ struct TileSegs {
     uint32_t total;                  // length of the concatenation
 };
 
+template <bool EARLY>
 __device__ __forceinline__ TileSegs tile_segments_warp(const uint32_t *bstart, int nt, int tx, int ty, int tz)
 {
     const int l = threadIdx.x & 31;
@@ -76,8 +77,8 @@ __device__ __forceinline__ TileSegs tile_segments_warp(const uint32_t *bstart, i
             const int ny = ty - dy < 0 ? nt - 1 : ty - dy;
             const int nz = tz - dz < 0 ? nt - 1 : tz - dz;
             const uint32_t nb = (uint32_t)nx + (uint32_t)nt * ((uint32_t)ny + (uint32_t)nt * (uint32_t)nz);
-            lo = bstart[8 * nb + c];
-            hi = bstart[8 * nb + c + 1];
+            lo = ld<EARLY>(bstart + 8 * nb + c);
+            hi = ld<EARLY>(bstart + 8 * nb + c + 1);
         }
         hi = hi > lo ? hi : lo;
         s.lo[h] = lo;

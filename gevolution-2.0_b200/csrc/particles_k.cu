@@ -80,14 +80,14 @@ __device__ __forceinline__ uint32_t bucket_slot(uint32_t b, uint32_t *counts)
     return base + (uint32_t)__popc(peers & lanemask_lt());
 }
 
-template <class R>
-__global__ void __launch_bounds__(KD_NT, sizeof(R) == 4 ? 4 : 2) k_kick_drift(PView<R> p, const uint32_t *__restrict__ bstart, int N, int nt,
-                                                      const R *__restrict__ phi, const R *__restrict__ chi,
-                                                      const R *__restrict__ Bi, int64_t n3, KickDriftParams kp,
+template <class R, bool EARLY>
+__global__ void __launch_bounds__(KD_NT, sizeof(R) == 4 ? 4 : 2) k_kick_drift(PView<R> p, const uint32_t *bstart, int N, int nt,
+                                                      const R *phi, const R *chi,
+                                                      const R *Bi, int64_t n3, KickDriftParams kp,
                                                       uint32_t *counts, uint32_t *bucket, uint32_t *rank,
                                                       unsigned long long *vmax_bits, int *err, FastDiv fN)
 {
-    pdl_entry();
+    pdl_entry<EARLY>();
     extern __shared__ __align__(16) unsigned char kd_smem[];
     R *sf = reinterpret_cast<R *>(kd_smem);
     __shared__ double wmax[KD_NT / 32];
@@ -116,12 +116,12 @@ __global__ void __launch_bounds__(KD_NT, sizeof(R) == 4 ? 4 : 2) k_kick_drift(PV
         }
 #pragma unroll
         for (int k = 0; k < PER; k++) {
-            if (need_phi) v[k][0] = __ldg(phi + gi[k]);
-            if (need_chi) v[k][1] = __ldg(chi + gi[k]);
+            if (need_phi) v[k][0] = ld<EARLY>(phi + gi[k]);
+            if (need_chi) v[k][1] = ld<EARLY>(chi + gi[k]);
             if (need_B) {
-                v[k][2] = __ldg(Bi + gi[k]);
-                v[k][3] = __ldg(Bi + n3 + gi[k]);
-                v[k][4] = __ldg(Bi + 2 * n3 + gi[k]);
+                v[k][2] = ld<EARLY>(Bi + gi[k]);
+                v[k][3] = ld<EARLY>(Bi + n3 + gi[k]);
+                v[k][4] = ld<EARLY>(Bi + 2 * n3 + gi[k]);
             }
         }
 #pragma unroll
@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(KD_NT, sizeof(R) == 4 ? 4 : 2) k_kick_drift(PV
     const R *P_ = sf + KdLayout<R>::field(0), *X_ = sf + KdLayout<R>::field(1);
     const R *B0 = sf + KdLayout<R>::field(2), *B1 = sf + KdLayout<R>::field(3), *B2 = sf + KdLayout<R>::field(4);
 
-    const uint32_t lo = bstart[8 * tile], hi = bstart[8 * tile + 8];
+    const uint32_t lo = ld<EARLY>(bstart + 8 * tile), hi = ld<EARLY>(bstart + 8 * tile + 8);
     R lmax = 0;   // max of q^2 / a^2 (converted to FP64 once, at the end)
     const R ib_k = (R)(1.0 / kp.b_k), ib_d = (R)(1.0 / kp.b_d);
     const R ia2_k = (R)(1.0 / (kp.a_k * kp.a_k));
@@ -359,9 +359,11 @@ void launch_kick_drift(const PView<R> &p, const uint32_t *bstart, int N, const R
 {
     int nt = N / 8;
     const size_t smem = KdLayout<R>::TOTAL * sizeof(R);
-    static bool attr_set[SMEM_ATTR_DEVICES] = {};
-    raise_smem_limit(k_kick_drift<R>, smem, attr_set);
-    pdl_launch(k_kick_drift<R>, (unsigned)nt * nt * nt, KD_NT, smem, st, p, bstart, N, nt, phi, chi, Bi, n3, kp, counts, bucket, rank, vmax_bits, err, FastDiv((uint32_t)N));
+    static bool attr_set[2][SMEM_ATTR_DEVICES] = {};
+    raise_smem_limit(k_kick_drift<R, true>, smem, attr_set[0]);
+    raise_smem_limit(k_kick_drift<R, false>, smem, attr_set[1]);
+    pdl_launch(k_kick_drift<R, true>, k_kick_drift<R, false>, (unsigned)nt * nt * nt, KD_NT, smem, st, p, bstart, N, nt, phi,
+               chi, Bi, n3, kp, counts, bucket, rank, vmax_bits, err, FastDiv((uint32_t)N));
 }
 
 // ---- particle I/O: host layout (box-unit positions, AoS triples) <-> cell + offset ----
@@ -495,9 +497,9 @@ __global__ void k_scan_add(uint32_t *start, int64_t nb, const uint32_t *block_su
 // thread and round, SCAN_ROUNDS rounds scanned side by side.
 constexpr int SCAN_ROUNDS = 8;
 
-__global__ void __launch_bounds__(SCAN_NT) k_scan_one(const uint32_t *__restrict__ counts, uint32_t *start, int nb)
+__global__ void __launch_bounds__(SCAN_NT) k_scan_one(const uint32_t *counts, uint32_t *start, int nb)
 {
-    pdl_entry();
+    pdl_entry<true>();   // one block
     __shared__ uint32_t wsum[SCAN_ROUNDS][SCAN_NT / 32];
     const int t = threadIdx.x, lane = t & 31, w = t >> 5;
     uint4 v[SCAN_ROUNDS];
@@ -563,14 +565,13 @@ int launch_scan(const uint32_t *counts, uint32_t *start, int64_t nb, uint32_t *b
 
 // ---- re-binning into bucket order, each bucket in (cell, ID) order ----
 // Step 1: every particle's destination j = start[bucket] + slot; inv[j] = i.
-// EARLY: launched by pdl_launch with a grid that asks for it.  A block lives for
-// a microsecond, so even the test of the grid size shows (512^3: 502 us
-// without it, 511 with)
+// A block lives for a microsecond, so even the test of the grid size shows
+// (512^3: 502 us without it, 511 with): one kernel for each kind of launch
 template <bool EARLY>
-__global__ void k_scatter_index(const uint32_t *__restrict__ bstart, const uint32_t *__restrict__ bucket,
-                                const uint32_t *__restrict__ rank, int64_t n, uint32_t *inv)
+__global__ void k_scatter_index(const uint32_t *bstart, const uint32_t *bucket,
+                                const uint32_t *rank, int64_t n, uint32_t *inv)
 {
-    if constexpr (EARLY) pdl_wait();
+    pdl_entry<EARLY>();
     int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
     const uint32_t j = bstart[bucket[i]] + rank[i];
@@ -597,8 +598,8 @@ template <class R> constexpr size_t rb_smem_bytes()
 // 241 us by insertion, 84 us by rank).  A bucket larger than
 // REBIN_SORT_MAX is copied in slot order.
 template <class R>
-__global__ void __launch_bounds__(RB_NT, 3) k_rebin_tile(PView<R> src, PView<R> dst, const uint32_t *__restrict__ bstart,
-                                                      const uint32_t *__restrict__ inv, int nt, int *err, FastDiv fN)
+__global__ void __launch_bounds__(RB_NT, 3) k_rebin_tile(PView<R> src, PView<R> dst, const uint32_t *bstart,
+                                                      const uint32_t *inv, int nt, int *err, FastDiv fN)
 {
     pdl_entry();
     constexpr int M = REBIN_SORT_MAX;
@@ -739,8 +740,7 @@ void launch_rebin(const PView<R> &src, PView<R> dst, const uint32_t *bstart, con
                   const uint32_t *rank, uint32_t *inv, int N, int *err, cudaStream_t st)
 {
     if (src.n <= 0) return;
-    const unsigned nb = cdiv(src.n, 256);
-    pdl_launch(nb <= PDL_BLOCKS ? k_scatter_index<true> : k_scatter_index<false>, nb, 256, 0, st, bstart, bucket, rank, src.n, inv);
+    pdl_launch(k_scatter_index<true>, k_scatter_index<false>, cdiv(src.n, 256), 256, 0, st, bstart, bucket, rank, src.n, inv);
     static bool attr_set[SMEM_ATTR_DEVICES] = {};
     raise_smem_limit(k_rebin_tile<R>, rb_smem_bytes<R>(), attr_set);
     const int nt = N / 8;

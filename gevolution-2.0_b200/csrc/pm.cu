@@ -98,7 +98,7 @@ __device__ __forceinline__ int pm_wrap1(int i, int N) { return i >= N ? i - N : 
 struct Vec3 {
     double v[3];
 };
-__device__ __forceinline__ Vec3 pm_get(const double *__restrict__ p, int64_t np, int64_t i)
+__device__ __forceinline__ Vec3 pm_get(const double *p, int64_t np, int64_t i)
 {
     return Vec3{{p[i], p[np + i], p[2 * np + i]}};
 }
@@ -118,7 +118,7 @@ __global__ void k_pm_planes(const double *__restrict__ in, double *__restrict__ 
         pm_put(out, np, i, v);
     }
 }
-__global__ void k_pm_triples(const double *__restrict__ in, double *__restrict__ out, int64_t np)
+__global__ void k_pm_triples(const double *in, double *out, int64_t np)
 {
     pdl_entry();
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < np; i += (int64_t)gridDim.x * blockDim.x) {
@@ -149,7 +149,7 @@ struct PmSite {
     __device__ __forceinline__ double w(int axis, int b) const { return b ? d[axis] : 1.0 - d[axis]; }
 };
 
-template <class R> __device__ __forceinline__ double pm_ld(const R *__restrict__ f, int i) { return (double)__ldg(f + i); }
+template <bool EARLY, class R> __device__ __forceinline__ double pm_ld(const R *f, int i) { return (double)ld<EARLY>(f + i); }
 
 // CIC deposit of cst at the particle's 8 corners
 template <class R> __device__ __forceinline__ void pm_scatter(const PmSite &s, double cst, R *out)
@@ -177,18 +177,18 @@ __device__ __forceinline__ void pm_add3(double *out, double a, double b, double 
 
 // G[i][k] = (psi(c_k + e_i) - psi(c_k - e_i)) / 2 at the 8 corners c_k of the
 // cell: 32 distinct values (the 8 corners and the 24 one step outside them)
-template <class R>
-__device__ __forceinline__ void pm_grad_corners(const R *__restrict__ psi, const PmSite &s, double G[3][8])
+template <bool EARLY, class R>
+__device__ __forceinline__ void pm_grad_corners(const R *psi, const PmSite &s, double G[3][8])
 {
     double in[8];
 #pragma unroll
-    for (int k = 0; k < 8; k++) in[k] = pm_ld(psi, s.at((k >> 2) & 1, (k >> 1) & 1, k & 1));
+    for (int k = 0; k < 8; k++) in[k] = pm_ld<EARLY>(psi, s.at((k >> 2) & 1, (k >> 1) & 1, k & 1));
 #pragma unroll
     for (int k = 0; k < 8; k++) {
         const int bx = (k >> 2) & 1, by = (k >> 1) & 1, bz = k & 1;
         // the neighbour inside the cell is a corner, the other one lies outside
-        const double ox = pm_ld(psi, s.at(bx ? 2 : -1, by, bz)), oy = pm_ld(psi, s.at(bx, by ? 2 : -1, bz)),
-                     oz = pm_ld(psi, s.at(bx, by, bz ? 2 : -1));
+        const double ox = pm_ld<EARLY>(psi, s.at(bx ? 2 : -1, by, bz)), oy = pm_ld<EARLY>(psi, s.at(bx, by ? 2 : -1, bz)),
+                     oz = pm_ld<EARLY>(psi, s.at(bx, by, bz ? 2 : -1));
         G[0][k] = 0.5 * (bx ? ox - in[k & 3] : in[k | 4] - ox);
         G[1][k] = 0.5 * (by ? oy - in[k & 5] : in[k | 2] - oy);
         G[2][k] = 0.5 * (bz ? oz - in[k & 6] : in[k | 1] - oz);
@@ -197,7 +197,7 @@ __device__ __forceinline__ void pm_grad_corners(const R *__restrict__ psi, const
 
 // mass deposit alone (the start of a run or of a recomputed segment)
 template <class R>
-__global__ void k_pm_deposit(const double *__restrict__ x, int64_t np, int N, double cst, R *out)
+__global__ void k_pm_deposit(const double *x, int64_t np, int N, double cst, R *out)
 {
     pdl_entry();
     const double invN = 1.0 / N;
@@ -209,11 +209,11 @@ __global__ void k_pm_deposit(const double *__restrict__ x, int64_t np, int N, do
 // to (xo, qo) (the same arrays or others), and the deposit of cst at the new
 // position that the next step (or the final density) needs: the moved
 // positions are not read back
-template <class R>
+template <class R, bool EARLY>
 __global__ void __launch_bounds__(PM_NT, 3) k_pm_kick_drift(const double *xi, const double *qi, double *xo, double *qo, int64_t np, int N,
-                                const R *__restrict__ psi, double kq, double kx, double cst, R *rho)
+                                const R *psi, double kq, double kx, double cst, R *rho)
 {
-    pdl_entry();
+    pdl_entry<EARLY>();
     const double invN = 1.0 / N;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < np; i += (int64_t)gridDim.x * blockDim.x) {
         double x[3], q[3];
@@ -225,7 +225,7 @@ __global__ void __launch_bounds__(PM_NT, 3) k_pm_kick_drift(const double *xi, co
         {
             const PmSite s(x, N, invN);
             double G[3][8];
-            pm_grad_corners(psi, s, G);
+            pm_grad_corners<EARLY>(psi, s, G);
             double g[3] = {0.0, 0.0, 0.0};
 #pragma unroll
             for (int k = 0; k < 8; k++) {
@@ -268,12 +268,12 @@ __device__ __forceinline__ void pm_weight_grad(const PmSite &s, const double v[8
 //      lq' is deposited into lam (three interleaved components) for the field
 //      part of the step.
 // (lxi, lqi) null: the cotangents start at zero.
-template <class R>
-__global__ void __launch_bounds__(PM_NT, 2) k_pm_reverse(const double *__restrict__ xb, const R *__restrict__ f, double mf, const double *__restrict__ xa,
-                             const R *__restrict__ psi, double kq, double kx, const double *lxi, const double *lqi,
+template <class R, bool EARLY>
+__global__ void __launch_bounds__(PM_NT, 2) k_pm_reverse(const double *xb, const R *f, double mf, const double *xa,
+                             const R *psi, double kq, double kx, const double *lxi, const double *lqi,
                              double *lxo, double *lqo, R *lam, int64_t np, int N)
 {
-    pdl_entry();
+    pdl_entry<EARLY>();
     const double invN = 1.0 / N;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < np; i += (int64_t)gridDim.x * blockDim.x) {
         double lx[3], lq[3];
@@ -286,7 +286,7 @@ __global__ void __launch_bounds__(PM_NT, 2) k_pm_reverse(const double *__restric
             const PmSite s(pm_get(xb, np, i).v, N, invN);
             double v[8], gm[3];
 #pragma unroll
-            for (int k = 0; k < 8; k++) v[k] = pm_ld(f, s.at((k >> 2) & 1, (k >> 1) & 1, k & 1));
+            for (int k = 0; k < 8; k++) v[k] = pm_ld<EARLY>(f, s.at((k >> 2) & 1, (k >> 1) & 1, k & 1));
             pm_weight_grad(s, v, gm);
 #pragma unroll
             for (int a = 0; a < 3; a++) lx[a] += mf * (double)N * gm[a];
@@ -296,7 +296,7 @@ __global__ void __launch_bounds__(PM_NT, 2) k_pm_reverse(const double *__restric
 #pragma unroll
             for (int a = 0; a < 3; a++) lq[a] += kx * lx[a];
             double G[3][8], v[8], gm[3];
-            pm_grad_corners(psi, s, G);
+            pm_grad_corners<EARLY>(psi, s, G);
             // lx_m -= kq N sum_k dw_k/dd_m (sum_a lq'_a G[a][k])
 #pragma unroll
             for (int k = 0; k < 8; k++) v[k] = lq[0] * G[0][k] + lq[1] * G[1][k] + lq[2] * G[2][k];
@@ -316,15 +316,15 @@ __global__ void __launch_bounds__(PM_NT, 2) k_pm_reverse(const double *__restric
 }
 
 // lpsi(v) = -kq sum_i (Lam_i(v - e_i) - Lam_i(v + e_i)) / 2; grid (N/32 or 1, N/4, N/2), block (min(N,32), 4, 2)
-template <class R>
-__global__ void k_pm_adj_div(const R *__restrict__ lam, int N, double kq, R *lpsi)
+template <class R, bool EARLY>
+__global__ void k_pm_adj_div(const R *lam, int N, double kq, R *lpsi)
 {
-    pdl_entry();
+    pdl_entry<EARLY>();
     const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y,
               z = blockIdx.z * blockDim.z + threadIdx.z;
     if (x >= N || y >= N || z >= N) return;
     auto at = [&](int xx, int yy, int zz, int c) {
-        return (double)__ldg(lam + 4 * (int64_t)(pm_wrap1(xx, N) + N * (pm_wrap1(yy, N) + N * pm_wrap1(zz, N))) + c);
+        return (double)ld<EARLY>(lam + 4 * (int64_t)(pm_wrap1(xx, N) + N * (pm_wrap1(yy, N) + N * pm_wrap1(zz, N))) + c);
     };
     double s = at(x - 1, y, z, 0) - at(x + 1, y, z, 0);
     s += at(x, y - 1, z, 1) - at(x, y + 1, z, 1);
@@ -333,7 +333,7 @@ __global__ void k_pm_adj_div(const R *__restrict__ lam, int N, double kq, R *lps
 }
 
 template <class R>
-__global__ void k_pm_contrast(const R *__restrict__ rho, int64_t n3, double *out)
+__global__ void k_pm_contrast(const R *rho, int64_t n3, double *out)
 {
     pdl_entry();
     for (int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; g < n3; g += (int64_t)gridDim.x * blockDim.x)
@@ -501,7 +501,7 @@ template <class R> struct Pm final : PmBase {
             // before steps 0, every, 2 every, ... are the checkpoints
             const bool from = n % every == 0, to = (n + 1) % every == 0 && n + 1 < ns;
             const int cf = n / every, ct = (n + 1) / every;
-            pdl_launch(k_pm_kick_drift<R>, pgrid(), PM_NT, 0, st, from ? ckx[cf]->p : x, from ? ckq[cf]->p : q, to ? ckx[ct]->p : x, to ? ckq[ct]->p : q, np, N, fld, coefs[3 * n], coefs[3 * n + 1], n + 1 < ns ? mcell : contrast, rho);
+            pdl_launch(k_pm_kick_drift<R, true>, k_pm_kick_drift<R, false>, pgrid(), PM_NT, 0, st, from ? ckx[cf]->p : x, from ? ckq[cf]->p : q, to ? ckx[ct]->p : x, to ? ckq[ct]->p : q, np, N, fld, coefs[3 * n], coefs[3 * n + 1], n + 1 < ns ? mcell : contrast, rho);
         }
         // final CIC density contrast: mass N^3/Np per particle, minus one
         pdl_launch(k_pm_contrast<R>, fgrid(), PM_NT, 0, st, rho, n3, delta);
@@ -541,21 +541,21 @@ template <class R> struct Pm final : PmBase {
                 potential(coefs[3 * n + 2], sp.p);
                 if (n + 1 < n1) {
                     segx[n + 1 - n0]->alloc(3 * np, "segment");
-                    pdl_launch(k_pm_kick_drift<R>, pgrid(), PM_NT, 0, st, xn(n), n == n0 ? ckq[s]->p : q, xn(n + 1), q, np, N, sp.p, coefs[3 * n], coefs[3 * n + 1], mcell, rho);
+                    pdl_launch(k_pm_kick_drift<R, true>, k_pm_kick_drift<R, false>, pgrid(), PM_NT, 0, st, xn(n), n == n0 ? ckq[s]->p : q, xn(n + 1), q, np, N, sp.p, coefs[3 * n], coefs[3 * n + 1], mcell, rho);
                 }
             }
             for (int n = n1 - 1; n >= n0; n--) {
                 const double kq = coefs[3 * n], kx = coefs[3 * n + 1], pc = coefs[3 * n + 2];
                 clear(lam, 4 * n3);
-                pdl_launch(k_pm_reverse<R>, pgrid(), PM_NT, 0, st, xb, fld, mb, xn(n), segpsi[n - n0]->p, kq, kx, first ? nullptr : lx, first ? nullptr : lq, lx, lq, lam, np, N);
+                pdl_launch(k_pm_reverse<R, true>, k_pm_reverse<R, false>, pgrid(), PM_NT, 0, st, xb, fld, mb, xn(n), segpsi[n - n0]->p, kq, kx, first ? nullptr : lx, first ? nullptr : lq, lx, lq, lam, np, N);
                 first = false;
-                pdl_launch(k_pm_adj_div<R>, dg, db, 0, st, lam, N, kq, fld);
+                pdl_launch(k_pm_adj_div<R, true>, k_pm_adj_div<R, false>, dg, db, 0, st, lam, N, kq, fld);
                 poisson(fld, fld, pc);
                 mb = mcell;
                 xb = xn(n);   // of the segment's first step the checkpoint, which outlives the segment
             }
         }
-        pdl_launch(k_pm_reverse<R>, pgrid(), PM_NT, 0, st, xb, fld, mb, nullptr, nullptr, 0.0, 0.0, lx, lq, lx, lq, nullptr, np, N);
+        pdl_launch(k_pm_reverse<R, true>, k_pm_reverse<R, false>, pgrid(), PM_NT, 0, st, xb, fld, mb, nullptr, nullptr, 0.0, 0.0, lx, lq, lx, lq, nullptr, np, N);
         pdl_launch(k_pm_triples, pgrid(), PM_NT, 0, st, lx, gx0, np);
         pdl_launch(k_pm_triples, pgrid(), PM_NT, 0, st, lq, gq0, np);
         pck(cudaGetLastError(), "adjoint launch");

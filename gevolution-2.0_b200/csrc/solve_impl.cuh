@@ -82,6 +82,7 @@ void fx_fwd_n(const FxArgs<R> &a, int ncomp, int64_t in_stride, int64_t out_stri
 {
     using C = typename CT<R>::C;
     constexpr int T = PASS_TX, NT = RegPlan<N / 2>::R2 * T;
+    static_assert((uint64_t)N * (N / T) > PDL_BLOCKS, "compiled for launches that are not early");
     constexpr size_t smem = (size_t)T * exch_size<N / 2, 1>() * sizeof(C);
     auto k = k_fx_fwd<R, N, T, MODE, resident<R>(NT, regs_fx<R, N, MODE>())>;
     set_smem<smem>(k);
@@ -92,15 +93,13 @@ template <class R, int N>
 void fx_tij6_n(const FxArgs<R> &a, int64_t in_stride, int64_t out_stride, const FftTables<R> &tb, cudaStream_t st)
 {
     using C = typename CT<R>::C;
+    static_assert((uint64_t)N * (N / PASS_TIJ) > PDL_BLOCKS, "compiled for launches that are not early");
     constexpr int T = cols<R>(PASS_TIJ), G = PASS_TIJ_G, NT = RegPlan<N / 2>::R2 * T * G;
     constexpr size_t smem = (size_t)6 * T * exch_size<N / 2, 1>() * sizeof(C);
     auto k = k_fx_fwd_tij6<R, N, T, G, resident<R>(NT, regs_for<R, N / 2>(REGS_TIJ<R>))>;
     set_smem<smem>(k);
     pdl_launch(k, dim3(N / T, N), NT, smem, st, a.in, in_stride, a.phi, a.c, a.out, out_stride, tb.tw_half, tb.tw_full);
 }
-
-// the x and y transforms of whole planes in one kernel (fftpass.cuh)
-template <int N> constexpr bool plane_pass() { return N <= 128; }
 
 template <class R, int N, int MODE>
 void plane_fwd_n(const FxArgs<R> &a, int ncomp, int64_t in_stride, int64_t out_stride, const FftTables<R> &tb, cudaStream_t st)
@@ -120,6 +119,7 @@ void fy_n(typename CT<R>::C *data, int64_t stride, int ncomp, const FftTables<R>
 {
     using C = typename CT<R>::C;
     constexpr int T = cols<R>(PASS_TY);
+    static_assert((uint64_t)N * (N / 2 / T) > PDL_BLOCKS, "compiled for launches that are not early");
     const dim3 grid((N / 2 + 1 + T - 1) / T, N, ncomp);
     if constexpr (y_staged<R, N>()) {
         constexpr size_t smem = (size_t)N * T * sizeof(C) + 128;
@@ -174,6 +174,7 @@ void fxi_n(const typename CT<R>::C *in, int64_t in_stride, R *out, int64_t out_s
 {
     using C = typename CT<R>::C;
     constexpr int T = PASS_TX, NT = RegPlan<N / 2>::R2 * T;
+    static_assert((uint64_t)N * (N / T) > PDL_BLOCKS, "compiled for launches that are not early");
     constexpr size_t smem = (size_t)T * exch_size<N / 2, 1>() * sizeof(C);
     auto k = k_fx_inv<R, N, T, resident<R>(NT, regs_for<R, N / 2>(REGS_X))>;
     set_smem<smem>(k);
@@ -228,6 +229,7 @@ void fz_n(const FzArgs<R> &a, const FftTables<R> &tb, cudaStream_t st)
     using C = typename CT<R>::C;
     using S = OpShape<OP, EXTRA>;
     if constexpr (z_staged<R, N, OP, EXTRA>()) {
+        static_assert((uint64_t)N * (N / 2 / 8) > PDL_BLOCKS, "compiled for launches that are not early");
         constexpr int T = S::CMAX == 1 ? cols<R>(8) : 4, NT = 256, MINB = fz_staged_minb<R, N, OP, EXTRA>();
         constexpr size_t dense = (size_t)S::CTMA * N * T * sizeof(C) + 128;
         constexpr size_t padded = (size_t)S::CTMA * (N + N / 8) * T * sizeof(C) + 128;

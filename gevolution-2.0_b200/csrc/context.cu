@@ -189,7 +189,7 @@ struct CtxBase {
     virtual double kick_drift(const KickDriftParams &kp) = 0;
     // kick_drift and lightcone without waiting for their results; those of a
     // whole cycle come with one synchronisation (cycle_results, then lightcone_count)
-    virtual void kick_drift_async(const KickDriftParams &kp) = 0;
+    virtual void kick_drift_async(const KickDriftParams &kp, bool whole_cycle) = 0;
     virtual bool lightcone_async(const gev_lightcone_args &lc, double tau, double dtau, double dtau_old, double a,
                                  double dadtau, int64_t cap) = 0;
     virtual void cycle_results(double *sum, double *phom, double *maxvel) = 0;
@@ -222,7 +222,7 @@ template <class R> struct Ctx final : CtxBase {
     // The device scalars that the host reads, in one block with the bucket
     // counts behind them (cleared together with the largest velocity): one
     // copy brings all of a cycle's results.
-    enum { BX_SUM = 0, BX_PHIHOM = 1, BX_ERR = 2, BX_LC = 3, BX_VMAX = 4, BX_WORDS = 5, BX_COUNTS = 6 };
+    enum { BX_SUM = 0, BX_PHIHOM = 1, BX_ERR = 2, BX_LC = 3, BX_VMAX = 4, BX_STOP = 5, BX_WORDS = 6, BX_COUNTS = 6 };
     DBuf<unsigned long long> box;
     unsigned long long *hbox = nullptr;  // pinned host copy of the block
     double *dsum = nullptr, *dphihom = nullptr;
@@ -998,18 +998,25 @@ template <class R> struct Ctx final : CtxBase {
 
     double kick_drift(const KickDriftParams &kp) override
     {
-        kick_drift_async(kp);
+        kick_drift_async(kp, false);
         if (!kp.do_kick) return 0.0;
         sync();
         return std::sqrt(held(BX_VMAX));
     }
 
-    void kick_drift_async(const KickDriftParams &kp) override
+    // whole_cycle: the stages before have not been looked at for errors; after
+    // one the particles stay (cycle_results puts their order right)
+    void kick_drift_async(const KickDriftParams &kp, bool whole_cycle) override
     {
         need_particles();
         // the largest velocity and, behind it, the bucket counts
-        const size_t words = 2 * (BX_COUNTS - BX_VMAX) + (kp.do_bin ? g.ntiles * 8 : 0);
-        ck(cudaMemsetAsync(dvmax, 0, words * sizeof(uint32_t), st), "memset");
+        if (whole_cycle) {
+            launch_kick_clear(dvmax, g.ntiles * 8, derr, bstart.p, st);
+            launched("clear");
+        } else {
+            const size_t words = 2 * (BX_COUNTS - BX_VMAX) + (kp.do_bin ? g.ntiles * 8 : 0);
+            ck(cudaMemsetAsync(dvmax, 0, words * sizeof(uint32_t), st), "memset");
+        }
         launch_kick_drift<R>(cur(), bstart.p, g.N, phi.p, chi.p, Bi.p, g.n3, kp, dcounts, bucket.p, rank.p, dvmax, derr, st);
         launched("kick/drift");
         if (kp.do_bin) finish_rebin();
@@ -1017,7 +1024,17 @@ template <class R> struct Ctx final : CtxBase {
 
     void cycle_results(double *sum, double *phom, double *maxvel) override
     {
-        sync();
+        try {
+            sync();
+        } catch (const DeviceError &) {
+            if (hbox[BX_STOP]) {
+                // the error came before the kick: the particles are still in the
+                // buffer that the re-binning read, their bucket ranges are gone
+                cur_is_A = !cur_is_A;
+                rebin_from_cells();
+            }
+            throw;
+        }
         *sum = held(BX_SUM);
         *phom = held(BX_PHIHOM);
         *maxvel = std::sqrt(held(BX_VMAX));
@@ -1484,7 +1501,7 @@ int step_cycle(gev_ctx *ctx, const gev_cosmo *cosmo, gev_state *s, const gev_lig
         kp.a_d = a;
         kp.b_d = a * a * N;
         kp.nfield_d = (1. / a < cm.z_relax + 1.) ? 3 : 0;
-        c.kick_drift_async(kp);
+        c.kick_drift_async(kp, true);
         gev::rk4bg(a, cm.fourpiG, cm, 0.5 * s->dtau);
         // the cycle's one synchronisation: every stage is queued by now
         double sum = 0.0, ph = 0.0, mv = 0.0;

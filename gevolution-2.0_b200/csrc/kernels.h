@@ -43,6 +43,12 @@ void launch_kick_drift(const PView<R> &p, const uint32_t *bstart, int N, const R
                        int64_t n3, const KickDriftParams &kp, uint32_t *counts, uint32_t *bucket, uint32_t *rank,
                        unsigned long long *vmax_bits, int *err, cudaStream_t st);
 
+// Clears the largest velocity, the word behind it and the nb bucket counts
+// behind that (vmax[0], vmax[1], counts) for a cycle's kick.  If an earlier
+// stage has set the error word, the kick must not move particles on its
+// fields: their bucket ranges bstart[0..nb] are emptied and vmax[1] is set.
+void launch_kick_clear(unsigned long long *vmax, int64_t nb, const int *err, uint32_t *bstart, cudaStream_t st);
+
 template <class R>
 void launch_load_particles(PView<R> p, const double *pos, const double *q, const int64_t *id, int64_t n, int N,
                            int *err, cudaStream_t st);

@@ -366,6 +366,25 @@ void launch_kick_drift(const PView<R> &p, const uint32_t *bstart, int N, const R
                chi, Bi, n3, kp, counts, bucket, rank, vmax_bits, err, FastDiv((uint32_t)N));
 }
 
+// In place of a memset, so that the kick need not look at the error word itself:
+// a load that every block waits for costs it 3 to 6 % (512^3: 5.56 -> 5.75 ms
+// and more), an empty bucket range nothing.
+__global__ void k_kick_clear(uint4 *w, int64_t n4, const int *err, uint32_t *bstart, int64_t nb)
+{
+    pdl_entry();
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const bool stop = *err != 0;
+    if (i < n4) w[i] = make_uint4(0u, 0u, i == 0 && stop ? 1u : 0u, 0u);
+    if (stop)
+        for (int64_t j = i; j <= nb; j += (int64_t)gridDim.x * blockDim.x) bstart[j] = 0u;
+}
+
+void launch_kick_clear(unsigned long long *vmax, int64_t nb, const int *err, uint32_t *bstart, cudaStream_t st)
+{
+    const int64_t n4 = 1 + nb / 4;   // nb is a multiple of 8
+    pdl_launch(k_kick_clear, cdiv(n4, 256), 256, 0, st, reinterpret_cast<uint4 *>(vmax), n4, err, bstart, nb);
+}
+
 // ---- particle I/O: host layout (box-unit positions, AoS triples) <-> cell + offset ----
 template <class R>
 __global__ void k_load_particles(PView<R> p, const double *pos, const double *q, const int64_t *id, int64_t n, int N,

@@ -242,6 +242,12 @@ typedef struct {
     double T00hom, phi_hom, maxvel;
 } gev_state;
 
+/* The call looks for device errors once, at its end.  When it returns
+ * GEV_ERR_DEVICE, *st is as before the call.  If the error arose before the
+ * kick, the particles are too; if in the kick, the drift or the re-binning
+ * (gev_last_error: a non-finite coordinate), they have moved.  Either way phi,
+ * chi, B_i, h_ij and the lightcone logs are those of the failed cycle: load a
+ * checkpoint, or the particles and fields, before going on. */
 int gev_step(gev_ctx *ctx, const gev_cosmo *cosmo, gev_state *st);
 /* gev_step with one lightcone shell written where main.cu writes it: after
  * the field solves and before the kick (writeLightcones, main.cu:1040-1100),

@@ -188,3 +188,38 @@ def test_pm_positions_far_outside_the_box(N, n):
     # (up to 6e5 here) larger than those of a single deposit (N x |w|, about 5e2)
     for k, (a, b) in enumerate(zip(*res)):
         assert rel_err(a.cpu().numpy(), b.cpu().numpy()) < (1e-10 if k < 3 else 6e-13 * 1.2e3 * 4), k
+
+
+@pytest.mark.parametrize("prec", PRECS)
+@pytest.mark.parametrize("N", [64, 128])
+def test_failed_cycle_leaves_the_particles(N, prec):
+    """An error that arises before the kick (here the lightcone's ID log, sized
+    for the one particle that was there at first, overflows) leaves particles
+    and state as they were, on both sides of the size from which the kick can
+    be launched early; the next call finds the error cleared and the particles
+    in order."""
+    n = 100000
+    rng = np.random.default_rng(9)
+    r = np.abs(rng.standard_normal((n, 3))) + 0.05
+    pos = np.ascontiguousarray(0.971 * r / np.linalg.norm(r, axis=1)[:, None])
+    q = 1e-4 * rng.standard_normal((n, 3))
+    ids = np.arange(n, dtype=np.int64)
+    fpg = 1.5 * (5.0 * N) ** 2 / 2997.92458 ** 2
+    cosmo = gev.Cosmo(0.32, 0.68, 0.0, fpg, 48.0, 0.04, 200.0, 5.0 * N)
+    shell = gev.LightconeArgs((0.0, 0.0, 0.0), (1.0 / np.sqrt(3.0),) * 3, -1.0, (1.0, 0.3), 1.98, 1, 0)
+    with gev.Context(N, precision=prec, capacity=n, boxsize=5.0 * N) as c:
+        c.set_particles(np.full((1, 3), 0.5), np.zeros((1, 3)))
+        c.lightcone(shell, 1.0, 0.02, 0.02, 0.5, 0.1, 16)
+        c.set_particles(pos, q, ids, 0.32 / n)
+        before = [x[np.argsort(c.get_particles()[2])] for x in c.get_particles()]
+        st = gev.State(0.5, 1.0, 0.02, 0.02, 7, 0.0, 0.0, 0.0)
+        with pytest.raises(gev.GevError) as e:
+            c.step_lightcone(cosmo, st, shell, n)
+        assert e.value.code == 4 and "0x2 " in str(e.value), str(e.value)
+        assert (st.a, st.tau, st.dtau, st.cycle, st.maxvel) == (0.5, 1.0, 0.02, 7, 0.0)
+        after = [x[np.argsort(c.get_particles()[2])] for x in c.get_particles()]
+        assert all(np.array_equal(x, y) for x, y in zip(before, after))
+        c.step(cosmo, st)
+        assert st.cycle == 8
+        moved = [x[np.argsort(c.get_particles()[2])] for x in c.get_particles()]
+        assert np.array_equal(moved[2], ids) and not np.array_equal(moved[0], before[0])

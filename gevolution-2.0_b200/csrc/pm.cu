@@ -480,6 +480,7 @@ template <class R> struct Pm final : PmBase {
     void forward(int ns, const double *coef, const double *x0, const double *q0, double *delta, double *xo,
                  double *qo) override
     {
+        have_forward = false;   // until the checkpoints of this run are all there
         nsteps = ns;
         coefs.assign(coef, coef + 3 * (size_t)ns);
         const int nck = (ns + every - 1) / every;

@@ -45,11 +45,9 @@ struct PmError : std::runtime_error {
 
 void pck(cudaError_t e, const char *what)
 {
-    if (e == cudaErrorMemoryAllocation) {
-        cudaGetLastError();
-        throw PmError(GEV_ERR_NOMEM, std::string(what) + ": " + cudaGetErrorString(e));
-    }
-    if (e != cudaSuccess) throw PmError(GEV_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
+    if (e == cudaSuccess) return;
+    cudaGetLastError();   // reported here: not to be found by the next call's launch check
+    throw PmError(e == cudaErrorMemoryAllocation ? GEV_ERR_NOMEM : GEV_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
 }
 
 template <class T> struct PBuf {
@@ -362,6 +360,7 @@ template <class R> struct Pm final : PmBase {
     int64_t np, n3, nk;
     double mass;
     int every;
+    int device;
     cudaStream_t st = nullptr;
     PBuf<R> fields;          // one allocation for rho, fld and lam
     R *rho = nullptr;        // deposited density of the step
@@ -380,7 +379,7 @@ template <class R> struct Pm final : PmBase {
     int nsteps = 0;
     bool have_forward = false;
 
-    Pm(const gev_pm_config &cfg) : N(cfg.N), np(cfg.np), mass(cfg.mass), every(cfg.checkpoint_every)
+    Pm(const gev_pm_config &cfg) : N(cfg.N), np(cfg.np), mass(cfg.mass), every(cfg.checkpoint_every), device(cfg.device)
     {
         pck(cudaSetDevice(cfg.device), "cudaSetDevice");
         pck(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking), "stream");
@@ -477,6 +476,37 @@ template <class R> struct Pm final : PmBase {
         poisson(rho, out, pc, true);
     }
 
+    // whether the kernels may address a caller's array themselves: doubles on
+    // their boundary, in this device's memory (or managed)
+    bool direct(const double *a) const
+    {
+        cudaPointerAttributes at;
+        if (reinterpret_cast<uintptr_t>(a) % sizeof(double) != 0) return false;
+        if (cudaPointerGetAttributes(&at, a) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        return at.type == cudaMemoryTypeManaged || (at.type == cudaMemoryTypeDevice && at.device == device);
+    }
+    // a caller's triples to planes and back; through a copy into `spare` (3 np
+    // values) where the array is not direct, so that whatever a copy accepts
+    // (another device's memory, any alignment) is accepted and all else is an
+    // error of the copy, not a fault of the kernel
+    void from_caller(const double *in, double *planes, double *spare)
+    {
+        if (!direct(in)) {
+            pck(cudaMemcpyAsync(spare, in, 3 * np * sizeof(double), cudaMemcpyDeviceToDevice, st), "copy in");
+            in = spare;
+        }
+        pdl_launch(k_pm_planes, pgrid(), PM_NT, 0, st, in, planes, np);
+    }
+    void to_caller(const double *planes, double *out, double *spare)
+    {
+        double *to = direct(out) ? out : spare;
+        pdl_launch(k_pm_triples, pgrid(), PM_NT, 0, st, planes, to, np);
+        if (to != out) pck(cudaMemcpyAsync(out, to, 3 * np * sizeof(double), cudaMemcpyDeviceToDevice, st), "copy out");
+    }
+
     void forward(int ns, const double *coef, const double *x0, const double *q0, double *delta, double *xo,
                  double *qo) override
     {
@@ -492,8 +522,8 @@ template <class R> struct Pm final : PmBase {
             ckx[s]->alloc(3 * np, "checkpoint");
             ckq[s]->alloc(3 * np, "checkpoint");
         }
-        pdl_launch(k_pm_planes, pgrid(), PM_NT, 0, st, x0, ckx[0]->p, np);
-        pdl_launch(k_pm_planes, pgrid(), PM_NT, 0, st, q0, ckq[0]->p, np);
+        from_caller(x0, ckx[0]->p, x);
+        from_caller(q0, ckq[0]->p, q);
         const double mcell = mass * (double)n3, contrast = (double)n3 / (double)np;
         deposit(ckx[0]->p, mcell);
         for (int n = 0; n < ns; n++) {
@@ -502,12 +532,14 @@ template <class R> struct Pm final : PmBase {
             // before steps 0, every, 2 every, ... are the checkpoints
             const bool from = n % every == 0, to = (n + 1) % every == 0 && n + 1 < ns;
             const int cf = n / every, ct = (n + 1) / every;
-            pdl_launch(k_pm_kick_drift<R, true>, k_pm_kick_drift<R, false>, pgrid(), PM_NT, 0, st, from ? ckx[cf]->p : x, from ? ckq[cf]->p : q, to ? ckx[ct]->p : x, to ? ckq[ct]->p : q, np, N, fld, coefs[3 * n], coefs[3 * n + 1], n + 1 < ns ? mcell : contrast, rho);
+            pdl_launch(k_pm_kick_drift<R, true>, k_pm_kick_drift<R, false>, pgrid(), PM_NT, 0, st, from ? ckx[cf]->p : x,
+                       from ? ckq[cf]->p : q, to ? ckx[ct]->p : x, to ? ckq[ct]->p : q, np, N, fld, coefs[3 * n],
+                       coefs[3 * n + 1], n + 1 < ns ? mcell : contrast, rho);
         }
         // final CIC density contrast: mass N^3/Np per particle, minus one
         pdl_launch(k_pm_contrast<R>, fgrid(), PM_NT, 0, st, rho, n3, delta);
-        if (xo) pdl_launch(k_pm_triples, pgrid(), PM_NT, 0, st, x, xo, np);
-        if (qo) pdl_launch(k_pm_triples, pgrid(), PM_NT, 0, st, q, qo, np);
+        if (xo) to_caller(x, xo, lx);
+        if (qo) to_caller(q, qo, lq);
         pck(cudaGetLastError(), "forward launch");
         pck(cudaStreamSynchronize(st), "forward");
         check_device("forward");
@@ -557,8 +589,8 @@ template <class R> struct Pm final : PmBase {
             }
         }
         pdl_launch(k_pm_reverse<R, true>, k_pm_reverse<R, false>, pgrid(), PM_NT, 0, st, xb, fld, mb, nullptr, nullptr, 0.0, 0.0, lx, lq, lx, lq, nullptr, np, N);
-        pdl_launch(k_pm_triples, pgrid(), PM_NT, 0, st, lx, gx0, np);
-        pdl_launch(k_pm_triples, pgrid(), PM_NT, 0, st, lq, gq0, np);
+        to_caller(lx, gx0, q);   // q is free by now
+        to_caller(lq, gq0, q);
         pck(cudaGetLastError(), "adjoint launch");
         pck(cudaStreamSynchronize(st), "adjoint");
         check_device("adjoint");

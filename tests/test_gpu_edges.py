@@ -223,3 +223,62 @@ def test_failed_cycle_leaves_the_particles(N, prec):
         assert st.cycle == 8
         moved = [x[np.argsort(c.get_particles()[2])] for x in c.get_particles()]
         assert np.array_equal(moved[2], ids) and not np.array_equal(moved[0], before[0])
+
+
+@pytest.mark.parametrize("prec", PRECS)
+def test_pm_arrays_off_the_double_boundary(prec):
+    """Caller's particle arrays at any byte address, as the copies of the run
+    have always taken them: the results are those of aligned arrays, bit for
+    bit where no atomics are summed in between (one step, few particles far
+    apart)."""
+    from gevb200 import pm as gevpm
+
+    N, n = 16, 5
+    x = (torch.arange(3 * n, device="cuda", dtype=torch.float64).reshape(n, 3) * 3.0 % 15.0 + 0.25) / N
+    q = 1e-3 * torch.ones((n, 3), device="cuda", dtype=torch.float64)
+    run = gevpm.PM(N, n, 0.32 / n, prec, checkpoint_every=1)
+    coef = np.array([0.1, 0.2, 1.0])
+
+    class At:
+        """3 n doubles whose first byte lies `off` bytes into a buffer."""
+
+        def __init__(self, values, off):
+            self.raw = torch.zeros(24 * n + 16, dtype=torch.uint8, device="cuda")
+            self.off = off
+            if values is not None:
+                self.raw[off:off + 24 * n] = values.reshape(-1).view(torch.uint8)
+
+        def data_ptr(self):
+            return self.raw.data_ptr() + self.off
+
+        def values(self):
+            return self.raw[self.off:self.off + 24 * n].clone().view(torch.float64)
+
+    out = []
+    for off in (0, 4):
+        a = [At(v, off) for v in (x, q, None, None, None, None)]
+        delta = torch.empty(N ** 3, dtype=torch.float64, device="cuda")
+        torch.cuda.synchronize()
+        run.forward(coef, a[0], a[1], delta, a[2], a[3])
+        run.adjoint(torch.ones_like(delta), a[4], a[5])
+        out.append([delta] + [v.values() for v in a[2:]])
+    for u, v in zip(*out):
+        assert torch.isfinite(u).all() and torch.equal(u, v)
+
+
+def test_pm_host_array_is_no_gpu_fault():
+    """A pageable host array, which the run does not take, is an error of the
+    call (or, where the driver can copy it, taken), and the context goes on."""
+    from gevb200 import pm as gevpm
+
+    N, n = 16, 5
+    run = gevpm.PM(N, n, 0.32 / n, gev.FP64, checkpoint_every=1)
+    delta = torch.empty(N ** 3, dtype=torch.float64, device="cuda")
+    host = torch.full((n, 3), 0.5, dtype=torch.float64)
+    torch.cuda.synchronize()
+    try:
+        run.forward(np.array([0.1, 0.2, 1.0]), host, host, delta)
+    except gev.GevError as e:
+        assert e.code == 2, str(e)
+    run.forward(np.array([0.1, 0.2, 1.0]), host.cuda(), host.cuda(), delta)
+    assert torch.isfinite(delta).all()

@@ -1053,12 +1053,13 @@ template <class R> struct Ctx final : CtxBase {
             t *= t;
             kmax = std::sqrt(3.0 * t);
         }
-        if ((int64_t)occ.n < (int64_t)BIN_COPIES * nb) {
-            bins.alloc((size_t)BIN_COPIES * 4 * nb, "bins");
-            occ.alloc((size_t)BIN_COPIES * nb, "bins");
+        const int copies = bin_copies(nb);
+        if ((int64_t)occ.n < (int64_t)copies * nb) {
+            bins.alloc((size_t)copies * 4 * nb, "bins");
+            occ.alloc((size_t)copies * nb, "bins");
         }
-        ck(cudaMemsetAsync(bins.p, 0, (size_t)BIN_COPIES * 4 * nb * sizeof(double), st), "memset");
-        ck(cudaMemsetAsync(occ.p, 0, (size_t)BIN_COPIES * nb * sizeof(unsigned long long), st), "memset");
+        ck(cudaMemsetAsync(bins.p, 0, (size_t)copies * 4 * nb * sizeof(double), st), "memset");
+        ck(cudaMemsetAsync(occ.p, 0, (size_t)copies * nb * sizeof(unsigned long long), st), "memset");
         if (!sinc.p) {   // the CIC deconvolution's sinc (tools.hpp:118-127)
             std::vector<double> h(N / 2 + 1, 1.0);
             for (int i = 1; i <= N / 2; i++)
@@ -1102,8 +1103,10 @@ template <class R> struct Ctx final : CtxBase {
             fz_pass<double>(N, fp, W64, g.nk, nullptr, nullptr, nullptr, tb, st);
             launched("fz binning (FP64)");
         }
-        launch_bin_reduce(bins.p, occ.p, nb, st);
-        launched("bin sums");
+        if (copies > 1) {
+            launch_bin_reduce(bins.p, occ.p, nb, copies, st);
+            launched("bin sums");
+        }
         std::vector<double> acc(4 * nb);
         std::vector<unsigned long long> oc(nb);
         ck(cudaMemcpyAsync(acc.data(), bins.p, 4 * nb * sizeof(double), cudaMemcpyDeviceToHost, st), "D2H");

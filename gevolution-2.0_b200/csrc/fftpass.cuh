@@ -652,8 +652,8 @@ template <class R> struct FzArgs {
     const double *partial;     // OP_POISSON: partial sums (npartial of them, null: none) summed into *sum
     int64_t npartial;
     double *sum;
-    double *bins;              // OP_BIN: BIN_COPIES x 4 x numbins accumulators (k, k^2, P, P^2)
-    unsigned long long *occ;   // OP_BIN: BIN_COPIES x numbins mode counts
+    double *bins;              // OP_BIN: copies x 4 x numbins accumulators (k, k^2, P, P^2)
+    unsigned long long *occ;   // OP_BIN: copies x numbins mode counts
     int *err;                  // device error word (may be null)
     const double *tab;         // OP_ZELD: ln k [h/Mpc] (ntab values) then ln P(k) (ntab values)
     int ntab;
@@ -865,7 +865,7 @@ template <class R, int NT> __device__ __forceinline__ void sum_partials(const Fz
 // bin does not decrease, so lanes of one bin are neighbours: each run of them
 // is summed by shuffles and only its first lane adds to the bins.  Five
 // global additions per mode on a few hundred addresses take 1450 us at 256^3
-// (FP64); this takes a few of them per warp, spread over BIN_COPIES copies.
+// (FP64); this takes a few of them per warp, spread over bin_copies copies.
 template <class R>
 __device__ __forceinline__ void bin_modes(const FzArgs<R> &a, int N, int kx, int ky, int kz, bool on, bool two,
                                           typename CT<R>::C v0, typename CT<R>::C v1, int copy)
@@ -1031,7 +1031,7 @@ __global__ void __launch_bounds__(RegPlan<N>::R2 *T *G, MINB) k_fz(FzArgs<R> a, 
                 const int z = z0 + (threadIdx.x & 31);
                 const bool on = kxl < P && z <= N / 2, two = z > 0 && z < N / 2;
                 const C v0 = on ? smem[slot(z, l)] : mk(R(0), R(0)), v1 = on && two ? smem[slot(N - z, l)] : mk(R(0), R(0));
-                bin_modes(a, N, kxl, ky, z, on, two, v0, v1, (int)((blockIdx.x + gridDim.x * blockIdx.y) % BIN_COPIES));
+                bin_modes(a, N, kxl, ky, z, on, two, v0, v1, (int)((blockIdx.x + gridDim.x * blockIdx.y) % bin_copies((int)a.p0)));
             }
         }
     } else if constexpr (CT1 == 1) {

@@ -95,10 +95,12 @@ int fyx_inverse(int N, typename CT<R>::C *in, int64_t in_stride, R *out, int64_t
 int64_t fxy_partials(int N);
 
 // copies of the spectrum's bins that the z pass adds into (by block), against
-// contention on a bin: bins [BIN_COPIES][4][nb], occ [BIN_COPIES][nb]
-constexpr int BIN_COPIES = 16;
+// contention on a bin: bins [copies][4][nb], occ [copies][nb].  With thousands
+// of bins there is none, and the copies would be most of the work and memory.
+constexpr int BIN_COPIES = 16, BIN_COPIES_MAX_BINS = 4096;
+__host__ __device__ constexpr int bin_copies(int nb) { return nb <= BIN_COPIES_MAX_BINS ? BIN_COPIES : 1; }
 // sums the copies (in a fixed order) into the first one
-void launch_bin_reduce(double *bins, unsigned long long *occ, int nb, cudaStream_t st);
+void launch_bin_reduce(double *bins, unsigned long long *occ, int nb, int copies, cudaStream_t st);
 
 struct FzParams {
     int op, extra;

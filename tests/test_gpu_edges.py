@@ -282,3 +282,21 @@ def test_pm_host_array_is_no_gpu_fault():
         assert e.code == 2, str(e)
     run.forward(np.array([0.1, 0.2, 1.0]), host.cuda(), host.cuda(), delta)
     assert torch.isfinite(delta).all()
+
+
+@pytest.mark.parametrize("prec", PRECS)
+@pytest.mark.parametrize("bins", [4096, 4097, 200001])
+def test_power_spectrum_many_bins(prec, bins):
+    """On each side of the number of bins from which they are kept once."""
+    test_power_spectrum_bins(prec, 16, bins)
+
+
+def test_power_spectrum_workspace():
+    """The device memory of a spectrum with very many bins is that of the five
+    sums per bin (160 MB here), with some room for the allocator."""
+    with gev.Context(16, precision=gev.FP64, capacity=8) as c:
+        c.set_particles(np.full((1, 3), 0.5), np.zeros((1, 3)))
+        c.power_spectrum(16)
+        free = torch.cuda.mem_get_info()[0]
+        c.power_spectrum(4000000)
+        assert free - torch.cuda.mem_get_info()[0] < 2 * 160e6

@@ -511,7 +511,9 @@ template <class R> struct Ctx final : CtxBase {
         if (ip.noise_out) field_get(GEV_FIELD_SOURCE, ip.noise_out);
         // 2. displacement field into the B_i planes
         const FftTables<R> tb = tables();
-        launched("forward x, y passes", fxy_forward<R>(N, FX_COPY, source.p, g.n3, 1, nullptr, nullptr, 0, 0, 0, 0, W.p, g.nk, nullptr, tb, st));
+        launched("forward x, y passes",
+                 fxy_forward<R>(N, FX_COPY, source.p, g.n3, 1, nullptr, nullptr, 0, 0, 0, 0, W.p, g.nk, nullptr, tb,
+                                st));
         FzParams fz{};
         fz.err = derr;
         fz.op = OP_ZELD;
@@ -546,7 +548,9 @@ template <class R> struct Ctx final : CtxBase {
         project(GEV_PROJ_CIC, 1.0, 1.0, 0, 0);
         gev_cosmo cm{Om, OL, Orad, fourpiG, 0.0, 0.0, 0.0, boxsize};
         const double H = hconf(a, fourpiG, cm);
-        launched("forward x, y passes", fxy_forward<R>(N, FX_COPY, source.p, g.n3, 1, nullptr, nullptr, 0, 0, 0, 0, W.p, g.nk, nullptr, tb, st));
+        launched("forward x, y passes",
+                 fxy_forward<R>(N, FX_COPY, source.p, g.n3, 1, nullptr, nullptr, 0, 0, 0, 0, W.p, g.nk, nullptr, tb,
+                                st));
         FzParams fp{};
         fp.err = derr;
         fp.op = OP_POISSON;
@@ -621,7 +625,9 @@ template <class R> struct Ctx final : CtxBase {
         launch_ics_modes(modes.p, N, ip.seed, ip.ksphere, (float)(ip.gr ? H * H : 0.0), sp, derr, st);
         launched("ics modes");
         // 3. kernel transform, numerator / kernel, backward transform: the displacement potential in chi
-        launched("forward x, y passes", fxy_forward<R>(N, FX_COPY, source.p, g.n3, 1, nullptr, nullptr, 0, 0, 0, 0, W.p, g.nk, nullptr, tb, st));
+        launched("forward x, y passes",
+                 fxy_forward<R>(N, FX_COPY, source.p, g.n3, 1, nullptr, nullptr, 0, 0, 0, 0, W.p, g.nk, nullptr, tb,
+                                st));
         FzParams fz{};
         fz.err = derr;
         fz.op = OP_ICS;
@@ -906,7 +912,9 @@ template <class R> struct Ctx final : CtxBase {
     {
         const int N = g.N;
         const FftTables<R> tb = tables();
-        launched("forward x, y passes", fxy_forward<R>(N, prepare ? FX_PREP_T00 : FX_COPY, source.p, g.n3, 1, phi.p, chi.p, bg, c, c2, c3, W.p, g.nk, partial.p, tb, st));
+        launched("forward x, y passes",
+                 fxy_forward<R>(N, prepare ? FX_PREP_T00 : FX_COPY, source.p, g.n3, 1, phi.p, chi.p, bg, c, c2, c3,
+                                W.p, g.nk, partial.p, tb, st));
         FzParams fp{};
         fp.err = derr;
         fp.op = OP_POISSON;
@@ -961,7 +969,9 @@ template <class R> struct Ctx final : CtxBase {
     {
         const int N = g.N;
         const FftTables<R> tb = tables();
-        launched("forward x, y passes", fxy_forward<R>(N, FX_PREP_TIJ, Sij.p, g.n3, 6, phi.p, chi.p, 0, coeff, 0, 0, W.p, g.nk, nullptr, tb, st));
+        launched("forward x, y passes",
+                 fxy_forward<R>(N, FX_PREP_TIJ, Sij.p, g.n3, 6, phi.p, chi.p, 0, coeff, 0, 0, W.p, g.nk, nullptr, tb,
+                                st));
         FzParams fp{};
         fp.err = derr;
         fp.op = OP_SCALAR;
@@ -984,7 +994,9 @@ template <class R> struct Ctx final : CtxBase {
         // T0i straight from project(T0I), or completed from project_step's sums with the current phi
         if (t0i_pending) project(GEV_PROJ_T0I, 1.0, t0i_coeff, 1, 0);
         t0i_pending = false;
-        launched("forward x, y passes", fxy_forward<R>(N, bi_sums ? FX_PREP_T0I : FX_COPY, Bi.p, g.n3, 3, phi.p, nullptr, 0, 0, 0, 0, W.p, g.nk, nullptr, tb, st));
+        launched("forward x, y passes",
+                 fxy_forward<R>(N, bi_sums ? FX_PREP_T0I : FX_COPY, Bi.p, g.n3, 3, phi.p, nullptr, 0, 0, 0, 0, W.p,
+                                g.nk, nullptr, tb, st));
         bi_sums = false;
         FzParams fp{};
         fp.err = derr;
@@ -1078,7 +1090,9 @@ template <class R> struct Ctx final : CtxBase {
         if constexpr (sizeof(R) == 8) {
             project(GEV_PROJ_CIC, 1.0, 1.0, 0, 0);
             const FftTables<R> tb = tables();
-            launched("forward x, y passes", fxy_forward<R>(N, FX_COPY, source.p, g.n3, 1, nullptr, nullptr, 0, 0, 0, 0, W.p, g.nk, nullptr, tb, st));
+            launched("forward x, y passes",
+                     fxy_forward<R>(N, FX_COPY, source.p, g.n3, 1, nullptr, nullptr, 0, 0, 0, 0, W.p, g.nk, nullptr,
+                                    tb, st));
             fz_pass<R>(N, fp, W.p, g.nk, nullptr, nullptr, nullptr, tb, st);
             launched("fz binning");
         } else {
@@ -1099,7 +1113,9 @@ template <class R> struct Ctx final : CtxBase {
             launched("density to FP32");
             const FftTables<double> tb{tw64_full.p, tw64_half.p, k2.p, ks.p, derr};
             double2 *W64 = reinterpret_cast<double2 *>(W.p);   // W holds 6 FP32 components = 3 FP64 ones
-            launched("forward x, y passes", fxy_forward<double>(N, FX_COPY, rho64.p, g.n3, 1, nullptr, nullptr, 0, 0, 0, 0, W64, g.nk, nullptr, tb, st));
+            launched("forward x, y passes",
+                     fxy_forward<double>(N, FX_COPY, rho64.p, g.n3, 1, nullptr, nullptr, 0, 0, 0, 0, W64, g.nk,
+                                         nullptr, tb, st));
             fz_pass<double>(N, fp, W64, g.nk, nullptr, nullptr, nullptr, tb, st);
             launched("fz binning (FP64)");
         }

@@ -1,4 +1,4 @@
-// fft.cuh -- batched in-shared-memory FFTs of the staged z pass (k_fz_tma), and
+// fft.cuh -- batched in-shared-memory FFTs of the staged passes (k_fz_tma, k_fy_tma), and
 // the small in-register DFTs that the two-step transforms (fftreg.cuh) use too.
 //
 // T independent lines of length L sit in shared memory as buf[n*ld + t]

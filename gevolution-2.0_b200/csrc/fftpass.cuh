@@ -430,7 +430,10 @@ __global__ void __launch_bounds__(RegPlan<N / 2>::R2 *T, MINB) k_fx_inv(const ty
 // Small grids (N <= 128): the x and y transforms of a whole z plane in one
 // kernel, the plane in shared memory between them.  At these sizes a pass is
 // bound by its launch and by latency, not by its traffic: two launches of a
-// solve and one pass over the spectrum go in each direction.
+// solve and one pass over the spectrum go in each direction.  At 128^3 this is
+// at its end: phi, chi and B_i solves take 37, 84 and 66 us in FP32 and 59, 152
+// and 210 us in FP64; with the forward transforms as two passes 39, 83 and 69
+// us, and 53, 142 and 205 us.
 // ---------------------------------------------------------------------------
 template <int N> struct PlaneShape {
     static constexpr int M = N / 2, P = M + 1;

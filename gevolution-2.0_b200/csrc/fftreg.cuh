@@ -9,11 +9,14 @@
 //   step 2  row q (threads take the rows q = u, u + R2, ...) holds R2 values:
 //           R2-point DFT over j gives X[q + R1 p], p < R2, in natural order.
 // The inverse runs the same two steps backwards (step 2 over p first), so a
-// pass that transforms, solves point by point and transforms back touches
-// shared memory four times per value and needs two block barriers: the
-// values of row q belong to one thread from the exchange to the exchange back.
-// Passes bound by shared memory when they run radix-8 steps through it (two
-// accesses per step and direction) become bound by their global traffic.
+// pass over one component that transforms, solves point by point and transforms
+// back touches shared memory four times per value and needs two block barriers:
+// the values of row q belong to one thread from the exchange to the exchange
+// back.  (Several components meet in shared memory for their solve: four more
+// accesses and two more barriers.)  Passes bound by shared memory when they run
+// radix-8 steps through it (two accesses per step and direction) become bound
+// by their global traffic, as long as the 2 R1 or 2 R2 values of a thread leave
+// registers for enough warps.
 //
 // Rows of the exchange buffer have the pitch (R2 + 1) * T (T lines side by
 // side, line index fastest): step 1 writes along a row, step 2 reads rows a

@@ -574,13 +574,15 @@ template <class R> struct Pm final : PmBase {
                 potential(coefs[3 * n + 2], sp.p);
                 if (n + 1 < n1) {
                     segx[n + 1 - n0]->alloc(3 * np, "segment");
-                    pdl_launch(k_pm_kick_drift<R, true>, k_pm_kick_drift<R, false>, pgrid(), PM_NT, 0, st, xn(n), n == n0 ? ckq[s]->p : q, xn(n + 1), q, np, N, sp.p, coefs[3 * n], coefs[3 * n + 1], mcell, rho);
+                    pdl_launch(k_pm_kick_drift<R, true>, k_pm_kick_drift<R, false>, pgrid(), PM_NT, 0, st, xn(n),
+                               n == n0 ? ckq[s]->p : q, xn(n + 1), q, np, N, sp.p, coefs[3 * n], coefs[3 * n + 1], mcell, rho);
                 }
             }
             for (int n = n1 - 1; n >= n0; n--) {
                 const double kq = coefs[3 * n], kx = coefs[3 * n + 1], pc = coefs[3 * n + 2];
                 clear(lam, 4 * n3);
-                pdl_launch(k_pm_reverse<R, true>, k_pm_reverse<R, false>, pgrid(), PM_NT, 0, st, xb, fld, mb, xn(n), segpsi[n - n0]->p, kq, kx, first ? nullptr : lx, first ? nullptr : lq, lx, lq, lam, np, N);
+                pdl_launch(k_pm_reverse<R, true>, k_pm_reverse<R, false>, pgrid(), PM_NT, 0, st, xb, fld, mb, xn(n),
+                           segpsi[n - n0]->p, kq, kx, first ? nullptr : lx, first ? nullptr : lq, lx, lq, lam, np, N);
                 first = false;
                 pdl_launch(k_pm_adj_div<R, true>, k_pm_adj_div<R, false>, dg, db, 0, st, lam, N, kq, fld);
                 poisson(fld, fld, pc);
@@ -588,7 +590,8 @@ template <class R> struct Pm final : PmBase {
                 xb = xn(n);   // of the segment's first step the checkpoint, which outlives the segment
             }
         }
-        pdl_launch(k_pm_reverse<R, true>, k_pm_reverse<R, false>, pgrid(), PM_NT, 0, st, xb, fld, mb, nullptr, nullptr, 0.0, 0.0, lx, lq, lx, lq, nullptr, np, N);
+        pdl_launch(k_pm_reverse<R, true>, k_pm_reverse<R, false>, pgrid(), PM_NT, 0, st, xb, fld, mb, nullptr,
+                   nullptr, 0.0, 0.0, lx, lq, lx, lq, nullptr, np, N);
         to_caller(lx, gx0, q);   // q is free by now
         to_caller(lq, gq0, q);
         pck(cudaGetLastError(), "adjoint launch");

@@ -2,9 +2,10 @@
 
 The kernels that the 512^3 cycle runs are specialised per N: the transforms'
 radices, rows and columns per block and twiddle tables, and the z pass, which
-in FP32 loads its pencils by bulk tensor boxes for some solves (one box up to
+loads its pencils by bulk tensor boxes for some solves (one box up to
 N = 256; N = 384: three boxes of 128; N = 512: two of 256; N = 768: three of
-256) and through registers for the others.  These
+256) and through registers for the others, and the y pass, which is staged in
+FP64 at N = 512 alone.  These
 tests compare each solve with an independent FP64 reference at those sizes:
 pocketfft (scipy.fft, the same transform numpy uses, pinned to the oracle's
 FFT in test_oracle_pin.py) for the transforms and the oracle's C restatements

@@ -114,7 +114,7 @@ __device__ __forceinline__ R prep_tij(const R *T, const R *phi, R coeff, int c, 
 // zo = (Z[k] - conj Z[M-k]) / 2i: kx = k gets ze + w zo, kx = M - k its mirror
 // conj(ze - w zo), from the same two values.  dst(l) is the output row of
 // line l.
-template <int M, int LINES, int NT, class C, class DST>
+template <int M, int LINES, int NT, bool EX, class C, class DST>
 __device__ __forceinline__ void fx_finish(C *smem, const C *__restrict__ tw_full, DST &&dst)
 {
     using R = decltype(smem->x);
@@ -126,7 +126,7 @@ __device__ __forceinline__ void fx_finish(C *smem, const C *__restrict__ tw_full
         C *buf = smem + l * ES;
         for (int q = u; q < R1; q += R2) {
             C v[R2];
-            step2_load<M, -1, 1>(v, buf, q);
+            step2_load<M, -1, EX, 1>(v, buf, q);
 #pragma unroll
             for (int p = 0; p < R2; p++) buf[q * (R2 + 1) + p] = v[p];
         }
@@ -252,7 +252,7 @@ __device__ __forceinline__ void fx_clear(const R *in, int u, int y, int z)
     }
 }
 
-template <class R, int N, int T, int MODE, int MINB>
+template <class R, int N, int T, int MODE, bool EX, int MINB>
 __global__ void __launch_bounds__(RegPlan<N / 2>::R2 *T, MINB) k_fx_fwd(FxArgs<R> a, int64_t in_stride, int64_t out_stride,
                                                                        const typename CT<R>::C *__restrict__ tw_half,
                                                                        const typename CT<R>::C *__restrict__ tw_full)
@@ -278,10 +278,10 @@ __global__ void __launch_bounds__(RegPlan<N / 2>::R2 *T, MINB) k_fx_fwd(FxArgs<R
         else if (comp == 1) load(IntC<1>{});
         else load(IntC<2>{});
         if (MODE == FX_COPY && a.clear) fx_clear<R, N>(in, u, y0 + l, z);
-        step1_store<M, -1, 1>(v, smem + l * ES, u, tw_half);
+        step1_store<M, -1, EX, 1>(v, smem + l * ES, u, tw_half);
     }
     __syncthreads();
-    fx_finish<M, T, NT>(smem, tw_full, [&](int i) { return out + (int64_t)PP * (y0 + i + (int64_t)N * z); });
+    fx_finish<M, T, NT, EX>(smem, tw_full, [&](int i) { return out + (int64_t)PP * (y0 + i + (int64_t)N * z); });
 
     if constexpr (MODE == FX_PREP_T00) block_sum<NT>(lsum, a.partial + blockIdx.x + gridDim.x * blockIdx.y);
 }
@@ -319,6 +319,7 @@ __global__ void __launch_bounds__(RegPlan<N / 2>::R2 *T *G, MINB) k_fx_fwd_tij6(
                                                                               const typename CT<R>::C *__restrict__ tw_full)
 {
     pdl_entry<false>();
+    constexpr bool EX = true;   // fftreg.cuh: not a vector field
     using C = typename CT<R>::C;
     constexpr int M = N / 2, PP = N / 2 + 2, R1 = RegPlan<M>::R1, R2 = RegPlan<M>::R2, NT = R2 * T * G, ES = exch_size<M, 1>();
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -365,10 +366,10 @@ __global__ void __launch_bounds__(RegPlan<N / 2>::R2 *T *G, MINB) k_fx_fwd_tij6(
         C v[R1];
 #pragma unroll
         for (int r = 0; r < R1; r++) v[r] = b[r * (R2 + 1) + u];
-        step1_store<M, -1, 1>(v, b, u, tw_half);
+        step1_store<M, -1, EX, 1>(v, b, u, tw_half);
     }
     __syncthreads();
-    fx_finish<M, 6 * T, NT>(smem, tw_full, [&](int i) {
+    fx_finish<M, 6 * T, NT, EX>(smem, tw_full, [&](int i) {
         return out + (i / T) * out_stride + (int64_t)PP * (y0 + i % T + (int64_t)N * z);
     });
 }
@@ -377,7 +378,7 @@ __global__ void __launch_bounds__(RegPlan<N / 2>::R2 *T *G, MINB) k_fx_fwd_tij6(
 // x pass, inverse: half spectrum -> real rows (imaginary parts of the kx = 0
 // and kx = N/2 entries do not contribute).  grid (N/T, N, ncomp)
 // ---------------------------------------------------------------------------
-template <class R, int N, int T, int MINB>
+template <class R, int N, int T, bool EX, int MINB>
 __global__ void __launch_bounds__(RegPlan<N / 2>::R2 *T, MINB) k_fx_inv(const typename CT<R>::C *in, int64_t in_stride, R *out,
                                                                        int64_t out_stride,
                                                                        const typename CT<R>::C *__restrict__ tw_half,
@@ -404,7 +405,7 @@ __global__ void __launch_bounds__(RegPlan<N / 2>::R2 *T, MINB) k_fx_inv(const ty
             const C dd = cmul(csub(A, B), w), s = cadd(A, B);
             v[r] = mk(s.x - dd.y, s.y + dd.x);         // (A+B) + i (A-B) w
         }
-        step1_store<M, 1, 1>(v, buf, u, tw_half);
+        step1_store<M, 1, EX, 1>(v, buf, u, tw_half);
     }
     __syncthreads();
     R *dst = out + (int64_t)blockIdx.z * out_stride + sidx(N, 0, y, z);
@@ -412,7 +413,7 @@ __global__ void __launch_bounds__(RegPlan<N / 2>::R2 *T, MINB) k_fx_inv(const ty
     const bool pairs = reinterpret_cast<uintptr_t>(out) % sizeof(C) == 0;
     for (int q = u; q < R1; q += R2) {
         C v[R2];
-        step2_load<M, 1, 1>(v, buf, q);
+        step2_load<M, 1, EX, 1>(v, buf, q);
 #pragma unroll
         for (int p = 0; p < R2; p++) {
             R *d = dst + 2 * (q + R1 * p);
@@ -455,7 +456,7 @@ template <int N> struct PlaneShape {
 template <class R, int N> constexpr int plane_minb() { return sizeof(R) == 4 && N == 128 ? 2 : 1; }
 
 // forward: rows (with their source preparation), then columns; grid (N, ncomp)
-template <class R, int N, int MODE>
+template <class R, int N, int MODE, bool EX>
 __global__ void __launch_bounds__(PlaneShape<N>::NT, plane_minb<R, N>()) k_plane_fwd(FxArgs<R> a, int64_t in_stride, int64_t out_stride,
                                                                  const typename CT<R>::C *__restrict__ tw_half,
                                                                  const typename CT<R>::C *__restrict__ tw_full)
@@ -478,7 +479,7 @@ __global__ void __launch_bounds__(PlaneShape<N>::NT, plane_minb<R, N>()) k_plane
 #pragma unroll
             for (int r = 0; r < XR1; r++) v[r] = fx_pair<R, N, MODE, decltype(cc)::v>(a, in, u + XR2 * r, y, z, lsum);
             if (MODE == FX_COPY && a.clear) fx_clear<R, N>(in, u, y, z);
-            step1_store<M, -1, 1>(v, smem + y * S::XES, u, tw_half);
+            step1_store<M, -1, EX, 1>(v, smem + y * S::XES, u, tw_half);
         }
     };
     if constexpr (MODE == FX_PREP_T0I || MODE == FX_PREP_TIJ) {
@@ -499,7 +500,7 @@ __global__ void __launch_bounds__(PlaneShape<N>::NT, plane_minb<R, N>()) k_plane
         C *buf = smem + (w / XR2) * S::XES;
         for (int q = w % XR2; q < XR1; q += XR2) {
             C v[XR2];
-            step2_load<M, -1, 1>(v, buf, q);
+            step2_load<M, -1, EX, 1>(v, buf, q);
 #pragma unroll
             for (int p = 0; p < XR2; p++) buf[q * (XR2 + 1) + p] = v[p];
         }
@@ -537,14 +538,14 @@ __global__ void __launch_bounds__(PlaneShape<N>::NT, plane_minb<R, N>()) k_plane
         C v[YR1];
 #pragma unroll
         for (int r = 0; r < YR1; r++) v[r] = buf[(r * (YR2 + 1) + u) * P];
-        step1_store<N, -1, P>(v, buf, u, tw_full);
+        step1_store<N, -1, EX, P>(v, buf, u, tw_full);
     }
     __syncthreads();
     if (u < YR2) {
         C *out = a.out + (int64_t)comp * out_stride + (int64_t)PP * N * z + k;
         for (int q = u; q < YR1; q += YR2) {
             C v[YR2];
-            step2_load<N, -1, P>(v, smem + k, q);
+            step2_load<N, -1, EX, P>(v, smem + k, q);
 #pragma unroll
             for (int p = 0; p < YR2; p++) out[PP * (q + YR1 * p)] = v[p];
         }
@@ -553,7 +554,7 @@ __global__ void __launch_bounds__(PlaneShape<N>::NT, plane_minb<R, N>()) k_plane
 }
 
 // inverse: columns, then rows; grid (N, ncomp)
-template <class R, int N>
+template <class R, int N, bool EX>
 __global__ void __launch_bounds__(PlaneShape<N>::NT, plane_minb<R, N>()) k_plane_inv(const typename CT<R>::C *in, int64_t in_stride, R *out,
                                                                  int64_t out_stride,
                                                                  const typename CT<R>::C *__restrict__ tw_half,
@@ -573,13 +574,13 @@ __global__ void __launch_bounds__(PlaneShape<N>::NT, plane_minb<R, N>()) k_plane
         C v[YR1];
 #pragma unroll
         for (int r = 0; r < YR1; r++) v[r] = ld(col + PP * (u0 + YR2 * r));
-        step1_store<N, 1, P>(v, smem + k0, u0, tw_full);
+        step1_store<N, 1, EX, P>(v, smem + k0, u0, tw_full);
     }
     __syncthreads();
     if (u0 < YR2) {
         for (int q = u0; q < YR1; q += YR2) {
             C v[YR2];
-            step2_load<N, 1, P>(v, smem + k0, q);
+            step2_load<N, 1, EX, P>(v, smem + k0, q);
 #pragma unroll
             for (int p = 0; p < YR2; p++) smem[(q * (YR2 + 1) + p) * P + k0] = v[p];
         }
@@ -607,7 +608,7 @@ __global__ void __launch_bounds__(PlaneShape<N>::NT, plane_minb<R, N>()) k_plane
 #pragma unroll
     for (int i = 0; i < S::XPER; i++) {
         const int w = threadIdx.x + i * NT;
-        if (w < S::XITEMS) step1_store<M, 1, 1>(v[i], smem + (w / XR2) * S::XES, w % XR2, tw_half);
+        if (w < S::XITEMS) step1_store<M, 1, EX, 1>(v[i], smem + (w / XR2) * S::XES, w % XR2, tw_half);
     }
     __syncthreads();
     // a caller's own array (gev_poisson_noalloc) may be aligned to single values only
@@ -618,7 +619,7 @@ __global__ void __launch_bounds__(PlaneShape<N>::NT, plane_minb<R, N>()) k_plane
         R *dst = out + (int64_t)blockIdx.y * out_stride + sidx(N, 0, y, z);
         for (int q = w % XR2; q < XR1; q += XR2) {
             C x[XR2];
-            step2_load<M, 1, 1>(x, smem + y * S::XES, q);
+            step2_load<M, 1, EX, 1>(x, smem + y * S::XES, q);
 #pragma unroll
             for (int p = 0; p < XR2; p++) {
                 R *d = dst + 2 * (q + XR1 * p);
@@ -949,6 +950,7 @@ __global__ void __launch_bounds__(RegPlan<N>::R2 *T *G, MINB) k_fz(FzArgs<R> a, 
 {
     constexpr bool EARLY = (uint64_t)((N / 2 + 1 + T - 1) / T) * N <= PDL_BLOCKS;   // the launch's grid
     pdl_entry<EARLY>();
+    constexpr bool EX = OP != OP_VECTOR;   // fftreg.cuh
     using C = typename CT<R>::C;
     constexpr int P = N / 2 + 1, PP = N / 2 + 2;
     constexpr int R1 = RegPlan<N>::R1, R2 = RegPlan<N>::R2;
@@ -1007,13 +1009,13 @@ __global__ void __launch_bounds__(RegPlan<N>::R2 *T *G, MINB) k_fz(FzArgs<R> a, 
             C v[R1];
 #pragma unroll
             for (int r = 0; r < R1; r++) v[r] = buf[c * ES + (r * (R2 + 1) + u) * T];
-            step1_store<N, -1, T>(v, buf + c * ES, u, tw);
+            step1_store<N, -1, EX, T>(v, buf + c * ES, u, tw);
         }
     } else {
         C v[R1];
 #pragma unroll
         for (int r = 0; r < R1; r++) v[r] = live ? __ldcs(a.data + col + PLANE * (u + R2 * r)) : mk(R(0), R(0));
-        step1_store<N, -1, T>(v, buf, u, tw);
+        step1_store<N, -1, EX, T>(v, buf, u, tw);
     }
     __syncthreads();
 
@@ -1021,7 +1023,7 @@ __global__ void __launch_bounds__(RegPlan<N>::R2 *T *G, MINB) k_fz(FzArgs<R> a, 
     if constexpr (OP == OP_BIN) {
         for (int q = u; q < R1; q += R2) {
             C v[R2];
-            step2_load<N, -1, T>(v, buf, q);
+            step2_load<N, -1, EX, T>(v, buf, q);
 #pragma unroll
             for (int p = 0; p < R2; p++) buf[(q * (R2 + 1) + p) * T] = v[p];
         }
@@ -1040,7 +1042,7 @@ __global__ void __launch_bounds__(RegPlan<N>::R2 *T *G, MINB) k_fz(FzArgs<R> a, 
     } else if constexpr (CT1 == 1) {
         for (int q = u; q < R1; q += R2) {
             C v[R2];
-            step2_load<N, -1, T>(v, buf, q);
+            step2_load<N, -1, EX, T>(v, buf, q);
             if (live) {
 #pragma unroll
                 for (int p = 0; p < R2; p++) {
@@ -1054,12 +1056,12 @@ __global__ void __launch_bounds__(RegPlan<N>::R2 *T *G, MINB) k_fz(FzArgs<R> a, 
                         buf[c * ES + (q * (R2 + 1) + p) * T] = mk(R(w[c].x), R(w[c].y));
                 }
             }
-            if constexpr (COUT > 0) step2_store<N, 1, T>(v, buf, q, tw);
+            if constexpr (COUT > 0) step2_store<N, 1, EX, T>(v, buf, q, tw);
 #pragma unroll 1
             for (int c = 1; c < COUT; c++) {
 #pragma unroll
                 for (int p = 0; p < R2; p++) v[p] = buf[c * ES + (q * (R2 + 1) + p) * T];
-                step2_store<N, 1, T>(v, buf + c * ES, q, tw);
+                step2_store<N, 1, EX, T>(v, buf + c * ES, q, tw);
             }
         }
     } else {
@@ -1067,7 +1069,7 @@ __global__ void __launch_bounds__(RegPlan<N>::R2 *T *G, MINB) k_fz(FzArgs<R> a, 
         for (int w = u + R2 * g; w < CT1 * R1; w += R2 * G) {
             C *row = buf + (w / R1) * ES;
             C v[R2];
-            step2_load<N, -1, T>(v, row, w % R1);
+            step2_load<N, -1, EX, T>(v, row, w % R1);
 #pragma unroll
             for (int p = 0; p < R2; p++) row[((w % R1) * (R2 + 1) + p) * T] = v[p];
         }
@@ -1105,7 +1107,7 @@ __global__ void __launch_bounds__(RegPlan<N>::R2 *T *G, MINB) k_fz(FzArgs<R> a, 
             C v[R2];
 #pragma unroll
             for (int p = 0; p < R2; p++) v[p] = row[((w % R1) * (R2 + 1) + p) * T];
-            step2_store<N, 1, T>(v, row, w % R1, tw);
+            step2_store<N, 1, EX, T>(v, row, w % R1, tw);
         }
     }
     if constexpr (COUT > 0) {
@@ -1114,7 +1116,7 @@ __global__ void __launch_bounds__(RegPlan<N>::R2 *T *G, MINB) k_fz(FzArgs<R> a, 
 #pragma unroll 1
         for (int c = g; c < COUT; c += G) {
             C v[R1];
-            step1_load<N, 1, T>(v, buf + c * ES, u);
+            step1_load<N, 1, EX, T>(v, buf + c * ES, u);
             if (live) {
 #pragma unroll
                 for (int r = 0; r < R1; r++) a.data[c * a.stride + col + PLANE * (u + R2 * r)] = v[r];
@@ -1285,7 +1287,7 @@ __global__ void __launch_bounds__(NT, MINB)
 }
 
 // y pass (in place): T kx-columns over all ky at one kz; grid (ceil(P/T), N, ncomp)
-template <class R, int N, int T, int S, int MINB>
+template <class R, int N, int T, int S, bool EX, int MINB>
 __global__ void __launch_bounds__(RegPlan<N>::R2 *T, MINB) k_fy(typename CT<R>::C *data, int64_t stride,
                                                                const typename CT<R>::C *__restrict__ tw)
 {
@@ -1302,12 +1304,12 @@ __global__ void __launch_bounds__(RegPlan<N>::R2 *T, MINB) k_fy(typename CT<R>::
         C v[R1];
 #pragma unroll
         for (int r = 0; r < R1; r++) v[r] = live ? d[PP * (u + R2 * r)] : mk(R(0), R(0));
-        step1_store<N, S, T>(v, buf, u, tw);
+        step1_store<N, S, EX, T>(v, buf, u, tw);
     }
     __syncthreads();
     for (int q = u; q < R1; q += R2) {
         C v[R2];
-        step2_load<N, S, T>(v, buf, q);
+        step2_load<N, S, EX, T>(v, buf, q);
         if (live) {
 #pragma unroll
             for (int p = 0; p < R2; p++) d[PP * (q + R1 * p)] = v[p];

@@ -52,16 +52,19 @@ __host__ __device__ constexpr double root_cos(int k)   // cos(2 pi k / 96), any 
 __host__ __device__ constexpr double root_sin(int k) { return root_cos(k + 72); }
 
 // a * exp(S 2 pi i K / R), R a divisor of 96.
-// FP32 radices of 16 and 32 carry the rounding errors of the root's two
-// constants along, four operations more: such a radix multiplies by one root
-// per value more than the radix-8 steps of a Stockham transform, and without
-// this the FP32 transforms were the less exact ones (forward and back of white
-// noise against 64 bits, x 1e-7; Stockham / two-step / with the constants:
-// 128^3 2.49 / 2.50 / 2.36, 256^3 2.71 / 2.77 / 2.43, 384^3 3.05 / 3.13 / 2.87,
-// 512^3 2.86 / 2.96 / 2.63, 768^3 3.14 / 3.28 / 3.04).  Time: a phi solve at
-// 384^3 917 -> 926 us, none that shows at the other sizes.  With the radices of
-// 12 and 24 too it would be 933 us.
-template <int R, int K, int S, class C> __device__ __forceinline__ C mul_root(C a)
+// EXACT: in FP32, radices of 16 and 32 carry the rounding errors of the root's
+// two constants along, four operations more: such a radix multiplies by one
+// root per value more than the radix-8 steps of a Stockham transform, and
+// without this the FP32 transforms were the less exact ones (forward and back
+// of white noise against 64 bits, x 1e-7; Stockham / two-step / EXACT: 128^3
+// 2.49 / 2.50 / 2.36, 256^3 2.71 / 2.77 / 2.43, 384^3 3.05 / 3.13 / 2.87, 512^3
+// 2.86 / 2.96 / 2.63, 768^3 3.14 / 3.28 / 3.05).  Time: a phi solve at 384^3 909
+// -> 917 us, none that shows at the other sizes; with the radices of 12 and 24
+// too it would be 15 us more.  Not for vector fields: what is left of B_i after
+// its longitudinal part is gone carries the FP32 rounding of the z pass's last
+// sums in a few long modes, ten times all other errors of its transforms (256^3
+// at z = 100: 8.4e-5 / 8.6e-5 / 8.5e-5), and its z pass would take 2 % longer.
+template <int R, int K, int S, bool EXACT, class C> __device__ __forceinline__ C mul_root(C a)
 {
     static_assert(96 % R == 0, "roots are tabulated for divisors of 96");
     using F = decltype(a.x);
@@ -79,7 +82,7 @@ template <int R, int K, int S, class C> __device__ __forceinline__ C mul_root(C 
         return o;
     } else {
         constexpr F c = F(root_cos(k)), s = F(S * root_sin(k));
-        if constexpr (sizeof(F) == 4 && (R == 16 || R == 32)) {
+        if constexpr (EXACT && sizeof(F) == 4 && (R == 16 || R == 32)) {
             constexpr F cl = F(root_cos(k) - (double)c), sl = F(S * root_sin(k) - (double)s);
             o.x = fmaf(a.x, c, fmaf(-a.y, s, a.x * cl - a.y * sl));
             o.y = fmaf(a.y, c, fmaf(a.x, s, a.y * cl + a.x * sl));
@@ -105,7 +108,7 @@ template <int N, class FN> __device__ __forceinline__ void static_for(FN &&f)
 template <int R> __host__ __device__ constexpr int radix_a() { return R == 16 ? 4 : (R == 32 ? 4 : (R == 24 ? 3 : (R == 12 ? 3 : (R == 6 ? 2 : 1)))); }
 
 // R-point DFT in registers, natural order in and out, exponent sign S
-template <int R, int S, class C> __device__ __forceinline__ void dft_reg(C (&v)[R])
+template <int R, int S, bool EXACT, class C> __device__ __forceinline__ void dft_reg(C (&v)[R])
 {
     if constexpr (R == 1) {
         return;
@@ -123,7 +126,7 @@ template <int R, int S, class C> __device__ __forceinline__ void dft_reg(C (&v)[
             dftR<A, S>(t);
             static_for<A>([&](auto ac) {
                 constexpr int a = decltype(ac)::v;
-                v[b + B * a] = mul_root<R, b * a, S>(t[a]);
+                v[b + B * a] = mul_root<R, b * a, S, EXACT>(t[a]);
             });
         });
 #pragma unroll
@@ -176,11 +179,11 @@ template <int L, int T> __host__ __device__ constexpr int exch_size() { return R
 
 // step 1, forward or the end of an inverse: values of thread j to / from the
 // exchange column at position j (buf already offset to line t)
-template <int L, int S, int T, class C>
+template <int L, int S, bool EXACT, int T, class C>
 __device__ __forceinline__ void step1_store(C (&v)[RegPlan<L>::R1], C *buf, int j, const C *__restrict__ tw)
 {
     constexpr int R1 = RegPlan<L>::R1, R2 = RegPlan<L>::R2;
-    dft_reg<R1, S>(v);
+    dft_reg<R1, S, EXACT>(v);
 #pragma unroll
     for (int q = 0; q < R1; q++) {
         if (q > 0) {
@@ -192,31 +195,31 @@ __device__ __forceinline__ void step1_store(C (&v)[RegPlan<L>::R1], C *buf, int 
     }
 }
 
-template <int L, int S, int T, class C>
+template <int L, int S, bool EXACT, int T, class C>
 __device__ __forceinline__ void step1_load(C (&v)[RegPlan<L>::R1], const C *buf, int j)
 {
     constexpr int R1 = RegPlan<L>::R1, R2 = RegPlan<L>::R2;
 #pragma unroll
     for (int q = 0; q < R1; q++) v[q] = buf[(q * (R2 + 1) + j) * T];
-    dft_reg<R1, S>(v);
+    dft_reg<R1, S, EXACT>(v);
 }
 
 // step 2: row q of the exchange buffer, transformed over its R2 values
-template <int L, int S, int T, class C>
+template <int L, int S, bool EXACT, int T, class C>
 __device__ __forceinline__ void step2_load(C (&v)[RegPlan<L>::R2], const C *buf, int q)
 {
     constexpr int R2 = RegPlan<L>::R2;
 #pragma unroll
     for (int j = 0; j < R2; j++) v[j] = buf[(q * (R2 + 1) + j) * T];
-    dft_reg<R2, S>(v);
+    dft_reg<R2, S, EXACT>(v);
 }
 
 // inverse of step 2: transform the row over p, twiddle, back to the buffer
-template <int L, int S, int T, class C>
+template <int L, int S, bool EXACT, int T, class C>
 __device__ __forceinline__ void step2_store(C (&v)[RegPlan<L>::R2], C *buf, int q, const C *__restrict__ tw)
 {
     constexpr int R2 = RegPlan<L>::R2;
-    dft_reg<R2, S>(v);
+    dft_reg<R2, S, EXACT>(v);
 #pragma unroll
     for (int j = 0; j < R2; j++) {
         if (j > 0) {

@@ -77,14 +77,14 @@ template <class R, int N, int MODE> constexpr int regs_fx()
     return MODE == FX_PREP_T00 && sizeof(R) == 4 && RegPlan<N / 2>::R1 >= 24 ? 80 : regs_for<R, N / 2>(REGS_X);
 }
 
-template <class R, int N, int MODE>
+template <class R, int N, int MODE, bool EX>
 void fx_fwd_n(const FxArgs<R> &a, int ncomp, int64_t in_stride, int64_t out_stride, const FftTables<R> &tb, cudaStream_t st)
 {
     using C = typename CT<R>::C;
     constexpr int T = PASS_TX, NT = RegPlan<N / 2>::R2 * T;
     static_assert((uint64_t)N * (N / T) > PDL_BLOCKS, "compiled for launches that are not early");
     constexpr size_t smem = (size_t)T * exch_size<N / 2, 1>() * sizeof(C);
-    auto k = k_fx_fwd<R, N, T, MODE, resident<R>(NT, regs_fx<R, N, MODE>())>;
+    auto k = k_fx_fwd<R, N, T, MODE, EX, resident<R>(NT, regs_fx<R, N, MODE>())>;
     set_smem<smem>(k);
     pdl_launch(k, dim3(N / T, N, ncomp), NT, smem, st, a, in_stride, out_stride, tb.tw_half, tb.tw_full);
 }
@@ -101,12 +101,12 @@ void fx_tij6_n(const FxArgs<R> &a, int64_t in_stride, int64_t out_stride, const 
     pdl_launch(k, dim3(N / T, N), NT, smem, st, a.in, in_stride, a.phi, a.c, a.out, out_stride, tb.tw_half, tb.tw_full);
 }
 
-template <class R, int N, int MODE>
+template <class R, int N, int MODE, bool EX>
 void plane_fwd_n(const FxArgs<R> &a, int ncomp, int64_t in_stride, int64_t out_stride, const FftTables<R> &tb, cudaStream_t st)
 {
     using C = typename CT<R>::C;
     constexpr size_t smem = (size_t)PlaneShape<N>::VALUES * sizeof(C);
-    auto k = k_plane_fwd<R, N, MODE>;
+    auto k = k_plane_fwd<R, N, MODE, EX>;
     set_smem<smem>(k);
     pdl_launch(k, dim3(N, ncomp), PlaneShape<N>::NT, smem, st, a, in_stride, out_stride, tb.tw_half, tb.tw_full);
 }
@@ -114,7 +114,7 @@ void plane_fwd_n(const FxArgs<R> &a, int ncomp, int64_t in_stride, int64_t out_s
 // y pass staged by bulk copies (k_fy_tma) or the two-step one (k_fy)
 template <class R, int N> constexpr bool y_staged() { return sizeof(R) == 8 && N == 512; }
 
-template <class R, int N, int S>
+template <class R, int N, int S, bool EX>
 void fy_n(typename CT<R>::C *data, int64_t stride, int ncomp, const FftTables<R> &tb, cudaStream_t st)
 {
     using C = typename CT<R>::C;
@@ -130,24 +130,34 @@ void fy_n(typename CT<R>::C *data, int64_t stride, int ncomp, const FftTables<R>
     } else {
         constexpr int NT = RegPlan<N>::R2 * T;
         constexpr size_t smem = (size_t)exch_size<N, T>() * sizeof(C);
-        auto k = k_fy<R, N, T, S, resident<R>(NT, regs_for<R, N>(REGS_Y))>;
+        auto k = k_fy<R, N, T, S, EX, resident<R>(NT, regs_for<R, N>(REGS_Y))>;
         set_smem<smem>(k);
         pdl_launch(k, grid, NT, smem, st, data, stride, tb.tw_full);
     }
 }
 
-template <class R, int N, int MODE>
-int fxy_fwd_n(const FxArgs<R> &a, int ncomp, int64_t in_stride, int64_t out_stride, const FftTables<R> &tb, cudaStream_t st)
+template <class R, int N, int MODE, bool EX>
+int fxy_fwd_ex(const FxArgs<R> &a, int ncomp, int64_t in_stride, int64_t out_stride, const FftTables<R> &tb, cudaStream_t st)
 {
     if constexpr (plane_pass<N>()) {
-        plane_fwd_n<R, N, MODE>(a, ncomp, in_stride, out_stride, tb, st);
+        plane_fwd_n<R, N, MODE, EX>(a, ncomp, in_stride, out_stride, tb, st);
         return 1;
     } else {
         if constexpr (MODE == FX_PREP_TIJ) fx_tij6_n<R, N>(a, in_stride, out_stride, tb, st);
-        else fx_fwd_n<R, N, MODE>(a, ncomp, in_stride, out_stride, tb, st);
-        fy_n<R, N, -1>(a.out, out_stride, ncomp, tb, st);
+        else fx_fwd_n<R, N, MODE, EX>(a, ncomp, in_stride, out_stride, tb, st);
+        fy_n<R, N, -1, EX>(a.out, out_stride, ncomp, tb, st);
         return 2;
     }
+}
+
+// three components are a vector field: no exact roots (fftreg.cuh)
+template <class R, int N, int MODE>
+int fxy_fwd_n(const FxArgs<R> &a, int ncomp, int64_t in_stride, int64_t out_stride, const FftTables<R> &tb, cudaStream_t st)
+{
+    if constexpr (MODE == FX_PREP_T0I) return fxy_fwd_ex<R, N, MODE, false>(a, ncomp, in_stride, out_stride, tb, st);
+    else if constexpr (MODE != FX_COPY || sizeof(R) == 8) return fxy_fwd_ex<R, N, MODE, true>(a, ncomp, in_stride, out_stride, tb, st);
+    else if (ncomp == 3) return fxy_fwd_ex<R, N, MODE, false>(a, ncomp, in_stride, out_stride, tb, st);
+    else return fxy_fwd_ex<R, N, MODE, true>(a, ncomp, in_stride, out_stride, tb, st);
 }
 
 template <class R>
@@ -168,7 +178,7 @@ int fxy_forward(int N, int mode, const R *in, int64_t in_stride, int ncomp, cons
     return n;
 }
 
-template <class R, int N>
+template <class R, int N, bool EX>
 void fxi_n(const typename CT<R>::C *in, int64_t in_stride, R *out, int64_t out_stride, int ncomp, const FftTables<R> &tb,
            cudaStream_t st)
 {
@@ -176,27 +186,37 @@ void fxi_n(const typename CT<R>::C *in, int64_t in_stride, R *out, int64_t out_s
     constexpr int T = PASS_TX, NT = RegPlan<N / 2>::R2 * T;
     static_assert((uint64_t)N * (N / T) > PDL_BLOCKS, "compiled for launches that are not early");
     constexpr size_t smem = (size_t)T * exch_size<N / 2, 1>() * sizeof(C);
-    auto k = k_fx_inv<R, N, T, resident<R>(NT, regs_for<R, N / 2>(REGS_X))>;
+    auto k = k_fx_inv<R, N, T, EX, resident<R>(NT, regs_for<R, N / 2>(REGS_X))>;
     set_smem<smem>(k);
     pdl_launch(k, dim3(N / T, N, ncomp), NT, smem, st, in, in_stride, out, out_stride, tb.tw_half, tb.tw_full);
+}
+
+template <class R, int N, bool EX>
+int fyx_inv_ex(typename CT<R>::C *in, int64_t in_stride, R *out, int64_t out_stride, int ncomp, const FftTables<R> &tb,
+              cudaStream_t st)
+{
+    using C = typename CT<R>::C;
+    if constexpr (plane_pass<N>()) {
+        constexpr size_t smem = (size_t)PlaneShape<N>::VALUES * sizeof(C);
+        auto k = k_plane_inv<R, N, EX>;
+        set_smem<smem>(k);
+        pdl_launch(k, dim3(N, ncomp), PlaneShape<N>::NT, smem, st, in, in_stride, out, out_stride, tb.tw_half, tb.tw_full);
+        return 1;
+    } else {
+        fy_n<R, N, 1, EX>(in, in_stride, ncomp, tb, st);
+        fxi_n<R, N, EX>(in, in_stride, out, out_stride, ncomp, tb, st);
+        return 2;
+    }
 }
 
 template <class R, int N>
 int fyx_inv_n(typename CT<R>::C *in, int64_t in_stride, R *out, int64_t out_stride, int ncomp, const FftTables<R> &tb,
               cudaStream_t st)
 {
-    using C = typename CT<R>::C;
-    if constexpr (plane_pass<N>()) {
-        constexpr size_t smem = (size_t)PlaneShape<N>::VALUES * sizeof(C);
-        auto k = k_plane_inv<R, N>;
-        set_smem<smem>(k);
-        pdl_launch(k, dim3(N, ncomp), PlaneShape<N>::NT, smem, st, in, in_stride, out, out_stride, tb.tw_half, tb.tw_full);
-        return 1;
-    } else {
-        fy_n<R, N, 1>(in, in_stride, ncomp, tb, st);
-        fxi_n<R, N>(in, in_stride, out, out_stride, ncomp, tb, st);
-        return 2;
+    if constexpr (sizeof(R) == 4) {
+        if (ncomp == 3) return fyx_inv_ex<R, N, false>(in, in_stride, out, out_stride, ncomp, tb, st);
     }
+    return fyx_inv_ex<R, N, true>(in, in_stride, out, out_stride, ncomp, tb, st);
 }
 
 template <class R>
